@@ -121,16 +121,21 @@ int launch_fc_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, cons
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 __device__ __forceinline__ uint16_t f2h_rn(float f) { return __half_as_ushort(__float2half_rn(f)); }
 
-// x / y for a constant y in {7, 15, 127} and x >= 0, correctly rounded like the IEEE division the
-// reference performs, without the division sequence: q = x*c, r = fma(-y, q, x), q' = fma(r, c, q) with
-// c = fl(1/y).  Checked exhaustively on the host against x / y for every non-negative finite fp32 x
-// (all three constants): no mismatch.  Infinite / NaN x fall through to q.
+// x / y for a constant y in {7, 15, 127} and x >= 0, correctly rounded like the IEEE division the reference performs:
+// division by a divisor known in advance (P. Markstein, IBM J. Res. Dev. 34(1), 1990; N. Brisebarre, J.-M. Muller,
+// S. K. Raina, IEEE Trans. Computers 53(8), 2004).  With c = RN(1/y): q = RN(x c), r = RN(x - y q), result
+// RN(q + r c).  Checked exhaustively on the host against x / y for every
+// non-negative finite fp32 x (all three constants): no mismatch.  Infinite / NaN x fall through to q.
 __device__ __forceinline__ float div_const_rn(float x, float y, float c) {
     const float q = __fmul_rn(x, c);
     const float r = __fmaf_rn(-y, q, x);
     const float q2 = __fmaf_rn(r, c, q);
     return (r == r) ? q2 : q;
 }
+// Nearest integer, ties away from zero.  |v| + 1/2 rounded toward zero never falls below an integer that the exact sum
+// reaches (integers below 2^23 are representable, and from there on the sum rounds back to v), so truncating it gives
+// floor(|v| + 1/2).
+__device__ __forceinline__ int round_half_away(float v) { return __float2int_rz(__fadd_rz(v, copysignf(0.5f, v))); }
 // 1 / d as the reference computes it (IEEE division), 0 for d == 0
 __device__ __forceinline__ float inv_or_zero(float d) { return (d != 0.0f) ? __frcp_rn(d) : 0.0f; }
 

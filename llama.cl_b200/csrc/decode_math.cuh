@@ -65,8 +65,7 @@ __device__ __forceinline__ void q8_quantize_rows_v(const float (&v)[ROWS][4], in
                 if (e0 + j < (lens[m] & ~7)) {
                     q = __float2int_rn(tq);  // nearest even
                 } else {
-                    const float h = __int_as_float((__float_as_int(tq) & 0x80000000) | 0x3F000000);
-                    q = __float2int_rz(__fadd_rz(tq, h));  // half away from zero, exact for every fp32
+                    q = round_half_away(tq);  // std::round
                 }
                 q = min(127, max(-128, q));
             }

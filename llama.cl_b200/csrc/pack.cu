@@ -16,9 +16,8 @@
 //
 // Arithmetic is the reference's, in fp32 with IEEE division: Q4_1
 // d=(max-min)/15, m=min, q=clamp(roundf((w-m)/d'),0,15) with d'=1/d computed
-// first; Q4_0 d=max(|min|,|max|)/7, q=clamp(roundf(w*d'),-7,7).  roundf
-// (half away from zero) is done as trunc(v +- 0.5) with the addition rounded
-// toward zero, which is exact for every fp32 v.
+// first; Q4_0 d=max(|min|,|max|)/7, q=clamp(roundf(w*d'),-7,7), roundf as
+// round_half_away of common.cuh.
 #include "common.cuh"
 
 namespace q4fc {
@@ -35,12 +34,6 @@ struct MinMax {
 __device__ __forceinline__ void mm_take(MinMax& a, float v) {  // sequential step of get_min_max
     if (a.vmax < v) a.vmax = v;
     if (a.vmin > v) a.vmin = v;
-}
-
-__device__ __forceinline__ int round_half_away(float v) {
-    // trunc(v + copysign(0.5, v)) with a round-toward-zero add == roundf(v)
-    float h = __int_as_float((__float_as_int(v) & 0x80000000) | 0x3F000000);
-    return __float2int_rz(__fadd_rz(v, h));
 }
 
 template <int G, int QTYPE>

@@ -40,11 +40,6 @@ __device__ __forceinline__ void mma_s8s8(int (&c)[4], uint32_t a0, uint32_t a1, 
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ float round_half_away(float t) {
-    const float h = __int_as_float((__float_as_int(t) & 0x80000000) | 0x3F000000);
-    return truncf(__fadd_rz(t, h));
-}
-
 // ---- pack ----------------------------------------------------------------------------------------------------------
 // Two launches.  q8c_scale_kernel: one warp per column n (a row of W) finds amax and stores d = amax / 127.
 // q8c_pack_kernel: grid (stripes, chunks of kPackBlocks K groups); per block the CTA reads 32 columns x 32 k with
@@ -99,7 +94,7 @@ __global__ void __launch_bounds__(256) q8c_pack_kernel(const float* __restrict__
             }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int q = (int)round_half_away(__fmul_rn(v[j], id));  // 0 beyond K
+                const int q = round_half_away(__fmul_rn(v[j], id));  // 0 beyond K
                 word |= (uint32_t)(q & 0xFF) << (8 * j);
             }
         }
@@ -241,7 +236,7 @@ __global__ void __launch_bounds__(256) emb_q8c_quant_kernel(const float* __restr
     const int64_t body = E & ~(int64_t)7;
     for (int64_t k = threadIdx.x; k < E; k += 256) {
         const float tv = __fmul_rn(__ldg(src + k), id);
-        const int q = (k < body) ? __float2int_rn(tv) : (int)round_half_away(tv);
+        const int q = (k < body) ? __float2int_rn(tv) : round_half_away(tv);
         dst[k] = (int8_t)min(127, max(-128, q));
     }
 }

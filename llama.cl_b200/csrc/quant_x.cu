@@ -81,8 +81,7 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_kernel(const float* __r
             if (e < body) {
                 q = sat8(__float2int_rn(t));  // nearest even, as _mm256_round_ps + packs
             } else {
-                const float h = __int_as_float((__float_as_int(t) & 0x80000000) | 0x3F000000);
-                q = sat8(__float2int_rz(__fadd_rz(t, h)));  // std::round: half away
+                q = sat8(round_half_away(t));  // std::round
             }
         }
         packed |= (uint32_t)(q & 0xFF) << (8 * j);
@@ -208,8 +207,7 @@ __device__ __forceinline__ void quant_pre_unit(const float* __restrict__ x, int 
             if (e0 + j < body) {
                 q = __float2int_rn(t);
             } else {
-                const float h = __int_as_float((__float_as_int(t) & 0x80000000) | 0x3F000000);
-                q = __float2int_rz(__fadd_rz(t, h));
+                q = round_half_away(t);  // std::round
             }
             q = sat8(q);
         }

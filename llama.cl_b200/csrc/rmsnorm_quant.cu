@@ -123,8 +123,7 @@ __global__ void __launch_bounds__(kRnThreads) rmsnorm_quant_kernel(const float* 
                 if (e0 + j < body) {
                     q = __float2int_rn(t);
                 } else {
-                    const float h = __int_as_float((__float_as_int(t) & 0x80000000) | 0x3F000000);
-                    q = __float2int_rz(__fadd_rz(t, h));
+                    q = round_half_away(t);  // std::round
                 }
                 q = sat8(q);
             }
