@@ -10,6 +10,7 @@ import os
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "lib", "libq4fc_b200.so")
+FRONT_PATH = os.path.join(PKG, "lib", "_q4fc_front.so")
 
 Q4_0, Q4_1 = 0, 1
 FLAG_NIBBLE_SIGNED = 1
@@ -180,6 +181,28 @@ def lib() -> C.CDLL:
                                         C.POINTER(i64), i32, vp, vp, vp]
     _lib = L
     return L
+
+
+_front = None
+
+
+def front():
+    """The native front of the ops (``csrc/front.cpp``), loaded on first use; ``llmops`` binds its workspace makers."""
+    global _front
+    if _front is None:
+        lib()  # the front is linked with it
+        if not os.path.exists(FRONT_PATH):
+            raise RuntimeError(f"{FRONT_PATH} is missing: build it with `python llama.cl_b200/build.py`")
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries come first)
+
+        loader = importlib.machinery.ExtensionFileLoader("_q4fc_front", FRONT_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_q4fc_front", loader))
+        loader.exec_module(mod)
+        _front = mod
+    return _front
 
 
 def check(rc: int, what: str) -> None:

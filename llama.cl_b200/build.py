@@ -1,8 +1,10 @@
-"""Build the sm_100a shared library ``lib/libq4fc_b200.so`` from ``csrc/*.cu``.
+"""Build the sm_100a shared library ``lib/libq4fc_b200.so`` from ``csrc/*.cu``
+and the Python front ``lib/_q4fc_front.so`` from ``csrc/front.cpp``.
 
-In-tree build with nvcc only (no torch headers: the library has a plain C
-ABI).  Each translation unit is compiled to an object in ``build/`` (in
-parallel) and linked with the static CUDA runtime.
+In-tree build.  The library needs nvcc only (no torch headers: it has a plain C
+ABI); each translation unit is compiled to an object in ``build/`` (in
+parallel) and linked with the static CUDA runtime.  The front is host code
+against the headers of the installed torch; it is linked with the library.
 """
 from __future__ import annotations
 
@@ -18,6 +20,8 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIB_DIR, "libq4fc_b200.so")
+FRONT_SRC = os.path.join(CSRC, "front.cpp")
+FRONT = os.path.join(LIB_DIR, "_q4fc_front.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
@@ -37,6 +41,21 @@ def _stale(target: str, deps: list[str]) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def front_command() -> list[str]:
+    import sysconfig
+
+    import torch
+
+    tdir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(nvcc()))
+    inc = [f"-I{os.path.join(tdir, 'include')}", f"-I{os.path.join(tdir, 'include', 'torch', 'csrc', 'api', 'include')}",
+           f"-I{os.path.join(cuda, 'include')}", f"-I{sysconfig.get_paths()['include']}"]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *inc, FRONT_SRC, "-o", FRONT,
+            f"-L{os.path.join(tdir, 'lib')}", "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10_cuda", "-lc10",
+            f"-L{os.path.join(cuda, 'lib64')}", "-lcudart", f"-L{LIB_DIR}", "-lq4fc_b200", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -63,6 +82,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-cudart", "static",
                *objs, "-o", LIB]
         subprocess.run(cmd, check=True)
+    if force or _stale(FRONT, [FRONT_SRC, headers[-1]]):
+        subprocess.run(front_command(), check=True)
     return LIB
 
 

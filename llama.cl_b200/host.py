@@ -2,8 +2,8 @@
 
 The reference's ``fc_Q4A`` takes and returns host memory.  ``HostFC`` keeps the
 packed weight resident on the GPU (as the reference keeps it resident in RAM
-after ``llmop_fc_q4a.__init__``) and, per call, copies the activations from
-pinned host memory to the device, runs the FC and copies the result back to
+after ``llmop_fc_q4a.__init__``) and, per call, brings the activations from
+pinned host memory to the device, runs the FC and brings the result back to
 pinned host memory."""
 from __future__ import annotations
 
@@ -16,9 +16,10 @@ from . import _cabi, llmops
 class HostFC:
     """``y_host = HostFC(wq, N)(x_host)``.
 
-    With ``graph=True`` (default) the three steps of a call -- copy in, FC kernel, copy out -- are captured
-    once per row count into a CUDA graph over fixed pinned staging buffers and replayed, which takes the
-    per-call cost on the CPU from several framework calls to one graph launch.  ``stream``: the stream the
+    With ``graph=True`` (default) the steps of a call are captured once per row count into a CUDA graph over fixed
+    pinned staging buffers and replayed, which takes the per-call cost on the CPU from several framework calls to
+    one graph launch.  Up to 8 rows the kernels read and write the pinned buffers themselves (the quantizing launch
+    reads every activation once, the FC kernel writes every output once), beyond that a copy each way frames the FC.  ``stream``: the stream the
     call runs on (default: a stream of its own); independent FCs on different streams overlap their copies
     and kernels.  With ``sync=False`` the caller synchronizes ``stream`` before reading the result or
     calling the same object again."""
@@ -41,7 +42,8 @@ class HostFC:
         self._y_host = torch.empty((1, max_rows, self.N), dtype=torch.float32).pin_memory()
         self.max_rows = max_rows
         self.use_graph = bool(graph)
-        self._graphs: dict[int, torch.cuda.CUDAGraph] = {}
+        self._graphs: dict[int, tuple] = {}  # rows -> (graph, executable, staging view, output view)
+        self._front, self._stream_ptr, self._dev_index = llmops._front(), self.stream.cuda_stream, llmops._index(dev)
         if self.fc_kwargs.get("workspace") is None:
             # captured graphs hold the workspace's address: own one, sized once for the largest call
             with torch.cuda.device(dev):
@@ -53,22 +55,39 @@ class HostFC:
         straight into it and passing it to ``__call__`` saves the host-side copy."""
         return self._x_host[:, :M]
 
+    def _reads_host(self, M: int) -> bool:
+        """Whether a call of ``M`` rows works on the pinned buffers in place.  A copy node costs 3-5 us of latency on
+        each side of a kernel that runs 5-20 us, and the bytes cross PCIe once either way; the prefill kernels and the
+        stream-K form re-read or re-write their buffers, so they get copies."""
+        return M <= 8 and set(self.fc_kwargs) <= {"workspace", "nibble_signed", "pdl", "prequant"}
+
     def _enqueue(self, M: int) -> None:
+        if self._reads_host(M):
+            kw, ws = self.fc_kwargs, self.fc_kwargs["workspace"]
+            flags = _cabi.FLAG_PREQUANT | (_cabi.FLAG_NIBBLE_SIGNED if kw.get("nibble_signed") else 0) | \
+                (_cabi.FLAG_PDL if kw.get("pdl") else 0)
+            Ng, Kg, _ = self.wq.shape
+            with torch.cuda.device(self.device):
+                _cabi.check(_cabi.lib().q4fc_fc_decode(
+                    self._x_host.data_ptr(), M, self.K, self.K, self.wq.data_ptr(), Ng, Kg, self.qtype, self.G, self.N,
+                    self._y_host.data_ptr(), self.N, ws.ptr, ws.nbytes, flags,
+                    torch.cuda.current_stream(self.device).cuda_stream), "HostFC")
+            return
         xd, yd = self._x_dev[:, :M], self._y_dev[:, :M]
         xd.copy_(self._x_host[:, :M], non_blocking=True)
         llmops.fc_Q4A(xd, self.wq, self.N, out=yd, **self.fc_kwargs)
         self._y_host[:, :M].copy_(yd, non_blocking=True)
 
-    def _graph(self, M: int) -> torch.cuda.CUDAGraph:
+    def _graph(self, M: int) -> tuple:
         g = self._graphs.get(M)
         if g is None:
             with torch.cuda.stream(self.stream):
                 self._enqueue(M)  # eager once: kernel attributes and lazy look-ups happen outside the capture
                 self.stream.synchronize()
-                g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g, stream=self.stream):
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=self.stream):
                     self._enqueue(M)
-            self._graphs[M] = g
+            g = self._graphs[M] = (graph, graph.raw_cuda_graph_exec(), self._x_host[:, :M], self._y_host[:, :M])
         return g
 
     def __call__(self, x_host: torch.Tensor, sync: bool = True) -> torch.Tensor:
@@ -77,16 +96,19 @@ class HostFC:
         M = x_host.shape[1]
         if M > self.max_rows or x_host.shape[2] != self.K:
             raise RuntimeError(f"HostFC: input {tuple(x_host.shape)} does not fit [1, <={self.max_rows}, {self.K}]")
+        if self.use_graph:
+            _, ex, stage, y = self._graph(M)
+            # one native call: activations into the staging buffer, graph launch, wait
+            if self._front.graph_step(stage, x_host, ex, self._stream_ptr, self._dev_index, sync):
+                return y
+            stage.copy_(x_host)
+            self._front.graph_step(stage, None, ex, self._stream_ptr, self._dev_index, sync)
+            return y
         stage = self._x_host[:, :M]
         if x_host.data_ptr() != stage.data_ptr():
             stage.copy_(x_host)
-        if self.use_graph:
-            g = self._graph(M)
-            with torch.cuda.stream(self.stream):
-                g.replay()
-        else:
-            with torch.cuda.stream(self.stream):
-                self._enqueue(M)
+        with torch.cuda.stream(self.stream):
+            self._enqueue(M)
         if sync:
             self.stream.synchronize()
         return self._y_host[:, :M]

@@ -27,8 +27,25 @@ __all__ = ["offline_FC_quant_Q4A", "offline_FC_dequant_Q4A", "fc_Q4A", "FC_dynam
            "QuantizedActivations", "QuantizeBatch", "FCChain", "FC_quant_Q8C", "FC_evaluate_Q8C", "embedding_q8c_quant_w", "embedding_q8c", "check_device_status"]
 
 
+def _index(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
+
+
 def _stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(_index(device))
+
+
+_native = None
+
+
+def _front():
+    """The native front (``csrc/front.cpp``) that checks, allocates, looks up and launches for the ops below."""
+    global _native
+    if _native is None:
+        f = _cabi.front()
+        f.bind(_make_fc_workspace, _make_q8c_scratch)
+        _native = f
+    return _native
 
 
 def _require_cuda(t: torch.Tensor, name: str, dtype: torch.dtype, rank: int) -> None:
@@ -89,26 +106,16 @@ def fc_workspace(rows: int, K: int, N: int, qtype: int, group_k: int, device: to
     return ws
 
 
+def _make_fc_workspace(rows: int, K: int, N: int, qtype: int, group_k: int, index: int):
+    """Called by the front when a call on the current stream finds no workspace, or too small a one."""
+    ws = fc_workspace(rows, K, N, qtype, group_k, torch.device("cuda", index))
+    return ws, ws.ptr, ws.nbytes
+
+
 def offline_FC_quant_Q4A(wei: torch.Tensor, *, qtype="q4_1", group_k: int = 32,
                          out: torch.Tensor | None = None) -> torch.Tensor:
     """fp32 ``[N, K]`` -> int8 ``[ceil(N/32), ceil(K/group_k), block_bytes]`` (ops/op_fc.hpp:151-219)."""
-    q = _cabi.parse_qtype(qtype)
-    _require_cuda(wei, "wei", torch.float32, 2)
-    N, K = wei.shape
-    bs = _cabi.lib().q4fc_block_bytes(q, group_k)
-    if bs < 0:
-        raise RuntimeError(f"unsupported block type: qtype={qtype!r}, group_k={group_k}")
-    Ng, Kg = (N + 31) // 32, (K + group_k - 1) // group_k
-    if out is None:
-        out = torch.empty((Ng, Kg, bs), dtype=torch.int8, device=wei.device)
-    else:
-        _require_cuda(out, "out", torch.int8, 3)
-        if tuple(out.shape) != (Ng, Kg, bs):
-            raise RuntimeError(f"out: expected shape {(Ng, Kg, bs)}, got {tuple(out.shape)}")
-    with torch.cuda.device(wei.device):
-        _cabi.check(_cabi.lib().q4fc_pack(wei.data_ptr(), N, K, q, group_k, out.data_ptr(), _stream_ptr(wei.device)),
-                    "offline_FC_quant_Q4A")
-    return out
+    return _front().pack(wei, _cabi.parse_qtype(qtype), group_k, out)
 
 
 def offline_FC_dequant_Q4A(weiq: torch.Tensor, *, nibble_signed: bool = False) -> torch.Tensor:
@@ -161,50 +168,7 @@ def fc_Q4A(input: torch.Tensor, wei_quantized: torch.Tensor, N: int, *, nibble_s
     different streams; by default that happens only for large rows x K.  ``addend`` (decode kernel, B*M <= 8):
     fp32 ``[N]`` (a bias) or ``[B, M, N]`` (a residual; may be ``out``), added to the result inside the kernel
     with one fp32 add per output, as the reference's ``llmops.iadd`` after the FC does."""
-    _require_cuda(input, "input", torch.float32, 3)
-    _require_cuda(wei_quantized, "wei_quantized", torch.int8, 3)
-    if wei_quantized.device != input.device:
-        raise RuntimeError("input and wei_quantized live on different devices")
-    B, M, K = input.shape
-    Ng, Kg, bs = wei_quantized.shape
-    q, G = _cabi.infer_variant(bs)
-    N = int(N)
-    rows = B * M
-    if out is None:
-        out = torch.empty((B, M, N), dtype=torch.float32, device=input.device)
-    else:
-        _require_cuda(out, "out", torch.float32, 3)
-        if tuple(out.shape) != (B, M, N):
-            raise RuntimeError(f"out: expected shape {(B, M, N)}, got {tuple(out.shape)}")
-    if workspace is None:
-        workspace = fc_workspace(rows, K, N, q, G, input.device)
-    flags = (FLAG_NIBBLE_SIGNED if nibble_signed else 0) | (FLAG_PDL if pdl else 0)
-    if path == "streamk":
-        flags |= FLAG_STREAMK
-    if prequant:
-        flags |= _cabi.FLAG_PREQUANT
-    L = _cabi.lib()
-    if addend is not None:
-        _require_cuda(addend, "addend", torch.float32, addend.dim())
-        if rows > 8 or path in ("streamk", "prefill"):
-            raise RuntimeError("addend is folded into the decode kernel only (B*M <= 8, path auto or decode)")
-        if tuple(addend.shape) == (N,):
-            ld_add = 0
-        elif tuple(addend.shape) == (B, M, N) and addend.is_contiguous():
-            ld_add = N
-        else:
-            raise RuntimeError(f"addend: expected contiguous shape {(N,)} or {(B, M, N)}, got {tuple(addend.shape)}")
-        with torch.cuda.device(input.device):
-            _cabi.check(L.q4fc_fc_decode_add(input.data_ptr(), rows, K, K, wei_quantized.data_ptr(), Ng, Kg, q, G, N,
-                                             out.data_ptr(), N, addend.data_ptr(), ld_add, workspace.ptr,
-                                             workspace.nbytes, flags, _stream_ptr(input.device)), "fc_Q4A")
-        return out
-    fn = {"auto": L.q4fc_fc, "decode": L.q4fc_fc_decode, "streamk": L.q4fc_fc_decode,
-          "prefill": L.q4fc_fc_prefill}[path]
-    with torch.cuda.device(input.device):
-        _cabi.check(fn(input.data_ptr(), rows, K, K, wei_quantized.data_ptr(), Ng, Kg, q, G, N, out.data_ptr(), N,
-                       workspace.ptr, workspace.nbytes, flags, _stream_ptr(input.device)), "fc_Q4A")
-    return out
+    return _front().fc(input, wei_quantized, N, nibble_signed, out, workspace, pdl, path, prequant, addend)
 
 
 class QuantizedActivations:
@@ -278,11 +242,10 @@ class QuantizeBatch:
             a = self._args[i]
             a.x, a.rows, a.K, a.ldx, a.xq = x.data_ptr(), xq.rows, xq.K, xq.K, xq.buf.data_ptr()
         self.group_k, self.signed, self.flags = G, signed, (FLAG_PDL if pdl else 0)
+        self._address, self._dev_index = _cabi.C.addressof(self._args), _index(self.device)
 
     def run(self) -> None:
-        with torch.cuda.device(self.device):
-            _cabi.check(_cabi.lib().q4fc_quant_x_q8_batch(self._args, self.n, self.group_k, int(self.signed), self.flags,
-                                                          _stream_ptr(self.device)), "quant_x_q8_batch")
+        _front().quant_batch(self._address, self.n, self.group_k, self.signed, self.flags, self._dev_index)
 
 
 def rmsnorm_quantize(input: torch.Tensor, weight: torch.Tensor, eps: float, group_k: int, *,
@@ -488,11 +451,10 @@ class FCBatch:
             self.outs.append(out)
         self.qtype, self.group_k = q, G
         self.flags = (FLAG_PDL if pdl else 0) | (FLAG_NIBBLE_SIGNED if (signed and q == Q4_0) else 0)
+        self._address, self._dev_index = _cabi.C.addressof(self._args), _index(self.device)
 
     def run(self):
-        with torch.cuda.device(self.device):
-            _cabi.check(_cabi.lib().q4fc_fc_decode_batch(self._args, self.n, self.qtype, self.group_k, self.flags,
-                                                         _stream_ptr(self.device)), "fc_decode_batch")
+        _front().fc_batch(self._address, self.n, self.qtype, self.group_k, self.flags, self._dev_index)
         return self.outs
 
 
@@ -614,7 +576,14 @@ class FCChain:
 
 
 # ---- per-channel int8 weights ("Q8C") and the quantized embedding table ---------------------------------------------
-_q8c_scratch: dict = {}
+_q8c_scratch: dict = {}  # (device index, stream) -> codes and scales of the largest call so far
+
+
+def _make_q8c_scratch(index: int, stream: int, need: int):
+    """Called by the front when a call on ``stream`` finds no scratch, or too small a one."""
+    ws = torch.empty(max(need, 1 << 16), dtype=torch.uint8, device=torch.device("cuda", index))
+    _q8c_scratch[(index, stream)] = ws
+    return ws, ws.data_ptr(), ws.numel()
 
 
 def FC_quant_Q8C(wei: torch.Tensor):
@@ -635,35 +604,7 @@ def FC_evaluate_Q8C(input: torch.Tensor, wei_quantized: torch.Tensor, wei_scales
                     out: torch.Tensor | None = None) -> torch.Tensor:
     """``[B, M, K]`` x Q8C weights -> ``[B, M, N]`` (ext/llama_ext.cpp:336-371).  The scratch for the quantized
     activations is kept per (device, stream) and grows to the largest call; calls on one stream are ordered."""
-    _require_cuda(input, "input", torch.float32, 3)
-    _require_cuda(wei_quantized, "wei_quantized", torch.int8, 3)
-    _require_cuda(wei_scales, "wei_scales", torch.float32, 1)
-    B, M, K = input.shape
-    Ng, Kg, bs = wei_quantized.shape
-    if bs != 1024:
-        raise RuntimeError(f"assert wei_quantized.size(2) == sizeof(q8_c_block) failed: got {bs}")
-    if Kg != (K + 31) // 32 or N > Ng * 32 or wei_scales.numel() < N:
-        raise RuntimeError(f"FC_evaluate_Q8C: weights {tuple(wei_quantized.shape)} / scales {tuple(wei_scales.shape)} "
-                           f"do not match K={K}, N={N}")
-    dev = input.device
-    if out is None:
-        out = torch.empty((B, M, N), dtype=torch.float32, device=dev)
-    else:
-        _require_cuda(out, "out", torch.float32, 3)
-        if tuple(out.shape) != (B, M, N):
-            raise RuntimeError(f"out: expected shape {(B, M, N)}, got {tuple(out.shape)}")
-    L = _cabi.lib()
-    need = L.q4fc_q8c_workspace_bytes(B * M, K)
-    with torch.cuda.device(dev):
-        stream = _stream_ptr(dev)
-        key = (dev.index, stream)
-        ws = _q8c_scratch.get(key)
-        if ws is None or ws.numel() < need:
-            ws = torch.empty(max(need, 1 << 16), dtype=torch.uint8, device=dev)
-            _q8c_scratch[key] = ws
-        _cabi.check(L.q4fc_q8c_fc(input.data_ptr(), B * M, K, K, wei_quantized.data_ptr(), wei_scales.data_ptr(), Ng,
-                                  Kg, N, out.data_ptr(), N, ws.data_ptr(), ws.numel(), stream), "FC_evaluate_Q8C")
-    return out
+    return _front().q8c_fc(input, wei_quantized, wei_scales, N, out)
 
 
 def embedding_q8c_quant_w(weight: torch.Tensor):
@@ -683,24 +624,7 @@ def embedding_q8c(output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
     """``output[..., :] = scales[id] * weight[id, :]`` for the ids in ``input`` (int32 or int64, any rank), with the
     reference's argument order and in-place result (ops/op_embedding.hpp:108-137).  An id outside the table gives a
     row of zeros and makes ``check_device_status`` raise."""
-    _require_cuda(weight, "weight", torch.int8, 2)
-    _require_cuda(scales, "scales", torch.float32, 1)
-    if not isinstance(input, torch.Tensor) or input.dtype not in (torch.int32, torch.int64):
-        raise RuntimeError("assert input.is<int64_t>() failed: ids must be int32 or int64")
-    if not input.is_cuda or not input.is_contiguous():
-        raise RuntimeError("input: must be a contiguous CUDA tensor")
-    V, E = weight.shape
-    if not isinstance(output, torch.Tensor) or output.dtype != torch.float32:
-        raise RuntimeError("assert output.is<float>() failed")
-    if tuple(output.shape) != tuple(input.shape) + (E,):
-        raise RuntimeError(f"assert infer_shape() == output.shape() failed: {tuple(output.shape)} vs "
-                           f"{tuple(input.shape) + (E,)}")
-    if not output.is_cuda or not output.is_contiguous():
-        raise RuntimeError("output: must be a contiguous CUDA tensor")
-    with torch.cuda.device(weight.device):
-        _cabi.check(_cabi.lib().q4fc_emb_q8c(input.data_ptr(), int(input.dtype == torch.int32), input.numel(),
-                                             weight.data_ptr(), scales.data_ptr(), V, E, output.data_ptr(), E,
-                                             _stream_ptr(weight.device)), "embedding_q8c")
+    _front().embedding(input, weight, scales, output)
 
 
 def check_device_status(device: torch.device | None = None) -> None:

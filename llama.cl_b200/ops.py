@@ -54,9 +54,7 @@ class llmop_embedding_q8c:
 
     def __call__(self, input_ids: torch.Tensor) -> torch.Tensor:
         ids = input_ids.to(self.weight.device).contiguous()
-        output = torch.empty(tuple(ids.shape) + (self.weight.shape[1],), dtype=torch.float32, device=self.weight.device)
-        llmops.embedding_q8c(output, ids, self.weight, self.scales)
-        return output
+        return llmops._front().embedding(ids, self.weight, self.scales, None)
 
     def __repr__(self) -> str:
         return f"llmop_embedding_q8c(weight: {list(self.weight.shape)})"

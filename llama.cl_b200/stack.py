@@ -84,6 +84,8 @@ class DecodeFCStack:
             self.xq_m = QA(1, R, I, self.G, False, dev)  # silu(gate) * up
         self.stream = torch.cuda.Stream(dev)
         self._graph = None
+        self._exec = None  # its executable graph, where forward() may launch it directly
+        self._front, self._stream_ptr, self._dev_index = llmops._front(), self.stream.cuda_stream, llmops._index(dev)
         self.use_graph = bool(graph)
         self.launches_per_token = (8 * len(layers) + 2) if glue == "llama" else (4 * len(layers) + 1)
         self.chains = None
@@ -191,6 +193,10 @@ class DecodeFCStack:
         """``x``: fp32 ``[1, rows, hidden]`` on the device (copied into the stack's input buffer), or None to run
         on what ``self.x`` holds.  Returns ``self.logits`` ``[1, rows, vocab]`` (valid once ``self.stream`` has
         been waited for, which ``sync=True`` does)."""
+        # A captured token is one native call: input copy, graph launch, wait.  (An ``attention`` callable may hold
+        # random-number kernels, whose state only CUDAGraph.replay() advances.)
+        if self._exec is not None and self._front.graph_step(self.x, x, self._exec, self._stream_ptr, self._dev_index, sync):
+            return self.logits
         with torch.cuda.stream(self.stream):
             if x is not None:
                 self.x.copy_(x, non_blocking=True)
@@ -204,6 +210,8 @@ class DecodeFCStack:
                     with torch.cuda.graph(g, stream=self.stream):
                         self.enqueue()
                     self._graph = g
+                    if self.attention is None:
+                        self._exec = g.raw_cuda_graph_exec()
                 self._graph.replay()
         if sync:
             self.stream.synchronize()
