@@ -54,6 +54,9 @@ int launch_dequant(const uint8_t* wq, int64_t Ng, int64_t Kg, int qtype, int G, 
                    cudaStream_t s);
 int launch_quant_x(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, float scale, int8_t* codes,
                    float* scales, float* gsums, cudaStream_t s);
+// the prefill GEMM's quantizer: scales (and group sums) by row tile of 64 or 128 (quant_x.cu)
+int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, bool sums, int tile, int8_t* codes,
+                        float* sc, cudaStream_t s);
 constexpr size_t kWsCounterCapacity = 64 * 1024;  // stripe counters of N <= 524288 end before the quantizer scratch
 size_t decode_workspace_bytes(int64_t N);
 size_t decode_prequant_offset();
@@ -116,6 +119,10 @@ size_t prefill_workspace_bytes(int64_t rows, int64_t K, int64_t N, int qtype, in
 int launch_fc_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, const uint8_t* wq, int64_t Ng,
                       int64_t Kg, int qtype, int G, int64_t N, float* y, int64_t ldy, void* ws, size_t ws_bytes,
                       unsigned flags, cudaStream_t s);
+// the same GEMM over per-channel int8 weights; `sc`: scratch of q8c_prefill_scale_bytes
+size_t q8c_prefill_scale_bytes(int64_t rows, int64_t Kg);
+int launch_q8c_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, const int8_t* wq, const float* wscales,
+                       int64_t Ng, int64_t Kg, int64_t N, float* y, int64_t ldy, int8_t* codes, float* sc, cudaStream_t s);
 
 #ifdef __CUDACC__
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }

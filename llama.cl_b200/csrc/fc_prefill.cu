@@ -1,115 +1,130 @@
-// Prefill FC (rows > 8): dense int8 contraction on the 5th-generation tensor
-// cores.  Replaces fc_Q4A (ops/op_fc.hpp:286-426) for large B*M.
+// FC over many activation rows (prefill): dense int8 contraction on the 5th-generation tensor cores.  Replaces fc_Q4A
+// (ops/op_fc.hpp:286-426) for B*M > 8 and, with FMT = kQ8C, FC_evaluate_Q8C (ext/llama_ext.cpp:232-371).
 //
-//   y[m][n] = sum_kb  fp32(wd[n,kb]) * xs[m,kb] * I[m,n,kb]  (+ fp32(wm[n,kb]) * gsum[m,kb], Q4_1)
-//   I[m,n,kb] = sum_{k in group kb} nibble(n,k) * code(m,k)      exact int32
+//   Q4:   y[m][n] = sum_kb  fp32(wd[n,kb]) * xs[m,kb] * I[m,n,kb]  (+ fp32(wm[n,kb]) * gsum[m,kb], Q4_1)
+//   Q8C:  y[m][n] = wscale[n] * sum_kb xs[m,kb] * I[m,n,kb]
+//   I[m,n,kb] = sum_{k in group kb} weight code(n,k) * activation code(m,k)      exact int32
 //
-// Two launches: the Q8 quantizer (quant_x.cu) writes codes / scales / group
-// sums of all rows to the workspace, then this kernel runs the GEMM.
+// Two launches: quant_x_tile_kernel (quant_x.cu) writes codes, scales and group sums of all rows to the workspace; this
+// kernel, started while that one runs (programmatic launch: its weight copies do not depend on it), runs the GEMM.
 //
-// One CTA computes a 128 (columns n) x 128 (rows m) output tile.
-//   * operand A = weights: the packed nibbles of 4 stripes are unpacked to
-//     one byte per weight in shared memory, K-major rows of 128 bytes, in the
-//     128-byte-swizzle canonical layout that tcgen05.mma reads;
-//   * operand B = activation codes (int8), same layout;
-//   * D = int32 accumulators in tensor memory, lane = weight column,
-//     column = activation row.
-// Every K group has its own pair of scales, so a group's MMA(s) (one K=32
-// instruction for group 32, four for group 128) write a fresh TMEM buffer
-// (4 buffers x 128 columns = all 512 columns) and the epilogue warps read the
-// buffer back with tcgen05.ld, turn the exact integers into fp32 (magic-number
-// add, no cvt), scale them and accumulate the tile in registers.  The CUDA-core
-// work per (m, n, group) -- one int add, one fp add, one mul, one or two fma --
-// is what bounds this kernel: the tensor pipe waits for the epilogue.
+// One CTA computes 128 columns n x TM rows m:
+//   * operand A = weights: the packed blocks come in by bulk copies, are unpacked to one byte per weight in shared
+//     memory, K-major rows of 128 bytes, in the 128-byte-swizzle canonical layout that tcgen05.mma reads;
+//   * operand B = activation codes (int8), same layout, straight from the code matrix by TMA;
+//   * D = int32 accumulators in tensor memory, lane = weight column, column = activation row.
+// Every K group has its own pair of scales, so a group's MMA(s) (one K=32 instruction for group 32, four for group
+// 128) write a fresh TMEM buffer (4 buffers of TM columns), and the epilogue warps read the buffer back with
+// tcgen05.ld, turn the exact integers into fp32, scale them and accumulate the tile in registers.
 //
-// Warp roles (24 warps, 21 of them busy): 0-15 epilogue (warp%4 = TMEM lane quarter, warp/4 =
-// which 32 of the 128 tile rows), 16-19 producers (unpack A and stage the
-// scales of one 128-k stage: generic-proxy stores + fence.proxy.async; one of
-// them also issues the TMA load of the B tile from the code matrix), 20 MMA
-// issue (one elected lane).  mbarriers: full/empty per shared-memory stage,
-// tfull/tempty per TMEM buffer.  Every wait is bounded: when a wait runs out
-// the CTA sets the workspace status word, every role leaves its loop, TMEM is
-// freed and the kernel returns.
+// What bounds it: the CUDA-core work per (m, n, group) -- one conversion, one mul, one or two fma -- against 32 or 128
+// tensor MACs.  Everything else is arranged to stay behind that: the packed bytes are prefetched several stages ahead
+// (a warp re-arms its own slot as soon as it has unpacked it), a lane unpacks one column so that both its 32-bit loads
+// and its 128-bit stores are free of bank conflicts without selects, scales arrive in the layout in which the epilogue
+// reads four rows per load, and weights, codes and scales have rings of their own, so that operands are released by the
+// MMA and not by the epilogue.
+//
+// Measured (whole call, quantizer included; before: unpacking straight from global memory without prefetch, one 128 x 128
+// tile per CTA whatever the row count, epilogue of 5 operations per integer):
+//   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 us   Q4_0 g32, 512 rows 280 -> 223 us (207 TOPS)
+//                   Q4_1 g128, 2048 rows 517 -> 323 us (572 TOPS)   Q8C, 256 rows 296 -> 132 us (175 TOPS)
+// A group of 32 k takes about 1100 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
+// convert, scale is latency-bound with the 16 warps that the registers allow.  Tried and dropped: handing registers
+// between roles with setmaxnreg (spills around it; 260 us for the 512-row case), both chunks in registers at once
+// (320 us), the add-a-constant conversion instead of I2F (30 % more issue slots), scalar instead of packed fp32 (5 % slower).
+//
+// Warp roles: epilogue (warp % 4 = TMEM lane quarter, warp / 4 = which 16-row chunks), 4 unpacking warps (one stripe
+// each), one MMA issuer, one loader.  Every wait is bounded: when a wait runs out the CTA sets the status word, every
+// role leaves its loop, TMEM is freed and the kernel returns.
+//
+// Few tiles: a cluster of `split` CTAs shares a tile and divides its K stages; the partial tiles meet in shared memory
+// and are added in rank order (fixed order, no atomics).
 #include <cuda.h>  // CUtensorMap and the cuTensorMapEncodeTiled prototype (resolved at run time, libcuda is not linked)
+
+#include <cooperative_groups.h>
 
 #include <atomic>
 
 #include "common.cuh"
+#include "ring_ptx.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace q4fc {
 namespace {
 
-constexpr int kTileN = 128;            // weight columns per tile = TMEM lanes
-constexpr int kTileM = 128;            // activation rows per tile = TMEM columns per buffer
-constexpr int kStageK = 128;           // k per shared-memory stage (one 128-byte swizzle row)
-constexpr int kStages = 4;
+constexpr int kTileN = 128;    // weight columns per tile = TMEM lanes
+constexpr int kStageK = 128;   // k per shared-memory stage (one 128-byte swizzle row)
 constexpr int kTmemBufs = 4;
-constexpr int kEpiWarps = 16, kProdWarps = 4;
-constexpr int kProdThreads = kProdWarps * 32;
-constexpr int kThreads = (kEpiWarps + kProdWarps + 4) * 32;  // the MMA warp's warpgroup is filled up with idle warps
-constexpr int kMmaWarp = kEpiWarps + kProdWarps;
-constexpr uint64_t kWaitLimitNs = 1000000000ull;  // every mbarrier wait gives up after one second
+constexpr int kProdWarps = 4;  // one stripe of the tile each
+constexpr int kMaxSplit = 8;
 
-// stage layout in shared memory (bytes); A and B tiles are 1024-byte aligned (swizzle atom)
-constexpr int kABytes = kTileN * kStageK;          // 16 KB
-constexpr int kBBytes = kTileM * kStageK;          // 16 KB
-constexpr int kWscBytes = 4 * kTileN * 8;          // [group in stage][n] {wd, wm} fp32
-constexpr int kXscBytes = 4 * kTileM * 8;          // [group in stage][row pair] {xs0, xs1, gsum0, gsum1} fp32
-constexpr int kStageBytes = kABytes + kBBytes + kWscBytes + kXscBytes;  // 40 KB
-constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
+enum Format { kQ4_0 = 0, kQ4_1 = 1, kQ4_0Signed = 2, kQ8C = 3 };
+
+template <int FMT, int G, int TM>
+struct PrefillShape {
+    static constexpr int kBlock = FMT == kQ8C ? 1024 : block_bytes(FMT == kQ4_1, G);
+    static constexpr int kGroups = kStageK / G;           // K groups per stage: 4 (group 32) or 1 (group 128)
+    static constexpr int kSums = FMT == kQ4_1 ? 2 : 1;    // per group and row: scale (and group sum)
+    static constexpr int kEpiWarps = TM / 8;              // 32 rows of the tile per warp and TMEM lane quarter
+    static constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
+    static constexpr int kLoadWidth = TM == 128 ? 16 : 8; // rows a thread takes from tensor memory at a time
+    static constexpr int kA = TM == 128 ? 3 : 2;          // stages of unpacked weights
+    static constexpr int kB = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;    // stages of activation codes
+    static constexpr int kRaw = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;  // stages of packed bytes
+    static constexpr int kScs = 4;                        // stages of scales
+    static constexpr int kRawStripe = kGroups * kBlock;   // packed bytes of one stripe in a stage
+    static constexpr int kABytes = kTileN * kStageK, kBBytes = TM * kStageK;
+    static constexpr int kXscBytes = kGroups * kSums * TM * 4;                // [group][scale | sum][row] fp32
+    static constexpr int kWscBytes = FMT == kQ8C ? 0 : kGroups * kTileN * 4;  // [group][n] {wd, wm} fp16
+    static constexpr int kScBytes = kXscBytes + kWscBytes;
+    static constexpr int kBOff = kA * kABytes;
+    static constexpr int kRawOff = kBOff + kB * kBBytes;
+    static constexpr int kScOff = kRawOff + kRaw * 4 * kRawStripe;
+    static constexpr int kBarOff = kScOff + kScs * kScBytes;
+    static constexpr int kSmem = kBarOff + 512 + 1024 /*alignment slack*/;
+    static_assert(TM == 128 || kSmem <= 113 * 1024, "two CTAs on an SM");
+    static_assert(TM * kTileN * 4 <= kRawOff, "the partial tile of a K split takes the operand stages' place");
+};
 
 struct PrefillParams {
     const uint8_t* wq;
-    const int8_t* codes;   // [rows][Kp]
-    const float* xs;       // [rows][Kg]
-    const float* gs;       // [rows][Kg]
+    const float* sc;       // [row tile][Kg][scale | sum][TM]
+    const float* wscales;  // Q8C
     float* y;
     int* status;
-    int64_t rows, N, ldy, Kp;
-    int Ng, Kg;
+    int64_t rows, N, ldy;
+    int Ng, Kg, split;
 };
 
 // ---- PTX helpers -------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(1000u) /* suspend-time hint, ns */
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
 // bounded wait: gives up after kWaitLimitNs, or as soon as another role has raised the abort flag
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t t0 = global_ns();
+    unsigned long long t0 = 0;
+#pragma unroll 1
     for (uint32_t i = 1;; i++) {
         if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 31) == 0) {
+        if ((i & 63) == 0) {
             if (*abort_flag) return false;
-            if (global_ns() - t0 > kWaitLimitNs) break;
+            const unsigned long long now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > kWaitLimitNs) break;
         }
     }
     *abort_flag = 1;
     return false;
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+// one lane of a converged warp.  (The compiler knows that exactly one lane runs the branch and keeps descriptors in
+// uniform registers; behind `lane == 0` it cannot, and issuing an MMA takes about a third longer.)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(p));
+    return p != 0;
 }
 // 2-D tiled TMA load (no multicast): box at (x, y) of the tensor map -> shared memory, completion on `bar`
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
@@ -123,14 +138,12 @@ __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
 __device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
     uint64_t r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
@@ -152,19 +165,35 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint6
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
         : "memory");
 }
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t addr) {
+    uint16_t v;
+    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 
 // K-major operand tile with 128-byte rows and 128-byte swizzle: rows 128 B apart, 8-row groups
 // 1024 B apart (stride byte offset), descriptor version 1, layout type 2 (SWIZZLE_128B)
@@ -172,47 +201,95 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
     return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
            (2ull << 61);
 }
-// byte address of (row, byte-in-row) inside a swizzled tile
-__device__ __forceinline__ uint32_t swz(uint32_t row, uint32_t byte) {
-    return (row >> 3) * 1024 + (row & 7) * 128 + ((((byte >> 4) ^ (row & 7)) & 7) << 4) + (byte & 15);
+// the eight nibbles of a word as bytes: k = 0..3 (low nibbles) and 4..7 (high nibbles)
+template <bool SIGNED>
+__device__ __forceinline__ void unpack_nibbles(uint32_t word, uint32_t& lo, uint32_t& hi) {
+    lo = word & 0x0F0F0F0Fu, hi = (word >> 4) & 0x0F0F0F0Fu;
+    if (SIGNED) {  // sign-extend each nibble into its byte
+        lo |= (lo & 0x08080808u) * 0x1Eu;
+        hi |= (hi & 0x08080808u) * 0x1Eu;
+    }
 }
 
-template <int G, int QTYPE, bool SIGNED>
-__global__ void __launch_bounds__(kThreads, 1) fc_prefill_kernel(const PrefillParams p,
-                                                                 const __grid_constant__ CUtensorMap codes_map) {
-    constexpr int BS = block_bytes(QTYPE, G);
-    constexpr int GPS = kStageK / G;  // K groups per stage: 4 (group 32) or 1 (group 128)
-    constexpr int MMAS = G / 32;      // K=32 instructions per group
+// acc[P .. P + W/2) += scaled integers of W rows (+ wm * their group sums); `xs`: the rows' scales, the group sums
+// follow at xs + TM
+template <int FMT, int TM, int P, int W>
+__device__ __forceinline__ void accumulate(uint64_t (&acc)[8], const uint32_t (&v)[W], const float* xs, uint64_t wd2,
+                                           uint64_t wm2) {
+#pragma unroll
+    for (int j = 0; j < W / 4; j++) {
+        const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(xs + 4 * j);
+        const uint64_t i01 = pack2(__int2float_rn((int)v[4 * j]), __int2float_rn((int)v[4 * j + 1]));
+        const uint64_t i23 = pack2(__int2float_rn((int)v[4 * j + 2]), __int2float_rn((int)v[4 * j + 3]));
+        uint64_t &a = acc[P + 2 * j], &b = acc[P + 2 * j + 1];
+        a = ffma2(FMT == kQ8C ? x4.x : fmul2(wd2, x4.x), i01, a);
+        b = ffma2(FMT == kQ8C ? x4.y : fmul2(wd2, x4.y), i23, b);
+        if (FMT == kQ4_1) {
+            const ulonglong2 g4 = *reinterpret_cast<const ulonglong2*>(xs + TM + 4 * j);
+            a = ffma2(wm2, g4.x, a);
+            b = ffma2(wm2, g4.y, b);
+        }
+    }
+}
+
+template <int FMT, int G, int TM>
+__global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 ? 1 : 2)
+    fc_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap codes_map) {
+    using S = PrefillShape<FMT, G, TM>;
+    constexpr int BS = S::kBlock;
+    constexpr int GPS = S::kGroups;
+    constexpr int MMAS = G / 32;  // K=32 instructions per group
+    constexpr int CGN = S::kEpiWarps / 4;
+    constexpr int kUnpackWarp = S::kEpiWarps, kMmaWarp = kUnpackWarp + kProdWarps;
 
     extern __shared__ uint8_t smem_raw[];
+    // (the same offset in every CTA of a cluster: the dynamic shared memory starts at the same address)
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t* bars = smem + kStages * kStageBytes;
-    const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * kStages;
-    const uint32_t bar_tfull = bar_empty + 8 * kStages, bar_tempty = bar_tfull + 8 * kTmemBufs;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8 * (2 * kStages + 2 * kTmemBufs));
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint8_t* bars = smem + S::kBarOff;
+    const uint32_t smem0 = smem_u32(smem);
+    const uint32_t bar_raw = smem0 + S::kBarOff;  // [raw stage][stripe]
+    const uint32_t bar_afull = bar_raw + 8 * 4 * S::kRaw, bar_aempty = bar_afull + 8 * S::kA;
+    const uint32_t bar_bfull = bar_aempty + 8 * S::kA, bar_bempty = bar_bfull + 8 * S::kB;
+    const uint32_t bar_sfull = bar_bempty + 8 * S::kB, bar_sempty = bar_sfull + 8 * S::kScs;
+    const uint32_t bar_tfull = bar_sempty + 8 * S::kScs, bar_tempty = bar_tfull + 8 * kTmemBufs;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 496);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 500);
+    static_assert(8 * (4 * S::kRaw + 2 * S::kA + 2 * S::kB + 2 * S::kScs + 2 * kTmemBufs) <= 496, "barriers");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tile = blockIdx.x, m_tile = blockIdx.y;
-    const int64_t n0 = (int64_t)n_tile * kTileN, m0 = (int64_t)m_tile * kTileM;
-    const int nb0 = n_tile * 4;
+    const int cs = p.split, rank = (int)(blockIdx.x % cs);
+    const int n_tile = (int)(blockIdx.x / cs), m_tile = blockIdx.y;
+    const int64_t n0 = (int64_t)n_tile * kTileN, m0 = (int64_t)m_tile * TM;
+    const int live = (int)min((int64_t)TM, p.rows - m0);  // rows of this tile that exist
     const int nstage = (p.Kg + GPS - 1) / GPS;
+    const int it0 = (int)((int64_t)nstage * rank / cs), it1 = (int)((int64_t)nstage * (rank + 1) / cs);
+    const int iters = it1 - it0;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStages; i++) {
-            mbar_init(bar_full + 8 * i, kProdThreads + 1);  // producer threads + the TMA issuer's expect_tx
-            mbar_init(bar_empty + 8 * i, 1 + kEpiWarps);
+        for (int i = 0; i < 4 * S::kRaw; i++) mbar_init(bar_raw + 8 * i, 1);
+        for (int i = 0; i < S::kA; i++) {
+            mbar_init(bar_afull + 8 * i, kProdWarps);
+            mbar_init(bar_aempty + 8 * i, 1);  // tcgen05.commit
+        }
+        for (int i = 0; i < S::kB; i++) {
+            mbar_init(bar_bfull + 8 * i, 1);
+            mbar_init(bar_bempty + 8 * i, 1);  // tcgen05.commit
+        }
+        for (int i = 0; i < S::kScs; i++) {
+            mbar_init(bar_sfull + 8 * i, kProdWarps + 1);  // unpacking warps + the loader's expect_tx
+            mbar_init(bar_sempty + 8 * i, S::kEpiWarps);
         }
         for (int i = 0; i < kTmemBufs; i++) {
             mbar_init(bar_tfull + 8 * i, 1);
-            mbar_init(bar_tempty + 8 * i, kEpiWarps);
+            mbar_init(bar_tempty + 8 * i, S::kEpiWarps);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_proxy_async();
     }
-    if (warp == kMmaWarp) {  // one warp allocates all 512 TMEM columns (this kernel runs one CTA per SM)
+    if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(512u)
+                     "r"((uint32_t)(kTmemBufs * TM))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -221,202 +298,282 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_kernel(const PrefillPa
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    // Register budget per role (whole warpgroups): the launch gives every thread 80; producers and the
-    // MMA warpgroup hand registers back, the epilogue warpgroups take 96 each (what is handed back,
-    // 4*32*16 + 4*32*56 = 9216, covers what is taken, 16*32*16 = 8192, so no request can block).
-    if (warp >= kEpiWarps && warp < kMmaWarp) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-        // =================== producers: one 128-k stage at a time ===================
-        const int pt = threadIdx.x - kEpiWarps * 32;  // 0..127
-        const int pw = pt >> 5;                       // stripe of the tile handled by this warp
-        const int c = lane & 7, rr = lane >> 3;       // 16-byte chunk (columns 4c..4c+3), row inside a 4-row set
-        const int nb = nb0 + pw;
-        const bool stripe_live = nb < p.Ng;
-        // columns are stored in a rotated order so that a half warp covers all 8 swizzle rows
-        // (conflict-free 8-byte stores); rows and the rotation do not change from stage to stage
-        uint32_t row_off[4];
-        int col_of[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            col_of[i] = (i + (c >> 1)) & 3;
-            const uint32_t row = pw * 32 + 4 * c + col_of[i];
-            row_off[i] = (row >> 3) * 1024 + (row & 7) * 128 + ((row & 7) << 16);  // low half: offset, high half: row&7
-        }
-        const uint8_t* stripe_base = p.wq + (int64_t)nb * p.Kg * BS;
-        const int64_t m_mine = m0 + pt;
-        for (int it = 0; it < nstage; it++) {
-            const int s = it % kStages;
-            if (!mbar_wait(bar_empty + 8 * s, ((it / kStages) & 1) ^ 1, abort_flag)) break;
-            uint8_t* st = smem + s * kStageBytes;
-            const uint32_t a_base = smem_u32(st), b_base = a_base + kABytes;
-            float2* wsc = reinterpret_cast<float2*>(st + kABytes + kBBytes);
-            float* xsc = reinterpret_cast<float*>(st + kABytes + kBBytes + kWscBytes);
-            const int kb0 = it * GPS;
-            if (pt == 0) {  // B: 128 rows x 128 bytes of codes, swizzled by the TMA unit; rows beyond the matrix read 0
-                mbar_arrive_expect_tx(bar_full + 8 * s, kBBytes);
-                tma_load_2d(b_base, &codes_map, bar_full + 8 * s, it * kStageK, (int)m0);
-            }
-            // ---- A: unpack nibbles of stripe nb: 16 word-rows (8 k each) x 32 columns
-            uint4 w[4];
-#pragma unroll
-            for (int i4 = 0; i4 < 4; i4++) {
-                const int r = 4 * i4 + rr;  // word-row inside the stage: k = 8r .. 8r+7
-                w[i4] = make_uint4(0u, 0u, 0u, 0u);
-                const int kb = (G == 128) ? kb0 : kb0 + i4;
-                if (stripe_live && kb < p.Kg) {
-                    const int row_in_block = (G == 128) ? r : rr;
-                    w[i4] = ldg_stream_v4(stripe_base + (int64_t)kb * BS + row_in_block * 128 + c * 16);
-                }
-            }
-            // ---- scales of the stage's groups (loads issued before the unpack stores)
-            float2 wv[GPS];
-            float xv[GPS], gv[GPS];
-#pragma unroll
-            for (int gi = 0; gi < GPS; gi++) {
-                const int kb = kb0 + gi;
-                wv[gi] = make_float2(0.f, 0.f);
-                xv[gi] = 0.f, gv[gi] = 0.f;
-                if (kb < p.Kg) {
-                    if (stripe_live) {
-                        const uint8_t* tail = stripe_base + (int64_t)kb * BS + 16 * G;
-                        wv[gi].x = h2f(*reinterpret_cast<const uint16_t*>(tail + 2 * lane));
-                        if (QTYPE == 1) wv[gi].y = h2f(*reinterpret_cast<const uint16_t*>(tail + 64 + 2 * lane));
-                    }
-                    if (m_mine < p.rows) {
-                        xv[gi] = __ldg(p.xs + m_mine * p.Kg + kb);
-                        if (QTYPE == 1) gv[gi] = __ldg(p.gs + m_mine * p.Kg + kb);
-                    }
-                }
-            }
-#pragma unroll
-            for (int i4 = 0; i4 < 4; i4++) {
-                const int r = 4 * i4 + rr;
-                const uint32_t chunk = (uint32_t)(r >> 1), sub = (uint32_t)(r & 1) * 8;
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const uint32_t word = col_of[i] == 0 ? w[i4].x : col_of[i] == 1 ? w[i4].y : col_of[i] == 2 ? w[i4].z : w[i4].w;
-                    uint32_t lo = word & 0x0F0F0F0Fu, hi = (word >> 4) & 0x0F0F0F0Fu;
-                    if (SIGNED) {  // sign-extend each nibble into its byte
-                        lo |= (lo & 0x08080808u) * 0x1Eu;
-                        hi |= (hi & 0x08080808u) * 0x1Eu;
-                    }
-                    const uint32_t addr = a_base + (row_off[i] & 0xFFFFu) + (((chunk ^ (row_off[i] >> 16)) & 7) << 4) + sub;
-                    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(lo), "r"(hi) : "memory");
-                }
-            }
-#pragma unroll
-            for (int gi = 0; gi < GPS; gi++) {
-                wsc[gi * kTileN + pt] = wv[gi];
-                // row pairs are kept as {xs0, xs1, gs0, gs1} for the packed epilogue arithmetic
-                float* q = xsc + (gi * (kTileM / 2) + (pt >> 1)) * 4 + (pt & 1);
-                q[0] = xv[gi];
-                q[2] = gv[gi];
-            }
-            fence_proxy_async();  // generic-proxy stores above -> visible to the tensor core's async proxy
-            mbar_arrive(bar_full + 8 * s);
-        }
-    } else if (warp >= kMmaWarp) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
-        // =================== MMA issue: one elected lane of one warp ===================
-        if (warp == kMmaWarp && lane == 0) {
-            // instruction descriptor: D = s32, A = u8 (s8 when sign-extended), B = s8, both K-major, N = 128, M = 128
-            const uint32_t idesc = (2u << 4) | ((SIGNED ? 1u : 0u) << 7) | (1u << 10) | ((uint32_t)(kTileM >> 3) << 17) |
-                                   ((uint32_t)(kTileN >> 4) << 24);
-            int gcount = 0;
-            bool ok = true;
-            for (int it = 0; it < nstage && ok; it++) {
-                const int s = it % kStages;
-                if (!mbar_wait(bar_full + 8 * s, (it / kStages) & 1, abort_flag)) break;
-                tc_fence_after();
-                const uint32_t a_base = smem_u32(smem + s * kStageBytes), b_base = a_base + kABytes;
-                const int ng = min(GPS, p.Kg - it * GPS);
-                for (int gi = 0; gi < ng; gi++, gcount++) {
-                    const int b = gcount % kTmemBufs;
-                    if (!mbar_wait(bar_tempty + 8 * b, ((gcount / kTmemBufs) & 1) ^ 1, abort_flag)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t d = tmem_base + b * kTileM;
-#pragma unroll
-                    for (int ks = 0; ks < MMAS; ks++) {
-                        const uint32_t koff = (uint32_t)(gi * G + ks * 32);  // bytes into the 128-byte row
-                        tc_mma_i8(d, make_desc(a_base + koff), make_desc(b_base + koff), idesc, ks > 0 ? 1u : 0u);
-                    }
-                    tc_commit(bar_tfull + 8 * b);  // the group's integers are complete in TMEM
-                }
-                tc_commit(bar_empty + 8 * s);  // the stage's operands have been consumed
-            }
-        }
-        __syncwarp();
-    } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 96;");
-        // =================== epilogue: 16 warps, 32 lanes x 32 columns each ===================
+    if (warp < kUnpackWarp) {
+        // =================== epilogue: 32 lanes x (16 + 16) rows per warp ===================
+        uint64_t acc[2][8];  // 2 x 16 rows as packed pairs
         const int quarter = warp & 3, cgrp = warp >> 2;
         const int nrow = quarter * 32 + lane;  // tile column n handled by this thread (= TMEM lane)
-        uint64_t acc[16];                      // 32 fp32 accumulators as 16 packed pairs (rows 2j, 2j+1)
+        if (iters == 0) pdl_wait_prior_grid();  // no K group: nothing else orders the stores behind earlier work
+        // chunks of 16 rows are dealt out to the warps of a quarter in turn, so that few rows still occupy all of them
+        const bool live0 = cgrp * 16 < live, live1 = (cgrp + CGN) * 16 < live;
 #pragma unroll
-        for (int i = 0; i < 16; i++) acc[i] = 0ull;
-        const uint64_t neg_magic = pack2(-12582912.0f, -12582912.0f);
-        int gcount = 0;
-        bool ok = true;
-        for (int it = 0; it < nstage && ok; it++) {
-            const int s = it % kStages;
-            const uint8_t* st = smem + s * kStageBytes;
-            const float2* wsc = reinterpret_cast<const float2*>(st + kABytes + kBBytes);
-            const ulonglong2* xsc2 = reinterpret_cast<const ulonglong2*>(st + kABytes + kBBytes + kWscBytes);
-            const int ng = min(GPS, p.Kg - it * GPS);
-            for (int gi = 0; gi < ng; gi++, gcount++) {
-                const int b = gcount % kTmemBufs;
-                if (!mbar_wait(bar_tfull + 8 * b, (gcount / kTmemBufs) & 1, abort_flag)) {
+        for (int i = 0; i < 8; i++) acc[0][i] = acc[1][i] = 0ull;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + cgrp * 16;
+        const int groups = min(p.Kg, it1 * GPS) - it0 * GPS;
+#pragma unroll 1
+        for (int g = 0; g < groups; g++) {
+            const int i = g / GPS, sl = i % S::kScs, gi = g % GPS, b = g % kTmemBufs;
+            if (gi == 0 && !wait_or_abort(bar_sfull + 8 * sl, (i / S::kScs) & 1, abort_flag)) break;
+            const uint8_t* sc = smem + S::kScOff + sl * S::kScBytes;
+            const float* xs = reinterpret_cast<const float*>(sc) + gi * (S::kSums * TM) + cgrp * 16;
+            uint64_t wd2 = 0, wm2 = 0;
+            if constexpr (FMT != kQ8C) {
+                const uint32_t w = reinterpret_cast<const uint32_t*>(sc + S::kXscBytes)[gi * kTileN + nrow];
+                const float wd = h2f((uint16_t)w), wm = h2f((uint16_t)(w >> 16));
+                wd2 = pack2(wd, wd), wm2 = pack2(wm, wm);
+            }
+            if (!wait_or_abort(bar_tfull + 8 * b, (g / kTmemBufs) & 1, abort_flag)) break;
+            tc_fence_after();
+            // W integers at a time: what the two chunks would take together is what the register file has left, and the
+            // compiler then serialises the arithmetic (37 rows, one CTA an SM: 84 us with W = 16 in 72 registers, 78 with 8)
+            auto release = [&] {  // the buffer can be overwritten
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_tempty + 8 * b);
+            };
+            constexpr int W = S::kLoadWidth;
+            uint32_t v[W];
+            if (live0) {
+                tc_ld(taddr + b * TM, v);
+                tc_wait_ld();
+                accumulate<FMT, TM, 0, W>(acc[0], v, xs, wd2, wm2);
+                if constexpr (W == 8) {
+                    tc_ld(taddr + b * TM + 8, v);
+                    tc_wait_ld();
+                    accumulate<FMT, TM, 4, W>(acc[0], v, xs + 8, wd2, wm2);
+                }
+            }
+            if (live1) {
+                tc_ld(taddr + b * TM + CGN * 16, v);
+                tc_wait_ld();
+                if constexpr (W == 8) {
+                    accumulate<FMT, TM, 0, W>(acc[1], v, xs + CGN * 16, wd2, wm2);
+                    tc_ld(taddr + b * TM + CGN * 16 + 8, v);
+                    tc_wait_ld();
+                }
+            }
+            release();
+            if (live1) accumulate<FMT, TM, W == 8 ? 4 : 0, W>(acc[1], v, xs + CGN * 16 + 16 - W, wd2, wm2);
+            if (gi == GPS - 1) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_sempty + 8 * sl);  // done with the stage's scales
+            }
+        }
+        if (cs == 1) {
+            const int64_t n = n0 + nrow;
+            if (n < p.N && !*abort_flag) {
+                const float ws = FMT == kQ8C ? __ldg(p.wscales + n) : 1.0f;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int mc = (cgrp + h * CGN) * 16;
+                    float* dst = p.y + (m0 + mc) * p.ldy + n;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        float lo, hi;
+                        unpack2(acc[h][j], lo, hi);
+                        if (FMT == kQ8C) lo = __fmul_rn(ws, lo), hi = __fmul_rn(ws, hi);
+                        if (mc + 2 * j < live) *dst = lo;
+                        dst += p.ldy;
+                        if (mc + 2 * j + 1 < live) *dst = hi;
+                        dst += p.ldy;
+                    }
+                }
+            }
+        } else if (!*abort_flag) {
+            // this CTA's partial tile; every operand of this CTA has been consumed (all groups' integers were seen)
+            float* red = reinterpret_cast<float*>(smem);
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int m = (cgrp + h * CGN) * 16 + 2 * j;
+                    float lo, hi;
+                    unpack2(acc[h][j], lo, hi);
+                    red[m * kTileN + nrow] = lo, red[(m + 1) * kTileN + nrow] = hi;
+                }
+        }
+    } else if (warp < kMmaWarp) {
+        // =================== unpacking: one stripe per warp, one column per lane ===================
+        const int pw = warp - kUnpackWarp;
+        const int nb = n_tile * 4 + pw;
+        const bool stripe_live = nb < p.Ng;  // (columns beyond the weights: nothing is read, nothing is stored)
+        const uint8_t* stripe = p.wq + (int64_t)nb * p.Kg * BS;
+        auto issue_raw = [&](int i) {
+            const int it = it0 + i, slot = (i % S::kRaw) * 4 + pw;
+            const uint32_t bytes = (uint32_t)(min(GPS, p.Kg - it * GPS) * BS);
+            mbar_expect_tx(bar_raw + 8 * slot, bytes);
+            bulk_g2s(smem0 + S::kRawOff + slot * S::kRawStripe, stripe + (int64_t)it * GPS * BS, bytes, bar_raw + 8 * slot);
+        };
+        if (stripe_live && lane == 0) {
+#pragma unroll 1
+            for (int i = 0; i < min(S::kRaw, iters); i++) issue_raw(i);
+        }
+        const uint32_t row = (uint32_t)(pw * 32 + lane);
+        const uint32_t row_off = (row >> 3) * 1024 + (row & 7) * 128, sw = (row & 7) << 4;
+#pragma unroll 1
+        for (int i = 0; i < iters; i++) {
+            const int s = i % S::kA, sl = i % S::kScs, rs = (i % S::kRaw) * 4 + pw;
+            const int ng = min(GPS, p.Kg - (it0 + i) * GPS);
+            if (stripe_live && !wait_or_abort(bar_raw + 8 * rs, (i / S::kRaw) & 1, abort_flag)) break;
+            if (!wait_or_abort(bar_aempty + 8 * s, ((i / S::kA) & 1) ^ 1, abort_flag)) break;
+            const uint32_t dst = smem0 + s * S::kABytes + row_off;
+            const uint32_t src = smem0 + S::kRawOff + rs * S::kRawStripe + lane * 4;
+            if (stripe_live) {
+                // 16 words at a time: the loads in one batch, then the stores
+                // (groups beyond Kg: stale bytes that no MMA reads)
+                if constexpr (FMT == kQ8C) {
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        uint32_t w[16];
+#pragma unroll
+                        for (int c = 0; c < 16; c++) w[c] = lds32(src + (h * 16 + c) * 128);
+#pragma unroll
+                        for (int c = 0; c < 4; c++)
+                            sts128(dst + ((uint32_t)((h * 4 + c) << 4) ^ sw), w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+                    }
+                } else {
+                    uint32_t w[16];
+#pragma unroll
+                    for (int c = 0; c < 16; c++) w[c] = lds32(src + (G == 128 ? c * 128 : (c / 4) * BS + (c % 4) * 128));
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        uint32_t lo0, hi0, lo1, hi1;
+                        unpack_nibbles<FMT == kQ4_0Signed>(w[2 * c], lo0, hi0);
+                        unpack_nibbles<FMT == kQ4_0Signed>(w[2 * c + 1], lo1, hi1);
+                        sts128(dst + ((uint32_t)(c << 4) ^ sw), lo0, hi0, lo1, hi1);
+                    }
+                }
+            }
+            if (!wait_or_abort(bar_sempty + 8 * sl, ((i / S::kScs) & 1) ^ 1, abort_flag)) break;
+            if constexpr (FMT != kQ8C) {
+                uint32_t* wsc = reinterpret_cast<uint32_t*>(smem + S::kScOff + sl * S::kScBytes + S::kXscBytes);
+                if (stripe_live) {
+#pragma unroll
+                    for (int gi = 0; gi < GPS; gi++)
+                        if (gi < ng) {
+                            const uint32_t tail = src - lane * 2 + gi * BS + 16 * G;
+                            uint32_t w = lds16(tail);
+                            if (FMT == kQ4_1) w |= lds16(tail + 64) << 16;
+                            wsc[gi * kTileN + row] = w;
+                        }
+                }
+            }
+            fence_proxy_async();  // generic-proxy stores above -> visible to the tensor core's async proxy
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(bar_afull + 8 * s);
+                mbar_arrive(bar_sfull + 8 * sl);
+                if (stripe_live && i + S::kRaw < iters) issue_raw(i + S::kRaw);  // this warp has read the slot
+            }
+        }
+    } else if (warp == kMmaWarp) {
+        // =================== MMA issue: one lane ===================
+        if (elect_one()) {
+            // instruction descriptor: D = s32, A = u8 (s8 where codes are signed), B = s8, both K-major, M = 128,
+            // N = the tile's existing rows rounded up to 16
+            const uint32_t ncols = (uint32_t)((live + 15) & ~15);
+            const uint32_t idesc = (2u << 4) | ((FMT == kQ4_0Signed || FMT == kQ8C ? 1u : 0u) << 7) | (1u << 10) |
+                                   ((ncols >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
+            const uint64_t desc0 = make_desc(smem0);  // (the start address counts 16-byte units from bit 0)
+            int gcount = 0;
+            bool ok = true;
+#pragma unroll 1
+            for (int i = 0; i < iters && ok; i++) {
+                const int sa = i % S::kA, sb = i % S::kB;
+                if (!wait_or_abort(bar_afull + 8 * sa, (i / S::kA) & 1, abort_flag) ||
+                    !wait_or_abort(bar_bfull + 8 * sb, (i / S::kB) & 1, abort_flag)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                uint32_t v[32];
-                tc_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + b * kTileM + cgrp * 32, v);
-                tc_wait_ld();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_tempty + 8 * b);  // the buffer can be overwritten
-                const float2 w = wsc[gi * kTileN + nrow];          // wd, wm of this thread's column
-                const uint64_t wd2 = pack2(w.x, w.x), wm2 = pack2(w.y, w.y);
+                const uint64_t a_desc = desc0 + (uint64_t)(sa * (S::kABytes / 16));
+                const uint64_t b_desc = desc0 + (uint64_t)((S::kBOff + sb * S::kBBytes) / 16);
+                const int ng = min(GPS, p.Kg - (it0 + i) * GPS);
+#pragma unroll 1
+                for (int gi = 0; gi < ng; gi++, gcount++) {
+                    const int b = gcount % kTmemBufs;
+                    const uint64_t ad = a_desc + (uint64_t)(gi * (G / 16)), bd = b_desc + (uint64_t)(gi * (G / 16));
+                    if (!wait_or_abort(bar_tempty + 8 * b, ((gcount / kTmemBufs) & 1) ^ 1, abort_flag)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const ulonglong2 xg = xsc2[gi * (kTileM / 2) + cgrp * 16 + j];  // {xs0, xs1}, {gs0, gs1}
-                    // exact int -> float: |I| < 2^22, so (I + 0x4B400000) reinterpreted is 12582912 + I
-                    const uint64_t i2 = fadd2(pack2(__int_as_float((int)v[2 * j] + 0x4B400000),
-                                                    __int_as_float((int)v[2 * j + 1] + 0x4B400000)),
-                                              neg_magic);
-                    acc[j] = ffma2(fmul2(wd2, xg.x), i2, acc[j]);
-                    if (QTYPE == 1) acc[j] = ffma2(wm2, xg.y, acc[j]);
+                    for (int ks = 0; ks < MMAS; ks++)
+                        tc_mma_i8(tmem_base + b * TM, ad + ks * 2, bd + ks * 2, idesc, ks > 0 ? 1u : 0u);
+                    tc_commit(bar_tfull + 8 * b);  // the group's integers are complete in TMEM
                 }
+                tc_commit(bar_aempty + 8 * sa);  // the stage's operands have been consumed
+                tc_commit(bar_bempty + 8 * sb);
             }
-            __syncwarp();
-            if (ok && lane == 0) mbar_arrive(bar_empty + 8 * s);  // done with the stage's scales
-        }
-        if (ok) {
-            const int64_t n = n0 + nrow;
-            if (n < p.N) {
-#pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int64_t m = m0 + cgrp * 32 + 2 * j;
-                    float lo, hi;
-                    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[j]));
-                    if (m < p.rows) p.y[m * p.ldy + n] = lo;
-                    if (m + 1 < p.rows) p.y[(m + 1) * p.ldy + n] = hi;
-                }
+            // the last commits' arrivals land before this CTA's shared memory can be handed on
+            if (ok && iters > 0) {
+                wait_or_abort(bar_aempty + 8 * ((iters - 1) % S::kA), ((iters - 1) / S::kA) & 1, abort_flag);
+                wait_or_abort(bar_bempty + 8 * ((iters - 1) % S::kB), ((iters - 1) / S::kB) & 1, abort_flag);
             }
         }
+    } else {
+        // =================== loader: codes and scales of the rows ===================
+        if (elect_one()) {
+            pdl_wait_prior_grid();  // the quantizer's results are complete
+#pragma unroll 1
+            for (int i = 0; i < iters; i++) {
+                const int s = i % S::kB, sl = i % S::kScs, it = it0 + i;
+                if (!wait_or_abort(bar_bempty + 8 * s, ((i / S::kB) & 1) ^ 1, abort_flag)) break;
+                mbar_expect_tx(bar_bfull + 8 * s, S::kBBytes);
+                // rows and k beyond the matrix read 0
+                tma_load_2d(smem0 + S::kBOff + s * S::kBBytes, &codes_map, bar_bfull + 8 * s, it * kStageK, (int)m0);
+                if (!wait_or_abort(bar_sempty + 8 * sl, ((i / S::kScs) & 1) ^ 1, abort_flag)) break;
+                const uint32_t bytes = (uint32_t)(min(GPS, p.Kg - it * GPS) * S::kSums * TM * 4);
+                mbar_expect_tx(bar_sfull + 8 * sl, bytes);
+                bulk_g2s(smem0 + S::kScOff + sl * S::kScBytes,
+                         p.sc + ((int64_t)m_tile * p.Kg + (int64_t)it * GPS) * (S::kSums * TM), bytes, bar_sfull + 8 * sl);
+            }
+        }
+    }
+    __syncwarp();
+    if (cs > 1) {
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        if (warp < kUnpackWarp && !*abort_flag) {
+            // rows rank, rank + cs, ... of the tile: the partial sums of all ranks in rank order
+            const float* red = reinterpret_cast<const float*>(smem);
+#pragma unroll 1
+            for (int m = rank + cs * warp; m < live; m += cs * S::kEpiWarps) {
+                float sum[4] = {};
+#pragma unroll 1
+                for (int q = 0; q < cs; q++) {
+                    const float* src = cluster.map_shared_rank(red, q) + m * kTileN + lane;
+#pragma unroll
+                    for (int c = 0; c < 4; c++) sum[c] = q ? __fadd_rn(sum[c], src[32 * c]) : src[32 * c];
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int64_t n = n0 + lane + 32 * c;
+                    if (n < p.N)
+                        p.y[(m0 + m) * p.ldy + n] = FMT == kQ8C ? __fmul_rn(__ldg(p.wscales + n), sum[c]) : sum[c];
+                }
+            }
+        }
+        __syncwarp();
+        cluster.sync();  // nobody leaves while its partial tile is being read
     }
 
     // ---- teardown: everyone meets, then the allocating warp frees TMEM
     tc_fence_before();
     __syncthreads();
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(p.status, 0x50524546);  // 'PREF': a bounded wait ran out
+    if (*abort_flag) {
+        if (threadIdx.x == 0) atomicExch(p.status, 0x50524546);  // 'PREF': a bounded wait ran out
+        // copies that may still be in flight land before the shared memory is handed to another CTA
+#pragma unroll 1
+        for (int i = 0; i < 64; i++) __nanosleep(32000);
+    }
     if (warp == kMmaWarp) {
+        __syncwarp();
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
+                     "r"((uint32_t)(kTmemBufs * TM))
+                     : "memory");
     }
 }
 
@@ -438,9 +595,9 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// the code matrix [rows][Kp] int8 as a 2-D tensor; boxes of 128 bytes x 128 rows land in the
+// the code matrix [rows][Kp] int8 as a 2-D tensor; boxes of 128 bytes x `tile` rows land in the
 // 128-byte-swizzle layout that the MMA descriptors describe; out-of-range rows and k read as 0
-int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t Kp) {
+int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t Kp, int tile) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) {
         set_error("fc_prefill: cuTensorMapEncodeTiled is not available from this driver");
@@ -448,7 +605,7 @@ int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t 
     }
     const cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)Kp};
-    const cuuint32_t box[2] = {(cuuint32_t)kStageK, (cuuint32_t)kTileM};
+    const cuuint32_t box[2] = {(cuuint32_t)kStageK, (cuuint32_t)tile};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(codes), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -461,41 +618,105 @@ int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t 
     return Q4FC_OK;
 }
 
-template <int G, int QTYPE, bool SIGNED>
-int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, cudaStream_t s) {
+template <int FMT, int G, int TM>
+int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, int64_t n_tiles, int64_t m_tiles, cudaStream_t s) {
+    using S = PrefillShape<FMT, G, TM>;
     static std::atomic<bool> attr_done[64] = {};  // set once per device; a second setter repeats the same call
     int dev = 0;
     Q4FC_CUDA_OK(cudaGetDevice(&dev));
-    auto* fn = fc_prefill_kernel<G, QTYPE, SIGNED>;
-    if (dev < 64 && !attr_done[dev]) {
-        Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        attr_done[dev] = true;
+    auto* fn = fc_prefill_kernel<FMT, G, TM>;
+    if (dev >= 64 || !attr_done[dev]) {
+        Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem));
+        Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        if (dev < 64) attr_done[dev] = true;
     }
-    const int64_t n_tiles = ((int64_t)p.Ng * 32 + kTileN - 1) / kTileN;
-    const int64_t m_tiles = (p.rows + kTileM - 1) / kTileM;
-    if (n_tiles > 0x7fffffffLL || m_tiles > 65535) {
-        set_error("fc_prefill: %lld x %lld tiles exceed the grid limit", (long long)n_tiles, (long long)m_tiles);
-        return Q4FC_ELIMIT;
-    }
-    fn<<<dim3((unsigned)n_tiles, (unsigned)m_tiles), kThreads, kSmemBytes, s>>>(p, map);
-    Q4FC_CUDA_OK(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_tiles * p.split), (unsigned)m_tiles);
+    cfg.blockDim = dim3(S::kThreads);
+    cfg.dynamicSmemBytes = S::kSmem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    // starts beside the quantizer in front of it and waits for that one's results where it needs them
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.split;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, fn, p, map));
     return Q4FC_OK;
 }
 
+template <int FMT, int G>
+int launch_prefill_tile(int tile, const PrefillParams& p, const CUtensorMap& map, int64_t n_tiles, int64_t m_tiles,
+                        cudaStream_t s) {
+    return tile == 128 ? launch_prefill_variant<FMT, G, 128>(p, map, n_tiles, m_tiles, s)
+                       : launch_prefill_variant<FMT, G, 64>(p, map, n_tiles, m_tiles, s);
+}
+
+// scales and group sums of a format, padded to whole row tiles of either size
+size_t scale_bytes(int64_t rows, int64_t Kg, int sums) { return (size_t)((rows + 127) / 128 * 128) * Kg * sums * 4; }
+
+// Quantizer and GEMM; `codes` and `sc` are scratch for [rows][Kg * G] bytes and scale_bytes().
+int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t ldx, int8_t* codes, float* sc,
+                PrefillParams p, cudaStream_t s) {
+    const DeviceInfo* di = device_info();
+    if (!di) return Q4FC_ECUDA;
+    p.rows = rows, p.sc = sc;
+    const int64_t Kp = (int64_t)p.Kg * G;
+    if (rows > 0x7fffffffLL || Kp > 0x7fffffffLL) {
+        set_error("fc_prefill: rows=%lld or K=%lld beyond the 2^31 coordinate range", (long long)rows, (long long)K);
+        return Q4FC_ELIMIT;
+    }
+    const int64_t n_tiles = (p.N + kTileN - 1) / kTileN;
+    const int64_t nstage = (Kp + kStageK - 1) / kStageK;
+    // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM and can share K out: the large tile as
+    // soon as such tiles occupy every SM (512 rows x 11008 columns, group 32: 223 us, with 64 rows 234; 256 rows, Q8C:
+    // equal; 200 x 4096, group 128: 37 us on 64 CTAs, 64-row tiles with K halved 29).  K is divided while that fills the
+    // two places on every SM and leaves a CTA four stages (37 rows x 11008: 78 us undivided, 62 by two, 41 by three, 55 by
+    // four, which needs a second wave).
+    const int tile = (rows > 64 && n_tiles * ((rows + 127) / 128) >= di->sm_count) ? 128 : 64;
+    const int64_t m_tiles = (rows + tile - 1) / tile;
+    int64_t split = 1;
+    if (tile == 64) {
+        split = 2 * (int64_t)di->sm_count / (n_tiles * m_tiles);
+        if (split > nstage / 4) split = nstage / 4;
+        if (split > kMaxSplit) split = kMaxSplit;
+        if (split < 1) split = 1;
+    }
+    if (n_tiles * split > 0x7fffffffLL || m_tiles > 65535) {
+        set_error("fc_prefill: %lld x %lld tiles exceed the grid limit", (long long)n_tiles, (long long)m_tiles);
+        return Q4FC_ELIMIT;
+    }
+    p.split = (int)split;
+    if (int rc = launch_quant_x_tile(x, rows, K, ldx, G, fmt == kQ4_1, tile, codes, sc, s)) return rc;
+    CUtensorMap map = {};
+    if (Kp > 0)  // (no K group: no stage reads the map)
+        if (int rc = make_codes_map(&map, codes, rows, Kp, tile)) return rc;
+    if (fmt == kQ8C) return launch_prefill_tile<kQ8C, 32>(tile, p, map, n_tiles, m_tiles, s);
+    if (fmt == kQ4_1 && G == 32) return launch_prefill_tile<kQ4_1, 32>(tile, p, map, n_tiles, m_tiles, s);
+    if (fmt == kQ4_1) return launch_prefill_tile<kQ4_1, 128>(tile, p, map, n_tiles, m_tiles, s);
+    if (fmt == kQ4_0 && G == 32) return launch_prefill_tile<kQ4_0, 32>(tile, p, map, n_tiles, m_tiles, s);
+    if (fmt == kQ4_0) return launch_prefill_tile<kQ4_0, 128>(tile, p, map, n_tiles, m_tiles, s);
+    if (G == 32) return launch_prefill_tile<kQ4_0Signed, 32>(tile, p, map, n_tiles, m_tiles, s);
+    return launch_prefill_tile<kQ4_0Signed, 128>(tile, p, map, n_tiles, m_tiles, s);
+}
+
 // workspace: [status 256][what the decode kernels keep between calls: decode_prequant_offset() bytes]
-//            [codes rows x Kp, 256-aligned][xs rows x Kg f32][gs rows x Kg f32]
+//            [codes rows x Kp, 256-aligned][scales and group sums]
 // The quantized activations start where the decode path's own quantizer scratch starts: calls on one
 // workspace are ordered, so the two can share that space, and neither lands on the stream-K stripe
 // counters, which must stay zero between calls.
 struct WsLayout {
-    size_t codes, xs, gs, total;
+    size_t codes, sc, total;
 };
 WsLayout ws_layout(int64_t rows, int64_t Kg, int G) {
     WsLayout l;
     l.codes = decode_prequant_offset();
-    l.xs = align_up(l.codes + (size_t)rows * Kg * G, 256);
-    l.gs = align_up(l.xs + (size_t)rows * Kg * 4, 256);
-    l.total = align_up(l.gs + (size_t)rows * Kg * 4, 256);
+    l.sc = align_up(l.codes + (size_t)rows * Kg * G, 256);
+    l.total = align_up(l.sc + scale_bytes(rows, Kg, 2), 256);
     return l;
 }
 
@@ -516,33 +737,25 @@ int launch_fc_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, cons
         return Q4FC_EWORKSPACE;
     }
     uint8_t* base = static_cast<uint8_t*>(ws);
-    PrefillParams p;
-    p.wq = wq;
-    p.codes = reinterpret_cast<const int8_t*>(base + l.codes);
-    p.xs = reinterpret_cast<const float*>(base + l.xs);
-    p.gs = reinterpret_cast<const float*>(base + l.gs);
-    p.y = y;
-    p.status = reinterpret_cast<int*>(base);
-    p.rows = rows, p.N = N, p.ldy = ldy, p.Kp = Kg * G;
-    p.Ng = (int)Ng, p.Kg = (int)Kg;
-    // the reference's 1/16 activation scale of Q4_0 pairs with its x16 nibble shift; neither is materialised
-    int rc = launch_quant_x(x, rows, K, ldx, G, 1.0f, reinterpret_cast<int8_t*>(base + l.codes),
-                            reinterpret_cast<float*>(base + l.xs), reinterpret_cast<float*>(base + l.gs), s);
-    if (rc) return rc;
-    if (rows > 0x7fffffffLL || p.Kp > 0x7fffffffLL) {
-        set_error("fc_prefill: rows=%lld or K=%lld beyond the 2^31 coordinate range", (long long)rows, (long long)K);
-        return Q4FC_ELIMIT;
-    }
-    CUtensorMap map;
-    rc = make_codes_map(&map, p.codes, rows, p.Kp);
-    if (rc) return rc;
+    PrefillParams p = {};
+    p.wq = wq, p.y = y, p.status = reinterpret_cast<int*>(base);
+    p.N = N, p.ldy = ldy, p.Ng = (int)Ng, p.Kg = (int)Kg;
     const bool sgn = (flags & Q4FC_FLAG_NIBBLE_SIGNED) && qtype == 0;
-    if (qtype == 1 && G == 32) return launch_prefill_variant<32, 1, false>(p, map, s);
-    if (qtype == 1 && G == 128) return launch_prefill_variant<128, 1, false>(p, map, s);
-    if (qtype == 0 && G == 32 && !sgn) return launch_prefill_variant<32, 0, false>(p, map, s);
-    if (qtype == 0 && G == 128 && !sgn) return launch_prefill_variant<128, 0, false>(p, map, s);
-    if (qtype == 0 && G == 32) return launch_prefill_variant<32, 0, true>(p, map, s);
-    return launch_prefill_variant<128, 0, true>(p, map, s);
+    // the reference's 1/16 activation scale of Q4_0 pairs with its x16 nibble shift; neither is materialised
+    return launch_gemm(qtype == 1 ? kQ4_1 : sgn ? kQ4_0Signed : kQ4_0, G, x, rows, K, ldx,
+                       reinterpret_cast<int8_t*>(base + l.codes), reinterpret_cast<float*>(base + l.sc), p, s);
+}
+
+size_t q8c_prefill_scale_bytes(int64_t rows, int64_t Kg) { return scale_bytes(rows, Kg, 1); }
+
+int launch_q8c_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, const int8_t* wq, const float* wscales,
+                       int64_t Ng, int64_t Kg, int64_t N, float* y, int64_t ldy, int8_t* codes, float* sc, cudaStream_t s) {
+    PrefillParams p = {};
+    p.status = ring_status_word();
+    if (!p.status) return Q4FC_ECUDA;
+    p.wq = reinterpret_cast<const uint8_t*>(wq), p.wscales = wscales, p.y = y;
+    p.N = N, p.ldy = ldy, p.Ng = (int)Ng, p.Kg = (int)Kg;
+    return launch_gemm(kQ8C, 32, x, rows, K, ldx, codes, sc, p, s);
 }
 
 }  // namespace q4fc

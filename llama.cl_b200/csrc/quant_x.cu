@@ -15,8 +15,9 @@
 // G/4 lanes of a group.  The raw values are parked in shared memory so that
 // one lane per group can walk them in order for the sequential sum; many
 // resident warps hide that serial chain.  The decode FC kernel has its own
-// fused copy of this arithmetic (tree-ordered sums); this kernel serves the
-// prefill path and callers that want the quantized activations themselves.
+// fused copy of this arithmetic (tree-ordered sums), the prefill path its own
+// kernel below; this one serves callers that want the quantized activations
+// themselves and the per-channel int8 FC.
 #include "common.cuh"
 
 namespace q4fc {
@@ -104,6 +105,70 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_kernel(const float* __r
                 for (int i = 0; i < len2; i++) s = __fadd_rn(s, mine[lane * PADG + i]);
                 gsums[row * Kg + kb2] = s;
             }
+        }
+    }
+}
+
+// The prefill GEMM's quantizer: the codes and scales of quant_x_kernel, scales (and, `sums`, group sums, tree-ordered)
+// in the layout in which the GEMM's tiles of 2^log2tile rows read them: [row tile][Kg][scale | sum][row in tile].
+// The eight warps of a CTA take the same 128 k of eight neighbouring rows, whose scales share a 32-byte sector.
+template <int G>
+__global__ void __launch_bounds__(kQxWarps * 32) quant_x_tile_kernel(const float* __restrict__ x, int64_t rows, int64_t K,
+                                                                     int64_t ldx, int64_t Kg, int vec_ok, int sums,
+                                                                     int log2tile, int8_t* __restrict__ codes,
+                                                                     float* __restrict__ sc) {
+    constexpr int SEG = G / 4;    // lanes per group
+    constexpr int GPC = 128 / G;  // groups per 128-k chunk
+    pdl_launch_dependents();      // the GEMM's weight copies run beside this launch
+    const int lane = threadIdx.x & 31;
+    const int64_t row_sets = (rows + kQxWarps - 1) / kQxWarps;
+    const int64_t c = blockIdx.x / row_sets;
+    const int64_t row = (blockIdx.x - c * row_sets) * kQxWarps + (threadIdx.x >> 5);
+    if (row >= rows) return;
+    const int64_t k = c * 128 + lane * 4;
+    const float* src = x + row * ldx + k;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (vec_ok && k + 4 <= K) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(src));
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (k + j < K) v[j] = __ldg(src + j);
+    }
+    const int64_t kb = c * GPC + lane / SEG;
+    const bool exists = kb < Kg;
+    const int len = exists ? (int)min((int64_t)G, K - kb * G) : 0;
+    const int body = len & ~7;
+    const int e0 = (lane % SEG) * 4;
+    float amax = 0.0f, sum = (v[0] + v[1]) + (v[2] + v[3]);  // (0 beyond K)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (e0 + j < len) amax = fmaxf(amax, fabsf(v[j]));
+#pragma unroll
+    for (int off = SEG / 2; off > 0; off >>= 1) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+        sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    }
+    const float d = div_const_rn(amax, 127.0f, 1.0f / 127.0f);
+    const float id = inv_or_zero(d);
+    uint32_t packed = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        int q = 0;
+        if (e0 + j < len) {
+            const float t = __fmul_rn(v[j], id);
+            q = sat8(e0 + j < body ? __float2int_rn(t) : round_half_away(t));
+        }
+        packed |= (uint32_t)(q & 0xFF) << (8 * j);
+    }
+    if (exists) {
+        *reinterpret_cast<uint32_t*>(codes + row * (Kg * G) + k) = packed;
+        if (e0 == 0) {
+            const int64_t tile = (int64_t)1 << log2tile, per = tile << sums;
+            float* dst = sc + ((row >> log2tile) * Kg + kb) * per + (row & (tile - 1));
+            dst[0] = d;
+            if (sums) dst[tile] = sum;
         }
     }
 }
@@ -332,6 +397,25 @@ int launch_quant_x_pre(const float* x, int rows, int64_t K, int64_t ldx, int G, 
     else
         Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_x_pre_kernel<128>, x, rows, K, ldx, Kg, vec_ok, (int)want_isum,
                                         (int)pdl, codes, sc, up, prod, ldp));
+    return Q4FC_OK;
+}
+
+int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, bool sums, int tile, int8_t* codes,
+                        float* sc, cudaStream_t s) {
+    const int64_t Kg = (K + G - 1) / G;
+    if (rows == 0 || Kg == 0) return Q4FC_OK;
+    const int64_t grid = (rows + kQxWarps - 1) / kQxWarps * ((Kg * G + 127) / 128);
+    if (grid > 0x7fffffffLL) {
+        set_error("quant_x: %lld x %lld exceeds the grid limit", (long long)rows, (long long)K);
+        return Q4FC_ELIMIT;
+    }
+    const int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
+    const int l2 = tile == 128 ? 7 : 6;
+    if (G == 32)
+        quant_x_tile_kernel<32><<<(unsigned)grid, kQxWarps * 32, 0, s>>>(x, rows, K, ldx, Kg, vec_ok, sums, l2, codes, sc);
+    else
+        quant_x_tile_kernel<128><<<(unsigned)grid, kQxWarps * 32, 0, s>>>(x, rows, K, ldx, Kg, vec_ok, sums, l2, codes, sc);
+    Q4FC_CUDA_OK(cudaGetLastError());
     return Q4FC_OK;
 }
 

@@ -26,3 +26,32 @@ def test_host_fc_in_place_and_copied(pkg, rows):
         x = torch.randn(1, rows, 640, generator=g)
         want = pkg.llmops.fc_Q4A(x.cuda(), wq, 1003).cpu()
         assert torch.equal(fc(x), want)
+
+
+@pytest.mark.parametrize("rows,N,K", [
+    (9, 4096, 512),     # one 16-row chunk
+    (16, 130, 4128),    # a last stage with one K group; K divided unevenly; stripes that fill no tile of four
+    (17, 97, 2080),     # two chunks, the second one row
+    (64, 1000, 1056), (65, 1000, 1056),       # one 64-row tile, one row more
+    (128, 20000, 160), (129, 10000, 160),     # 128-row tiles on every SM, one row more
+    (33, 40, 33),       # less than a stage
+])
+@pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "q8c"])
+def test_many_rows_on_tile_edges(pkg, oracle, fmt, rows, N, K):
+    """Both tile sizes and every K split of the tensor-core FC, against the oracle.  At most 2 Kg <= 264 fp32 roundings
+    of 2^-24 on either side of a sum: 2e-5 of its largest value."""
+    g = torch.Generator().manual_seed(rows + N + K)
+    W = torch.randn(N, K, generator=g) * 0.02
+    x = torch.randn(1, rows, K, generator=g)
+    if fmt == "q8c":
+        wq, ws = oracle.restated.q8c_pack(W.numpy())
+        want = oracle.restated.q8c_fc(x.numpy(), wq, ws, N)
+        run = lambda: pkg.c_ext.FC_evaluate_Q8C(x.cuda(), torch.from_numpy(wq).cuda(), torch.from_numpy(ws).cuda(), N)
+    else:
+        wq = oracle.restated.pack(W.numpy(), *fmt)
+        want = oracle.restated.fc(x.numpy(), wq, N)
+        run = lambda: pkg.llmops.fc_Q4A(x.cuda(), torch.from_numpy(wq).cuda(), N)
+    got = run()
+    assert torch.equal(got, run())  # fixed summation order
+    assert np.abs(got.cpu().numpy() - want).max() <= 2e-5 * np.abs(want).max()
+    pkg.llmops.check_device_status()
