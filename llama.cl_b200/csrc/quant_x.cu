@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_kernel(const float* __r
     constexpr int PADG = G + 1;    // padded group pitch in shared memory
     __shared__ float raw[kQxWarps][GPC * PADG + 3];
 
+    pdl_launch_dependents();  // (an FC launched for it starts beside this kernel and waits for its results)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t chunks = (Kg * G + 127) / 128;
     const int64_t unit = (int64_t)blockIdx.x * kQxWarps + warp;
