@@ -36,6 +36,14 @@ __device__ __forceinline__ void mm_take(MinMax& a, float v) {  // sequential ste
     if (a.vmin > v) a.vmin = v;
 }
 
+// 256-bit load (sm_100): a lane's eight weights in one request, 32-byte aligned (as two 128-bit loads each request
+// uses half of the sectors that it touches: 11008 x 4096, Q4_1 group 128, 46.7 us, now 45.2)
+__device__ __forceinline__ void ldg_v8(const float* p, float (&v)[8]) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+
 template <int G, int QTYPE>
 __global__ void __launch_bounds__(kPackThreads) pack_kernel(const float* __restrict__ w, int64_t N, int64_t K,
                                                             int64_t Kg, int tiles_k, int vec_ok,
@@ -70,7 +78,9 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(const float* __restr
         if (n < N && kb0 + kb_l < Kg) {
             cnt = (int)min((int64_t)8, max((int64_t)0, K - k));
             const float* src = w + n * K + k;
-            if (cnt == 8 && vec_ok) {
+            if (cnt == 8 && vec_ok == 2) {
+                ldg_v8(src, v[it]);
+            } else if (cnt == 8 && vec_ok) {
                 float4 a = __ldg(reinterpret_cast<const float4*>(src));
                 float4 b = __ldg(reinterpret_cast<const float4*>(src) + 1);
                 v[it][0] = a.x, v[it][1] = a.y, v[it][2] = a.z, v[it][3] = a.w;
@@ -213,7 +223,9 @@ int launch_pack(const float* w, int64_t N, int64_t K, int qtype, int G, uint8_t*
         set_error("pack: %lld x %lld tiles exceed the grid limit", (long long)Ng, (long long)tiles_k);
         return Q4FC_ELIMIT;
     }
-    const int vec_ok = (K % 4 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
+    // widest load that every row's start allows: 2 = 32 bytes, 1 = 16, 0 = 4
+    const uintptr_t wa = reinterpret_cast<uintptr_t>(w);
+    const int vec_ok = (K % 8 == 0 && (wa & 31) == 0) ? 2 : (K % 4 == 0 && (wa & 15) == 0) ? 1 : 0;
     dim3 grid((unsigned)(Ng * tiles_k));
 #define Q4FC_PACK(GG, QQ) \
     pack_kernel<GG, QQ><<<grid, kPackThreads, 0, s>>>(w, N, K, Kg, (int)tiles_k, vec_ok, wq)

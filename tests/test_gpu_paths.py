@@ -55,3 +55,17 @@ def test_many_rows_on_tile_edges(pkg, oracle, fmt, rows, N, K):
     assert torch.equal(got, run())  # fixed summation order
     assert np.abs(got.cpu().numpy() - want).max() <= 2e-5 * np.abs(want).max()
     pkg.llmops.check_device_status()
+
+
+@pytest.mark.parametrize("qtype,G", [(0, 32), (1, 128)])
+@pytest.mark.parametrize("K", [264, 260, 259])
+@pytest.mark.parametrize("offset", [0, 4, 1])
+def test_pack_load_widths(pkg, oracle, qtype, G, K, offset):
+    """Rows that start on 32, 16 and 4 bytes take three widths of load: the same bytes."""
+    g = torch.Generator().manual_seed(K + offset)
+    W = torch.randn(33, K, generator=g) * 0.02
+    store = torch.empty(33 * K + offset, device="cuda")
+    w = store[offset:].view(33, K)
+    w.copy_(W)
+    got = pkg.llmops.offline_FC_quant_Q4A(w, qtype="q4_1" if qtype else "q4_0", group_k=G)
+    assert np.array_equal(got.cpu().numpy(), oracle.restated.pack(W.numpy(), qtype, G))
