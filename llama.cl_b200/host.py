@@ -63,6 +63,7 @@ class HostFC:
 
     def _enqueue(self, M: int) -> None:
         if self._reads_host(M):
+            llmops._require_cuda(self.wq, "wei_quantized", torch.int8, 3)
             kw, ws = self.fc_kwargs, self.fc_kwargs["workspace"]
             flags = _cabi.FLAG_PREQUANT | (_cabi.FLAG_NIBBLE_SIGNED if kw.get("nibble_signed") else 0) | \
                 (_cabi.FLAG_PDL if kw.get("pdl") else 0)

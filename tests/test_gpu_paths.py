@@ -28,6 +28,17 @@ def test_host_fc_in_place_and_copied(pkg, rows):
         assert torch.equal(fc(x), want)
 
 
+@pytest.mark.parametrize("rows", [1, 9])
+def test_host_fc_refuses_unfit_weights(pkg, rows):
+    """A slice of a packed tensor has the pitch of the whole; unsigned bytes are no packed tensor: both are refused."""
+    full = torch.zeros(8, 16, 640, dtype=torch.int8, device="cuda")
+    for wq, text in ((full[:, 4:12], "dense row-major"), (full.view(torch.uint8), r"is<int8>\(3\)")):
+        for graph in (True, False):
+            with pytest.raises(RuntimeError, match=text):
+                fc = pkg.host.HostFC(wq, 256, max_rows=16, graph=graph)
+                fc(torch.zeros(1, rows, fc.K))
+
+
 @pytest.mark.parametrize("rows,N,K", [
     (9, 4096, 512),     # one 16-row chunk
     (16, 130, 4128),    # a last stage with one K group; K divided unevenly; stripes that fill no tile of four
