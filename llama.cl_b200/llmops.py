@@ -82,7 +82,16 @@ class Workspace:
 
 
 _workspaces: dict = {}
-_retired: list = []  # replaced workspaces stay allocated: CUDA graphs captured earlier hold their raw pointers
+_retired: list = []  # replaced scratch stays allocated: CUDA graphs captured earlier hold its raw pointer
+
+
+def _put(table: dict, key, scratch) -> None:
+    """Make ``scratch`` the one of ``key``.  Whatever it replaces is kept: a captured graph, or another thread that is
+    launching with it, may still use it."""
+    old = table.get(key)
+    if old is not None:
+        _retired.append(old)
+    table[key] = scratch
 
 
 def fc_workspace(rows: int, K: int, N: int, qtype: int, group_k: int, device: torch.device) -> Workspace:
@@ -99,10 +108,8 @@ def fc_workspace(rows: int, K: int, N: int, qtype: int, group_k: int, device: to
            torch.cuda.current_stream(device).cuda_stream)
     ws = _workspaces.get(key)
     if ws is None or ws.nbytes < need:
-        if ws is not None:
-            _retired.append(ws)
         ws = Workspace(need, device)
-        _workspaces[key] = ws
+        _put(_workspaces, key, ws)
     return ws
 
 
@@ -580,9 +587,13 @@ _q8c_scratch: dict = {}  # (device index, stream) -> codes and scales of the lar
 
 
 def _make_q8c_scratch(index: int, stream: int, need: int):
-    """Called by the front when a call on ``stream`` finds no scratch, or too small a one."""
-    ws = torch.empty(max(need, 1 << 16), dtype=torch.uint8, device=torch.device("cuda", index))
-    _q8c_scratch[(index, stream)] = ws
+    """Called by the front when a call on ``stream`` finds no scratch, or too small a one.  What is replaced stays
+    allocated (see ``_put``); each scratch is at least twice the one before, so that all of them together stay below
+    twice the last one."""
+    old = _q8c_scratch.get((index, stream))
+    need = max(need, 1 << 16, 2 * old.numel() if old is not None else 0)
+    ws = torch.empty(need, dtype=torch.uint8, device=torch.device("cuda", index))
+    _put(_q8c_scratch, (index, stream), ws)
     return ws, ws.data_ptr(), ws.numel()
 
 
@@ -603,7 +614,8 @@ def FC_quant_Q8C(wei: torch.Tensor):
 def FC_evaluate_Q8C(input: torch.Tensor, wei_quantized: torch.Tensor, wei_scales: torch.Tensor, N: int, *,
                     out: torch.Tensor | None = None) -> torch.Tensor:
     """``[B, M, K]`` x Q8C weights -> ``[B, M, N]`` (ext/llama_ext.cpp:336-371).  The scratch for the quantized
-    activations is kept per (device, stream) and grows to the largest call; calls on one stream are ordered."""
+    activations is kept per (device, stream) and grows with the calls, and stays where a captured graph has it; calls on
+    one stream are ordered."""
     return _front().q8c_fc(input, wei_quantized, wei_scales, N, out)
 
 

@@ -1,5 +1,7 @@
 """Branches of the host and kernel dispatch, each at the sizes where it can go wrong, against the other entry points or
 the oracle."""
+import weakref
+
 import numpy as np
 import pytest
 import torch
@@ -37,6 +39,32 @@ def test_host_fc_refuses_unfit_weights(pkg, rows):
             with pytest.raises(RuntimeError, match=text):
                 fc = pkg.host.HostFC(wq, 256, max_rows=16, graph=graph)
                 fc(torch.zeros(1, rows, fc.K))
+
+
+def test_q8c_graph_outlives_a_larger_call(pkg):
+    """A captured call keeps its scratch when a larger call on the stream needs another: the scratch is not handed out
+    again, and the replay gives the captured call's result."""
+    ops = pkg.llmops
+    g = torch.Generator().manual_seed(0)
+    w, s = pkg.c_ext.FC_quant_Q8C((torch.randn(200, 1024, generator=g) * 0.02).cuda())
+    small, large = (torch.randn(1, rows, 1024, generator=g).cuda() for rows in (8, 2000))
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        want = ops.FC_evaluate_Q8C(small, w, s, 200)
+        key = (torch.cuda.current_device(), stream.cuda_stream)
+        scratch = weakref.ref(ops._q8c_scratch[key])
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = ops.FC_evaluate_Q8C(small, w, s, 200)
+        for rows in (9, 700, 2000):
+            ops.FC_evaluate_Q8C(large[:, :rows].contiguous(), w, s, 200)
+        assert scratch() is not None and ops._q8c_scratch[key] is not scratch()
+        kept = sum(t.numel() for t in ops._retired if isinstance(t, torch.Tensor))
+        assert kept < sum(t.numel() for t in ops._q8c_scratch.values())
+        graph.replay()
+    stream.synchronize()
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("rows,N,K", [
