@@ -407,7 +407,8 @@ PyObject* quant_batch(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // ---- graph_step(dst, src, graph_exec, stream, device, sync): copy the step's input, replay its graph, wait -----------
 // The graph holds none of torch's random-number kernels (CUDAGraph.replay() would have to advance their state).
-// False: `src` is no plain tensor like `dst`; nothing has been done.
+// False: `src` is no plain tensor like `dst`, or shares a part of its memory (Tensor.copy_ refuses that); nothing has been
+// done.
 PyObject* graph_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!nargs_ok(n, 6)) return nullptr;
     FRONT_BEGIN
@@ -427,6 +428,8 @@ PyObject* graph_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
             !d.is_contiguous() || !s.is_contiguous() || d.is_neg() || s.is_neg())
             Py_RETURN_FALSE;
         dst = d.data_ptr(), src = s.data_ptr(), bytes = d.nbytes(), host_copy = both_host;
+        const uintptr_t da = reinterpret_cast<uintptr_t>(dst), sa = reinterpret_cast<uintptr_t>(src);
+        if (da != sa && da < sa + bytes && sa < da + bytes) Py_RETURN_FALSE;
     }
     c10::cuda::CUDAGuard guard(dev);
     const int rc = without_gil([&] {

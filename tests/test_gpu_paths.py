@@ -41,6 +41,20 @@ def test_host_fc_refuses_unfit_weights(pkg, rows):
                 fc(torch.zeros(1, rows, fc.K))
 
 
+def test_host_fc_refuses_overlapping_input(pkg):
+    """Rows 1..4 of the staging buffer cannot be copied onto rows 0..3; rows 4..7 can, rows 0..3 need no copy."""
+    g = torch.Generator().manual_seed(3)
+    wq = pkg.llmops.offline_FC_quant_Q4A((torch.randn(96, 512, generator=g) * 0.02).cuda())
+    fc = pkg.host.HostFC(wq, 96)
+    x = torch.randn(1, 8, 512, generator=g)
+    fc(x[:, :4])  # captured
+    for lo in (0, 4):
+        fc.x_staging(8).copy_(x)
+        assert torch.equal(fc(fc.x_staging(8)[:, lo: lo + 4]), pkg.llmops.fc_Q4A(x[:, lo: lo + 4].cuda(), wq, 96).cpu())
+    with pytest.raises(RuntimeError, match="single memory location"):
+        fc(fc.x_staging(8)[:, 1:5])
+
+
 def test_q8c_graph_outlives_a_larger_call(pkg):
     """A captured call keeps its scratch when a larger call on the stream needs another: the scratch is not handed out
     again, and the replay gives the captured call's result."""
