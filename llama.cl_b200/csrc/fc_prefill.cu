@@ -27,7 +27,7 @@
 // Measured (whole call, quantizer included; before: unpacking straight from global memory without prefetch, one 128 x 128
 // tile per CTA whatever the row count, epilogue of 5 operations per integer):
 //   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 us   Q4_0 g32, 512 rows 280 -> 223 us (207 TOPS)
-//                   Q4_1 g128, 2048 rows 517 -> 323 us (572 TOPS)   Q8C, 256 rows 296 -> 132 us (175 TOPS)
+//                   Q4_1 g128, 2048 rows 517 -> 323 us (572 TOPS)   Q8C, 256 rows 296 -> 151 us (153 TOPS)
 // A group of 32 k takes about 1100 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
 // convert, scale is latency-bound with the 16 warps that the registers allow.  Tried and dropped: handing registers
 // between roles with setmaxnreg (spills around it; 260 us for the 512-row case), both chunks in registers at once
@@ -37,6 +37,13 @@
 // each), one MMA issuer, one loader.  Every wait is bounded: when a wait runs out the CTA sets the status word, every
 // role leaves its loop, TMEM is freed and the kernel returns.
 //
+// Q8C sums K in two levels (FOLD): the 8-row kernel of q8c.cu adds chains of a few groups, and one chain over all of K is
+// less exact than that (K = 4096: 2.0e-7 of the result in the 2-norm, with 8 warps' chains 9.6e-8; K = 11008: 3.3e-7 and
+// 1.3e-7).  After 8 groups, or 12 where a CTA has more than 64, a thread moves its running sums to a second place and keeps
+// what that addition rounds off: 6.5e-8 to 7.5e-8 for K from 512 to 11008, below the 8-warp sums at every size tried.  It
+// costs 131 -> 151 us at 256 rows x 4096 x 11008 and 33 -> 35 at 37 rows; every 16 groups 146 us and 8.3e-8, at K = 3001 not
+// below the 8-warp sums.  (Staggering the moves over the warps: 156; as an outer loop around the groups' loop: 157.)
+//
 // Few tiles: a cluster of `split` CTAs shares a tile and divides its K stages; the partial tiles meet in shared memory
 // and are added in rank order (fixed order, no atomics).
 #include <cuda.h>  // CUtensorMap and the cuTensorMapEncodeTiled prototype (resolved at run time, libcuda is not linked)
@@ -44,6 +51,7 @@
 #include <cooperative_groups.h>
 
 #include <atomic>
+#include <cfloat>
 
 #include "common.cuh"
 #include "ring_ptx.cuh"
@@ -55,7 +63,7 @@ namespace {
 
 constexpr int kTileN = 128;    // weight columns per tile = TMEM lanes
 constexpr int kStageK = 128;   // k per shared-memory stage (one 128-byte swizzle row)
-constexpr int kTmemBufs = 4;
+constexpr int kTmemBufs = 4;   // of a tile's columns each
 constexpr int kProdWarps = 4;  // one stripe of the tile each
 constexpr int kMaxSplit = 8;
 
@@ -73,6 +81,7 @@ struct PrefillShape {
     static constexpr int kB = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;    // stages of activation codes
     static constexpr int kRaw = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;  // stages of packed bytes
     static constexpr int kScs = 4;                        // stages of scales
+    static constexpr int kBufs = FMT == kQ8C && TM == 64 ? kTmemBufs - 1 : kTmemBufs;  // buffers of integers (Q8C: one holds sums)
     static constexpr int kRawStripe = kGroups * kBlock;   // packed bytes of one stripe in a stage
     static constexpr int kABytes = kTileN * kStageK, kBBytes = TM * kStageK;
     static constexpr int kXscBytes = kGroups * kSums * TM * 4;                // [group][scale | sum][row] fp32
@@ -82,7 +91,8 @@ struct PrefillShape {
     static constexpr int kRawOff = kBOff + kB * kBBytes;
     static constexpr int kScOff = kRawOff + kRaw * 4 * kRawStripe;
     static constexpr int kBarOff = kScOff + kScs * kScBytes;
-    static constexpr int kSmem = kBarOff + 512 + 1024 /*alignment slack*/;
+    static constexpr int kSumOff = kBarOff + 512;
+    static constexpr int kSmem = kSumOff + (FMT == kQ8C && TM == 128 ? TM * kTileN * 4 : 0) + 1024 /*alignment slack*/;
     static_assert(TM == 128 || kSmem <= 113 * 1024, "two CTAs on an SM");
     static_assert(TM * kTileN * 4 <= kRawOff, "the partial tile of a K split takes the operand stages' place");
 };
@@ -151,6 +161,12 @@ __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fsub2(uint64_t a, uint64_t b) { return ffma2(b, 0xBF800000BF800000ull, a); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -180,6 +196,12 @@ __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&r)[8]) {
                  : "r"(taddr)
                  : "memory");
 }
+__device__ __forceinline__ void tc_st(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;
@@ -190,6 +212,12 @@ __device__ __forceinline__ uint32_t lds16(uint32_t addr) {
     uint16_t v;
     asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(addr));
     return v;
+}
+__device__ __forceinline__ void lds128(uint32_t addr, uint64_t& a, uint64_t& b) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void sts128(uint32_t addr, uint64_t a, uint64_t b) {
+    asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(addr), "l"(a), "l"(b) : "memory");
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
@@ -232,7 +260,85 @@ __device__ __forceinline__ void accumulate(uint64_t (&acc)[8], const uint32_t (&
     }
 }
 
-template <int FMT, int G, int TM>
+// ---- Q8C: sums in two levels --------------------------------------------------------------------------------------------
+// `sum` += `run`, and what the addition rounds off stays in `run` and starts the next running sum (T. J. Dekker, Numer.
+// Math. 18, 1971: exact where |sum| >= |run|; elsewhere a rounding of the smaller `run` is lost).
+__device__ __forceinline__ uint64_t move_sum(uint64_t sum, uint64_t& run) {
+    const uint64_t s = fadd2(sum, run);
+    run = fsub2(run, fsub2(s, sum));
+    return s;
+}
+__device__ __forceinline__ void finite_or_zero(uint64_t& v) {
+    float lo, hi;
+    unpack2(v, lo, hi);
+    v = pack2(fabsf(lo) <= FLT_MAX ? lo : 0.0f, fabsf(hi) <= FLT_MAX ? hi : 0.0f);
+}
+// Sixteen rows of a thread's running sums into the sums behind `at`: 128-row tiles keep them in shared memory (a thread's
+// own 16-byte places), 64-row tiles, whose shared memory is full, in the last of their four TMEM buffers.
+template <int TM, int THREADS>
+__device__ __forceinline__ void fold(uint64_t (&run)[8], uint32_t at, bool first) {
+    uint64_t odd = 0;  // not finite where a sum has left the finite numbers
+    if constexpr (TM == 128) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            uint64_t a = 0, b = 0;
+            if (!first) lds128(at + j * THREADS * 16, a, b);
+            a = move_sum(a, run[2 * j]), b = move_sum(b, run[2 * j + 1]);
+            odd = fadd2(odd, fadd2(run[2 * j], run[2 * j + 1]));
+            sts128(at + j * THREADS * 16, a, b);
+        }
+    } else {
+        tc_wait_st();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint32_t v[8] = {};
+            if (!first) {
+                tc_ld(at + 8 * h, v);
+                tc_wait_ld();
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                uint64_t a = pack2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                a = move_sum(a, run[4 * h + j]);
+                odd = fadd2(odd, run[4 * h + j]);
+                float lo, hi;
+                unpack2(a, lo, hi);
+                v[2 * j] = __float_as_uint(lo), v[2 * j + 1] = __float_as_uint(hi);
+            }
+            tc_st(at + 8 * h, v);
+        }
+    }
+    float lo, hi;
+    unpack2(odd, lo, hi);
+    if (!(fabsf(lo) <= FLT_MAX && fabsf(hi) <= FLT_MAX)) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) finite_or_zero(run[j]);
+    }
+}
+template <int TM, int THREADS>
+__device__ __forceinline__ void unfold(uint64_t (&run)[8], uint32_t at) {  // `run` += the sums behind `at`
+    if constexpr (TM == 128) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            uint64_t a, b;
+            lds128(at + j * THREADS * 16, a, b);
+            run[2 * j] = fadd2(a, run[2 * j]), run[2 * j + 1] = fadd2(b, run[2 * j + 1]);
+        }
+    } else {
+        tc_wait_st();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            uint32_t v[8];
+            tc_ld(at + 8 * h, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                run[4 * h + j] = fadd2(pack2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), run[4 * h + j]);
+        }
+    }
+}
+
+template <int FMT, int G, int TM, int FOLD>
 __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 ? 1 : 2)
     fc_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap codes_map) {
     using S = PrefillShape<FMT, G, TM>;
@@ -309,10 +415,14 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
 #pragma unroll
         for (int i = 0; i < 8; i++) acc[0][i] = acc[1][i] = 0ull;
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + cgrp * 16;
+        // the sums that FOLD K groups at a time are moved to
+        constexpr int kEpi = S::kEpiWarps * 32;
+        const uint32_t sum0 = TM == 128 ? smem0 + S::kSumOff + threadIdx.x * 16 : taddr + S::kBufs * TM;
+        const uint32_t sum1 = sum0 + (TM == 128 ? 4 * 16 * kEpi : CGN * 16);
         const int groups = min(p.Kg, it1 * GPS) - it0 * GPS;
 #pragma unroll 1
         for (int g = 0; g < groups; g++) {
-            const int i = g / GPS, sl = i % S::kScs, gi = g % GPS, b = g % kTmemBufs;
+            const int i = g / GPS, sl = i % S::kScs, gi = g % GPS, b = g % S::kBufs;
             if (gi == 0 && !wait_or_abort(bar_sfull + 8 * sl, (i / S::kScs) & 1, abort_flag)) break;
             const uint8_t* sc = smem + S::kScOff + sl * S::kScBytes;
             const float* xs = reinterpret_cast<const float*>(sc) + gi * (S::kSums * TM) + cgrp * 16;
@@ -322,7 +432,7 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                 const float wd = h2f((uint16_t)w), wm = h2f((uint16_t)(w >> 16));
                 wd2 = pack2(wd, wd), wm2 = pack2(wm, wm);
             }
-            if (!wait_or_abort(bar_tfull + 8 * b, (g / kTmemBufs) & 1, abort_flag)) break;
+            if (!wait_or_abort(bar_tfull + 8 * b, (g / S::kBufs) & 1, abort_flag)) break;
             tc_fence_after();
             // W integers at a time: what the two chunks would take together is what the register file has left, and the
             // compiler then serialises the arithmetic (37 rows, one CTA an SM: 84 us with W = 16 in 72 registers, 78 with 8)
@@ -358,6 +468,15 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_sempty + 8 * sl);  // done with the stage's scales
             }
+            if constexpr (FOLD > 0)
+                if (g % FOLD == FOLD - 1) {
+                    if (live0) fold<TM, kEpi>(acc[0], sum0, g == FOLD - 1);
+                    if (live1) fold<TM, kEpi>(acc[1], sum1, g == FOLD - 1);
+                }
+        }
+        if (FOLD > 0 && groups >= FOLD) {
+            if (live0) unfold<TM, kEpi>(acc[0], sum0);
+            if (live1) unfold<TM, kEpi>(acc[1], sum1);
         }
         if (cs == 1) {
             const int64_t n = n0 + nrow;
@@ -491,9 +610,9 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                 const int ng = min(GPS, p.Kg - (it0 + i) * GPS);
 #pragma unroll 1
                 for (int gi = 0; gi < ng; gi++, gcount++) {
-                    const int b = gcount % kTmemBufs;
+                    const int b = gcount % S::kBufs;
                     const uint64_t ad = a_desc + (uint64_t)(gi * (G / 16)), bd = b_desc + (uint64_t)(gi * (G / 16));
-                    if (!wait_or_abort(bar_tempty + 8 * b, ((gcount / kTmemBufs) & 1) ^ 1, abort_flag)) {
+                    if (!wait_or_abort(bar_tempty + 8 * b, ((gcount / S::kBufs) & 1) ^ 1, abort_flag)) {
                         ok = false;
                         break;
                     }
@@ -540,18 +659,31 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
             const float* red = reinterpret_cast<const float*>(smem);
 #pragma unroll 1
             for (int m = rank + cs * warp; m < live; m += cs * S::kEpiWarps) {
-                float sum[4] = {};
+                uint64_t sum[2] = {}, rest[2] = {};  // columns lane, lane + 32 and lane + 64, lane + 96
 #pragma unroll 1
                 for (int q = 0; q < cs; q++) {
                     const float* src = cluster.map_shared_rank(red, q) + m * kTileN + lane;
 #pragma unroll
-                    for (int c = 0; c < 4; c++) sum[c] = q ? __fadd_rn(sum[c], src[32 * c]) : src[32 * c];
+                    for (int c = 0; c < 2; c++) {
+                        const uint64_t v = pack2(src[64 * c], src[64 * c + 32]);
+                        if (FMT == kQ8C) {
+                            uint64_t r = fadd2(v, rest[c]);
+                            sum[c] = move_sum(sum[c], r);
+                            finite_or_zero(r);
+                            rest[c] = r;
+                        } else {
+                            sum[c] = q ? fadd2(sum[c], v) : v;
+                        }
+                    }
                 }
+                float out[4];
+#pragma unroll
+                for (int c = 0; c < 2; c++) unpack2(FMT == kQ8C ? fadd2(sum[c], rest[c]) : sum[c], out[2 * c], out[2 * c + 1]);
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     const int64_t n = n0 + lane + 32 * c;
                     if (n < p.N)
-                        p.y[(m0 + m) * p.ldy + n] = FMT == kQ8C ? __fmul_rn(__ldg(p.wscales + n), sum[c]) : sum[c];
+                        p.y[(m0 + m) * p.ldy + n] = FMT == kQ8C ? __fmul_rn(__ldg(p.wscales + n), out[c]) : out[c];
                 }
             }
         }
@@ -618,13 +750,13 @@ int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t 
     return Q4FC_OK;
 }
 
-template <int FMT, int G, int TM>
+template <int FMT, int G, int TM, int FOLD = 0>
 int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, int64_t n_tiles, int64_t m_tiles, cudaStream_t s) {
     using S = PrefillShape<FMT, G, TM>;
     static std::atomic<bool> attr_done[64] = {};  // set once per device; a second setter repeats the same call
     int dev = 0;
     Q4FC_CUDA_OK(cudaGetDevice(&dev));
-    auto* fn = fc_prefill_kernel<FMT, G, TM>;
+    auto* fn = fc_prefill_kernel<FMT, G, TM, FOLD>;
     if (dev >= 64 || !attr_done[dev]) {
         Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem));
         Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
@@ -695,7 +827,14 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     CUtensorMap map = {};
     if (Kp > 0)  // (no K group: no stage reads the map)
         if (int rc = make_codes_map(&map, codes, rows, Kp, tile)) return rc;
-    if (fmt == kQ8C) return launch_prefill_tile<kQ8C, 32>(tile, p, map, n_tiles, m_tiles, s);
+    if (fmt == kQ8C) {
+        const bool many = p.Kg > 64 * split;  // K groups of a CTA: see the file's head
+        if (tile == 128)
+            return many ? launch_prefill_variant<kQ8C, 32, 128, 12>(p, map, n_tiles, m_tiles, s)
+                        : launch_prefill_variant<kQ8C, 32, 128, 8>(p, map, n_tiles, m_tiles, s);
+        return many ? launch_prefill_variant<kQ8C, 32, 64, 12>(p, map, n_tiles, m_tiles, s)
+                    : launch_prefill_variant<kQ8C, 32, 64, 8>(p, map, n_tiles, m_tiles, s);
+    }
     if (fmt == kQ4_1 && G == 32) return launch_prefill_tile<kQ4_1, 32>(tile, p, map, n_tiles, m_tiles, s);
     if (fmt == kQ4_1) return launch_prefill_tile<kQ4_1, 128>(tile, p, map, n_tiles, m_tiles, s);
     if (fmt == kQ4_0 && G == 32) return launch_prefill_tile<kQ4_0, 32>(tile, p, map, n_tiles, m_tiles, s);

@@ -291,7 +291,7 @@ int launch_q8c_fc(const float* x, int64_t rows, int64_t K, int64_t ldx, const in
     int8_t* codes = static_cast<int8_t*>(ws);
     float* xs = reinterpret_cast<float*>(static_cast<char*>(ws) + align_up((size_t)(rows * Kg * 32), 256));
     // the kernel below holds 8 rows; with more of them in a CTA, on mma.sync, 256 rows x 4096 x 11008 took 296 us
-    // (the tensor-core GEMM: 132 us)
+    // (the tensor-core GEMM: 151 us)
     if (rows > 8) return launch_q8c_prefill(x, rows, K, ldx, wq, wscales, Ng, Kg, N, y, ldy, codes, xs, s);
     if (int rc = launch_quant_x(x, rows, K, ldx, 32, 1.0f, codes, xs, nullptr, s)) return rc;
     const int64_t stripes = (N + 31) / 32;

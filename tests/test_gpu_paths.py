@@ -110,6 +110,45 @@ def test_many_rows_on_tile_edges(pkg, oracle, fmt, rows, N, K):
     pkg.llmops.check_device_status()
 
 
+@pytest.mark.parametrize("rows,N,K", [
+    (256, 11008, 4096),               # 128-row tiles, groups by 12
+    (300, 9000, 2000),                # by 8, a last stage with three groups
+    (129, 10000, 11008),
+    (37, 11008, 4096),                # 64-row tiles, K divided by 3
+    (512, 4096, 11008),               # undivided
+    (17, 200, 1000), (9, 700, 4097),  # divided further
+])
+def test_q8c_many_rows_precision(pkg, rows, N, K):
+    """The sums over K against 64 bits on the same codes and scales.  A rounding to nearest is off by 2.5e-8 of its sum in
+    the root mean square; a chain of 12 groups holds 6.5 such errors of the whole sum's size (in squares), the second
+    level, the division of K and the column scale four more at most: 8.1e-8.  One chain over K = 4096 gives 2.0e-7."""
+    g = torch.Generator(device="cuda").manual_seed(rows + N + K)
+    x = torch.randn(1, rows, K, generator=g, device="cuda")
+    w, s = pkg.c_ext.FC_quant_Q8C(torch.randn(N, K, generator=g, device="cuda") * 0.02)
+    codes, xs, _ = pkg.llmops.FC_dynamic_quantize_x(x[0], 32)
+    Ng, Kg = w.shape[:2]
+    q = w.view(Ng, Kg, 8, 32, 4).permute(0, 3, 1, 2, 4).reshape(Ng * 32, Kg * 32)[:N]
+    want = (codes.double().view(rows, Kg, 32) * xs.double()[:, :, None]).view(rows, -1) @ q.double().t() * s[:N].double()
+    got = pkg.c_ext.FC_evaluate_Q8C(x, w, s, N)[0].double()
+    assert ((got - want).norm() / want.norm()).item() <= 8.1e-8
+
+
+@pytest.mark.parametrize("rows", [40, 400])
+def test_q8c_many_rows_beyond_the_finite_numbers(pkg, rows):
+    """Sums that overflow, and inputs that are not finite, end as in the 8-row kernel.  (Finite rows: 2 x 40 roundings of
+    2^-24, each of a part of the sum of the terms' sizes, about 16: 8e-5.)"""
+    g = torch.Generator().manual_seed(rows)
+    x = torch.randn(1, rows, 1000, generator=g)
+    x[0, 1], x[0, 2] = 1e38, -1e38
+    x[0, 3, 700:], x[0, 5, 300], x[0, 6, 999], x[0, 7] = 3e38, float("inf"), float("nan"), float("nan")
+    x = x.cuda()
+    w, s = pkg.c_ext.FC_quant_Q8C((torch.rand(5000, 1000, generator=g) * 0.02 + 0.01).cuda())
+    want = pkg.c_ext.FC_evaluate_Q8C(x[:, :8].contiguous(), w, s, 5000)
+    got = pkg.c_ext.FC_evaluate_Q8C(x, w, s, 5000)[:, :8]
+    assert torch.isinf(want[0, 1]).all() and torch.isinf(want[0, 2]).all() and torch.isinf(want[0, 3]).all()
+    assert torch.allclose(got, want, rtol=0, atol=8e-5, equal_nan=True)
+
+
 @pytest.mark.parametrize("qtype,G", [(0, 32), (1, 128)])
 @pytest.mark.parametrize("K", [264, 260, 259])
 @pytest.mark.parametrize("offset", [0, 4, 1])
