@@ -210,11 +210,9 @@ size_t q4fc_fc_workspace_bytes(int64_t rows, int64_t K, int64_t N, int qtype, in
         const size_t q = decode_prequant_offset() + quant_pre_bytes(rows, K, group_k);
         if (q > need) need = q;
     }
-    if (rows > kMaxDecodeRows) {
-        size_t p = prefill_workspace_bytes(rows, K, N, qtype, group_k);
-        if (p > need) need = p;
-    }
-    return need;
+    // q4fc_fc_prefill takes any row count
+    const size_t p = prefill_workspace_bytes(rows, K, N, qtype, group_k);
+    return p > need ? p : need;
 }
 
 int q4fc_fc_workspace_init(void* ws, size_t ws_bytes, q4fc_stream_t stream) {

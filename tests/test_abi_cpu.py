@@ -68,6 +68,23 @@ def test_argument_errors_without_gpu(lib_built):
     assert L.q4fc_strerror(4) == b"workspace missing or too small"
 
 
+@pytest.mark.parametrize("qtype,G", [(0, 32), (0, 128), (1, 32), (1, 128)])
+def test_workspace_serves_every_path(lib_built, qtype, G):
+    """q4fc_fc_workspace_bytes is enough for the prefill entry point at any row count, and never falls as rows grow.
+    (What the entry point needs is read from its refusal of a call without a workspace; nothing is launched.)"""
+    import llama_cl_b200 as pkg
+
+    L = pkg._cabi.lib()
+    for K in (1, 256, 4096, 4100):
+        sizes = []
+        for rows in (1, 5, 8, 9, 64, 65, 128, 129, 500):
+            assert L.q4fc_fc_prefill(16, rows, K, K, 16, 1, -(-K // G), qtype, G, 32, 16, 32, None, 0, 0, None) == 4
+            needed = int(re.search(rb"(\d+) needed", L.q4fc_last_error()).group(1))
+            sizes.append(L.q4fc_fc_workspace_bytes(rows, K, 32, qtype, G))
+            assert sizes[-1] >= needed, (rows, K)
+        assert sizes == sorted(sizes)
+
+
 def test_wrappers_reject_cpu_tensors(lib_built):
     """There is no CPU path: CPU tensors are an error, not a fallback."""
     import torch

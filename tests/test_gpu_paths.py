@@ -81,6 +81,26 @@ def test_q8c_graph_outlives_a_larger_call(pkg):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("qtype,G", [(0, 32), (1, 128)])
+@pytest.mark.parametrize("rows", [1, 5, 8])
+def test_few_rows_on_the_prefill_path(pkg, rows, qtype, G):
+    """A workspace of exactly the stated size serves the prefill path at any row count, here and through HostFC."""
+    ops, N, K = pkg.llmops, 96, 4100
+    g = torch.Generator().manual_seed(rows)
+    wq = ops.offline_FC_quant_Q4A((torch.randn(N, K, generator=g) * 0.02).cuda(), qtype=qtype, group_k=G)
+    x = torch.zeros(1, rows, -(-K // G) * G)
+    x[:, :, :K] = torch.randn(1, rows, K, generator=g)
+    size = pkg._cabi.lib().q4fc_fc_workspace_bytes(rows, x.shape[2], N, qtype, G)
+    ws = ops.Workspace(size, torch.device("cuda"))
+    assert ws.nbytes == size
+    got = ops.fc_Q4A(x.cuda(), wq, N, path="prefill", workspace=ws).cpu()
+    ws.check()
+    # 2 x 264 roundings of 2^-24 at most, which add up like a random walk: 1.4e-6 of the sum; a factor of ten on top
+    want = ops.fc_Q4A(x.cuda(), wq, N, path="decode").cpu()
+    assert (got - want).abs().max() <= 1.4e-5 * want.abs().max()
+    assert torch.equal(pkg.host.HostFC(wq, N, max_rows=rows, path="prefill")(x), got)
+
+
 @pytest.mark.parametrize("rows,N,K", [
     (9, 4096, 512),     # one 16-row chunk
     (16, 130, 4128),    # a last stage with one K group; K divided unevenly; stripes that fill no tile of four
