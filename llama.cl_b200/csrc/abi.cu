@@ -793,8 +793,9 @@ int q4fc_fc_check_status(void* ws, q4fc_stream_t stream) {
     Q4FC_CUDA_OK(cudaStreamSynchronize(s));
     if (status != 0) {
         Q4FC_CUDA_OK(cudaMemsetAsync(ws, 0, sizeof(int), s));
-        set_error("device status word = 0x%x (%s)", status,
-                  (status & 0x100) ? "an embedding id was out of range" : "a bounded wait ran out");
+        const bool bad_id = (status & kStatusBadId) != 0, wait = (status & ~kStatusBadId) != 0;
+        set_error("device status word = 0x%x (%s%s%s)", status, bad_id ? "an embedding id was out of range" : "",
+                  bad_id && wait ? "; " : "", wait ? "a bounded wait ran out" : "");
         return Q4FC_EDEVICE;
     }
     return Q4FC_OK;

@@ -45,6 +45,9 @@ const DeviceInfo* device_info();
 // then       CTA partials [ctas][2][8][32] fp32 (size fixed per device)
 // then       per-stripe arrival counters int[Ng], zero between calls
 constexpr size_t kWsStatusBytes = 256;
+// A status word holds the code of the first wait that ran out, four ASCII letters, and this bit, which no letter has, when
+// an embedding id was out of range.
+constexpr int kStatusBadId = 0x80;
 
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 

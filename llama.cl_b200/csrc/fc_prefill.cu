@@ -695,7 +695,8 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
     tc_fence_before();
     __syncthreads();
     if (*abort_flag) {
-        if (threadIdx.x == 0) atomicExch(p.status, 0x50524546);  // 'PREF': a bounded wait ran out
+        if (threadIdx.x == 0 && (atomicCAS(p.status, 0, 0x50524546) & ~kStatusBadId) == 0)  // 'PREF': a bounded wait ran out
+            atomicOr(p.status, 0x50524546);
         // copies that may still be in flight land before the shared memory is handed to another CTA
 #pragma unroll 1
         for (int i = 0; i < 64; i++) __nanosleep(32000);

@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(256) emb_q8c_quant_kernel(const float* __restr
 // One CTA per looked-up id: out[i][k] = scales[id] * (float)codes[id][k].  A lane takes four codes at a time, so that a
 // warp's loads and stores are whole lines (16 codes a lane left every 16-byte store 64 bytes from its neighbour: 2048 ids
 // of 4096 took 14.2 us, now 8.2), eight of them in flight.  An id outside [0, V) leaves a row of
-// zeros and sets bit 0x100 of the status word.
+// zeros and sets kStatusBadId in the status word.
 template <typename Tidx>
 __global__ void __launch_bounds__(128) emb_q8c_kernel(const Tidx* __restrict__ ids, const int8_t* __restrict__ codes,
                                                       const float* __restrict__ scales, int64_t V, int64_t E,
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(128) emb_q8c_kernel(const Tidx* __restrict__ i
     float* dst = out + i * ldo;
     if (id < 0 || id >= V) {
         for (int64_t k = threadIdx.x; k < E; k += 128) dst[k] = 0.0f;
-        if (threadIdx.x == 0 && status != nullptr) atomicOr(status, 0x100);
+        if (threadIdx.x == 0 && status != nullptr) atomicOr(status, kStatusBadId);
         return;
     }
     const int8_t* src = codes + id * E;

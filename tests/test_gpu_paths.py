@@ -81,6 +81,25 @@ def test_q8c_graph_outlives_a_larger_call(pkg):
     assert torch.equal(got, want)
 
 
+def test_status_word_texts(pkg):
+    """The code of a wait that ran out (here: written from the host) is no bad embedding id, whichever letters it has."""
+    ws = pkg.llmops.Workspace(4096, torch.device("cuda"))
+    word = ws.buf[:4].view(torch.int32)
+    for code in (b"PREF", b"RFUL", b"REMP", b"TPWT", b"CFUL", b"RXBQ"):
+        word.fill_(int.from_bytes(code, "big"))
+        with pytest.raises(RuntimeError, match=r"\(a bounded wait ran out\)"):
+            ws.check()
+        word.fill_(int.from_bytes(code, "big") | 0x80)
+        with pytest.raises(RuntimeError, match=r"\(an embedding id was out of range; a bounded wait ran out\)"):
+            ws.check()
+        ws.check()  # cleared
+    op = pkg.ops.llmop_embedding_q8c(torch.randn(10, 64, device="cuda"))
+    op(torch.tensor([3, 10, -1], device="cuda"))
+    with pytest.raises(RuntimeError, match=r"\(an embedding id was out of range\)"):
+        pkg.llmops.check_device_status()
+    pkg.llmops.check_device_status()
+
+
 @pytest.mark.parametrize("qtype,G", [(0, 32), (1, 128)])
 @pytest.mark.parametrize("rows", [1, 5, 8])
 def test_few_rows_on_the_prefill_path(pkg, rows, qtype, G):
