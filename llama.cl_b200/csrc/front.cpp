@@ -405,12 +405,13 @@ PyObject* quant_batch(PyObject*, PyObject* const* a, Py_ssize_t n) {
     FRONT_END
 }
 
-// ---- graph_step(dst, src, graph_exec, stream, device, sync): copy the step's input, replay its graph, wait -----------
+// ---- graph_step(dst, src, graph_exec, stream, device, sync, result): copy the step's input, replay its graph, wait -----
+// Returns a new view of the tensor `result`, made while the graph runs, or True where that is None.
 // The graph holds none of torch's random-number kernels (CUDAGraph.replay() would have to advance their state).
 // False: `src` is no plain tensor like `dst`, or shares a part of its memory (Tensor.copy_ refuses that); nothing has been
 // done.
 PyObject* graph_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (!nargs_ok(n, 6)) return nullptr;
+    if (!nargs_ok(n, 7)) return nullptr;
     FRONT_BEGIN
     cudaGraphExec_t exec = static_cast<cudaGraphExec_t>(PyLong_AsVoidPtr(a[2]));
     cudaStream_t stream = static_cast<cudaStream_t>(PyLong_AsVoidPtr(a[3]));
@@ -432,18 +433,23 @@ PyObject* graph_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (da != sa && da < sa + bytes && sa < da + bytes) Py_RETURN_FALSE;
     }
     c10::cuda::CUDAGuard guard(dev);
-    const int rc = without_gil([&] {
+    int rc = without_gil([&] {
         cudaError_t e = cudaSuccess;
         if (src != dst) {
             if (host_copy) memcpy(dst, src, bytes);
             else e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, stream);
         }
         if (e == cudaSuccess) e = cudaGraphLaunch(exec, stream);
-        if (e == cudaSuccess && sync) e = cudaStreamSynchronize(stream);
         return (int)e;
     });
+    if (a[6] == Py_None) {
+        ret = new_ref(Py_True);
+    } else {
+        ret = THPVariable_Wrap(THPVariable_Unpack(a[6]).detach());
+        if (!ret) throw PyFailed();
+    }
+    if (rc == cudaSuccess && sync) rc = without_gil([&] { return (int)cudaStreamSynchronize(stream); });
     if (rc != cudaSuccess) fail(std::string("CUDA error: ") + cudaGetErrorString((cudaError_t)rc));
-    ret = new_ref(Py_True);
     FRONT_END
 }
 

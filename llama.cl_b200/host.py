@@ -99,12 +99,12 @@ class HostFC:
             raise RuntimeError(f"HostFC: input {tuple(x_host.shape)} does not fit [1, <={self.max_rows}, {self.K}]")
         if self.use_graph:
             _, ex, stage, y = self._graph(M)
-            # one native call: activations into the staging buffer, graph launch, wait
-            if self._front.graph_step(stage, x_host, ex, self._stream_ptr, self._dev_index, sync):
-                return y
+            # one native call: activations into the staging buffer, graph launch, a new view of the output, wait
+            got = self._front.graph_step(stage, x_host, ex, self._stream_ptr, self._dev_index, sync, y)
+            if got is not False:
+                return got
             stage.copy_(x_host)
-            self._front.graph_step(stage, None, ex, self._stream_ptr, self._dev_index, sync)
-            return y
+            return self._front.graph_step(stage, None, ex, self._stream_ptr, self._dev_index, sync, y)
         stage = self._x_host[:, :M]
         if x_host.data_ptr() != stage.data_ptr():
             stage.copy_(x_host)

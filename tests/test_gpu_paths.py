@@ -41,6 +41,18 @@ def test_host_fc_refuses_unfit_weights(pkg, rows):
                 fc(torch.zeros(1, rows, fc.K))
 
 
+def test_host_fc_results_are_views_of_their_own(pkg):
+    """What a caller does to the tensor that a call returned changes no later call's."""
+    wq = pkg.llmops.offline_FC_quant_Q4A(torch.randn(96, 512).cuda())
+    for graph in (True, False):
+        fc = pkg.host.HostFC(wq, 96, graph=graph)
+        x = torch.randn(1, 4, 512)
+        y = fc(x)
+        y.squeeze_(0).requires_grad_()
+        z = fc(x)
+        assert z is not y and z.shape == (1, 4, 96) and not z.requires_grad and z.data_ptr() == y.data_ptr()
+
+
 def test_host_fc_refuses_overlapping_input(pkg):
     """Rows 1..4 of the staging buffer cannot be copied onto rows 0..3; rows 4..7 can, rows 0..3 need no copy."""
     g = torch.Generator().manual_seed(3)
