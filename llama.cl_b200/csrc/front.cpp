@@ -12,11 +12,13 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cuda_runtime_api.h>
 
 #include <cstring>
+#include <exception>
 #include <string>
 #include <string_view>
 #include <vector>
@@ -178,7 +180,7 @@ int without_gil(F f) {
 #define FRONT_END                                        \
     return ret; }                                        \
     catch (const PyFailed&) {}                           \
-    catch (const std::exception& e) { PyErr_SetString(PyExc_RuntimeError, e.what()); } \
+    catch (...) { torch::translate_exception_to_python(std::current_exception()); } /* as torch's own functions do */ \
     Py_XDECREF(ret);                                     \
     return nullptr;
 

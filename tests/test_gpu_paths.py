@@ -93,6 +93,14 @@ def test_q8c_graph_outlives_a_larger_call(pkg):
     assert torch.equal(got, want)
 
 
+def test_out_of_memory_is_torchs_own_error(pkg):
+    """A result that no card holds (549 GB): torch.OutOfMemoryError, as torch.empty raises it, without a C++ trace."""
+    op = pkg.ops.llmop_embedding_q8c(torch.randn(4, 4096, device="cuda"))
+    with pytest.raises(torch.OutOfMemoryError) as e:
+        op(torch.zeros(1 << 25, dtype=torch.int32, device="cuda"))
+    assert "Exception raised from" not in str(e.value)
+
+
 def test_status_word_texts(pkg):
     """The code of a wait that ran out (here: written from the host) is no bad embedding id, whichever letters it has."""
     ws = pkg.llmops.Workspace(4096, torch.device("cuda"))
