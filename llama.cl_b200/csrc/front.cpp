@@ -80,17 +80,24 @@ void check(int rc, const char* what) {
     fail(std::string(what) + ": " + q4fc_strerror(rc) + " (" + std::to_string(rc) + "): " + q4fc_last_error());
 }
 
+// an integer (anything with __index__); nothing else is one
 int64_t as_int(PyObject* o) {
     const int64_t v = PyLong_AsLongLong(o);
-    if (v == -1 && PyErr_Occurred()) {
-        PyErr_Clear();
-        PyObject* l = PyNumber_Long(o);  // the int() of the Python signature
-        if (!l) throw PyFailed();
-        const int64_t w = PyLong_AsLongLong(l);
-        Py_DECREF(l);
-        if (w == -1 && PyErr_Occurred()) throw PyFailed();
-        return w;
-    }
+    if (v == -1 && PyErr_Occurred()) throw PyFailed();
+    return v;
+}
+int as_c_int(PyObject* o) {
+    const int64_t v = as_int(o);
+    if (v != (int)v) fail("integer out of range: " + std::to_string(v));
+    return (int)v;
+}
+// int(o)
+int64_t to_int(PyObject* o) {
+    PyObject* l = PyNumber_Long(o);
+    if (!l) throw PyFailed();
+    const int64_t v = PyLong_AsLongLong(l);
+    Py_DECREF(l);
+    if (v == -1 && PyErr_Occurred()) throw PyFailed();
     return v;
 }
 bool truth(PyObject* o) {
@@ -200,12 +207,15 @@ PyObject* fc(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t B = x.size(0), M = x.size(1), K = x.size(2), Ng = w.size(0), Kg = w.size(1), rows = B * M;
     int q = 0, G = 0;
     variant_of(w.size(2), &q, &G);
-    const int64_t N = as_int(a[2]);
-    const char* path = PyUnicode_AsUTF8(a[7]);
-    if (!path) throw PyFailed();
-    const std::string_view pv(path);
+    const int64_t N = to_int(a[2]);
+    std::string_view pv;
+    if (PyUnicode_Check(a[7])) {
+        const char* path = PyUnicode_AsUTF8(a[7]);
+        if (!path) throw PyFailed();
+        pv = path;
+    }
     const bool streamk = pv == "streamk", prefill = pv == "prefill";
-    if (!streamk && !prefill && pv != "auto" && pv != "decode") {
+    if (a[9] == Py_None && !streamk && !prefill && pv != "auto" && pv != "decode") {  // (an addend has one path only)
         PyErr_SetObject(PyExc_KeyError, a[7]);
         throw PyFailed();
     }
@@ -273,7 +283,7 @@ PyObject* fc(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* pack(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!nargs_ok(n, 4)) return nullptr;
     FRONT_BEGIN
-    const int q = (int)as_int(a[1]), G = (int)as_int(a[2]);
+    const int q = as_c_int(a[1]), G = as_c_int(a[2]);
     const Tensor& w = tensor(a[0], "wei", at::kFloat, 2);
     const int bs = q4fc_block_bytes(q, G);
     if (bs < 0) fail("unsupported block type: qtype=" + std::to_string(q) + ", group_k=" + std::to_string(G));

@@ -93,6 +93,33 @@ def test_q8c_graph_outlives_a_larger_call(pkg):
     assert torch.equal(got, want)
 
 
+def test_argument_forms(pkg):
+    """Sizes are integers (fc_Q4A alone takes what int() takes); an unknown path is a KeyError unless an addend, which has
+    one path, makes it meaningless."""
+    ops = pkg.llmops
+    W, x = torch.randn(64, 512).cuda(), torch.randn(1, 1, 512).cuda()
+    wq, (w8, s8) = ops.offline_FC_quant_Q4A(W), pkg.c_ext.FC_quant_Q8C(W)
+    for bad in (63.5, 64.0, "64", None):
+        with pytest.raises(TypeError):
+            ops.FC_evaluate_Q8C(x, w8, s8, bad)
+    for bad in (32.0, "32", None):
+        with pytest.raises(TypeError):
+            ops.offline_FC_quant_Q4A(W, group_k=bad)
+    for bad in (33, (1 << 32) + 32):
+        with pytest.raises(RuntimeError):
+            ops.offline_FC_quant_Q4A(W, group_k=bad)
+    assert torch.equal(ops.FC_evaluate_Q8C(x, w8, s8, np.int64(60)), ops.FC_evaluate_Q8C(x, w8, s8, 60))
+    assert torch.equal(ops.offline_FC_quant_Q4A(W, group_k=np.int64(32)), wq)
+    want = ops.fc_Q4A(x, wq, 60)
+    for n in (60.5, "60", np.int64(60)):
+        assert torch.equal(ops.fc_Q4A(x, wq, n), want)
+    bias = torch.zeros(60, device="cuda")
+    for path in ("fast", None):
+        with pytest.raises(KeyError):
+            ops.fc_Q4A(x, wq, 60, path=path)
+        assert torch.equal(ops.fc_Q4A(x, wq, 60, path=path, addend=bias), want)
+
+
 def test_out_of_memory_is_torchs_own_error(pkg):
     """A result that no card holds (549 GB): torch.OutOfMemoryError, as torch.empty raises it, without a C++ trace."""
     op = pkg.ops.llmop_embedding_q8c(torch.randn(4, 4096, device="cuda"))
