@@ -58,8 +58,12 @@ class HostFC:
     def _reads_host(self, M: int) -> bool:
         """Whether a call of ``M`` rows works on the pinned buffers in place.  A copy node costs 3-5 us of latency on
         each side of a kernel that runs 5-20 us, and the bytes cross PCIe once either way; the prefill kernels and the
-        stream-K form re-read or re-write their buffers, so they get copies."""
-        return M <= 8 and set(self.fc_kwargs) <= {"workspace", "nibble_signed", "pdl", "prequant"}
+        stream-K form re-read or re-write their buffers, so they get copies.  So does a call whose workspace has no room
+        for the quantizing launch: every cluster of the FC kernel would read the activations over PCIe for itself."""
+        if M > 8 or not set(self.fc_kwargs) <= {"workspace", "nibble_signed", "pdl", "prequant"}:
+            return False
+        need = _cabi.lib().q4fc_fc_workspace_bytes(M, self.K, self.N, self.qtype, self.G)
+        return self.fc_kwargs["workspace"].nbytes >= need
 
     def _enqueue(self, M: int) -> None:
         if self._reads_host(M):

@@ -41,6 +41,19 @@ def test_host_fc_refuses_unfit_weights(pkg, rows):
                 fc(torch.zeros(1, rows, fc.K))
 
 
+def test_host_fc_with_a_small_workspace_copies(pkg):
+    """A workspace without room for the quantizer's codes: the kernel would read the host buffer once per cluster, so the
+    activations are copied."""
+    g = torch.Generator().manual_seed(5)
+    wq = pkg.llmops.offline_FC_quant_Q4A((torch.randn(300, 1024, generator=g) * 0.02).cuda())
+    x = torch.randn(1, 4, 1024, generator=g)
+    size = pkg._cabi.lib().q4fc_fc_workspace_bytes(4, 1024, 300, 1, 32)
+    for nbytes in (size - 256, size):
+        fc = pkg.host.HostFC(wq, 300, workspace=pkg.llmops.Workspace(nbytes, wq.device))
+        assert fc._reads_host(4) == (nbytes == size)
+        assert torch.equal(fc(x), pkg.llmops.fc_Q4A(x.cuda(), wq, 300).cpu())
+
+
 def test_host_fc_results_are_views_of_their_own(pkg):
     """What a caller does to the tensor that a call returned changes no later call's."""
     wq = pkg.llmops.offline_FC_quant_Q4A(torch.randn(96, 512).cuda())
