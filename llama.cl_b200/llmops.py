@@ -639,10 +639,10 @@ def embedding_q8c(output: torch.Tensor, input: torch.Tensor, weight: torch.Tenso
     _front().embedding(input, weight, scales, output)
 
 
-def check_device_status(device: torch.device | None = None) -> None:
+def check_device_status(device: torch.device | str | int | None = None) -> None:
     """Raises if a kernel launched without a workspace on this device reported a failure (a bounded wait that ran
     out, an embedding id outside its table).  Host-synchronous on the current stream."""
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else device
+    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(dev):
         _cabi.check(_cabi.lib().q4fc_fc_check_status(None, _stream_ptr(dev)), "check_device_status")
 

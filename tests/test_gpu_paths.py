@@ -141,6 +141,11 @@ def test_out_of_memory_is_torchs_own_error(pkg):
     assert "Exception raised from" not in str(e.value)
 
 
+@pytest.mark.parametrize("device", [None, 0, "cuda", "cuda:0", torch.device("cuda"), torch.device("cuda", 0)])
+def test_device_forms(pkg, device):
+    pkg.llmops.check_device_status(device)
+
+
 def test_status_word_texts(pkg):
     """The code of a wait that ran out (here: written from the host) is no bad embedding id, whichever letters it has."""
     ws = pkg.llmops.Workspace(4096, torch.device("cuda"))
