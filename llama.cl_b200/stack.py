@@ -195,8 +195,8 @@ class DecodeFCStack:
         been waited for, which ``sync=True`` does)."""
         # A captured token is one native call: input copy, graph launch, wait.  (An ``attention`` callable may hold
         # random-number kernels, whose state only CUDAGraph.replay() advances.)
-        if self._exec is not None and self._front.graph_step(self.x, x, self._exec, self._stream_ptr, self._dev_index, sync,
-                                                               None):
+        if self.use_graph and self._exec is not None and self._front.graph_step(
+                self.x, x, self._exec, self._stream_ptr, self._dev_index, sync, None):
             return self.logits
         with torch.cuda.stream(self.stream):
             if x is not None:

@@ -141,6 +141,25 @@ def test_out_of_memory_is_torchs_own_error(pkg):
     assert "Exception raised from" not in str(e.value)
 
 
+def test_stack_switches_its_graph_off(pkg):
+    """use_graph = False after a captured token: the steps are enqueued one by one, as without a graph from the start."""
+    H, I, V = 128, 256, 96
+    g = torch.Generator().manual_seed(8)
+    pack = lambda N, K: pkg.llmops.offline_FC_quant_Q4A((torch.randn(N, K, generator=g) * 0.02).cuda())
+    layer = {k: pack(*s) for k, s in dict(q=(H, H), k=(H, H), v=(H, H), o=(H, H), gate=(I, H), up=(I, H), down=(H, I)).items()}
+    st = pkg.stack.DecodeFCStack([layer], pack(V, H), hidden=H, intermediate=I, vocab=V)
+    x = torch.randn(1, 1, H, generator=g).cuda()
+    torch.cuda.synchronize()
+    want = st.forward(x, sync=True).clone()
+    assert torch.equal(st.forward(x, sync=True), want)
+    calls, enqueue = [], st.enqueue
+    st.enqueue = lambda: (calls.append(1), enqueue())
+    st.use_graph = False
+    assert torch.equal(st.forward(x, sync=True), want) and calls == [1]
+    st.use_graph = True
+    assert torch.equal(st.forward(x, sync=True), want) and calls == [1]
+
+
 @pytest.mark.parametrize("device", [None, 0, "cuda", "cuda:0", torch.device("cuda"), torch.device("cuda", 0)])
 def test_device_forms(pkg, device):
     pkg.llmops.check_device_status(device)
