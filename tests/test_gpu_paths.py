@@ -41,6 +41,27 @@ def test_host_fc_refuses_unfit_weights(pkg, rows):
                 fc(torch.zeros(1, rows, fc.K))
 
 
+def test_host_fc_in_place_forms(pkg):
+    """The in-place path without a graph, without waiting, on given streams, two at once and as a group."""
+    ops, HostFC = pkg.llmops, pkg.host.HostFC
+    g = torch.Generator().manual_seed(6)
+    shapes = [(300, 1024), (1003, 640)]
+    ws = [ops.offline_FC_quant_Q4A((torch.randn(*s, generator=g) * 0.02).cuda(), qtype="q4_0") for s in shapes]
+    xs = [[torch.randn(1, rows, K, generator=g) for _, K in shapes] for rows in (1, 8, 3, 1)]
+    want = [[ops.fc_Q4A(x.cuda(), w, n).cpu() for x, w, (n, _) in zip(row, ws, shapes)] for row in xs]
+    for graph in (True, False):
+        fcs = [HostFC(w, n, graph=graph, stream=torch.cuda.Stream()) for w, (n, _) in zip(ws, shapes)]
+        for row, ys in zip(xs, want):
+            got = [f(x, sync=False) for f, x in zip(fcs, row)]
+            for f in fcs:
+                f.stream.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(got, ys))
+            assert all(torch.equal(f(x), y) for f, x, y in zip(fcs, row, ys))
+    group = pkg.host.HostFCGroup([HostFC(w, n) for w, (n, _) in zip(ws, shapes)])
+    for row, ys in zip(xs, want):
+        assert all(torch.equal(a, b) for a, b in zip(group(row), ys))
+
+
 def test_host_fc_with_a_small_workspace_copies(pkg):
     """A workspace without room for the quantizer's codes: the kernel would read the host buffer once per cluster, so the
     activations are copied."""
@@ -214,8 +235,24 @@ def test_few_rows_on_the_prefill_path(pkg, rows, qtype, G):
 ])
 @pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "q8c"])
 def test_many_rows_on_tile_edges(pkg, oracle, fmt, rows, N, K):
-    """Both tile sizes and every K split of the tensor-core FC, against the oracle.  At most 2 Kg <= 264 fp32 roundings
-    of 2^-24 on either side of a sum: 2e-5 of its largest value."""
+    """Both tile sizes of the tensor-core FC and K divided by 1, 2, 4 and 8, against the oracle (the other divisions and
+    long K: below).  At most 2 Kg <= 264 fp32 roundings of 2^-24 on either side of a sum, which add up like a random walk:
+    1.4e-6 of its largest value; 2e-5 is a factor of ten and more on top."""
+    check_many_rows(pkg, oracle, fmt, rows, N, K)
+
+
+@pytest.mark.parametrize("rows,N,K", [
+    # 64-row tiles, 148 SMs: 296 places over the column tiles divide K by 3, 5, 6 and 7; 29 stages, the last one group
+    (20, 11000, 3600), (9, 7550, 3600), (9, 6270, 3600), (9, 5370, 3600),
+    (129, 10000, 1184),  # 128-row tiles on every SM: ten stages go around every ring, the last one group
+])
+@pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128", "q8c"])
+def test_many_rows_divisions_and_long_k(pkg, oracle, fmt, rows, N, K):
+    """Clusters that are no power of two, and tiles whose shared-memory rings wrap, in every format."""
+    check_many_rows(pkg, oracle, fmt, rows, N, K)
+
+
+def check_many_rows(pkg, oracle, fmt, rows, N, K):
     g = torch.Generator().manual_seed(rows + N + K)
     W = torch.randn(N, K, generator=g) * 0.02
     x = torch.randn(1, rows, K, generator=g)
@@ -224,13 +261,50 @@ def test_many_rows_on_tile_edges(pkg, oracle, fmt, rows, N, K):
         want = oracle.restated.q8c_fc(x.numpy(), wq, ws, N)
         run = lambda: pkg.c_ext.FC_evaluate_Q8C(x.cuda(), torch.from_numpy(wq).cuda(), torch.from_numpy(ws).cuda(), N)
     else:
-        wq = oracle.restated.pack(W.numpy(), *fmt)
-        want = oracle.restated.fc(x.numpy(), wq, N)
-        run = lambda: pkg.llmops.fc_Q4A(x.cuda(), torch.from_numpy(wq).cuda(), N)
+        signed = isinstance(fmt, str)
+        wq = oracle.restated.pack(W.numpy(), *((0, int(fmt[6:])) if signed else fmt))
+        want = oracle.restated.fc(x.numpy(), wq, N, nibble_signed=signed)
+        run = lambda: pkg.llmops.fc_Q4A(x.cuda(), torch.from_numpy(wq).cuda(), N, nibble_signed=signed)
     got = run()
     assert torch.equal(got, run())  # fixed summation order
     assert np.abs(got.cpu().numpy() - want).max() <= 2e-5 * np.abs(want).max()
     pkg.llmops.check_device_status()
+
+
+@pytest.mark.parametrize("fmt", ["q4", "q8c"])
+def test_many_rows_captured_and_on_two_streams(pkg, fmt):
+    """Calls with both tile sizes on one workspace, captured into a graph and replayed, and beside them eager calls on a
+    second stream: all bit-equal to calls one by one (fixed summation orders)."""
+    ops, N, K = pkg.llmops, 11008, 1056
+    g = torch.Generator(device="cuda").manual_seed(4)
+    W = torch.randn(N, K, generator=g, device="cuda") * 0.02
+    if fmt == "q8c":
+        w, s = pkg.c_ext.FC_quant_Q8C(W)
+        fc = lambda x: ops.FC_evaluate_Q8C(x, w, s, N)
+    else:
+        w = ops.offline_FC_quant_Q4A(W)
+        fc = lambda x: ops.fc_Q4A(x, w, N)
+    inputs = [[torch.randn(1, rows, K, generator=g, device="cuda") for rows in (300, 20, 200)] for _ in range(3)]
+    want = [[fc(x) for x in xs] for xs in inputs]
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    static = [x.clone() for x in inputs[0]]
+    with torch.cuda.stream(a):
+        [fc(x) for x in static]  # the stream's workspace, at its largest
+        a.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=a):
+            outs = [fc(x) for x in static]
+    for xs, ys in zip(inputs, want):
+        with torch.cuda.stream(a):
+            for t, x in zip(static, xs):
+                t.copy_(x)
+            graph.replay()
+        with torch.cuda.stream(b):
+            beside = [fc(x) for x in reversed(inputs[1])]
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, y) for o, y in zip(outs, ys))
+        assert all(torch.equal(o, y) for o, y in zip(beside, reversed(want[1])))
 
 
 @pytest.mark.parametrize("rows,N,K", [
