@@ -4,7 +4,8 @@ and the Python front ``lib/_q4fc_front.so`` from ``csrc/front.cpp``.
 In-tree build.  The library needs nvcc only (no torch headers: it has a plain C
 ABI); each translation unit is compiled to an object in ``build/`` (in
 parallel) and linked with the static CUDA runtime.  The front is host code
-against the headers of the installed torch; it is linked with the library.
+against the headers of the installed torch (g++, Python's and torch's headers);
+it is linked with the library, and built anew when torch is another one.
 """
 from __future__ import annotations
 
@@ -22,6 +23,7 @@ LIB_DIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIB_DIR, "libq4fc_b200.so")
 FRONT_SRC = os.path.join(CSRC, "front.cpp")
 FRONT = os.path.join(LIB_DIR, "_q4fc_front.so")
+FRONT_TORCH = os.path.join(OBJ, "front_torch.txt")  # the torch that FRONT was built against
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
@@ -41,6 +43,19 @@ def _stale(target: str, deps: list[str]) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _torch_build() -> str:
+    import torch
+
+    return f"{torch.__version__} {torch.version.git_version} {os.path.dirname(torch.__file__)}"
+
+
+def front_stale(deps: list[str]) -> bool:
+    if _stale(FRONT, deps) or not os.path.exists(FRONT_TORCH):
+        return True
+    with open(FRONT_TORCH) as f:
+        return f.read() != _torch_build()
 
 
 def front_command() -> list[str]:
@@ -82,8 +97,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-cudart", "static",
                *objs, "-o", LIB]
         subprocess.run(cmd, check=True)
-    if force or _stale(FRONT, [FRONT_SRC, headers[-1]]):
+    if force or front_stale([FRONT_SRC, headers[-1]]):
         subprocess.run(front_command(), check=True)
+        with open(FRONT_TORCH, "w") as f:
+            f.write(_torch_build())
     return LIB
 
 

@@ -29,13 +29,13 @@ def oracle():
 
 @pytest.fixture(scope="session")
 def lib_built():
-    """Make sure the CUDA library exists (compiles it when nvcc is here and it does not)."""
+    """Make sure the CUDA library and the native front exist (compiles them when nvcc is here and they do not)."""
     import importlib.util
 
     path = os.path.join(ROOT, "llama.cl_b200", "build.py")
     spec = importlib.util.spec_from_file_location("_q4fc_build", path)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
-    if not os.path.exists(mod.LIB):
+    if not (os.path.exists(mod.LIB) and os.path.exists(mod.FRONT)):
         mod.build()
     return mod.LIB

@@ -68,6 +68,24 @@ def test_argument_errors_without_gpu(lib_built):
     assert L.q4fc_strerror(4) == b"workspace missing or too small"
 
 
+def test_front_is_rebuilt_for_another_torch(tmp_path):
+    """The front is compiled against torch's headers: it is stale without its source, its target or the same torch."""
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("_q4fc_build", os.path.join(ROOT, "llama.cl_b200", "build.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    src, mod.FRONT, mod.FRONT_TORCH = (str(tmp_path / n) for n in ("front.cpp", "front.so", "front_torch.txt"))
+    open(src, "w").close()
+    assert mod.front_stale([src])
+    open(mod.FRONT, "w").close()
+    assert mod.front_stale([src])
+    for text, stale in ((mod._torch_build(), False), ("2.0.0 x /elsewhere", True)):
+        with open(mod.FRONT_TORCH, "w") as f:
+            f.write(text)
+        assert mod.front_stale([src]) is stale
+
+
 @pytest.mark.parametrize("qtype,G", [(0, 32), (0, 128), (1, 32), (1, 128)])
 def test_workspace_serves_every_path(lib_built, qtype, G):
     """q4fc_fc_workspace_bytes is enough for the prefill entry point at any row count, and never falls as rows grow.
