@@ -29,7 +29,9 @@
 //   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 us   Q4_0 g32, 512 rows 280 -> 223 us (207 TOPS)
 //                   Q4_1 g128, 2048 rows 517 -> 323 us (572 TOPS)   Q8C, 256 rows 296 -> 151 us (153 TOPS)
 // A group of 32 k takes about 1100 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
-// convert, scale is latency-bound with the 16 warps that the registers allow.  Tried and dropped: handing registers
+// convert, scale is latency-bound with the 16 warps that the registers allow (512 rows: issue slots 65 % busy, ALU 46 %, FMA
+// 41 %, XU, where the conversions are not, 0.2 %; per issue 2.2 warps wait for tensor or shared memory, 1.7 for the
+// instruction before).  Tried and dropped: handing registers
 // between roles with setmaxnreg (spills around it; 260 us for the 512-row case), both chunks in registers at once
 // (320 us), the add-a-constant conversion instead of I2F (30 % more issue slots), scalar instead of packed fp32 (5 % slower).
 //

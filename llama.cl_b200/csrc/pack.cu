@@ -5,7 +5,7 @@
 // 0.52-0.63 bytes written per weight.
 //
 // Work split: one thread owns one 32-bit output word = one column n x 8
-// consecutive k (two 128-bit loads).  The G/8 threads that share a (column,
+// consecutive k (one 256-bit load where the rows start on 32 bytes).  The G/8 threads that share a (column,
 // K group) sit in adjacent lanes, so the group minimum / maximum is a
 // segmented warp-shuffle reduction.  The reduction keeps the reference's
 // "first value wins a tie" rule of get_min_max (ops/op_fc.hpp:112-122) by
