@@ -1,5 +1,6 @@
 // FC over many activation rows (prefill): dense int8 contraction on the 5th-generation tensor cores.  Replaces fc_Q4A
-// (ops/op_fc.hpp:286-426) for B*M > 8 and, with FMT = kQ8C, FC_evaluate_Q8C (ext/llama_ext.cpp:232-371).
+// (ops/op_fc.hpp:286-426) for B*M > 8 and, with FMT = kQ8C, FC_evaluate_Q8C (ext/llama_ext.cpp:232-371) where q8c.cu's own
+// kernel has too much to do.
 //
 //   Q4:   y[m][n] = sum_kb  fp32(wd[n,kb]) * xs[m,kb] * I[m,n,kb]  (+ fp32(wm[n,kb]) * gsum[m,kb], Q4_1)
 //   Q8C:  y[m][n] = wscale[n] * sum_kb xs[m,kb] * I[m,n,kb]

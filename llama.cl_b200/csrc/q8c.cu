@@ -1,8 +1,8 @@
 // Per-channel int8 weights ("Q8C"): the FC of the reference's older extension and its quantized embedding table.
 //
 //   FC_quant_Q8C       ext/llama_ext.cpp:56-113    -> q8c_pack_kernel
-//   FC_evaluate_Q8C    ext/llama_ext.cpp:232-371   -> quant_x_kernel<32> (scale 1, no group sums) + q8c_fc_kernel up to
-//                                                     8 rows, the tensor-core GEMM of fc_prefill.cu beyond
+//   FC_evaluate_Q8C    ext/llama_ext.cpp:232-371   -> quant_x_kernel<32> (scale 1, no group sums) + q8c_fc_kernel for few
+//                                                     rows or little work, else the tensor-core GEMM of fc_prefill.cu
 //   embedding_q8c_quant_w   ops/op_embedding.hpp:51-78    -> emb_q8c_quant_kernel
 //   embedding_q8c           ops/op_embedding.hpp:80-137   -> emb_q8c_kernel
 //
@@ -107,36 +107,45 @@ __global__ void __launch_bounds__(256) q8c_pack_kernel(const float* __restrict__
 }
 
 // ---- FC ------------------------------------------------------------------------------------------------------------
-// Up to 8 rows (beyond: the tensor-core GEMM of fc_prefill.cu).  Grid: stripes * split; a cluster of `split` CTAs
-// shares one stripe and divides its K groups.
+// Grid: (stripes * split, row tiles); a cluster of `split` CTAs shares one stripe and divides its K groups.  NT times 8 rows
+// per CTA: the weights are loaded once for all of them.
+template <int NT>
 __global__ void __launch_bounds__(kFcWarps * 32) q8c_fc_kernel(const int8_t* codes, const float* xs, int64_t rows, int64_t Kg,
                                                                const int8_t* __restrict__ wq,
                                                                const float* __restrict__ wscales, int64_t N,
                                                                float* __restrict__ y, int64_t ldy, int split) {
-    __shared__ float part[kFcWarps][8][33];
+    __shared__ float part[kFcWarps][NT][8][33];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int64_t stripe = blockIdx.x / split;
     const int rank = blockIdx.x % split;
+    const int64_t row0 = (int64_t)blockIdx.y * (NT * 8);
     // K groups of this CTA: an even share, the first `rem` ranks one more
     const int64_t share = Kg / split, rem = Kg % split;
     const int64_t kb0 = rank * share + min((int64_t)rank, rem);
     const int64_t kb1 = kb0 + share + (rank < rem ? 1 : 0);
 
-    float acc[4][2];
+    float acc[NT][4][2];
 #pragma unroll
-    for (int c = 0; c < 4; c++) acc[c][0] = acc[c][1] = 0.0f;
+    for (int i = 0; i < NT; i++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc[i][c][0] = acc[i][c][1] = 0.0f;
 
     const int8_t* blk = wq + (stripe * Kg) * 1024 + t * 128 + g * 16;
     // rows whose codes (B fragment: row g) and scales (C fragment: rows 2t, 2t + 1) this lane reads
-    const bool clive = g < rows;
-    const int8_t* crow = codes + (clive ? g : 0) * (Kg * 32) + 4 * t;
-    bool slive[2];
-    const float* srow[2];
+    const int8_t* crow[NT];
+    const float* srow[NT][2];
+    bool clive[NT], slive[NT][2];
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        slive[j] = 2 * t + j < rows;
-        srow[j] = xs + (slive[j] ? 2 * t + j : 0) * Kg;
+    for (int i = 0; i < NT; i++) {
+        const int64_t rb = row0 + i * 8;
+        clive[i] = rb + g < rows;
+        crow[i] = codes + (clive[i] ? rb + g : 0) * (Kg * 32) + 4 * t;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            slive[i][j] = rb + 2 * t + j < rows;
+            srow[i][j] = xs + (slive[i][j] ? rb + 2 * t + j : 0) * Kg;
+        }
     }
 
     // Started beside the quantizer: ask for this warp's first blocks, then wait for the codes (lm_head of one token:
@@ -151,48 +160,64 @@ __global__ void __launch_bounds__(kFcWarps * 32) q8c_fc_kernel(const int8_t* cod
     for (int64_t kb = kb0 + warp; kb < kb1; kb += kFcWarps) {
         const uint4 lo = ldg_stream_v4(blk + kb * 1024);        // block row t: k = 4t..4t+3 of columns 4g..4g+3
         const uint4 hi = ldg_stream_v4(blk + kb * 1024 + 512);  // block row 4 + t: k = 16+4t..
-        uint32_t b0 = 0, b1 = 0;
-        if (clive) {
-            b0 = *reinterpret_cast<const uint32_t*>(crow + kb * 32);
-            b1 = *reinterpret_cast<const uint32_t*>(crow + kb * 32 + 16);
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            uint32_t b0 = 0, b1 = 0;
+            if (clive[i]) {
+                b0 = *reinterpret_cast<const uint32_t*>(crow[i] + kb * 32);
+                b1 = *reinterpret_cast<const uint32_t*>(crow[i] + kb * 32 + 16);
+            }
+            int c01[4] = {0, 0, 0, 0}, c23[4] = {0, 0, 0, 0};
+            mma_s8s8(c01, lo.x, lo.y, hi.x, hi.y, b0, b1);  // columns 4g (c0, c1) and 4g + 1 (c2, c3)
+            mma_s8s8(c23, lo.z, lo.w, hi.z, hi.w, b0, b1);  // columns 4g + 2 and 4g + 3
+            const float d0 = slive[i][0] ? srow[i][0][kb] : 0.0f;
+            const float d1 = slive[i][1] ? srow[i][1][kb] : 0.0f;
+            acc[i][0][0] = fmaf(d0, (float)c01[0], acc[i][0][0]);
+            acc[i][0][1] = fmaf(d1, (float)c01[1], acc[i][0][1]);
+            acc[i][1][0] = fmaf(d0, (float)c01[2], acc[i][1][0]);
+            acc[i][1][1] = fmaf(d1, (float)c01[3], acc[i][1][1]);
+            acc[i][2][0] = fmaf(d0, (float)c23[0], acc[i][2][0]);
+            acc[i][2][1] = fmaf(d1, (float)c23[1], acc[i][2][1]);
+            acc[i][3][0] = fmaf(d0, (float)c23[2], acc[i][3][0]);
+            acc[i][3][1] = fmaf(d1, (float)c23[3], acc[i][3][1]);
         }
-        int c01[4] = {0, 0, 0, 0}, c23[4] = {0, 0, 0, 0};
-        mma_s8s8(c01, lo.x, lo.y, hi.x, hi.y, b0, b1);  // columns 4g (c0, c1) and 4g + 1 (c2, c3)
-        mma_s8s8(c23, lo.z, lo.w, hi.z, hi.w, b0, b1);  // columns 4g + 2 and 4g + 3
-        const float d0 = slive[0] ? srow[0][kb] : 0.0f;
-        const float d1 = slive[1] ? srow[1][kb] : 0.0f;
-        acc[0][0] = fmaf(d0, (float)c01[0], acc[0][0]);
-        acc[0][1] = fmaf(d1, (float)c01[1], acc[0][1]);
-        acc[1][0] = fmaf(d0, (float)c01[2], acc[1][0]);
-        acc[1][1] = fmaf(d1, (float)c01[3], acc[1][1]);
-        acc[2][0] = fmaf(d0, (float)c23[0], acc[2][0]);
-        acc[2][1] = fmaf(d1, (float)c23[1], acc[2][1]);
-        acc[3][0] = fmaf(d0, (float)c23[2], acc[3][0]);
-        acc[3][1] = fmaf(d1, (float)c23[3], acc[3][1]);
     }
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-        part[warp][2 * t][4 * g + c] = acc[c][0];
-        part[warp][2 * t + 1][4 * g + c] = acc[c][1];
-    }
+    for (int i = 0; i < NT; i++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            part[warp][i][2 * t][4 * g + c] = acc[i][c][0];
+            part[warp][i][2 * t + 1][4 * g + c] = acc[i][c][1];
+        }
     __syncthreads();
-    // one thread per (row, column): the warps' sums in order
+    // one thread per (row of every 8, column): the warps' sums in order
     const int m = warp, c = lane;
     const int64_t n = stripe * 32 + c;
-    float s = part[0][m][c];
+    float s[NT];
 #pragma unroll
-    for (int w2 = 1; w2 < kFcWarps; w2++) s += part[w2][m][c];
+    for (int i = 0; i < NT; i++) {
+        s[i] = part[0][i][m][c];
+#pragma unroll
+        for (int w2 = 1; w2 < kFcWarps; w2++) s[i] += part[w2][i][m][c];
+    }
     if (split > 1) {
-        part[0][m][c] = s;
         cg::cluster_group cluster = cg::this_cluster();
+#pragma unroll
+        for (int i = 0; i < NT; i++) part[0][i][m][c] = s[i];
         cluster.sync();
-        if (rank == 0) {
-            for (int r = 1; r < split; r++) s += *cluster.map_shared_rank(&part[0][m][c], r);
-            if (m < rows && n < N) y[m * ldy + n] = __fmul_rn(__ldg(wscales + n), s);
-        }
+        if (rank == 0)
+            for (int r = 1; r < split; r++)
+#pragma unroll
+                for (int i = 0; i < NT; i++) s[i] += *cluster.map_shared_rank(&part[0][i][m][c], r);
         cluster.sync();  // the other CTAs' shared memory stays alive until rank 0 has read it
-    } else if (m < rows && n < N) {
-        y[m * ldy + n] = __fmul_rn(__ldg(wscales + n), s);
+    }
+    if (rank == 0 && n < N) {
+        const float ws = __ldg(wscales + n);
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            const int64_t row = row0 + i * 8 + m;
+            if (row < rows) y[row * ldy + n] = __fmul_rn(ws, s[i]);
+        }
     }
 }
 
@@ -290,20 +315,26 @@ int launch_q8c_fc(const float* x, int64_t rows, int64_t K, int64_t ldx, const in
     if (!di) return Q4FC_ECUDA;
     int8_t* codes = static_cast<int8_t*>(ws);
     float* xs = reinterpret_cast<float*>(static_cast<char*>(ws) + align_up((size_t)(rows * Kg * 32), 256));
-    // the kernel below holds 8 rows; with more of them in a CTA, on mma.sync, 256 rows x 4096 x 11008 took 296 us
-    // (the tensor-core GEMM: 151 us)
-    if (rows > 8) return launch_q8c_prefill(x, rows, K, ldx, wq, wscales, Ng, Kg, N, y, ldy, codes, xs, s);
-    if (int rc = launch_quant_x(x, rows, K, ldx, 32, 1.0f, codes, xs, nullptr, s)) return rc;
     const int64_t stripes = (N + 31) / 32;
+    const int nt = rows <= 8 ? 1 : rows <= 16 ? 2 : 4;
+    const int64_t tiles = (rows + 8 * nt - 1) / (8 * nt);
     // few stripes: a cluster of CTAs shares each one, until the grid holds about two CTAs per SM
     int split = 1;
     while (split < kMaxSplit && stripes * split < 2 * (int64_t)di->sm_count && Kg / (2 * split) >= kFcWarps) split *= 2;
+    // The tensor-core GEMM takes over beyond 16 rows as soon as this kernel's CTAs no longer find a place all at once, two
+    // on an SM (96 rows x 512 x 512: 5 us here, 12 there; 512 x 4096: 22 and 12; 256 x 4096 x 11008: 296 and 151).  Over 819
+    // sizes (K and N from 512 to 11008 and 30000, 17 to 128 rows) that line costs 0.6 % against the better of the two.  Up to
+    // 16 rows the weight stream decides and this kernel is ahead, with 16 rows in a CTA (9 x 4096 x 4096: 12 us, GEMM 15; 9 x
+    // 11008 x 30000: 108 and 148; behind only at 13 to 16 rows x 11008 columns, 27 and 25 at K = 4096).
+    if (rows > 16 && stripes * split * tiles > 2 * (int64_t)di->sm_count)
+        return launch_q8c_prefill(x, rows, K, ldx, wq, wscales, Ng, Kg, N, y, ldy, codes, xs, s);
+    if (int rc = launch_quant_x(x, rows, K, ldx, 32, 1.0f, codes, xs, nullptr, s)) return rc;
     if (stripes * split > 0x7fffffffLL) {
         set_error("q8c_fc: %lld columns exceed the grid limit", (long long)N);
         return Q4FC_ELIMIT;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(stripes * split));
+    cfg.gridDim = dim3((unsigned)(stripes * split), (unsigned)tiles);
     cfg.blockDim = dim3(kFcWarps * 32);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -317,7 +348,8 @@ int launch_q8c_fc(const float* x, int64_t rows, int64_t K, int64_t ldx, const in
     cfg.numAttrs = 2;
     const int8_t* ccodes = codes;
     const float* cxs = xs;
-    Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, q8c_fc_kernel, ccodes, cxs, rows, Kg, wq, wscales, N, y, ldy, split));
+    auto* fn = nt == 1 ? q8c_fc_kernel<1> : nt == 2 ? q8c_fc_kernel<2> : q8c_fc_kernel<4>;
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, fn, ccodes, cxs, rows, Kg, wq, wscales, N, y, ldy, split));
     return Q4FC_OK;
 }
 

@@ -17,7 +17,7 @@
 // resident warps hide that serial chain.  The decode FC kernel has its own
 // fused copy of this arithmetic (tree-ordered sums), the prefill path its own
 // kernel below; this one serves callers that want the quantized activations
-// themselves and the per-channel int8 FC of up to 8 rows.
+// themselves and the per-channel int8 FC on mma.sync (q8c.cu).
 #include "common.cuh"
 
 namespace q4fc {

@@ -243,7 +243,7 @@ def test_many_rows_on_tile_edges(pkg, oracle, fmt, rows, N, K):
 
 @pytest.mark.parametrize("rows,N,K", [
     # 64-row tiles, 148 SMs: 296 places over the column tiles divide K by 3, 5, 6 and 7; 29 stages, the last one group
-    (20, 11000, 3600), (9, 7550, 3600), (9, 6270, 3600), (9, 5370, 3600),
+    (20, 11000, 3600), (17, 7550, 3600), (17, 6270, 3600), (17, 5370, 3600),
     (129, 10000, 1184),  # 128-row tiles on every SM: ten stages go around every ring, the last one group
 ])
 @pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128", "q8c"])
@@ -269,6 +269,15 @@ def check_many_rows(pkg, oracle, fmt, rows, N, K):
     assert torch.equal(got, run())  # fixed summation order
     assert np.abs(got.cpu().numpy() - want).max() <= 2e-5 * np.abs(want).max()
     pkg.llmops.check_device_status()
+
+
+@pytest.mark.parametrize("rows,N,K", [
+    (8, 200, 520), (9, 200, 520), (16, 200, 520), (17, 200, 520), (32, 200, 520), (33, 200, 520),  # 1, 2 and 4 row tiles
+    (16, 9500, 100), (17, 9500, 100),   # 297 stripes: two places on each of 148 SMs hold one CTA less
+    (17, 9470, 100), (128, 1180, 250), (129, 1180, 250),  # as many CTAs as places; a row tile more
+])
+def test_q8c_row_tiles_and_the_line_to_the_gemm(pkg, oracle, rows, N, K):
+    check_many_rows(pkg, oracle, "q8c", rows, N, K)
 
 
 @pytest.mark.parametrize("fmt", ["q4", "q8c"])
@@ -313,7 +322,7 @@ def test_many_rows_captured_and_on_two_streams(pkg, fmt):
     (129, 10000, 11008),
     (37, 11008, 4096),                # 64-row tiles, K divided by 3
     (512, 4096, 11008),               # undivided
-    (17, 200, 1000), (9, 700, 4097),  # divided further
+    (17, 5000, 1000), (40, 2000, 4097),  # divided by 2 and 8
 ])
 def test_q8c_many_rows_precision(pkg, rows, N, K):
     """The sums over K against 64 bits on the same codes and scales.  A rounding to nearest is off by 2.5e-8 of its sum in
