@@ -4,15 +4,22 @@
 // W[N][K] -> int8 [Ng][Kg][BS].  HBM-bound streaming kernel: 4 bytes read and
 // 0.52-0.63 bytes written per weight.
 //
-// Work split: one thread owns one 32-bit output word = one column n x 8
-// consecutive k (one 256-bit load where the rows start on 32 bytes).  The G/8 threads that share a (column,
+// Work split: one thread owns two 32-bit output words = one column n x 16
+// consecutive k (two 256-bit loads where the rows start on 32 bytes).  The G/16 threads that share a (column,
 // K group) sit in adjacent lanes, so the group minimum / maximum is a
-// segmented warp-shuffle reduction.  The reduction keeps the reference's
+// segmented warp-shuffle reduction.  A CTA stages a tile of 32 columns x 256 k of packed output in
+// shared memory and writes it out with 128-bit stores.
+//
+// What bounds it: issue slots, then HBM.  One word per thread and one path for all values took 22 warp instructions per 32
+// weights; the instructions a group costs (shuffles, scale and its reciprocal, addresses) are now shared by 16 weights of a
+// thread, and full groups of ordinary finite values take a path without clamps and float-to-int conversions.
+// 11008 x 4096, Q4_1 group 128: 45.3 -> 36.8 us (5.5 TB/s).
+//
+// General path: the reduction keeps the reference's
 // "first value wins a tie" rule of get_min_max (ops/op_fc.hpp:112-122) by
 // always combining an earlier k range (left) with a later one (right) under
 // the same strict compares, which matters only for the sign of a zero
-// minimum.  A CTA stages a tile of 32 columns x 256 k of packed output in
-// shared memory and writes it out with 128-bit stores.
+// minimum.
 //
 // Arithmetic is the reference's, in fp32 with IEEE division: Q4_1
 // d=(max-min)/15, m=min, q=clamp(roundf((w-m)/d'),0,15) with d'=1/d computed
@@ -36,92 +43,132 @@ __device__ __forceinline__ void mm_take(MinMax& a, float v) {  // sequential ste
     if (a.vmin > v) a.vmin = v;
 }
 
-// 256-bit load (sm_100): a lane's eight weights in one request, 32-byte aligned (as two 128-bit loads each request
-// uses half of the sectors that it touches: 11008 x 4096, Q4_1 group 128, 46.7 us, now 45.2)
-__device__ __forceinline__ void ldg_v8(const float* p, float (&v)[8]) {
+// 256-bit load (sm_100), 32-byte aligned
+__device__ __forceinline__ void ldg_v8(const float* p, float* v) {
     asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                  : "l"(p));
 }
+// of three values (sm_100); NaN if one of them is
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float scale_of(int qtype, float vmin, float vmax) {
+    return qtype == 1 ? div_const_rn(__fsub_rn(vmax, vmin), 15.0f, 1.0f / 15.0f)
+                      : div_const_rn(fmaxf(fabsf(vmin), fabsf(vmax)), 7.0f, 1.0f / 7.0f);
+}
+// where code j of a word goes: byte (j&3), low nibble for j<4, high nibble for j>=4 (ops/op_fc.hpp:39-48)
+__host__ __device__ constexpr uint32_t place(int j) { return 1u << (8 * (j & 3) + 4 * (j >> 2)); }
+
+// Eight codes of values whose group has a scale between 2^-100 and 2^100: no clamp is needed, |w - m| / d and |w| / d exceed 15
+// and 7 by a few roundings at most.  The words are sums: nibbles do not overlap, a multiply-add places a code.
+template <int QTYPE>
+__device__ __forceinline__ uint32_t codes_of(const float* v, float m, float id) {
+    uint32_t word;
+    if (QTYPE == 1) {
+        // t >= 0: roundf is trunc(t + 0.5) with the add rounded toward zero; adding 2^23, rounded the same way, leaves the
+        // integer in the low bits (0x4B000000 above it, whose multiples the start value takes off again)
+        word = 0u - (0x4B000000u * place(0) + 0x4B000000u * place(4));
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const float t = __fmul_rn(__fsub_rn(v[j], m), id);
+            word += __float_as_uint(__fadd_rz(__fadd_rz(t, 0.5f), 8388608.0f)) * place(j);
+        }
+    } else {
+        word = 0x88888888u;  // code + 8 in every nibble, so that no borrow crosses
+#pragma unroll
+        for (int j = 0; j < 8; j++) word += (uint32_t)round_half_away(__fmul_rn(v[j], id)) * place(j);
+        word ^= 0x88888888u;
+    }
+    return word;
+}
+
+constexpr int kPerThread = 16;                    // consecutive k of a thread
+constexpr int kRowWords = 36;                     // staged block rows: 32 words and a gap, against bank conflicts
 
 template <int G, int QTYPE>
 __global__ void __launch_bounds__(kPackThreads) pack_kernel(const float* __restrict__ w, int64_t N, int64_t K,
                                                             int64_t Kg, int tiles_k, int vec_ok,
                                                             uint8_t* __restrict__ out) {
     constexpr int BS = block_bytes(QTYPE, G);
-    constexpr int SEG = G / 8;              // lanes sharing one (column, group)
+    constexpr int SEG = G / kPerThread;     // lanes sharing one (column, group)
     constexpr int NPW = 32 / SEG;           // columns per warp step
     constexpr int GB = kTileK / G;          // groups per CTA tile
-    constexpr int UNITS = GB * (32 / NPW);  // warp steps per tile
-    constexpr int ITERS = UNITS / (kPackThreads / 32);
-    static_assert(UNITS % (kPackThreads / 32) == 0, "tile must divide among the warps");
+    constexpr int STEPS = 32 / NPW;         // warp steps per group: the columns
+    constexpr int WARPS = kPackThreads / 32;
+    constexpr int ITERS = GB * STEPS / WARPS;
+    constexpr int STAGE = (G / 8 + 1) * kRowWords;  // words of a staged block: its rows, then scales (and minima)
+    static_assert(ITERS == 2 && WARPS % STEPS == 0, "a warp keeps its columns and moves on by half a tile");
 
-    __shared__ __align__(16) uint32_t stage[GB * BS / 4];
+    __shared__ __align__(16) uint32_t stage[GB * STAGE];
 
     const int64_t nb = blockIdx.x / tiles_k;
     const int tile = blockIdx.x % tiles_k;
     const int64_t kb0 = (int64_t)tile * GB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seg_lane = lane % SEG;  // = k8 inside the group
+    const int seg_lane = lane % SEG;
+    const int n_l = (warp % STEPS) * NPW + lane / SEG;
+    const int64_t n = nb * 32 + n_l;
 
-    float v[ITERS][8];
-    int nvalid[ITERS];  // valid elements of this thread's 8 (prefix), -1: column beyond N
-
+    float v[ITERS][kPerThread];
+    int nvalid[ITERS];  // valid elements of this thread's (prefix), -1: column beyond N, or group beyond Kg
 #pragma unroll
     for (int it = 0; it < ITERS; it++) {
-        const int u = warp + it * (kPackThreads / 32);
-        const int kb_l = u / (32 / NPW);
-        const int n_l = (u % (32 / NPW)) * NPW + lane / SEG;
-        const int64_t n = nb * 32 + n_l;
-        const int64_t k = (kb0 + kb_l) * G + seg_lane * 8;
-        int cnt = -1;
-        if (n < N && kb0 + kb_l < Kg) {
-            cnt = (int)min((int64_t)8, max((int64_t)0, K - k));
-            const float* src = w + n * K + k;
-            if (cnt == 8 && vec_ok == 2) {
-                ldg_v8(src, v[it]);
-            } else if (cnt == 8 && vec_ok) {
-                float4 a = __ldg(reinterpret_cast<const float4*>(src));
-                float4 b = __ldg(reinterpret_cast<const float4*>(src) + 1);
-                v[it][0] = a.x, v[it][1] = a.y, v[it][2] = a.z, v[it][3] = a.w;
-                v[it][4] = b.x, v[it][5] = b.y, v[it][6] = b.z, v[it][7] = b.w;
-            } else {
+        const int64_t kb = kb0 + warp / STEPS + it * (GB / ITERS);
+        const int64_t k = kb * G + seg_lane * kPerThread;
+        const float* src = w + n * K + k;
+        const int cnt = (n < N && kb < Kg) ? (int)min((int64_t)kPerThread, max((int64_t)0, K - k)) : -1;
+        if (cnt == kPerThread && vec_ok == 2) {
+            ldg_v8(src, v[it]);
+            ldg_v8(src + 8, v[it] + 8);
+        } else if (cnt == kPerThread && vec_ok) {
 #pragma unroll
-                for (int j = 0; j < 8; j++) v[it][j] = (j < cnt) ? __ldg(src + j) : 0.0f;
+            for (int i = 0; i < kPerThread / 4; i++) {
+                const float4 a = __ldg(reinterpret_cast<const float4*>(src) + i);
+                v[it][4 * i] = a.x, v[it][4 * i + 1] = a.y, v[it][4 * i + 2] = a.z, v[it][4 * i + 3] = a.w;
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; j++) v[it][j] = 0.0f;
+            for (int j = 0; j < kPerThread; j++) v[it][j] = (j < cnt) ? __ldg(src + j) : 0.0f;
         }
         nvalid[it] = cnt;
     }
 
 #pragma unroll
     for (int it = 0; it < ITERS; it++) {
-        const int u = warp + it * (kPackThreads / 32);
-        const int kb_l = u / (32 / NPW);
-        const int n_l = (u % (32 / NPW)) * NPW + lane / SEG;
+        const int kb_l = warp / STEPS + it * (GB / ITERS);
         const int cnt = nvalid[it];
-
-        // Fast path (whole warp has 8 valid values per lane): plain min / max and an xor butterfly.
-        // The value of a minimum / maximum does not depend on the scan order; only the SIGN of a zero
-        // does (get_min_max keeps the first of equal values), so when any lane of the warp ends up with
-        // a zero minimum or maximum, or values are missing, the warp redoes the reduction in order.
-        float vmin = v[it][0], vmax = v[it][0];
+        const float* x = v[it];
+        float vmin = min3(x[0], x[1], x[2]), vmax = max3(x[0], x[1], x[2]);
 #pragma unroll
-        for (int j = 1; j < 8; j++) vmin = fminf(vmin, v[it][j]), vmax = fmaxf(vmax, v[it][j]);
+        for (int j = 3; j + 1 < kPerThread; j += 2) vmin = min3(vmin, x[j], x[j + 1]), vmax = max3(vmax, x[j], x[j + 1]);
+        vmin = min3(vmin, x[15], x[15]), vmax = max3(vmax, x[15], x[15]);
 #pragma unroll
         for (int off = 1; off < SEG; off <<= 1) {
-            vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, off));
-            vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, off));
+            const float a = __shfl_xor_sync(0xffffffffu, vmin, off), b = __shfl_xor_sync(0xffffffffu, vmax, off);
+            vmin = min3(vmin, a, a), vmax = max3(vmax, b, b);
         }
-        if (__any_sync(0xffffffffu, cnt != 8 || vmin == 0.0f || vmax == 0.0f)) {
+        float d = scale_of(QTYPE, vmin, vmax);
+        uint32_t word[2];
+        // (the value of a minimum does not depend on the order of the scan, only the sign of a zero does)
+        if (__all_sync(0xffffffffu, cnt == kPerThread && vmin != 0.0f && vmax != 0.0f && d >= 0x1p-100f && d <= 0x1p100f)) {
+            const float id = __frcp_rn(d);
+            word[0] = codes_of<QTYPE>(x, vmin, id), word[1] = codes_of<QTYPE>(x + 8, vmin, id);
+        } else {
+            // missing values, zeros as extremes, NaN, infinities, scales near the ends of the range
             MinMax mm;
             mm.has = cnt > 0;
-            mm.vmin = mm.vmax = v[it][0];
+            mm.vmin = mm.vmax = x[0];
 #pragma unroll
-            for (int j = 1; j < 8; j++)
-                if (j < cnt) mm_take(mm, v[it][j]);
+            for (int j = 1; j < kPerThread; j++)
+                if (j < cnt) mm_take(mm, x[j]);
             // ordered segmented reduction: lane i absorbs lane i+off (later k)
 #pragma unroll
             for (int off = 1; off < SEG; off <<= 1) {
@@ -135,52 +182,41 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(const float* __restr
             }
             vmin = __shfl_sync(0xffffffffu, mm.vmin, 0, SEG);
             vmax = __shfl_sync(0xffffffffu, mm.vmax, 0, SEG);
-        }
-
-        float d, m, id;
-        if (QTYPE == 1) {
-            d = div_const_rn(__fsub_rn(vmax, vmin), 15.0f, 1.0f / 15.0f);
-            m = vmin;
-        } else {
-            d = div_const_rn(fmaxf(fabsf(vmin), fabsf(vmax)), 7.0f, 1.0f / 7.0f);
-            m = 0.0f;
-        }
-        id = inv_or_zero(d);
-
-        uint32_t word = 0;
-        if (cnt >= 0) {
+            d = scale_of(QTYPE, vmin, vmax);
+            const float id = inv_or_zero(d);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                if (j < cnt) {
-                    // byte (j&3), low nibble for j<4, high nibble for j>=4 (ops/op_fc.hpp:39-48)
-                    const uint32_t place = 1u << (8 * (j & 3) + 4 * (j >> 2));
-                    if (QTYPE == 1) {
-                        // (w - m) * id >= 0: roundf is trunc(t + 0.5) with the add rounded toward zero; clamp at 15
-                        const float t = __fmul_rn(__fsub_rn(v[it][j], m), id);
-                        const uint32_t q = (uint32_t)min(15, __float2int_rz(__fadd_rz(t, 0.5f)));
-                        word += q * place;  // nibbles do not overlap: a multiply-add places the code
-                    } else {
-                        const int q = min(7, max(round_half_away(__fmul_rn(v[it][j], id)), -7));
-                        word += (uint32_t)(q & 0xF) * place;
+            for (int h = 0; h < 2; h++) {
+                word[h] = 0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    if (8 * h + j < cnt) {
+                        const float e = x[8 * h + j];
+                        const int q = QTYPE == 1 ? min(15, __float2int_rz(__fadd_rz(__fmul_rn(__fsub_rn(e, vmin), id), 0.5f)))
+                                                 : min(7, max(round_half_away(__fmul_rn(e, id)), -7)) & 0xF;
+                        word[h] += (uint32_t)q * place(j);
                     }
                 }
             }
         }
-        stage[kb_l * (BS / 4) + seg_lane * 32 + n_l] = word;
+        uint32_t* block = stage + kb_l * STAGE;
+        block[(2 * seg_lane) * kRowWords + n_l] = word[0];
+        block[(2 * seg_lane + 1) * kRowWords + n_l] = word[1];
         if (seg_lane == 0) {
-            uint16_t* tail = reinterpret_cast<uint16_t*>(stage + kb_l * (BS / 4) + G * 4);
+            uint16_t* tail = reinterpret_cast<uint16_t*>(block + (G / 8) * kRowWords);
             const bool live = cnt >= 0;  // cnt==0 cannot occur at seg_lane 0 of an existing group
             tail[n_l] = live ? f2h_rn(d) : (uint16_t)0;
-            if (QTYPE == 1) tail[32 + n_l] = live ? f2h_rn(m) : (uint16_t)0;
+            if (QTYPE == 1) tail[32 + n_l] = live ? f2h_rn(vmin) : (uint16_t)0;
         }
     }
     __syncthreads();
 
-    const int groups_here = (int)min((int64_t)GB, Kg - kb0);
-    const int n16 = groups_here * BS / 16;
+    constexpr int N16 = BS / 16;  // 16-byte pieces of a block, eight to a staged row
+    const int n16 = (int)min((int64_t)GB, Kg - kb0) * N16;
     uint4* dst = reinterpret_cast<uint4*>(out + (nb * Kg + kb0) * (int64_t)BS);
-    const uint4* src4 = reinterpret_cast<const uint4*>(stage);
-    for (int i = threadIdx.x; i < n16; i += kPackThreads) dst[i] = src4[i];
+    for (int i = threadIdx.x; i < n16; i += kPackThreads) {
+        const int kb_l = i / N16, o = i % N16;
+        dst[i] = *reinterpret_cast<const uint4*>(stage + kb_l * STAGE + (o >> 3) * kRowWords + (o & 7) * 4);
+    }
 }
 
 template <int G, int QTYPE>

@@ -367,3 +367,20 @@ def test_pack_load_widths(pkg, oracle, qtype, G, K, offset):
     w.copy_(W)
     got = pkg.llmops.offline_FC_quant_Q4A(w, qtype="q4_1" if qtype else "q4_0", group_k=G)
     assert np.array_equal(got.cpu().numpy(), oracle.restated.pack(W.numpy(), qtype, G))
+
+
+@pytest.mark.parametrize("qtype,G", [(0, 32), (0, 128), (1, 32), (1, 128)])
+@pytest.mark.parametrize("N,K", [(64, 512), (33, 520), (40, 516), (37, 515)])  # 32-, 16- and 4-byte loads; a column beyond N
+def test_pack_scales_at_the_ends(pkg, oracle, qtype, G, N, K):
+    """Groups on both sides of the scales between which the packer clamps nothing, in warps of ordinary ones; ties of the
+    rounding (the values are multiples of half a step).  Bytes, so no tolerance."""
+    g = torch.Generator().manual_seed(N * 7 + K + G)
+    W = torch.randint(-14, 15, (N, K), generator=g).float() * 0.5
+    # (where 1 / scale is infinite, what the reference's conversion to int makes of that is not defined)
+    for row, scale in enumerate((2.0**-122, 2.0**-118, 2.0**-106, 2.0**-103, 2.0**-100, 2.0**-97, 2.0**97, 2.0**100, 2.0**103, 2.0**123)):
+        W[row] *= scale
+    W[10] = W[10].abs() + 1.0   # no zero among the extremes
+    W[11, : K // 2] = 3.25      # equal values: scale 0 (Q4_1)
+    want = oracle.restated.pack(W.numpy(), qtype, G)
+    got = pkg.llmops.offline_FC_quant_Q4A(W.cuda(), qtype=("q4_0", "q4_1")[qtype], group_k=G).cpu().numpy()
+    assert np.array_equal(got, want)
