@@ -56,10 +56,10 @@ enum {
      * reference reads it unsigned (ops/op_fc.hpp:95-106, 364-376) and parity
      * is defined against that. */
     Q4FC_FLAG_NIBBLE_SIGNED = 1u,
-    /* Launch with programmatic stream serialization: the kernel may start
-     * while its predecessor on the stream drains; it touches activations,
-     * outputs and workspace only after the predecessor has completed, and
-     * streams weights before that.  Use only when the predecessor does not
+    /* Stream weights while the predecessor on the stream drains.  (Calls may
+     * start before their predecessor has completed in any case; without this
+     * flag they touch no memory before it has, with it only activations,
+     * outputs and workspace wait.)  Use only when the predecessor does not
      * write this call's weights. */
     Q4FC_FLAG_PDL = 2u,
     /* q4fc_fc_decode only: use the stream-K kernel (one contiguous byte run

@@ -127,6 +127,21 @@ size_t q8c_prefill_scale_bytes(int64_t rows, int64_t Kg);
 int launch_q8c_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, const int8_t* wq, const float* wscales,
                        int64_t Ng, int64_t Kg, int64_t N, float* y, int64_t ldy, int8_t* codes, float* sc, cudaStream_t s);
 
+// A launch that may begin before the kernel in front of it has ended: the kernel waits (pdl_wait_prior_grid) before it touches
+// global memory, and lets its own successor begin only after that wait, so that a successor which begins early finds everything
+// in front of this kernel complete.
+struct DependentLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    DependentLaunch(dim3 grid, unsigned threads, cudaStream_t s) {
+        cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.stream = s;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attr, cfg.numAttrs = 1;
+    }
+    DependentLaunch(const DependentLaunch&) = delete;
+};
+
 #ifdef __CUDACC__
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 __device__ __forceinline__ uint16_t f2h_rn(float f) { return __half_as_ushort(__float2half_rn(f)); }
@@ -166,6 +181,17 @@ __device__ __forceinline__ uint2 ldg_stream_v2(const void* p) {
 // programmatic dependent launch: both are no-ops when the kernel was launched
 // without the programmatic-serialization attribute
 __device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of what the kernel in front may have written: never moved above pdl_wait_prior_grid().
+__device__ __forceinline__ float ld_after_wait(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_after_wait(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 

@@ -258,8 +258,10 @@ __global__ void __launch_bounds__(128) emb_q8c_kernel(const Tidx* __restrict__ i
                                                       const float* __restrict__ scales, int64_t V, int64_t E,
                                                       float* __restrict__ out, int64_t ldo, int vec_ok,
                                                       int* __restrict__ status) {
+    pdl_wait_prior_grid();
+    pdl_launch_dependents();
     const int64_t i = blockIdx.x;
-    const int64_t id = (int64_t)ids[i];
+    const int64_t id = (int64_t)*const_cast<const volatile Tidx*>(ids + i);  // (not read above the wait; nor is what it leads to)
     float* dst = out + i * ldo;
     if (id < 0 || id >= V) {
         for (int64_t k = threadIdx.x; k < E; k += 128) dst[k] = 0.0f;
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(128) emb_q8c_kernel(const Tidx* __restrict__ i
         return;
     }
     const int8_t* src = codes + id * E;
-    const float s = __ldg(scales + id);
+    const float s = ld_after_wait(scales + id);
     if (vec_ok) {
 #pragma unroll 8
         for (int64_t k = (int64_t)threadIdx.x * 4; k < E; k += 128 * 4) {
@@ -374,13 +376,13 @@ int launch_emb_q8c(const void* ids, int ids_are_i32, int64_t n, const int8_t* co
     const int vec_ok = (E % 4 == 0) && (ldo % 4 == 0) && ((reinterpret_cast<uintptr_t>(codes) & 3) == 0) &&
                        ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
     int* status = ring_status_word();
+    DependentLaunch l(dim3((unsigned)n), 128, s);
     if (ids_are_i32)
-        emb_q8c_kernel<int32_t><<<(unsigned)n, 128, 0, s>>>(static_cast<const int32_t*>(ids), codes, scales, V, E, out,
-                                                            ldo, vec_ok, status);
+        Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, emb_q8c_kernel<int32_t>, static_cast<const int32_t*>(ids), codes, scales, V, E, out,
+                                        ldo, vec_ok, status));
     else
-        emb_q8c_kernel<int64_t><<<(unsigned)n, 128, 0, s>>>(static_cast<const int64_t*>(ids), codes, scales, V, E, out,
-                                                            ldo, vec_ok, status);
-    Q4FC_CUDA_OK(cudaGetLastError());
+        Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, emb_q8c_kernel<int64_t>, static_cast<const int64_t*>(ids), codes, scales, V, E, out,
+                                        ldo, vec_ok, status));
     return Q4FC_OK;
 }
 

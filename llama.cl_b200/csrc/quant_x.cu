@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_kernel(const float* __r
     constexpr int PADG = G + 1;    // padded group pitch in shared memory
     __shared__ float raw[kQxWarps][GPC * PADG + 3];
 
+    pdl_wait_prior_grid();
     pdl_launch_dependents();  // (an FC launched for it starts beside this kernel and waits for its results)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t chunks = (Kg * G + 127) / 128;
@@ -49,11 +50,11 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_kernel(const float* __r
 
     float v[4];
     if (vec_ok && k + 4 <= K) {
-        float4 a = __ldg(reinterpret_cast<const float4*>(src));
+        float4 a = ld_after_wait(reinterpret_cast<const float4*>(src));
         v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
     } else {
 #pragma unroll
-        for (int j = 0; j < 4; j++) v[j] = (k + j < K) ? __ldg(src + j) : 0.0f;
+        for (int j = 0; j < 4; j++) v[j] = (k + j < K) ? ld_after_wait(src + j) : 0.0f;
     }
 
     const int g_l = lane / SEG;              // group inside the chunk
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_tile_kernel(const float
                                                                      float* __restrict__ sc) {
     constexpr int SEG = G / 4;    // lanes per group
     constexpr int GPC = 128 / G;  // groups per 128-k chunk
+    pdl_wait_prior_grid();
     pdl_launch_dependents();      // the GEMM's weight copies run beside this launch
     const int lane = threadIdx.x & 31;
     const int64_t row_sets = (rows + kQxWarps - 1) / kQxWarps;
@@ -130,12 +132,12 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_tile_kernel(const float
     const float* src = x + row * ldx + k;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     if (vec_ok && k + 4 <= K) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(src));
+        const float4 a = ld_after_wait(reinterpret_cast<const float4*>(src));
         v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
     } else {
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            if (k + j < K) v[j] = __ldg(src + j);
+            if (k + j < K) v[j] = ld_after_wait(src + j);
     }
     const int64_t kb = c * GPC + lane / SEG;
     const bool exists = kb < Kg;
@@ -363,7 +365,7 @@ int launch_quant_x_pre_batch(const q4fc_xq_call* calls, int n, int G, bool want_
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;  // (it waits before it reads, and without `pdl` releases the FC only after that)
     if (G == 32)
         Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_x_pre_batch_kernel<32>, b, (int)want_isum, (int)pdl));
     else
@@ -391,7 +393,7 @@ int launch_quant_x_pre(const float* x, int rows, int64_t K, int64_t ldx, int G, 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = 1;  // (it waits before it reads, and without `pdl` releases the FC only after that)
     if (G == 32)
         Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_x_pre_kernel<32>, x, rows, K, ldx, Kg, vec_ok, (int)want_isum,
                                         (int)pdl, codes, sc, up, prod, ldp));
@@ -412,11 +414,9 @@ int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, in
     }
     const int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const int l2 = tile == 128 ? 7 : 6;
-    if (G == 32)
-        quant_x_tile_kernel<32><<<(unsigned)grid, kQxWarps * 32, 0, s>>>(x, rows, K, ldx, Kg, vec_ok, sums, l2, codes, sc);
-    else
-        quant_x_tile_kernel<128><<<(unsigned)grid, kQxWarps * 32, 0, s>>>(x, rows, K, ldx, Kg, vec_ok, sums, l2, codes, sc);
-    Q4FC_CUDA_OK(cudaGetLastError());
+    DependentLaunch l(dim3((unsigned)grid), kQxWarps * 32, s);
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, G == 32 ? quant_x_tile_kernel<32> : quant_x_tile_kernel<128>, x, rows, K, ldx, Kg, vec_ok,
+                                    (int)sums, l2, codes, sc));
     return Q4FC_OK;
 }
 
@@ -431,13 +431,9 @@ int launch_quant_x(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, 
         return Q4FC_ELIMIT;
     }
     const int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    if (G == 32)
-        quant_x_kernel<32><<<(unsigned)grid, kQxWarps * 32, 0, s>>>(x, rows, K, ldx, Kg, scale, vec_ok, codes, scales,
-                                                                    gsums);
-    else
-        quant_x_kernel<128><<<(unsigned)grid, kQxWarps * 32, 0, s>>>(x, rows, K, ldx, Kg, scale, vec_ok, codes,
-                                                                     scales, gsums);
-    Q4FC_CUDA_OK(cudaGetLastError());
+    DependentLaunch l(dim3((unsigned)grid), kQxWarps * 32, s);
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, G == 32 ? quant_x_kernel<32> : quant_x_kernel<128>, x, rows, K, ldx, Kg, scale, vec_ok,
+                                    codes, scales, gsums));
     return Q4FC_OK;
 }
 

@@ -384,3 +384,37 @@ def test_pack_scales_at_the_ends(pkg, oracle, qtype, G, N, K):
     want = oracle.restated.pack(W.numpy(), qtype, G)
     got = pkg.llmops.offline_FC_quant_Q4A(W.cuda(), qtype=("q4_0", "q4_1")[qtype], group_k=G).cpu().numpy()
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 20])
+def test_kernels_that_start_early_wait_for_their_inputs(pkg, rows):
+    """Weights, activations and ids written by the kernel directly in front, again and again in the same buffers, give what they
+    give after a synchronisation."""
+    ops, g = pkg.llmops, torch.Generator().manual_seed(rows)
+    K = N = 2048
+    packed = [ops.offline_FC_quant_Q4A((torch.randn(N, K, generator=g) * 0.02).cuda()) for _ in range(2)]
+    q8 = [pkg.c_ext.FC_quant_Q8C((torch.randn(N, K, generator=g) * 0.02).cuda()) for _ in range(2)]
+    xs = [torch.randn(1, rows, K, generator=g).cuda() for _ in range(2)]
+    table = pkg.ops.llmop_embedding_q8c(torch.randn(100, K, generator=g).cuda())
+    ids = [torch.randint(0, 100, (1, rows), generator=g).cuda() for _ in range(2)]
+    w, w8, s8, x, i = packed[0].clone(), q8[0][0].clone(), q8[0][1].clone(), xs[0].clone(), ids[0].clone()
+
+    def step(k, wait):
+        out = []
+        for dst, src, f in ((w, packed[k], lambda: ops.fc_Q4A(x, w, N)), (x, xs[k], lambda: ops.fc_Q4A(x, w, N)),
+                            (w8, q8[k][0], lambda: pkg.c_ext.FC_evaluate_Q8C(x, w8, s8, N)),
+                            (s8, q8[k][1], lambda: pkg.c_ext.FC_evaluate_Q8C(x, w8, s8, N)), (i, ids[k], lambda: table(i))):
+            dst.copy_(src)
+            if wait:
+                torch.cuda.synchronize()
+            out.append(f())
+            if wait:
+                torch.cuda.synchronize()
+        out.append(ops.fc_Q4A(ops.fc_Q4A(out[0], w, N), w, N))
+        return out
+
+    step(1, True)
+    want = [step(k, True) for k in (0, 1)]
+    got = [step(k % 2, False) for k in range(20)]
+    for k in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(got[k], want[k % 2]))
