@@ -29,6 +29,7 @@
 // tile per CTA whatever the row count, epilogue of 5 operations per integer):
 //   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 us   Q4_0 g32, 512 rows 280 -> 223 us (207 TOPS)
 //                   Q4_1 g128, 2048 rows 517 -> 323 us (572 TOPS)   Q8C, 256 rows 296 -> 151 us (153 TOPS)
+// and, with K divided where the last round over the SMs would be nearly empty: 512 rows 187 us, 2048 rows 311, 256 rows 100.
 // A group of 32 k takes about 1100 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
 // convert, scale is latency-bound with the 16 warps that the registers allow (512 rows: issue slots 65 % busy, ALU 46 %, FMA
 // 41 %, XU, where the conversions are not, 0.2 %; per issue 2.2 warps wait for tensor or shared memory, 1.7 for the
@@ -47,7 +48,7 @@
 // costs 131 -> 151 us at 256 rows x 4096 x 11008 and 33 -> 35 at 37 rows; every 16 groups 146 us and 8.3e-8, at K = 3001 not
 // below the 8-warp sums.  (Staggering the moves over the warps: 156; as an outer loop around the groups' loop: 157.)
 //
-// Few tiles: a cluster of `split` CTAs shares a tile and divides its K stages; the partial tiles meet in shared memory
+// Few tiles, or the last of many: a cluster of `split` CTAs shares a tile and divides its K stages; the partial tiles meet in shared memory
 // and are added in rank order (fixed order, no atomics).
 #include <cuda.h>  // CUtensorMap and the cuTensorMapEncodeTiled prototype (resolved at run time, libcuda is not linked)
 
@@ -108,6 +109,10 @@ struct PrefillParams {
     int* status;
     int64_t rows, N, ldy;
     int Ng, Kg, split;
+    int n_tiles;         // column tiles; tiles are counted along them
+    int n_off, m_off;    // this launch's first tile
+    int n_end, m_end;    // and the one behind its last
+    int remainder;       // this launch does the tiles that are left of one in front of it
 };
 
 // ---- PTX helpers -------------------------------------------------------------
@@ -367,7 +372,9 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cs = p.split, rank = (int)(blockIdx.x % cs);
-    const int n_tile = (int)(blockIdx.x / cs), m_tile = blockIdx.y;
+    int n_tile = (int)(blockIdx.x / cs) + p.n_off, m_tile = (int)blockIdx.y + p.m_off;
+    if (n_tile >= p.n_tiles) n_tile -= p.n_tiles, m_tile++;
+    if (m_tile > p.m_end || (m_tile == p.m_end && n_tile >= p.n_end)) return;  // (the whole cluster)
     const int64_t n0 = (int64_t)n_tile * kTileN, m0 = (int64_t)m_tile * TM;
     const int live = (int)min((int64_t)TM, p.rows - m0);  // rows of this tile that exist
     const int nstage = (p.Kg + GPS - 1) / GPS;
@@ -637,7 +644,13 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
     } else {
         // =================== loader: codes and scales of the rows ===================
         if (elect_one()) {
-            pdl_wait_prior_grid();  // the quantizer's results are complete
+            // The quantizer's results are complete.  (It has let this launch, or the one whose remainder this one does, begin only
+            // when everything in front of it was complete; a remainder begins behind its first launch's wait, and waits for the
+            // rest of it before it ends.)
+            if (!p.remainder) {
+                pdl_wait_prior_grid();
+                pdl_launch_dependents();
+            }
 #pragma unroll 1
             for (int i = 0; i < iters; i++) {
                 const int s = i % S::kB, sl = i % S::kScs, it = it0 + i;
@@ -650,6 +663,10 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                 mbar_expect_tx(bar_sfull + 8 * sl, bytes);
                 bulk_g2s(smem0 + S::kScOff + sl * S::kScBytes,
                          p.sc + ((int64_t)m_tile * p.Kg + (int64_t)it * GPS) * (S::kSums * TM), bytes, bar_sfull + 8 * sl);
+            }
+            if (p.remainder) {
+                pdl_wait_prior_grid();
+                pdl_launch_dependents();
             }
         }
     }
@@ -755,7 +772,7 @@ int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t 
 }
 
 template <int FMT, int G, int TM, int FOLD = 0>
-int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, int64_t n_tiles, int64_t m_tiles, cudaStream_t s) {
+int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
     using S = PrefillShape<FMT, G, TM>;
     static std::atomic<bool> attr_done[64] = {};  // set once per device; a second setter repeats the same call
     int dev = 0;
@@ -767,7 +784,7 @@ int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, int64
         if (dev < 64) attr_done[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n_tiles * p.split), (unsigned)m_tiles);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(S::kThreads);
     cfg.dynamicSmemBytes = S::kSmem;
     cfg.stream = s;
@@ -786,10 +803,31 @@ int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, int64
 }
 
 template <int FMT, int G>
-int launch_prefill_tile(int tile, const PrefillParams& p, const CUtensorMap& map, int64_t n_tiles, int64_t m_tiles,
-                        cudaStream_t s) {
-    return tile == 128 ? launch_prefill_variant<FMT, G, 128>(p, map, n_tiles, m_tiles, s)
-                       : launch_prefill_variant<FMT, G, 64>(p, map, n_tiles, m_tiles, s);
+int launch_prefill_tile(int tile, const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
+    return tile == 128 ? launch_prefill_variant<FMT, G, 128>(p, map, grid, s)
+                       : launch_prefill_variant<FMT, G, 64>(p, map, grid, s);
+}
+
+// tiles first .. end - 1, K divided by p.split
+int launch_tiles(int fmt, int G, int tile, PrefillParams p, const CUtensorMap& map, int64_t first, int64_t end, cudaStream_t s) {
+    const int64_t wide = end - first < p.n_tiles ? end - first : p.n_tiles;
+    p.n_off = (int)(first % p.n_tiles), p.m_off = (int)(first / p.n_tiles);
+    p.n_end = (int)(end % p.n_tiles), p.m_end = (int)(end / p.n_tiles);
+    const dim3 grid((unsigned)(wide * p.split), (unsigned)((end - first + wide - 1) / wide));
+    if (fmt == kQ8C) {
+        const bool many = p.Kg > 64 * p.split;  // K groups of a CTA: see the file's head
+        if (tile == 128)
+            return many ? launch_prefill_variant<kQ8C, 32, 128, 12>(p, map, grid, s)
+                        : launch_prefill_variant<kQ8C, 32, 128, 8>(p, map, grid, s);
+        return many ? launch_prefill_variant<kQ8C, 32, 64, 12>(p, map, grid, s)
+                    : launch_prefill_variant<kQ8C, 32, 64, 8>(p, map, grid, s);
+    }
+    if (fmt == kQ4_1 && G == 32) return launch_prefill_tile<kQ4_1, 32>(tile, p, map, grid, s);
+    if (fmt == kQ4_1) return launch_prefill_tile<kQ4_1, 128>(tile, p, map, grid, s);
+    if (fmt == kQ4_0 && G == 32) return launch_prefill_tile<kQ4_0, 32>(tile, p, map, grid, s);
+    if (fmt == kQ4_0) return launch_prefill_tile<kQ4_0, 128>(tile, p, map, grid, s);
+    if (G == 32) return launch_prefill_tile<kQ4_0Signed, 32>(tile, p, map, grid, s);
+    return launch_prefill_tile<kQ4_0Signed, 128>(tile, p, map, grid, s);
 }
 
 // scales and group sums of a format, padded to whole row tiles of either size
@@ -815,36 +853,40 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     // four, which needs a second wave).
     const int tile = (rows > 64 && n_tiles * ((rows + 127) / 128) >= di->sm_count) ? 128 : 64;
     const int64_t m_tiles = (rows + tile - 1) / tile;
-    int64_t split = 1;
-    if (tile == 64) {
-        split = 2 * (int64_t)di->sm_count / (n_tiles * m_tiles);
-        if (split > nstage / 4) split = nstage / 4;
-        if (split > kMaxSplit) split = kMaxSplit;
-        if (split < 1) split = 1;
+    const int64_t tiles = n_tiles * m_tiles, places = (tile == 128 ? 1 : 2) * (int64_t)di->sm_count;
+    const int64_t most = nstage / 4 < 1 ? 1 : nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
+    int64_t split = 1, left = 0, left_split = 1;  // of the tiles, the last `left` with K divided by `left_split`
+    if (tiles < places) {
+        split = places / tiles < most ? places / tiles : most;
+    } else if (tiles % places != 0) {
+        // What is left after whole rounds over the places would take a round of its own, most places empty.  With K divided it
+        // takes ceil(left * c / places) rounds of 1/c, each with some stages' time for start-up and the adding; larger clusters
+        // do not fit everywhere.  (11008 columns, K = 4096: 512 rows, group 32, 48 of 344 tiles left, 220 -> 187 us; 256 rows, Q8C, 24
+        // of 172, 148 -> 100; 256 rows, group 128, 64 -> 47; 100 rows x 20000, group 32, 18 of 314, 180 -> 106.  Divided where this
+        // sum says no: 1000 rows, 96 of 688, Q8C, 360 -> 394.)
+        left = tiles % places;
+        int64_t best = nstage;  // undivided, in the launch of the others
+        for (int64_t c = 2; c <= most; c++) {
+            const int64_t fit = c == 2 ? places : c <= 4 ? places * 15 / 16 : places * 13 / 16;
+            const int64_t cost = (left * c + fit - 1) / fit * ((nstage + c - 1) / c + (G == 128 ? 8 : 4));
+            if (cost < best) best = cost, left_split = c;
+        }
+        if (left_split == 1) left = 0;
     }
-    if (n_tiles * split > 0x7fffffffLL || m_tiles > 65535) {
+    if (n_tiles * split > 0x7fffffffLL || m_tiles > 65535 || tiles > 0x7fffffffLL / kMaxSplit) {
         set_error("fc_prefill: %lld x %lld tiles exceed the grid limit", (long long)n_tiles, (long long)m_tiles);
         return Q4FC_ELIMIT;
     }
-    p.split = (int)split;
+    p.n_tiles = (int)n_tiles;
     if (int rc = launch_quant_x_tile(x, rows, K, ldx, G, fmt == kQ4_1, tile, codes, sc, s)) return rc;
     CUtensorMap map = {};
     if (Kp > 0)  // (no K group: no stage reads the map)
         if (int rc = make_codes_map(&map, codes, rows, Kp, tile)) return rc;
-    if (fmt == kQ8C) {
-        const bool many = p.Kg > 64 * split;  // K groups of a CTA: see the file's head
-        if (tile == 128)
-            return many ? launch_prefill_variant<kQ8C, 32, 128, 12>(p, map, n_tiles, m_tiles, s)
-                        : launch_prefill_variant<kQ8C, 32, 128, 8>(p, map, n_tiles, m_tiles, s);
-        return many ? launch_prefill_variant<kQ8C, 32, 64, 12>(p, map, n_tiles, m_tiles, s)
-                    : launch_prefill_variant<kQ8C, 32, 64, 8>(p, map, n_tiles, m_tiles, s);
-    }
-    if (fmt == kQ4_1 && G == 32) return launch_prefill_tile<kQ4_1, 32>(tile, p, map, n_tiles, m_tiles, s);
-    if (fmt == kQ4_1) return launch_prefill_tile<kQ4_1, 128>(tile, p, map, n_tiles, m_tiles, s);
-    if (fmt == kQ4_0 && G == 32) return launch_prefill_tile<kQ4_0, 32>(tile, p, map, n_tiles, m_tiles, s);
-    if (fmt == kQ4_0) return launch_prefill_tile<kQ4_0, 128>(tile, p, map, n_tiles, m_tiles, s);
-    if (G == 32) return launch_prefill_tile<kQ4_0Signed, 32>(tile, p, map, n_tiles, m_tiles, s);
-    return launch_prefill_tile<kQ4_0Signed, 128>(tile, p, map, n_tiles, m_tiles, s);
+    p.split = (int)split;
+    if (int rc = launch_tiles(fmt, G, tile, p, map, 0, tiles - left, s)) return rc;
+    if (left == 0) return Q4FC_OK;
+    p.split = (int)left_split, p.remainder = 1;
+    return launch_tiles(fmt, G, tile, p, map, tiles - left, tiles, s);
 }
 
 // workspace: [status 256][what the decode kernels keep between calls: decode_prequant_offset() bytes]

@@ -252,6 +252,17 @@ def test_many_rows_divisions_and_long_k(pkg, oracle, fmt, rows, N, K):
     check_many_rows(pkg, oracle, fmt, rows, N, K)
 
 
+@pytest.mark.parametrize("rows,N,K", [
+    (129, 9500, 2080),    # 150 tiles of 128 rows on 148 SMs: two left, K divided by four, the last stage one group
+    (12700, 300, 1056),   # 300 tiles, four left over three column tiles: the launch's rows of tiles wrap
+    (20, 37900, 1060),    # 297 tiles of 64 rows on 296 places: one left, columns and k beyond the weights
+])
+@pytest.mark.parametrize("fmt", [(0, 32), (1, 32), (1, 128), "signed32", "q8c"])
+def test_many_rows_last_tiles_divided(pkg, oracle, fmt, rows, N, K):
+    """Tiles left over after whole rounds go in a launch of their own with K divided (tolerance as above)."""
+    check_many_rows(pkg, oracle, fmt, rows, N, K)
+
+
 def check_many_rows(pkg, oracle, fmt, rows, N, K):
     g = torch.Generator().manual_seed(rows + N + K)
     W = torch.randn(N, K, generator=g) * 0.02
