@@ -13,7 +13,7 @@
 // What bounds it: issue slots, then HBM.  One word per thread and one path for all values took 22 warp instructions per 32
 // weights; the instructions a group costs (shuffles, scale and its reciprocal, addresses) are now shared by 16 weights of a
 // thread, and full groups of ordinary finite values take a path without clamps and float-to-int conversions.
-// 11008 x 4096, Q4_1 group 128: 45.3 -> 36.8 us (5.5 TB/s).
+// 11008 x 4096, Q4_1 group 128: 45.2 -> 36.5 us (5.6 TB/s).
 //
 // General path: the reduction keeps the reference's
 // "first value wins a tie" rule of get_min_max (ops/op_fc.hpp:112-122) by
@@ -48,6 +48,21 @@ __device__ __forceinline__ void ldg_v8(const float* p, float* v) {
     asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                  : "l"(p));
+}
+// Sixteen values from any 4-byte place: the 16-byte pieces around them, shifted by what they start too early.  (As sixteen
+// 4-byte loads, each of them 32 sectors wide for a warp, 8747 x 2816, Q4_0 group 128 took 41 us, so 28.)
+__device__ __forceinline__ void ldg_any16(const float* src, float* v) {
+    const int a = (int)(reinterpret_cast<uintptr_t>(src) >> 2) & 3;
+    float t[20];
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+        const float4 q = __ldg(reinterpret_cast<const float4*>(src - a) + i);
+        t[4 * i] = q.x, t[4 * i + 1] = q.y, t[4 * i + 2] = q.z, t[4 * i + 3] = q.w;
+    }
+#pragma unroll
+    for (int i = 0; i < 19; i++) t[i] = a & 1 ? t[i + 1] : t[i];
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = a & 2 ? t[i + 2] : t[i];
 }
 // of three values (sm_100); NaN if one of them is
 __device__ __forceinline__ float min3(float a, float b, float c) {
@@ -134,6 +149,8 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(const float* __restr
                 const float4 a = __ldg(reinterpret_cast<const float4*>(src) + i);
                 v[it][4 * i] = a.x, v[it][4 * i + 1] = a.y, v[it][4 * i + 2] = a.z, v[it][4 * i + 3] = a.w;
             }
+        } else if (cnt == kPerThread && n * K + k >= 4 && n * K + k + 20 <= N * K) {  // (the pieces lie inside the matrix)
+            ldg_any16(src, v[it]);
         } else {
 #pragma unroll
             for (int j = 0; j < kPerThread; j++) v[it][j] = (j < cnt) ? __ldg(src + j) : 0.0f;
