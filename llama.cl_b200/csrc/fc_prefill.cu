@@ -12,6 +12,9 @@
 // One CTA computes 128 columns n x TM rows m:
 //   * operand A = weights: the packed blocks come in by bulk copies, are unpacked to one byte per weight in shared
 //     memory, K-major rows of 128 bytes, in the 128-byte-swizzle canonical layout that tcgen05.mma reads;
+//     Group 128 in 128-row tiles: in tensor memory instead, in the fourth result buffer's place (a group's four MMAs and its
+//     long epilogue need no fourth buffer; 2048 rows x 4096 x 11008 312 -> 297 us, 512 rows 85 -> 82.  With group 32 the three
+//     buffers cost more than that: Q8C, 256 rows, 148 -> 176 undivided);
 //   * operand B = activation codes (int8), same layout, straight from the code matrix by TMA;
 //   * D = int32 accumulators in tensor memory, lane = weight column, column = activation row.
 // Every K group has its own pair of scales, so a group's MMA(s) (one K=32 instruction for group 32, four for group
@@ -81,17 +84,20 @@ struct PrefillShape {
     static constexpr int kEpiWarps = TM / 8;              // 32 rows of the tile per warp and TMEM lane quarter
     static constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
     static constexpr int kLoadWidth = TM == 128 ? 16 : 8; // rows a thread takes from tensor memory at a time
-    static constexpr int kA = TM == 128 ? 3 : 2;          // stages of unpacked weights
+    static constexpr bool kATmem = G == 128 && TM == 128; // unpacked weights in tensor memory, else in shared memory
+    static constexpr int kA = kATmem ? 4 : TM == 128 ? 3 : 2;  // stages of unpacked weights
     static constexpr int kB = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;    // stages of activation codes
     static constexpr int kRaw = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;  // stages of packed bytes
     static constexpr int kScs = 4;                        // stages of scales
-    static constexpr int kBufs = FMT == kQ8C && TM == 64 ? kTmemBufs - 1 : kTmemBufs;  // buffers of integers (Q8C: one holds sums)
+    // buffers of integers in the kTmemBufs x TM columns (the last one's place: Q8C, sums; kATmem, weights)
+    static constexpr int kBufs = (FMT == kQ8C && TM == 64) || kATmem ? kTmemBufs - 1 : kTmemBufs;
+    static_assert(!kATmem || kA * kStageK / 4 == TM, "weights take one buffer's columns");
     static constexpr int kRawStripe = kGroups * kBlock;   // packed bytes of one stripe in a stage
     static constexpr int kABytes = kTileN * kStageK, kBBytes = TM * kStageK;
     static constexpr int kXscBytes = kGroups * kSums * TM * 4;                // [group][scale | sum][row] fp32
     static constexpr int kWscBytes = FMT == kQ8C ? 0 : kGroups * kTileN * 4;  // [group][n] {wd, wm} fp16
     static constexpr int kScBytes = kXscBytes + kWscBytes;
-    static constexpr int kBOff = kA * kABytes;
+    static constexpr int kBOff = kATmem ? 0 : kA * kABytes;
     static constexpr int kRawOff = kBOff + kB * kBBytes;
     static constexpr int kScOff = kRawOff + kRaw * 4 * kRawStripe;
     static constexpr int kBarOff = kScOff + kScs * kScBytes;
@@ -189,6 +195,14 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint6
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
         : "memory");
 }
+__device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accum)
+        : "memory");
+}
 __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -208,6 +222,13 @@ __device__ __forceinline__ void tc_st(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
                  "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
+}
+__device__ __forceinline__ void tc_st(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
@@ -412,7 +433,7 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = *tmem_slot, a_tmem = tmem_base + S::kBufs * TM;
 
     if (warp < kUnpackWarp) {
         // =================== epilogue: 32 lanes x (16 + 16) rows per warp ===================
@@ -560,6 +581,18 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                         for (int c = 0; c < 4; c++)
                             sts128(dst + ((uint32_t)((h * 4 + c) << 4) ^ sw), w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
                     }
+                } else if constexpr (S::kATmem) {
+                    __syncwarp();
+                    tc_fence_after();
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        uint32_t w[8], o[16];
+#pragma unroll
+                        for (int c = 0; c < 8; c++) w[c] = lds32(src + (h * 8 + c) * 128);
+#pragma unroll
+                        for (int c = 0; c < 8; c++) unpack_nibbles<FMT == kQ4_0Signed>(w[c], o[2 * c], o[2 * c + 1]);
+                        tc_st(a_tmem + ((uint32_t)(pw * 32) << 16) + s * (kStageK / 4) + 16 * h, o);
+                    }
                 } else {
                     uint32_t w[16];
 #pragma unroll
@@ -587,7 +620,13 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                         }
                 }
             }
-            fence_proxy_async();  // generic-proxy stores above -> visible to the tensor core's async proxy
+            if constexpr (S::kATmem) {
+                __syncwarp();
+                tc_wait_st();
+                tc_fence_before();
+            } else {
+                fence_proxy_async();  // generic-proxy stores above -> visible to the tensor core's async proxy
+            }
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(bar_afull + 8 * s);
@@ -628,8 +667,12 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                     }
                     tc_fence_after();
 #pragma unroll
-                    for (int ks = 0; ks < MMAS; ks++)
-                        tc_mma_i8(tmem_base + b * TM, ad + ks * 2, bd + ks * 2, idesc, ks > 0 ? 1u : 0u);
+                    for (int ks = 0; ks < MMAS; ks++) {
+                        if constexpr (S::kATmem)
+                            tc_mma_i8(tmem_base + b * TM, a_tmem + sa * (kStageK / 4) + ks * 8, bd + ks * 2, idesc, ks > 0 ? 1u : 0u);
+                        else
+                            tc_mma_i8(tmem_base + b * TM, ad + ks * 2, bd + ks * 2, idesc, ks > 0 ? 1u : 0u);
+                    }
                     tc_commit(bar_tfull + 8 * b);  // the group's integers are complete in TMEM
                 }
                 tc_commit(bar_aempty + 8 * sa);  // the stage's operands have been consumed
