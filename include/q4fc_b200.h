@@ -58,9 +58,12 @@ enum {
     Q4FC_FLAG_NIBBLE_SIGNED = 1u,
     /* Stream weights while the predecessor on the stream drains.  (Calls may
      * start before their predecessor has completed in any case; without this
-     * flag they touch no memory before it has, with it only activations,
-     * outputs and workspace wait.)  Use only when the predecessor does not
-     * write this call's weights. */
+     * flag they touch no memory before it has, and let their successor start
+     * only then; with it only activations, outputs and workspace wait.)  Use
+     * only when no launch that may still be running writes this call's
+     * weights: not the predecessor and, where that one carries this flag too
+     * (or releases its successor before it has itself waited), not the ones in
+     * front of it up to the nearest that does neither. */
     Q4FC_FLAG_PDL = 2u,
     /* q4fc_fc_decode only: use the stream-K kernel (one contiguous byte run
      * per CTA, weights staged in registers, partial sums through the workspace)

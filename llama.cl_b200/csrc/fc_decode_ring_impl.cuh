@@ -14,8 +14,8 @@
 // (cp.async.bulk, global -> shared, completion counted on an mbarrier; this GPU's own memory, no multicast) of
 // up to SB blocks each into a ring of `depth` slots, as far ahead as the ring allows -- on B200 that is up to
 // ~190 KB per SM in flight with no register cost, and for most Llama-7B shapes the CTA's whole share.  The
-// first ring-full is issued before the programmatic-dependent-launch wait: weights never depend on the
-// preceding kernel, so they stream while that kernel drains and while this one quantizes its activations.
+// first ring-full is issued at once where nothing in front writes weights (the caller's Q4FC_FLAG_PDL, or behind this call's
+// own quantizing launch), so that weights stream while the kernel in front drains; else behind the wait for that kernel.
 // Warps 0-15 consume: every warp takes block(s) `warp` of each slot from shared memory into registers, frees
 // the slot with one mbarrier arrival per warp, feeds mma.sync.m16n8k32 (u8 x s8 -> s32, exact) and scales per
 // K group in fp32.
@@ -276,7 +276,9 @@ __global__ void __launch_bounds__(kRThreads, 1) fc_decode_ring_kernel(const __gr
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncwarp();
-    pdl_launch_dependents();
+    // The next launch may begin, and where its caller set Q4FC_FLAG_PDL read its weights, as soon as every CTA says so.  Here only
+    // where everything in front of this call's first launch is complete already or the caller vouches for it; else behind the wait.
+    if (TP || p.weights_early) pdl_launch_dependents();
     // "this CTA runs": nobody may store into a CTA's shared memory before that CTA has started
     if (cs > 1 || bq > 1) cluster_arrive_release();
 
@@ -332,6 +334,7 @@ __global__ void __launch_bounds__(kRThreads, 1) fc_decode_ring_kernel(const __gr
             // where weights do not depend on the preceding kernel: fill the ring now
             if (!p.weights_early) pdl_wait_prior_grid();
             while (p_filled < depth && p_li < r) issue_slot(), p_filled++;
+            if (!TP && !p.weights_early) pdl_launch_dependents();
             if constexpr (PREQ) {
                 pdl_wait_prior_grid();
                 if (r > 0) {

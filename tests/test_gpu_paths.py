@@ -429,3 +429,56 @@ def test_kernels_that_start_early_wait_for_their_inputs(pkg, rows):
     got = [step(k % 2, False) for k in range(20)]
     for k in range(20):
         assert all(torch.equal(a, b) for a, b in zip(got[k], want[k % 2]))
+
+
+class EarlyWriter:
+    """Rewrites a buffer with one of two contents by the embedding look-up, which lets its successor begin at once and then
+    stores for as long as it takes: few CTAs, so that others find places beside them.  The values are whole numbers in fp32:
+    bytes and halves of them are finite nibbles, codes and scales too."""
+
+    def __init__(self, pkg, nbytes, ctas, seed):
+        g, E = torch.Generator().manual_seed(seed), nbytes // 4 // ctas
+        assert E * ctas * 4 == nbytes and E % 4 == 0
+        self.table = torch.randint(-127, 128, (2 * ctas, E), generator=g).to(torch.int8).cuda()
+        self.ids = torch.arange(2 * ctas).view(2, ctas).cuda()
+        self.scales, self.out, self.pkg = torch.ones(2 * ctas, device="cuda"), torch.zeros(ctas, E, device="cuda"), pkg
+
+    def __call__(self, k):
+        self.pkg.llmops.embedding_q8c(self.out, self.ids[k], self.table, self.scales)
+
+
+@pytest.mark.parametrize("reader", ["multi", "batch"])
+@pytest.mark.parametrize("between", ["decode", "decode_quantizer", "prequantized", "prefill", "q8c", "quantizer", "look-up"])
+def test_calls_without_the_flag_hold_a_flagged_successor_back(pkg, between, reader):
+    """A kernel writes weights, a call without pdl=True follows, a call with it reads those weights, no copy or wait between:
+    the same results as with waits (the same kernels on the same inputs: equal)."""
+    ops, g = pkg.llmops, torch.Generator().manual_seed(3)
+    K, N = 4096, 16384
+    write = EarlyWriter(pkg, N // 32 * (K // 128) * 2176, 256, 1)
+    w2 = write.out.view(torch.int8).view(N // 32, K // 128, 2176)
+    x = torch.randn(1, 8, K, generator=g).cuda()
+    x2 = ops.quantize_activations(torch.randn(1, 2, K, generator=g).cuda(), 128)
+    w1 = ops.offline_FC_quant_Q4A((torch.randn(640, K, generator=g) * 0.02).cuda())
+    w8, s8 = pkg.c_ext.FC_quant_Q8C((torch.randn(640, K, generator=g) * 0.02).cuda())
+    x1, x32, w32 = ops.quantize_activations(x, 32), x.view(1, 32, K // 4), w1[:, :K // 128].contiguous()
+    table, ids = pkg.ops.llmop_embedding_q8c(torch.randn(100, K, generator=g).cuda()), torch.arange(50).cuda()
+    call = {"decode": lambda: ops.fc_Q4A(x[:, :1], w1, 640), "decode_quantizer": lambda: ops.fc_Q4A(x, w1, 640),
+            "prequantized": lambda: ops.fc_Q4A_q8(x1, w1, 640), "prefill": lambda: ops.fc_Q4A(x32, w32, 640),
+            "q8c": lambda: pkg.c_ext.FC_evaluate_Q8C(x, w8, s8, 640),
+            "quantizer": lambda: ops.quantize_activations(x, 32).codes(), "look-up": lambda: table(ids)}[between]
+    batch = ops.FCBatch([(x2, w2, N)], pdl=True)
+    read = (lambda: ops.fc_Q4A_multi(x2, [w2], [N], pdl=True)[0]) if reader == "multi" else (lambda: batch.run()[0].clone())
+
+    def step(k, wait):
+        out = []
+        for f in (lambda: write(k), call, read):
+            out.append(f())
+            if wait:
+                torch.cuda.synchronize()
+        return out[1:]
+
+    want = [step(k, True) for k in (0, 1)]
+    assert not torch.equal(want[0][1], want[1][1])
+    got = [step(k % 2, False) for k in range(20)]
+    for k in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(got[k], want[k % 2]))
