@@ -1,5 +1,6 @@
 """Branches of the host and kernel dispatch, each at the sizes where it can go wrong, against the other entry points or
 the oracle."""
+import ctypes
 import weakref
 
 import numpy as np
@@ -254,30 +255,52 @@ def test_many_rows_divisions_and_long_k(pkg, oracle, fmt, rows, N, K):
 
 @pytest.mark.parametrize("rows,N,K", [
     (129, 9500, 2080),    # 150 tiles of 128 rows on 148 SMs: two left, K divided by four, the last stage one group
-    (12700, 300, 1056),   # 300 tiles, four left over three column tiles: the launch's rows of tiles wrap
-    (20, 37900, 1060),    # 297 tiles of 64 rows on 296 places: one left, columns and k beyond the weights
+    (6500, 300, 2080),    # 153 tiles, five left over three column tiles: the launch's rows of tiles wrap, the last is not full
+    (20, 37900, 2084),    # 297 tiles of 64 rows on 296 places: one left, columns and k beyond the weights
 ])
-@pytest.mark.parametrize("fmt", [(0, 32), (1, 32), (1, 128), "signed32", "q8c"])
+@pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128", "q8c"])
 def test_many_rows_last_tiles_divided(pkg, oracle, fmt, rows, N, K):
     """Tiles left over after whole rounds go in a launch of their own with K divided (tolerance as above)."""
-    check_many_rows(pkg, oracle, fmt, rows, N, K)
+    check_many_rows(pkg, oracle, fmt, rows, N, K, launches=3)  # the quantizer, whole rounds, the remainder
 
 
-def check_many_rows(pkg, oracle, fmt, rows, N, K):
+def graph_nodes(graph):
+    """Nodes of a captured graph."""
+    n = ctypes.c_size_t()
+    assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(n)) == 0
+    return n.value
+
+
+def check_many_rows(pkg, oracle, fmt, rows, N, K, launches=None):
     g = torch.Generator().manual_seed(rows + N + K)
     W = torch.randn(N, K, generator=g) * 0.02
     x = torch.randn(1, rows, K, generator=g)
     if fmt == "q8c":
         wq, ws = oracle.restated.q8c_pack(W.numpy())
         want = oracle.restated.q8c_fc(x.numpy(), wq, ws, N)
-        run = lambda: pkg.c_ext.FC_evaluate_Q8C(x.cuda(), torch.from_numpy(wq).cuda(), torch.from_numpy(ws).cuda(), N)
+        xd, wd, sd = x.cuda(), torch.from_numpy(wq).cuda(), torch.from_numpy(ws).cuda()
+        run = lambda: pkg.c_ext.FC_evaluate_Q8C(xd, wd, sd, N)
     else:
         signed = isinstance(fmt, str)
         wq = oracle.restated.pack(W.numpy(), *((0, int(fmt[6:])) if signed else fmt))
         want = oracle.restated.fc(x.numpy(), wq, N, nibble_signed=signed)
-        run = lambda: pkg.llmops.fc_Q4A(x.cuda(), torch.from_numpy(wq).cuda(), N, nibble_signed=signed)
+        xd, wd = x.cuda(), torch.from_numpy(wq).cuda()
+        run = lambda: pkg.llmops.fc_Q4A(xd, wd, N, nibble_signed=signed)
     got = run()
     assert torch.equal(got, run())  # fixed summation order
+    if launches is not None:
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            run()  # the stream's workspace
+            stream.synchronize()
+            with torch.cuda.graph(graph, stream=stream):
+                again = run()
+        assert graph_nodes(graph) == launches
+        graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got, again)
     assert np.abs(got.cpu().numpy() - want).max() <= 2e-5 * np.abs(want).max()
     pkg.llmops.check_device_status()
 
@@ -291,11 +314,12 @@ def test_q8c_row_tiles_and_the_line_to_the_gemm(pkg, oracle, rows, N, K):
     check_many_rows(pkg, oracle, "q8c", rows, N, K)
 
 
+@pytest.mark.parametrize("K,sizes", [(1056, (300, 20, 200)), (2080, (200, 512, 20))])  # 200 and 512 rows: with a remainder
 @pytest.mark.parametrize("fmt", ["q4", "q8c"])
-def test_many_rows_captured_and_on_two_streams(pkg, fmt):
+def test_many_rows_captured_and_on_two_streams(pkg, fmt, K, sizes):
     """Calls with both tile sizes on one workspace, captured into a graph and replayed, and beside them eager calls on a
     second stream: all bit-equal to calls one by one (fixed summation orders)."""
-    ops, N, K = pkg.llmops, 11008, 1056
+    ops, N = pkg.llmops, 11008
     g = torch.Generator(device="cuda").manual_seed(4)
     W = torch.randn(N, K, generator=g, device="cuda") * 0.02
     if fmt == "q8c":
@@ -304,7 +328,7 @@ def test_many_rows_captured_and_on_two_streams(pkg, fmt):
     else:
         w = ops.offline_FC_quant_Q4A(W)
         fc = lambda x: ops.fc_Q4A(x, w, N)
-    inputs = [[torch.randn(1, rows, K, generator=g, device="cuda") for rows in (300, 20, 200)] for _ in range(3)]
+    inputs = [[torch.randn(1, rows, K, generator=g, device="cuda") for rows in sizes] for _ in range(3)]
     want = [[fc(x) for x in xs] for xs in inputs]
     a, b = torch.cuda.Stream(), torch.cuda.Stream()
     torch.cuda.synchronize()
