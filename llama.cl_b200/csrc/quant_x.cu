@@ -334,6 +334,27 @@ __global__ void __launch_bounds__(128) quant_x_pre_batch_kernel(const __grid_con
 
 }  // namespace
 
+bool begins_early(cudaStream_t s, const void* kernel) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t* front = nullptr;
+    const cudaGraphEdgeData* edges = nullptr;
+    size_t n = 0, followers = 0;
+    cudaGraphNodeType type = cudaGraphNodeTypeEmpty;
+    cudaKernelNodeParams node = {};
+    // (an error here is not the caller's; what there is to say about the stream the launch itself will say)
+    if (cudaStreamGetCaptureInfo_v3(s, &status, nullptr, nullptr, &front, &edges, &n) != cudaSuccess) cudaGetLastError();
+    if (status != cudaStreamCaptureStatusActive) return true;
+    if (n != 1) return false;
+    if (cudaGraphNodeGetType(front[0], &type) != cudaSuccess ||
+        cudaGraphNodeGetDependentNodes_v2(front[0], nullptr, nullptr, &followers) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (type != cudaGraphNodeTypeKernel || followers != 0) return false;
+    if (cudaGraphKernelNodeGetParams(front[0], &node) != cudaSuccess) cudaGetLastError();  // (a kernel of another library)
+    return node.func != kernel;
+}
+
 int launch_quant_x_pre_batch(const q4fc_xq_call* calls, int n, int G, bool want_isum, bool pdl, cudaStream_t s) {
     QuantBatch b = {};
     int units = 0;
@@ -357,19 +378,10 @@ int launch_quant_x_pre_batch(const q4fc_xq_call* calls, int n, int G, bool want_
     }
     if (b.n == 0) return Q4FC_OK;
     b.unit0[b.n] = units;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((units + 3) / 4));
-    cfg.blockDim = dim3(128);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;  // (it waits before it reads, and without `pdl` releases the FC only after that)
-    if (G == 32)
-        Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_x_pre_batch_kernel<32>, b, (int)want_isum, (int)pdl));
-    else
-        Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_x_pre_batch_kernel<128>, b, (int)want_isum, (int)pdl));
+    auto* kernel = G == 32 ? quant_x_pre_batch_kernel<32> : quant_x_pre_batch_kernel<128>;
+    // (it waits before it reads, and without `pdl` releases the FC only after that)
+    DependentLaunch l(reinterpret_cast<const void*>(kernel), dim3((unsigned)((units + 3) / 4)), 128, s, pdl);
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, kernel, b, (int)want_isum, (int)pdl));
     return Q4FC_OK;
 }
 
@@ -385,21 +397,10 @@ int launch_quant_x_pre(const float* x, int rows, int64_t K, int64_t ldx, int G, 
     const int64_t grid = (chunks * rows + 3) / 4;
     const int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0) &&
                        ((reinterpret_cast<uintptr_t>(up) & 15) == 0);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(128);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;  // (it waits before it reads, and without `pdl` releases the FC only after that)
-    if (G == 32)
-        Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_x_pre_kernel<32>, x, rows, K, ldx, Kg, vec_ok, (int)want_isum,
-                                        (int)pdl, codes, sc, up, prod, ldp));
-    else
-        Q4FC_CUDA_OK(cudaLaunchKernelEx(&cfg, quant_x_pre_kernel<128>, x, rows, K, ldx, Kg, vec_ok, (int)want_isum,
-                                        (int)pdl, codes, sc, up, prod, ldp));
+    auto* kernel = G == 32 ? quant_x_pre_kernel<32> : quant_x_pre_kernel<128>;
+    // (it waits before it reads, and without `pdl` releases the FC only after that)
+    DependentLaunch l(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), 128, s, pdl);
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, kernel, x, rows, K, ldx, Kg, vec_ok, (int)want_isum, (int)pdl, codes, sc, up, prod, ldp));
     return Q4FC_OK;
 }
 
@@ -414,9 +415,9 @@ int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, in
     }
     const int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const int l2 = tile == 128 ? 7 : 6;
-    DependentLaunch l(dim3((unsigned)grid), kQxWarps * 32, s);
-    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, G == 32 ? quant_x_tile_kernel<32> : quant_x_tile_kernel<128>, x, rows, K, ldx, Kg, vec_ok,
-                                    (int)sums, l2, codes, sc));
+    auto* kernel = G == 32 ? quant_x_tile_kernel<32> : quant_x_tile_kernel<128>;
+    DependentLaunch l(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), kQxWarps * 32, s);
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, kernel, x, rows, K, ldx, Kg, vec_ok, (int)sums, l2, codes, sc));
     return Q4FC_OK;
 }
 
@@ -431,9 +432,9 @@ int launch_quant_x(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, 
         return Q4FC_ELIMIT;
     }
     const int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    DependentLaunch l(dim3((unsigned)grid), kQxWarps * 32, s);
-    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, G == 32 ? quant_x_kernel<32> : quant_x_kernel<128>, x, rows, K, ldx, Kg, scale, vec_ok,
-                                    codes, scales, gsums));
+    auto* kernel = G == 32 ? quant_x_kernel<32> : quant_x_kernel<128>;
+    DependentLaunch l(reinterpret_cast<const void*>(kernel), dim3((unsigned)grid), kQxWarps * 32, s);
+    Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, kernel, x, rows, K, ldx, Kg, scale, vec_ok, codes, scales, gsums));
     return Q4FC_OK;
 }
 

@@ -271,6 +271,82 @@ def graph_nodes(graph):
     return n.value
 
 
+def early_edges(graph):
+    """Edges of a captured graph over which a kernel begins before the one in front of it has ended, and all of them."""
+    cu, n = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t()
+    g = ctypes.c_void_p(graph.raw_cuda_graph())
+    assert cu.cuGraphGetEdges_v2(g, None, None, None, ctypes.byref(n)) == 0
+    ends, data = [(ctypes.c_void_p * n.value)() for _ in range(2)], (ctypes.c_ubyte * (8 * n.value))()
+    assert cu.cuGraphGetEdges_v2(g, ends[0], ends[1], data, ctypes.byref(n)) == 0
+    return sum(data[8 * i + 2] == 1 for i in range(n.value)), n.value  # (bytes of an edge: from port, to port, type)
+
+
+def test_quantizers_on_a_side_branch_do_not_begin_early(pkg):
+    """Captured behind one another, or behind a kernel that something else follows already, quantizers are ordinary nodes; in
+    one line with FCs they begin early.  The results are those of the eager calls."""
+    ops, g = pkg.llmops, torch.Generator().manual_seed(9)
+    K, N, dev = 512, 256, torch.device("cuda")
+    w = ops.offline_FC_quant_Q4A((torch.randn(N, K, generator=g) * 0.02).cuda())
+    xs = [torch.randn(1, 2, K, generator=g).cuda() for _ in range(4)]
+    xq = [ops.QuantizedActivations(1, 2, K, 32, False, dev) for _ in xs]
+    quantizers = [ops.QuantizeBatch([(x, q)]) for x, q in zip(xs, xq)]
+    other = ops.QuantizeBatch([(xs[0], ops.QuantizedActivations(1, 2, K, 32, False, dev))])
+    fcs = [ops.FCBatch([(q, w, N)]) for q in xq]
+    want = [ops.fc_Q4A_q8(ops.quantize_activations(x, 32), w, N) for x in xs]
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def line():
+        for q, f in zip(quantizers, fcs):
+            q.run(), f.run()
+
+    def branch():
+        start = torch.cuda.Event()
+        start.record(main)
+        side.wait_event(start)
+        done = []
+        with torch.cuda.stream(side):
+            for q in quantizers:
+                q.run()
+                done.append(torch.cuda.Event())
+                done[-1].record(side)
+        for f, e in zip(fcs, done):
+            main.wait_event(e)
+            f.run()
+
+    def row():
+        for q in quantizers:
+            q.run()
+
+    def behind():  # the last quantizer behind an FC that another one follows already
+        line()
+        end = torch.cuda.Event()
+        end.record(main)
+        fcs[0].run()
+        side.wait_event(end)
+        with torch.cuda.stream(side):
+            other.run()
+            end.record(side)
+        main.wait_event(end)
+
+    torch.cuda.synchronize()
+    for form, count in ((line, (7, 7)), (row, (0, 3)), (behind, (8, 9)), (branch, None)):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.stream(main):
+            form()
+            main.synchronize()
+            with torch.cuda.graph(graph, stream=main):
+                form()
+        assert count is None or early_edges(graph) == count, form.__name__
+        for f, q in zip(fcs, xq):
+            f.outs[0].zero_(), q.buf.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        if form is row:
+            [f.run() for f in fcs]
+        torch.cuda.synchronize()
+        assert all(torch.equal(f.outs[0], y) for f, y in zip(fcs, want)), form.__name__
+
+
 def check_many_rows(pkg, oracle, fmt, rows, N, K, launches=None):
     g = torch.Generator().manual_seed(rows + N + K)
     W = torch.randn(N, K, generator=g) * 0.02
