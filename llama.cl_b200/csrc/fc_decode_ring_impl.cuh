@@ -620,11 +620,14 @@ int ring_max_clusters(RingVariant* v, int dev, int cl, int log2cl, const DeviceI
     return v->max_clusters[dev][log2cl];
 }
 
-// Above this many activation values (rows x K) a separate quantizing launch in front of the FC beats the
-// quantizer inside it, which every CTA (or cluster of sharers) runs for itself.  Needs scratch: used only when
-// the caller's workspace has room for it.  (K = 4096: 4 rows x 4096 columns, group 32, 8.5 -> 7.4 us, 8 rows x 32000 28.7 ->
-// 25.2; K = 11008, one row x 4096, group 32: inside 11.1, in a launch of its own 12.0.)
-constexpr int64_t kPreQuantMinValues = 16 * 1024;
+// Whether a quantizing launch in front of the FC beats the quantizer inside it, which every cluster of CTAs runs for itself: a
+// CTA's share is a quarter of the rows x K values where four CTAs share the work or K is divided by four, half with K divided by
+// two, an eighth with K divided by eight.  From 16K values (by eight: 40K) the launch costs less than that share.  Inside / in
+// front, us, call after call in a graph, Q4_1 group 32: 8 rows x 2048 x 4096 7.5 / 6.2, 4 x 4096 x 2048 6.2 / 6.5, 5 x 4096 x 2048
+// 8.4 / 6.6, 4 x 4096 x 11008 15.5 / 15.2, 4 x 4096 x 32000 29.6 / 26.4, 3 x 11008 x 1024 8.8 / 7.6; by eight, 8 x 4096 x 512 6.3 /
+// 7.0, 2 x 8192 x 512 5.1 / 6.4, 5 x 8192 x 512 6.7 / 7.0.  At the line with two rows both ways: 2 x 8192 x 4096
+// 10.3 / 11.6 and x 1024 5.4 / 6.6, x 2400 13.4 / 10.4.  Needs scratch: used only when the caller's workspace has room for it.
+bool quantizes_in_front(int64_t values, int k_parts) { return values >= (k_parts < 8 ? 16 : 40) * 1024; }
 
 // one FC of a launch, as the entry points describe it
 struct RingCall {
@@ -720,6 +723,12 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
     const bool sgn = (flags & Q4FC_FLAG_NIBBLE_SIGNED) && qtype == 0;
     const bool pdl = (flags & Q4FC_FLAG_PDL) != 0;
 
+    // ---- shape of the launch: K split (clusters) only when one input's stripes alone cannot fill the GPU
+    const int sms = di->sm_count;
+    int cs = 1;
+    if (p.ninputs == 1)
+        while (cs < 8 && cs * 2 <= kg_max && ng_total * cs * 2 <= sms) cs *= 2;
+
     // ---- one fp32 input: quantize it inside the FC kernel, or in a launch of its own in front of it
     bool preq = !any_fp32, own_quant_launch = false;
     if (any_fp32) {
@@ -729,7 +738,7 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
         if (TP && tp[0]->xq_scratch != nullptr && !tp[0]->x_stamped) {
             base = static_cast<uint8_t*>(tp[0]->xq_scratch);  // the caller's scratch
         } else if (!TP && ws != nullptr &&
-                   ((flags & Q4FC_FLAG_PREQUANT) || (int64_t)rows * K >= kPreQuantMinValues) &&
+                   ((flags & Q4FC_FLAG_PREQUANT) || quantizes_in_front(rows * K, cs)) &&
                    ws_bytes >= decode_prequant_offset() + quant_pre_bytes(rows, K, G)) {
             base = static_cast<uint8_t*>(ws) + decode_prequant_offset();  // its fixed place in the workspace
         }
@@ -747,14 +756,9 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
         return Q4FC_ELIMIT;
     }
 
-    // ---- shape of the launch: K split (clusters) only when one input's stripes alone cannot fill the GPU
-    const int sms = di->sm_count;
     const int BS = block_bytes(qtype, G);
     const int SB = kRW * (G == 32 ? 4 : 1);
     p.slot_bytes = SB * BS;
-    int cs = 1;
-    if (p.ninputs == 1)
-        while (cs < 8 && cs * 2 <= kg_max && ng_total * cs * 2 <= sms) cs *= 2;
     size_t fixed = 0;
     int nc = 0;
     for (;; cs *= 2) {

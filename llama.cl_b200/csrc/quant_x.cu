@@ -177,8 +177,8 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_tile_kernel(const float
 }
 
 // Quantizer in front of the decode FC when rows x K is large.  The decode kernel normally quantizes the
-// activations itself, every cluster for itself; beyond a few tens of thousands of values that repeated work
-// costs more than one extra small launch.  One warp owns 128 consecutive k of ONE row, so the whole input is
+// activations itself, every cluster for itself; from 16K values (quantizes_in_front in fc_decode_ring_impl.cuh)
+// that repeated work costs more than one extra small launch.  One warp owns 128 consecutive k of ONE row, so the whole input is
 // spread over hundreds of warps and the kernel is a single short latency chain.  Codes and scales follow
 // the same rules as quant_x_kernel; the group sums are formed in exactly the order of the decode kernel's
 // own quantizer (four values per lane in k order, then a butterfly over the group's lanes), so the FC

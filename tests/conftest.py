@@ -1,3 +1,4 @@
+import ctypes
 import os
 import sys
 
@@ -12,6 +13,13 @@ GOLDEN = os.path.join(ROOT, "tests", "golden")
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200); run with -m gpu")
+
+
+def graph_nodes(graph) -> int:
+    """Nodes of a torch.cuda.CUDAGraph(keep_graph=True): how many launches (and copies) the captured calls make."""
+    n = ctypes.c_size_t()
+    assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(n)) == 0
+    return n.value
 
 
 @pytest.fixture(scope="session")

@@ -12,6 +12,8 @@ import numpy as np
 import pytest
 import torch
 
+from conftest import graph_nodes
+
 pytestmark = pytest.mark.gpu
 
 VARIANTS = [(0, 32), (0, 128), (1, 32), (1, 128)]
@@ -452,7 +454,9 @@ def test_decode_prequantized_path_equals_fused_quantizer(lib_built, qname, q, G,
     g = torch.Generator().manual_seed(77)
     s = torch.cuda.current_stream().cuda_stream
     flags = 1 if signed else 0
-    for (N, K, rows) in [(4096, 11008, 8), (1000, 11008, 4), (640, 6152, 8), (96, 8192, 6)]:
+    # (the last five: 16384 values and one K group less, N for K divided by 1, 2 and 8; 40960 with K divided by 8, and less)
+    for (N, K, rows) in [(4096, 11008, 8), (1000, 11008, 4), (640, 6152, 8), (96, 8192, 6), (4200, 4096, 4), (2000, 8192, 2),
+                         (1300, 2048, 8), (4100, 4064, 4), (1300, 16352, 1), (96, 4096, 8), (500, 8192, 5)]:
         W = (torch.randn(N, K, generator=g) * 0.02).cuda()
         wq = pkg.llmops.offline_FC_quant_Q4A(W, qtype=qname, group_k=G)
         Ng, Kg, _ = wq.shape
@@ -467,7 +471,12 @@ def test_decode_prequantized_path_equals_fused_quantizer(lib_built, qname, q, G,
             assert rc == 0, L.q4fc_last_error()
             outs.append(y)
         torch.cuda.synchronize()
-        assert rows * K >= 40 * 1024  # the sizes above are meant to take the separate launch
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            assert 0 == L.q4fc_fc_decode(x.data_ptr(), rows, K, K, wq.data_ptr(), Ng, Kg, q, G, N, y.data_ptr(), N, ws.data_ptr(),
+                                         nbytes, flags, torch.cuda.current_stream().cuda_stream)
+        in_front = rows * K >= (40 * 1024 if N <= 576 else 16 * 1024)  # 148 SMs: up to 18 stripes K is divided by eight
+        assert graph_nodes(graph) == (2 if in_front else 1), (N, K, rows)
         assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]), (N, K, rows)
         want = pkg.llmops.fc_Q4A(x, wq, N, path="streamk", nibble_signed=signed)
         assert torch.allclose(outs[1], want, rtol=1e-3, atol=1e-4)

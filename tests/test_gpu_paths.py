@@ -7,6 +7,8 @@ import numpy as np
 import pytest
 import torch
 
+from conftest import graph_nodes
+
 pytestmark = pytest.mark.gpu
 
 
@@ -262,13 +264,6 @@ def test_many_rows_divisions_and_long_k(pkg, oracle, fmt, rows, N, K):
 def test_many_rows_last_tiles_divided(pkg, oracle, fmt, rows, N, K):
     """Tiles left over after whole rounds go in a launch of their own with K divided (tolerance as above)."""
     check_many_rows(pkg, oracle, fmt, rows, N, K, launches=3)  # the quantizer, whole rounds, the remainder
-
-
-def graph_nodes(graph):
-    """Nodes of a captured graph."""
-    n = ctypes.c_size_t()
-    assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(n)) == 0
-    return n.value
 
 
 def early_edges(graph):
