@@ -197,9 +197,10 @@ def test_stack_on_the_chain(pkg, oracle, rows):
 
 def test_chain_argument_checks(pkg):
     ops = pkg.llmops
-    W = ops.offline_FC_quant_Q4A(torch.randn(64, 64).cuda(), qtype="q4_1", group_k=32)
-    W2 = ops.offline_FC_quant_Q4A(torch.randn(64, 64).cuda(), qtype="q4_0", group_k=32)
-    x = torch.randn(1, 2, 64).cuda()
+    g = torch.Generator().manual_seed(12)
+    w, x = torch.randn(64, 64, generator=g).cuda(), torch.randn(1, 2, 64, generator=g).cuda()
+    W = ops.offline_FC_quant_Q4A(w, qtype="q4_1", group_k=32)
+    W2 = ops.offline_FC_quant_Q4A(torch.randn(64, 64, generator=g).cuda(), qtype="q4_0", group_k=32)
     y = torch.empty(1, 2, 64).cuda()
     with pytest.raises(RuntimeError):
         ops.FCChain([])
@@ -217,4 +218,9 @@ def test_chain_argument_checks(pkg):
     c = ops.FCChain([dict(x=x, jobs=[(W, 64, y)])])  # a chain of one step is a plain FC
     c.run()
     c.check()
-    assert np.allclose(y.cpu().numpy(), ops.fc_Q4A(x, W, 64).cpu().numpy(), rtol=1e-5, atol=1e-6)
+    # The same codes, scales and integers, the four terms of a sum (two groups, scale * I and minimum * sum of x in each) in
+    # another order: at most eight roundings on either side, each 2^-24 of a value of at most the terms' sum of magnitudes,
+    # 2 max|w| of the quantized and max|w| of the given sum of |x| (a code's rounding: 1/254 of its group's largest; fp16
+    # scales: 2^-11).
+    largest = 3.002 * w.abs().max() * (x.abs().sum(2).max() + 64 * x.abs().max() / 254)
+    assert (y - ops.fc_Q4A(x, W, 64)).abs().max() <= 16 * 2.0**-24 * largest
