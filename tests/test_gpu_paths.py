@@ -492,40 +492,6 @@ def test_pack_scales_at_the_ends(pkg, oracle, qtype, G, N, K):
     assert np.array_equal(got, want)
 
 
-@pytest.mark.parametrize("rows", [1, 8, 20])
-def test_kernels_that_start_early_wait_for_their_inputs(pkg, rows):
-    """Weights, activations and ids written by the kernel directly in front, again and again in the same buffers, give what they
-    give after a synchronisation."""
-    ops, g = pkg.llmops, torch.Generator().manual_seed(rows)
-    K = N = 2048
-    packed = [ops.offline_FC_quant_Q4A((torch.randn(N, K, generator=g) * 0.02).cuda()) for _ in range(2)]
-    q8 = [pkg.c_ext.FC_quant_Q8C((torch.randn(N, K, generator=g) * 0.02).cuda()) for _ in range(2)]
-    xs = [torch.randn(1, rows, K, generator=g).cuda() for _ in range(2)]
-    table = pkg.ops.llmop_embedding_q8c(torch.randn(100, K, generator=g).cuda())
-    ids = [torch.randint(0, 100, (1, rows), generator=g).cuda() for _ in range(2)]
-    w, w8, s8, x, i = packed[0].clone(), q8[0][0].clone(), q8[0][1].clone(), xs[0].clone(), ids[0].clone()
-
-    def step(k, wait):
-        out = []
-        for dst, src, f in ((w, packed[k], lambda: ops.fc_Q4A(x, w, N)), (x, xs[k], lambda: ops.fc_Q4A(x, w, N)),
-                            (w8, q8[k][0], lambda: pkg.c_ext.FC_evaluate_Q8C(x, w8, s8, N)),
-                            (s8, q8[k][1], lambda: pkg.c_ext.FC_evaluate_Q8C(x, w8, s8, N)), (i, ids[k], lambda: table(i))):
-            dst.copy_(src)
-            if wait:
-                torch.cuda.synchronize()
-            out.append(f())
-            if wait:
-                torch.cuda.synchronize()
-        out.append(ops.fc_Q4A(ops.fc_Q4A(out[0], w, N), w, N))
-        return out
-
-    step(1, True)
-    want = [step(k, True) for k in (0, 1)]
-    got = [step(k % 2, False) for k in range(20)]
-    for k in range(20):
-        assert all(torch.equal(a, b) for a, b in zip(got[k], want[k % 2]))
-
-
 class EarlyWriter:
     """Rewrites a buffer with one of two contents by the embedding look-up, which lets its successor begin at once and then
     stores for as long as it takes: few CTAs, so that others find places beside them.  The values are whole numbers in fp32:
@@ -540,6 +506,121 @@ class EarlyWriter:
 
     def __call__(self, k):
         self.pkg.llmops.embedding_q8c(self.out, self.ids[k], self.table, self.scales)
+
+
+def alternating(step):
+    """step(k, wait) twenty times for k = 0, 1, 0, ... without a wait or copy in between gives what it gives with waits (the same
+    kernels on the same inputs: equal)."""
+    step(1, True)
+    want = [step(k, True) for k in (0, 1)]
+    assert not torch.equal(want[0][-1], want[1][-1])
+    got = [step(k % 2, False) for k in range(20)]
+    torch.cuda.synchronize()
+    for k in range(20):
+        assert all(torch.equal(a, b) for a, b in zip(got[k], want[k % 2]))
+
+
+EARLY_READERS = {  # what is written in front: its bytes, by how many CTAs, and who reads it
+    **{f"weights, {rows} rows": (64 * 64 * 640, 16, lambda t, o, rows=rows: t.fc(t.x(rows, 2048), o.view(torch.int8).view(64, 64, 640), 2048))
+       for rows in (1, 8, 20, 300)},
+    **{f"activations, {rows} rows": (rows * 2048 * 4, 1 if rows < 4 else 4, lambda t, o, rows=rows: t.fc(o.view(1, rows, 2048), t.w, 2048))
+       for rows in (1, 2, 8, 20, 300)},
+    "activations, 129 rows and a remainder": (129 * 2080 * 4, 8, lambda t, o: t.fc(o.view(1, 129, 2080), t.wide, 9500)),
+    **{f"int8 weights, {rows} rows": (64 * 64 * 1024, 16, lambda t, o, rows=rows: t.q8(t.x(rows, 2048), o.view(torch.int8).view(64, 64, 1024), t.s8))
+       for rows in (1, 8, 300)},
+    **{f"int8 scales, {rows} rows": (2048 * 4, 1, lambda t, o, rows=rows: t.q8(t.x(rows, 2048), t.w8, o.view(2048))) for rows in (1, 300)},
+    **{f"int8 activations, {rows} rows": (rows * 2048 * 4, 1, lambda t, o, rows=rows: t.q8(o.view(1, rows, 2048), t.w8, t.s8))
+       for rows in (1, 300)},
+    "quantizer": (8 * 2048 * 4, 4, lambda t, o: t.ops.quantize_activations(o.view(1, 8, 2048), 32).codes()),
+    "quantizer of its own": (20 * 2048 * 4, 4, lambda t, o: t.ops.FC_dynamic_quantize_x(o.view(20, 2048), 32)[0]),
+    "table": (100 * 2048, 4, lambda t, o: t.look_up(o.view(torch.int8).view(100, 2048), t.s8[:100])),
+    "table scales": (400, 1, lambda t, o: t.look_up(t.table, o.view(100))),
+}
+
+
+class EarlyInputs:
+    def __init__(self, pkg):
+        self.ops, self.q8c, self.g = pkg.llmops, pkg.c_ext, torch.Generator(device="cuda").manual_seed(2)
+        r = lambda *s: torch.randn(*s, generator=self.g, device="cuda")
+        self.w, self.wide = (self.ops.offline_FC_quant_Q4A(r(*s) * 0.02) for s in ((2048, 2048), (9500, 2080)))
+        self.w8, self.s8 = pkg.c_ext.FC_quant_Q8C(r(2048, 2048) * 0.02)
+        self.table = torch.randint(-127, 128, (100, 2048), generator=self.g, device="cuda").to(torch.int8)
+        self.ids, self.kept = torch.arange(99, -1, -1, device="cuda"), {}
+        self.wait = False
+        self.fc = lambda x, w, N: self.done(self.ops.fc_Q4A(x, w, N))
+        self.q8 = lambda x, w, s: self.done(pkg.c_ext.FC_evaluate_Q8C(x, w, s, 2048))
+
+    def done(self, result):
+        if self.wait:
+            torch.cuda.synchronize()
+        return result
+
+    def x(self, rows, K):
+        if (rows, K) not in self.kept:
+            self.kept[rows, K] = torch.randn(1, rows, K, generator=self.g, device="cuda")
+        return self.kept[rows, K]
+
+    def look_up(self, table, scales):
+        out = torch.empty(100, 2048, device="cuda")
+        self.ops.embedding_q8c(out, self.ids, table, scales)
+        return self.done(out)
+
+
+@pytest.mark.parametrize("reader", EARLY_READERS)
+def test_kernels_that_begin_early_wait_for_their_inputs(pkg, reader):
+    """Weights, activations, scales and tables written by a kernel directly in front that releases its successor at once, again
+    and again in the same buffer, which the reader of the time before may still read."""
+    nbytes, ctas, read = EARLY_READERS[reader]
+    t, write = EarlyInputs(pkg), EarlyWriter(pkg, nbytes, ctas, 5)
+    t.x(1, 2048)
+
+    def step(k, wait):
+        t.wait = wait
+        t.done(write(k))
+        return [t.done(read(t, write.out))]
+
+    alternating(step)
+
+
+def test_kernels_that_begin_early_behind_one_another(pkg):
+    """Chains of calls, each reading what the one in front computes, in memory that calls before them have used."""
+    t, ops = EarlyInputs(pkg), pkg.llmops
+    pack = lambda N, K: ops.offline_FC_quant_Q4A(torch.randn(N, K, generator=t.g, device="cuda") * 0.02)
+    narrow = pack(64, 9500)
+    xs = [{rows: torch.randn(1, rows, K, generator=t.g, device="cuda") for rows, K in ((1, 2048), (8, 2048), (20, 2048), (129, 2080))}
+          for _ in range(2)]
+    # ids from the quantizer: eight bytes each, the first of every group the 127 that makes the scale one
+    ids = torch.randint(0, 127, (2, 8, 64, 4), generator=torch.Generator().manual_seed(1))
+    ids[..., 0] = 127
+    as_bytes = [ids[k].view(torch.int8).view(8, 2048).float().cuda() for k in (0, 1)]
+    big = torch.randint(-127, 128, (128, 2048), generator=torch.Generator().manual_seed(1)).to(torch.int8).cuda()
+    ones = torch.ones(128, device="cuda")
+
+    ids_of = lambda k: t.done(ops.FC_dynamic_quantize_x(as_bytes[k], 32)[0]).view(torch.int64)
+    codes = lambda x: t.done(ops.quantize_activations(x, 32)).codes()
+
+    def look_up(i):
+        out = torch.empty(*i.shape, 2048, device="cuda")
+        ops.embedding_q8c(out, i, big, ones)
+        return t.done(out)
+
+    chains = [
+        lambda k: t.fc(t.q8(t.fc(xs[k][8], t.w, 2048), t.w8, t.s8), t.w, 2048),
+        lambda k: codes(t.fc(t.fc(xs[k][1], t.w, 2048), t.w, 2048)),
+        lambda k: t.q8(t.fc(t.fc(xs[k][20], t.w, 2048), t.w, 2048), t.w8, t.s8),
+        lambda k: t.fc(t.fc(xs[k][129], t.wide, 9500)[:, :8], narrow, 64),  # (129 rows: with a remainder)
+        lambda k: t.fc(xs[k][129], t.wide, 9500),
+        lambda k: t.fc(look_up(ids_of(k).view(-1)[:8]).view(1, 8, 2048), t.w, 2048),
+        lambda k: look_up(ids_of(k)),
+    ]
+
+    def step(k, wait):
+        t.wait = wait
+        return [f(k) for f in chains]
+
+    assert torch.equal(look_up(ids_of(0)), big[ids[0].view(8, 256).cuda()].float())
+    alternating(step)
+    pkg.llmops.check_device_status()
 
 
 @pytest.mark.parametrize("reader", ["multi", "batch"])
@@ -572,8 +653,4 @@ def test_calls_without_the_flag_hold_a_flagged_successor_back(pkg, between, read
                 torch.cuda.synchronize()
         return out[1:]
 
-    want = [step(k, True) for k in (0, 1)]
-    assert not torch.equal(want[0][1], want[1][1])
-    got = [step(k % 2, False) for k in range(20)]
-    for k in range(20):
-        assert all(torch.equal(a, b) for a, b in zip(got[k], want[k % 2]))
+    alternating(step)
