@@ -913,16 +913,20 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     if (tiles < places) {
         split = places / tiles < most ? places / tiles : most;
     } else if (tiles % places != 0) {
-        // What is left after whole rounds over the places would take a round of its own, most places empty.  With K divided it
-        // takes ceil(left * c / places) rounds of 1/c, each with some stages' time for start-up and the adding; larger clusters
-        // do not fit everywhere.  (11008 columns, K = 4096: 512 rows, group 32, 48 of 344 tiles left, 220 -> 187 us; 256 rows, Q8C, 24
-        // of 172, 148 -> 100; 256 rows, group 128, 64 -> 47; 100 rows x 20000, group 32, 18 of 314, 180 -> 106.  Divided where this
-        // sum says no: 1000 rows, 96 of 688, Q8C, 360 -> 394.)
+        // What is left after whole rounds over the places would take a round of its own, most places empty.  With K divided by c it
+        // takes 1/c of one, and some stages' time for start-up and the adding, where that many clusters run at once.  (11008
+        // columns, K = 4096: 512 rows, group 32, 48 of 344 tiles left, 217 -> 186 us; 256 rows, Q8C, 24 of 172, 148 -> 100; 256 rows,
+        // group 128, 61 -> 47; 100 rows x 20000, group 32, 18 of 314, 174 -> 106.  Divided where this sum says no: 1000 rows, 96
+        // of 688, Q8C, 360 -> 394.)
         left = tiles % places;
         int64_t best = nstage;  // undivided, in the launch of the others
         for (int64_t c = 2; c <= most; c++) {
-            const int64_t fit = c == 2 ? places : c <= 4 ? places * 15 / 16 : places * 13 / 16;
-            const int64_t cost = (left * c + fit - 1) / fit * ((nstage + c - 1) / c + (G == 128 ? 8 : 4));
+            // Clusters of 2 .. 8 CTAs that run at once on 148 SMs, one CTA on an SM (two: twice as many at least): by the number of
+            // tiles left from which on the launch takes longer (rows x 4096, group 32: 33 tiles by four 100.5 us, 34 120.6; 22 by
+            // six 97.5, 23 114.3; 42 by three 112, 44 129).
+            constexpr int kAtOnce[kMaxSplit - 1] = {74, 42, 33, 24, 22, 15, 15};
+            const int64_t fit = kAtOnce[c - 2] * places / 148;
+            const int64_t cost = (left + fit - 1) / fit * ((nstage + c - 1) / c + (G == 128 ? 8 : 4));
             if (cost < best) best = cost, left_split = c;
         }
         if (left_split == 1) left = 0;

@@ -257,6 +257,7 @@ def test_many_rows_divisions_and_long_k(pkg, oracle, fmt, rows, N, K):
 
 @pytest.mark.parametrize("rows,N,K", [
     (129, 9500, 2080),    # 150 tiles of 128 rows on 148 SMs: two left, K divided by four, the last stage one group
+    (150, 11648, 2080),   # 182 tiles, 34 left: K divided by three
     (6500, 300, 2080),    # 153 tiles, five left over three column tiles: the launch's rows of tiles wrap, the last is not full
     (20, 37900, 2084),    # 297 tiles of 64 rows on 296 places: one left, columns and k beyond the weights
 ])
