@@ -10,7 +10,7 @@
 // boundary in it.  When a single input has fewer stripes than half the SMs, a thread-block cluster of cs CTAs
 // shares a stripe range and CTA rank j takes the K slice [j*Kg/cs, (j+1)*Kg/cs) of each of them.
 //
-// Streaming.  Warp 8 is the producer: one thread walks the CTA's byte stream and issues 1-D bulk copies
+// Streaming.  Warp 16 is the producer: one thread walks the CTA's byte stream and issues 1-D bulk copies
 // (cp.async.bulk, global -> shared, completion counted on an mbarrier; this GPU's own memory, no multicast) of
 // up to SB blocks each into a ring of `depth` slots, as far ahead as the ring allows -- on B200 that is up to
 // ~190 KB per SM in flight with no register cost, and for most Llama-7B shapes the CTA's whole share.  The
@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(kRThreads, 1) fc_decode_ring_kernel(const __gr
     }
     __syncwarp();
     // The next launch may begin, and where its caller set Q4FC_FLAG_PDL read its weights, as soon as every CTA says so.  Here only
-    // where everything in front of this call's first launch is complete already or the caller vouches for it; else behind the wait.
+    // where everything in front of this call's first launch is complete already or the caller vouches for it; else behind the wait,
+    // below.
     if (TP || p.weights_early) pdl_launch_dependents();
     // "this CTA runs": nobody may store into a CTA's shared memory before that CTA has started
     if (cs > 1 || bq > 1) cluster_arrive_release();
@@ -334,7 +335,6 @@ __global__ void __launch_bounds__(kRThreads, 1) fc_decode_ring_kernel(const __gr
             // where weights do not depend on the preceding kernel: fill the ring now
             if (!p.weights_early) pdl_wait_prior_grid();
             while (p_filled < depth && p_li < r) issue_slot(), p_filled++;
-            if (!TP && !p.weights_early) pdl_launch_dependents();
             if constexpr (PREQ) {
                 pdl_wait_prior_grid();
                 if (r > 0) {
@@ -386,6 +386,9 @@ __global__ void __launch_bounds__(kRThreads, 1) fc_decode_ring_kernel(const __gr
 
     if (warp == kRW) {
         if (lane == 0) {
+            // (behind the wait and the barrier: 1 row x 4096 x 4096, group 32, call after call 5.8 us; in front of the first copies or
+            // right behind them 5.9, 1 x 11008 x 4096 10.4 and 10.8, 1 x 1024 x 512 4.6 and 4.9; at once, as it used to be, 5.9, 10.4, 4.8)
+            if (!TP && !p.weights_early) pdl_launch_dependents();
             // refill: a slot is reused once all consumer warps have taken their blocks out of it
             uint32_t eph = 0;  // parity of the empty barrier's completion to wait for
             int wrapped = 0;
