@@ -127,24 +127,17 @@ size_t q8c_prefill_scale_bytes(int64_t rows, int64_t Kg);
 int launch_q8c_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, const int8_t* wq, const float* wscales,
                        int64_t Ng, int64_t Kg, int64_t N, float* y, int64_t ldy, int8_t* codes, float* sc, cudaStream_t s);
 
-// Whether a launch of `kernel`, small work that waits for what is in front of it, should begin before that has ended.  Eagerly:
-// yes.  In a capture only behind one other kernel that nothing else follows yet: a graph runs a node that begins early in one
-// line with the node in front, so that work prepared on a side branch (one quantizer behind the other, FCs behind each of them)
-// would wait for the FCs beside it.  (Four quantizers beside four FC launches 121.6 -> 112.6 us; in one line with them 126.4 as
-// without this rule, never early 129.2 and, as the decode FCs' own quantizers too, 4 rows x 4096 x 4096 7.6 -> 8.1.)
-bool begins_early(cudaStream_t s, const void* kernel);
-
 // A launch that may begin before the kernel in front of it has ended: the kernel waits (pdl_wait_prior_grid) before it touches
 // global memory, and lets its own successor begin only after that wait, so that a successor which begins early finds everything
 // in front of this kernel complete.
 struct DependentLaunch {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr = {};
-    DependentLaunch(const void* kernel, dim3 grid, unsigned threads, cudaStream_t s, bool always = false) {
+    DependentLaunch(dim3 grid, unsigned threads, cudaStream_t s, bool early = true) {
         cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.stream = s;
         attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr, cfg.numAttrs = always || begins_early(s, kernel);
+        cfg.attrs = &attr, cfg.numAttrs = early;
     }
     DependentLaunch(const DependentLaunch&) = delete;
 };

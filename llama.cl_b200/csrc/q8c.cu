@@ -376,8 +376,7 @@ int launch_emb_q8c(const void* ids, int ids_are_i32, int64_t n, const int8_t* co
     const int vec_ok = (E % 4 == 0) && (ldo % 4 == 0) && ((reinterpret_cast<uintptr_t>(codes) & 3) == 0) &&
                        ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
     int* status = ring_status_word();
-    DependentLaunch l(ids_are_i32 ? reinterpret_cast<const void*>(&emb_q8c_kernel<int32_t>)
-                                  : reinterpret_cast<const void*>(&emb_q8c_kernel<int64_t>), dim3((unsigned)n), 128, s);
+    DependentLaunch l(dim3((unsigned)n), 128, s);
     if (ids_are_i32)
         Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, emb_q8c_kernel<int32_t>, static_cast<const int32_t*>(ids), codes, scales, V, E, out,
                                         ldo, vec_ok, status));
