@@ -118,6 +118,9 @@ int q4fc_quant_x(const float* x, int64_t rows, int64_t K, int64_t ldx, int group
  *   q4fc_fc_decode  rows <= 8: weight-streaming GEMV, HBM-bound.
  *   q4fc_fc_prefill any rows:  int8 tensor-core GEMM.
  *   q4fc_fc         picks one of the two.
+ * The sums over K groups have a fixed order, the same from run to run.  It
+ * depends on the sizes and, in the GEMM (q4fc_q8c_fc's too), on where in y an
+ * output lies: equal rows of x in one call may differ in the last place.
  * ws: workspace of at least q4fc_fc_workspace_bytes() bytes, 256-byte
  * aligned, zeroed once with q4fc_fc_workspace_init() before its first use;
  * the kernels leave it ready for the next call.  Calls that may overlap on

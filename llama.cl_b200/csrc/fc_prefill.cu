@@ -18,7 +18,8 @@
 //   * operand B = activation codes (int8), same layout, straight from the code matrix by TMA;
 //   * D = int32 accumulators in tensor memory, lane = weight column, column = activation row.
 // Every K group has its own pair of scales, so a group's MMA(s) (one K=32 instruction for group 32, four for group
-// 128) write a fresh TMEM buffer (4 buffers of TM columns), and the epilogue warps read the buffer back with
+// 128) write a fresh TMEM buffer (four of TM columns, three where the fourth's place holds weights or Q8C's sums), and the
+// epilogue warps read the buffer back with
 // tcgen05.ld, turn the exact integers into fp32, scale them and accumulate the tile in registers.
 //
 // What bounds it: the CUDA-core work per (m, n, group) -- one conversion, one mul, one or two fma -- against 32 or 128
@@ -28,15 +29,15 @@
 // reads four rows per load, and weights, codes and scales have rings of their own, so that operands are released by the
 // MMA and not by the epilogue.
 //
-// Measured (whole call, quantizer included; before: unpacking straight from global memory without prefetch, one 128 x 128
-// tile per CTA whatever the row count, epilogue of 5 operations per integer):
-//   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 us   Q4_0 g32, 512 rows 280 -> 223 us (207 TOPS)
-//                   Q4_1 g128, 2048 rows 517 -> 323 us (572 TOPS)   Q8C, 256 rows 296 -> 151 us (153 TOPS)
-// and, with K divided where the last round over the SMs would be nearly empty: 512 rows 187 us, 2048 rows 311, 256 rows 100.
+// Measured (whole call, quantizer included; unpacking straight from global memory without prefetch, one 128 x 128 tile per CTA
+// whatever the row count, epilogue of 5 operations per integer -> this form -> with the last tiles divided, below, and weights in
+// tensor memory):
+//   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 -> 38.8 us   Q4_0 g32, 512 rows 280 -> 223 -> 186 us (248 TOPS)
+//                   Q4_1 g128, 2048 rows 517 -> 323 -> 296 us (624 TOPS)   Q8C, 256 rows 296 -> 151 -> 101 us (228 TOPS)
 // A group of 32 k takes about 1100 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
-// convert, scale is latency-bound with the 16 warps that the registers allow (512 rows: issue slots 65 % busy, ALU 46 %, FMA
-// 41 %, XU, where the conversions are not, 0.2 %; per issue 2.2 warps wait for tensor or shared memory, 1.7 for the
-// instruction before).  Tried and dropped: handing registers
+// convert, scale is latency-bound with the 16 warps that the registers allow (512 rows: issue slots 65 % busy, ALU 45 %, FMA
+// 43 %, XU, where the conversions are not, 0.2 %; per issue 2.1 warps wait for tensor or shared memory, 1.7 for the
+// instruction before).  Tried and dropped, in the 223 us form: handing registers
 // between roles with setmaxnreg (spills around it; 260 us for the 512-row case), both chunks in registers at once
 // (320 us), the add-a-constant conversion instead of I2F (30 % more issue slots), scalar instead of packed fp32 (5 % slower).
 //
@@ -48,11 +49,12 @@
 // less exact than that (K = 4096: 2.0e-7 of the result in the 2-norm, with 8 warps' chains 9.6e-8; K = 11008: 3.3e-7 and
 // 1.3e-7).  After 8 groups, or 12 where a CTA has more than 64, a thread moves its running sums to a second place and keeps
 // what that addition rounds off: 6.5e-8 to 7.5e-8 for K from 512 to 11008, below the 8-warp sums at every size tried.  It
-// costs 131 -> 151 us at 256 rows x 4096 x 11008 and 33 -> 35 at 37 rows; every 16 groups 146 us and 8.3e-8, at K = 3001 not
+// cost 131 -> 151 us at 256 rows x 4096 x 11008 (before the last tiles were divided) and 33 -> 35 at 37 rows; every 16 groups 146 us and 8.3e-8, at K = 3001 not
 // below the 8-warp sums.  (Staggering the moves over the warps: 156; as an outer loop around the groups' loop: 157.)
 //
 // Few tiles, or the last of many: a cluster of `split` CTAs shares a tile and divides its K stages; the partial tiles meet in shared memory
-// and are added in rank order (fixed order, no atomics).
+// and are added in rank order (fixed order, no atomics).  So the outputs of one call can be sums in two orders: equal rows of x, or
+// equal columns of W, in whole rounds and in the remainder may differ in the last place.
 #include <cuda.h>  // CUtensorMap and the cuTensorMapEncodeTiled prototype (resolved at run time, libcuda is not linked)
 
 #include <cooperative_groups.h>
@@ -900,11 +902,13 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     }
     const int64_t n_tiles = (p.N + kTileN - 1) / kTileN;
     const int64_t nstage = (Kp + kStageK - 1) / kStageK;
-    // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM and can share K out: the large tile as
-    // soon as such tiles occupy every SM (512 rows x 11008 columns, group 32: 223 us, with 64 rows 234; 256 rows, Q8C:
-    // equal; 200 x 4096, group 128: 37 us on 64 CTAs, 64-row tiles with K halved 29).  K is divided while that fills the
-    // two places on every SM and leaves a CTA four stages (37 rows x 11008: 78 us undivided, 62 by two, 41 by three, 55 by
-    // four, which needs a second wave).
+    // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM: the large tile as soon as such tiles occupy
+    // every SM (512 rows x 4096 x 11008, group 32: 186 us, with 64 rows 209; 256 rows, Q8C: 102 and 108), the small one for less
+    // work (320 x 2048 x 2048, group 32: 27.8 us, with 128 rows 35.6).  Over 264 sizes (65 to 1024 rows, K x N from 1000 x 9000 to
+    // 11008 x 4096) that line costs 4.5 % against the better of the two, with group 128 9 %: from half the SMs on large tiles with K
+    // divided are ahead (group 128, 512 x 4096 x 4096: 44.2 us, with 128 rows 34.9; group 32, 512 x 11008 x 4096 225 and 201).  K is
+    // divided while that fills the two places on every SM and leaves a CTA four stages (37 rows x 11008: 78 us undivided, 62 by
+    // two, 41 by three, 55 by four, which needs a second wave).
     const int tile = (rows > 64 && n_tiles * ((rows + 127) / 128) >= di->sm_count) ? 128 : 64;
     const int64_t m_tiles = (rows + tile - 1) / tile;
     const int64_t tiles = n_tiles * m_tiles, places = (tile == 128 ? 1 : 2) * (int64_t)di->sm_count;

@@ -324,10 +324,12 @@ int launch_q8c_fc(const float* x, int64_t rows, int64_t K, int64_t ldx, const in
     int split = 1;
     while (split < kMaxSplit && stripes * split < 2 * (int64_t)di->sm_count && Kg / (2 * split) >= kFcWarps) split *= 2;
     // The tensor-core GEMM takes over beyond 16 rows as soon as this kernel's CTAs no longer find a place all at once, two
-    // on an SM (96 rows x 512 x 512: 5 us here, 12 there; 512 x 4096: 22 and 12; 256 x 4096 x 11008: 296 and 151).  Over 819
-    // sizes (K and N from 512 to 11008 and 30000, 17 to 128 rows) that line costs 0.6 % against the better of the two.  Up to
-    // 16 rows the weight stream decides and this kernel is ahead, with 16 rows in a CTA (9 x 4096 x 4096: 12 us, GEMM 15; 9 x
-    // 11008 x 30000: 108 and 148; behind only at 13 to 16 rows x 11008 columns, 27 and 25 at K = 4096).
+    // on an SM (17 rows x 768 x 1664: 6 us here, 13 there; 105 x 6763 x 3330: 106 and 37).  Over 540 sizes (K
+    // from 512 to 11008, N to 32000, 9 to 128 rows) that line costs 0.8 % against the better of the two, 200 or 350 CTAs 1.9 %, a
+    // line from 9 rows on 1.8 %; it is behind by 27 % at most, just on it (32 x 8732 x 2354, 296 CTAs: 32 and 25; 34 x 768 x
+    // 2432, 304 CTAs: 12 and 15).  Up to 16 rows the weight stream decides and this kernel is ahead, with 16 rows in a CTA (9 x
+    // 4096 x 4096: 12 us, GEMM 15; 9 x 11008 x 30000: 108 and 148; behind only at 13 to 16 rows x 11008 columns, 27 and 25 at K =
+    // 4096).
     if (rows > 16 && stripes * split * tiles > 2 * (int64_t)di->sm_count)
         return launch_q8c_prefill(x, rows, K, ldx, wq, wscales, Ng, Kg, N, y, ldy, codes, xs, s);
     if (int rc = launch_quant_x(x, rows, K, ldx, 32, 1.0f, codes, xs, nullptr, s)) return rc;
