@@ -383,7 +383,9 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
 
     extern __shared__ uint8_t smem_raw[];
     // (the same offset in every CTA of a cluster: the dynamic shared memory starts at the same address)
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    // (An offset, and no cast through an integer behind which every load of a scale is a generic one: 37 rows x 4096 x 11008
+    // 39.1 -> 36.3 us, 200 x 4096 x 4096, group 128, 26.8 -> 25.5, Q8C, 512 x 4096 x 4096, 86.5 -> 82.0.)
+    uint8_t* smem = smem_raw + (-smem_u32(smem_raw) & 1023u);
     uint8_t* bars = smem + S::kBarOff;
     const uint32_t smem0 = smem_u32(smem);
     const uint32_t bar_raw = smem0 + S::kBarOff;  // [raw stage][stripe]
