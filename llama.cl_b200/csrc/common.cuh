@@ -57,9 +57,12 @@ int launch_dequant(const uint8_t* wq, int64_t Ng, int64_t Kg, int qtype, int G, 
                    cudaStream_t s);
 int launch_quant_x(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, float scale, int8_t* codes,
                    float* scales, float* gsums, cudaStream_t s);
-// the prefill GEMM's quantizer: scales (and group sums) by row tile of 64 or 128 (quant_x.cu)
-int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, bool sums, int tile, int8_t* codes,
-                        float* sc, cudaStream_t s);
+// the prefill GEMM's quantizer (quant_x.cu): scales (and group sums) by row tile of 64 or 128; codes int8 or, with `f16` (group
+// 32), fp16 against nibbles that stand in the lowest eight places of an fp16 as they are (n x 2^-24, or n x 2^-20 four places
+// up): eight k in the order 0,2,4,6,1,3,5,7, those with k % 8 < 4 times 256 and the others times 16, so that both products are
+// n x code x 2^-16, and the scales times 64 (which no finite row overflows); 2^10 in the weights' scales make up the rest.
+int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, bool sums, int tile, bool f16,
+                        int8_t* codes, float* sc, cudaStream_t s);
 constexpr size_t kWsCounterCapacity = 64 * 1024;  // stripe counters of N <= 524288 end before the quantizer scratch
 size_t decode_workspace_bytes(int64_t N);
 size_t decode_prequant_offset();

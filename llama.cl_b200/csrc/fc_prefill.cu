@@ -7,18 +7,16 @@
 //   I[m,n,kb] = sum_{k in group kb} weight code(n,k) * activation code(m,k)      exact int32
 //
 // Two launches: quant_x_tile_kernel (quant_x.cu) writes codes, scales and group sums of all rows to the workspace; this
-// kernel, started while that one runs (programmatic launch: its weight copies do not depend on it), runs the GEMM.
+// kernel, or that of fc_prefill_wide.cu (128-row tiles of Q4 weights), started while that one runs (programmatic launch: its weight
+// copies do not depend on it), runs the GEMM.
 //
-// One CTA computes 128 columns n x TM rows m:
+// One CTA computes 128 columns n x TM rows m, 64, or of Q8C weights also 128:
 //   * operand A = weights: the packed blocks come in by bulk copies, are unpacked to one byte per weight in shared
 //     memory, K-major rows of 128 bytes, in the 128-byte-swizzle canonical layout that tcgen05.mma reads;
-//     Group 128 in 128-row tiles: in tensor memory instead, in the fourth result buffer's place (a group's four MMAs and its
-//     long epilogue need no fourth buffer; 2048 rows x 4096 x 11008 312 -> 297 us, 512 rows 85 -> 82.  With group 32 the three
-//     buffers cost more than that: Q8C, 256 rows, 148 -> 176 undivided);
 //   * operand B = activation codes (int8), same layout, straight from the code matrix by TMA;
 //   * D = int32 accumulators in tensor memory, lane = weight column, column = activation row.
 // Every K group has its own pair of scales, so a group's MMA(s) (one K=32 instruction for group 32, four for group
-// 128) write a fresh TMEM buffer (four of TM columns, three where the fourth's place holds weights or Q8C's sums), and the
+// 128) write a fresh TMEM buffer (four of TM columns, three where the fourth's place holds Q8C's sums), and the
 // epilogue warps read the buffer back with
 // tcgen05.ld, turn the exact integers into fp32, scale them and accumulate the tile in registers.
 //
@@ -30,16 +28,15 @@
 // MMA and not by the epilogue.
 //
 // Measured (whole call, quantizer included; unpacking straight from global memory without prefetch, one 128 x 128 tile per CTA
-// whatever the row count, epilogue of 5 operations per integer -> this form -> with the last tiles divided, below, and weights in
-// tensor memory):
-//   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 -> 38.8 us   Q4_0 g32, 512 rows 280 -> 223 -> 186 us (248 TOPS)
-//                   Q4_1 g128, 2048 rows 517 -> 323 -> 296 us (624 TOPS)   Q8C, 256 rows 296 -> 151 -> 101 us (228 TOPS)
-// A group of 32 k takes about 1100 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
-// convert, scale is latency-bound with the 16 warps that the registers allow (512 rows: issue slots 65 % busy, ALU 45 %, FMA
-// 43 %, XU, where the conversions are not, 0.2 %; per issue 2.1 warps wait for tensor or shared memory, 1.7 for the
-// instruction before).  Tried and dropped, in the 223 us form: handing registers
+// whatever the row count, epilogue of 5 operations per integer -> this form -> with the last tiles divided, below, and scales read by
+// shared-memory loads):
+//   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 -> 36.3 us   Q8C, 256 rows 296 -> 151 -> 99 us (233 TOPS)
+// With 128-row tiles of Q4 weights, before they had a kernel of their own: Q4_0 g32, 512 rows 186 us; Q4_1 g128, 2048 rows 296.
+// A group of 32 k takes about 1000 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
+// convert, scale is latency-bound with the 16 warps that the registers allow.  Tried and dropped: handing registers
 // between roles with setmaxnreg (spills around it; 260 us for the 512-row case), both chunks in registers at once
-// (320 us), the add-a-constant conversion instead of I2F (30 % more issue slots), scalar instead of packed fp32 (5 % slower).
+// (320 us), the add-a-constant conversion instead of I2F (30 % more issue slots), scalar instead of packed fp32 (5 % slower), and
+// this file's work in the form of fc_prefill_wide.cu (Q8C, 256 rows: 102; 64-row tiles, 12 x 11008 x 4096: 27.4 -> 31).
 //
 // Warp roles: epilogue (warp % 4 = TMEM lane quarter, warp / 4 = which 16-row chunks), 4 unpacking warps (one stripe
 // each), one MMA issuer, one loader.  Every wait is bounded: when a wait runs out the CTA sets the status word, every
@@ -55,28 +52,22 @@
 // Few tiles, or the last of many: a cluster of `split` CTAs shares a tile and divides its K stages; the partial tiles meet in shared memory
 // and are added in rank order (fixed order, no atomics).  So the outputs of one call can be sums in two orders: equal rows of x, or
 // equal columns of W, in whole rounds and in the remainder may differ in the last place.
-#include <cuda.h>  // CUtensorMap and the cuTensorMapEncodeTiled prototype (resolved at run time, libcuda is not linked)
-
 #include <cooperative_groups.h>
 
 #include <atomic>
 #include <cfloat>
 
-#include "common.cuh"
-#include "ring_ptx.cuh"
+#include "prefill_common.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace q4fc {
 namespace {
 
-constexpr int kTileN = 128;    // weight columns per tile = TMEM lanes
 constexpr int kStageK = 128;   // k per shared-memory stage (one 128-byte swizzle row)
 constexpr int kTmemBufs = 4;   // of a tile's columns each
 constexpr int kProdWarps = 4;  // one stripe of the tile each
 constexpr int kMaxSplit = 8;
-
-enum Format { kQ4_0 = 0, kQ4_1 = 1, kQ4_0Signed = 2, kQ8C = 3 };
 
 template <int FMT, int G, int TM>
 struct PrefillShape {
@@ -86,20 +77,19 @@ struct PrefillShape {
     static constexpr int kEpiWarps = TM / 8;              // 32 rows of the tile per warp and TMEM lane quarter
     static constexpr int kThreads = (kEpiWarps + kProdWarps + 2) * 32;
     static constexpr int kLoadWidth = TM == 128 ? 16 : 8; // rows a thread takes from tensor memory at a time
-    static constexpr bool kATmem = G == 128 && TM == 128; // unpacked weights in tensor memory, else in shared memory
-    static constexpr int kA = kATmem ? 4 : TM == 128 ? 3 : 2;  // stages of unpacked weights
+    static_assert(TM == 64 || FMT == kQ8C, "128-row tiles of Q4 weights: fc_prefill_wide.cu");
+    static constexpr int kA = TM == 128 ? 3 : 2;          // stages of unpacked weights
     static constexpr int kB = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;    // stages of activation codes
     static constexpr int kRaw = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;  // stages of packed bytes
     static constexpr int kScs = 4;                        // stages of scales
-    // buffers of integers in the kTmemBufs x TM columns (the last one's place: Q8C, sums; kATmem, weights)
-    static constexpr int kBufs = (FMT == kQ8C && TM == 64) || kATmem ? kTmemBufs - 1 : kTmemBufs;
-    static_assert(!kATmem || kA * kStageK / 4 == TM, "weights take one buffer's columns");
+    // buffers of integers in the kTmemBufs x TM columns (Q8C in 64-row tiles keeps its sums in the last one's place)
+    static constexpr int kBufs = FMT == kQ8C && TM == 64 ? kTmemBufs - 1 : kTmemBufs;
     static constexpr int kRawStripe = kGroups * kBlock;   // packed bytes of one stripe in a stage
     static constexpr int kABytes = kTileN * kStageK, kBBytes = TM * kStageK;
     static constexpr int kXscBytes = kGroups * kSums * TM * 4;                // [group][scale | sum][row] fp32
     static constexpr int kWscBytes = FMT == kQ8C ? 0 : kGroups * kTileN * 4;  // [group][n] {wd, wm} fp16
     static constexpr int kScBytes = kXscBytes + kWscBytes;
-    static constexpr int kBOff = kATmem ? 0 : kA * kABytes;
+    static constexpr int kBOff = kA * kABytes;
     static constexpr int kRawOff = kBOff + kB * kBBytes;
     static constexpr int kScOff = kRawOff + kRaw * 4 * kRawStripe;
     static constexpr int kBarOff = kScOff + kScs * kScBytes;
@@ -107,21 +97,6 @@ struct PrefillShape {
     static constexpr int kSmem = kSumOff + (FMT == kQ8C && TM == 128 ? TM * kTileN * 4 : 0) + 1024 /*alignment slack*/;
     static_assert(TM == 128 || kSmem <= 113 * 1024, "two CTAs on an SM");
     static_assert(TM * kTileN * 4 <= kRawOff, "the partial tile of a K split takes the operand stages' place");
-};
-
-enum { kWhole, kFirst, kRemainder };
-struct PrefillParams {
-    const uint8_t* wq;
-    const float* sc;       // [row tile][Kg][scale | sum][TM]
-    const float* wscales;  // Q8C
-    float* y;
-    int* status;
-    int64_t rows, N, ldy;
-    int Ng, Kg, split;
-    int n_tiles;         // column tiles; tiles are counted along them
-    int n_off, m_off;    // this launch's first tile
-    int n_end, m_end;    // and the one behind its last
-    int part;            // kWhole, or of two launches kFirst (whole rounds) and kRemainder (the tiles that are left)
 };
 
 // ---- PTX helpers -------------------------------------------------------------
@@ -142,69 +117,13 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
     *abort_flag = 1;
     return false;
 }
-// one lane of a converged warp.  (The compiler knows that exactly one lane runs the branch and keeps descriptors in
-// uniform registers; behind `lane == 0` it cannot, and issuing an MMA takes about a third longer.)
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}"
-        : "=r"(p));
-    return p != 0;
-}
-// 2-D tiled TMA load (no multicast): box at (x, y) of the tensor map -> shared memory, completion on `bar`
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
-                 : "memory");
-}
-// packed fp32 pairs (sm_100): one issue slot for two fused multiply-adds
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 __device__ __forceinline__ uint64_t fsub2(uint64_t a, uint64_t b) { return ffma2(b, 0xBF800000BF800000ull, a); }
-__device__ __forceinline__ void fence_gpu_and_copies() { asm volatile("fence.acq_rel.gpu;\n\tfence.proxy.async.global;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
 __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum)
-        : "memory");
-}
-__device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accum)
         : "memory");
 }
 __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&r)[16]) {
@@ -227,14 +146,6 @@ __device__ __forceinline__ void tc_st(uint32_t taddr, const uint32_t (&r)[8]) {
                  "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                  : "memory");
 }
-__device__ __forceinline__ void tc_st(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     uint32_t v;
@@ -254,22 +165,6 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint64_t a, uint64_t b) {
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
-// K-major operand tile with 128-byte rows and 128-byte swizzle: rows 128 B apart, 8-row groups
-// 1024 B apart (stride byte offset), descriptor version 1, layout type 2 (SWIZZLE_128B)
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
-}
-// the eight nibbles of a word as bytes: k = 0..3 (low nibbles) and 4..7 (high nibbles)
-template <bool SIGNED>
-__device__ __forceinline__ void unpack_nibbles(uint32_t word, uint32_t& lo, uint32_t& hi) {
-    lo = word & 0x0F0F0F0Fu, hi = (word >> 4) & 0x0F0F0F0Fu;
-    if (SIGNED) {  // sign-extend each nibble into its byte
-        lo |= (lo & 0x08080808u) * 0x1Eu;
-        hi |= (hi & 0x08080808u) * 0x1Eu;
-    }
 }
 
 // acc[P .. P + W/2) += scaled integers of W rows (+ wm * their group sums); `xs`: the rows' scales, the group sums
@@ -439,7 +334,7 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot, a_tmem = tmem_base + S::kBufs * TM;
+    const uint32_t tmem_base = *tmem_slot;
 
     if (warp < kUnpackWarp) {
         // =================== epilogue: 32 lanes x (16 + 16) rows per warp ===================
@@ -587,18 +482,6 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                         for (int c = 0; c < 4; c++)
                             sts128(dst + ((uint32_t)((h * 4 + c) << 4) ^ sw), w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
                     }
-                } else if constexpr (S::kATmem) {
-                    __syncwarp();
-                    tc_fence_after();
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        uint32_t w[8], o[16];
-#pragma unroll
-                        for (int c = 0; c < 8; c++) w[c] = lds32(src + (h * 8 + c) * 128);
-#pragma unroll
-                        for (int c = 0; c < 8; c++) unpack_nibbles<FMT == kQ4_0Signed>(w[c], o[2 * c], o[2 * c + 1]);
-                        tc_st(a_tmem + ((uint32_t)(pw * 32) << 16) + s * (kStageK / 4) + 16 * h, o);
-                    }
                 } else {
                     uint32_t w[16];
 #pragma unroll
@@ -626,13 +509,7 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                         }
                 }
             }
-            if constexpr (S::kATmem) {
-                __syncwarp();
-                tc_wait_st();
-                tc_fence_before();
-            } else {
-                fence_proxy_async();  // generic-proxy stores above -> visible to the tensor core's async proxy
-            }
+            fence_proxy_async();  // generic-proxy stores above -> visible to the tensor core's async proxy
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(bar_afull + 8 * s);
@@ -674,10 +551,7 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
                     tc_fence_after();
 #pragma unroll
                     for (int ks = 0; ks < MMAS; ks++) {
-                        if constexpr (S::kATmem)
-                            tc_mma_i8(tmem_base + b * TM, a_tmem + sa * (kStageK / 4) + ks * 8, bd + ks * 2, idesc, ks > 0 ? 1u : 0u);
-                        else
-                            tc_mma_i8(tmem_base + b * TM, ad + ks * 2, bd + ks * 2, idesc, ks > 0 ? 1u : 0u);
+                        tc_mma_i8(tmem_base + b * TM, ad + ks * 2, bd + ks * 2, idesc, ks > 0 ? 1u : 0u);
                     }
                     tc_commit(bar_tfull + 8 * b);  // the group's integers are complete in TMEM
                 }
@@ -806,24 +680,24 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// the code matrix [rows][Kp] int8 as a 2-D tensor; boxes of 128 bytes x `tile` rows land in the
+// the code matrix, rows of `row_bytes`, as a 2-D tensor; boxes of 128 bytes x `tile` rows land in the
 // 128-byte-swizzle layout that the MMA descriptors describe; out-of-range rows and k read as 0
-int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t Kp, int tile) {
+int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t row_bytes, int tile) {
     EncodeTiledFn enc = encode_tiled_fn();
     if (!enc) {
         set_error("fc_prefill: cuTensorMapEncodeTiled is not available from this driver");
         return Q4FC_ECUDA;
     }
-    const cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)Kp};
-    const cuuint32_t box[2] = {(cuuint32_t)kStageK, (cuuint32_t)tile};
+    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)kStageRow, (cuuint32_t)tile};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(codes), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
-        set_error("fc_prefill: cuTensorMapEncodeTiled failed with %d (rows=%lld, Kp=%lld)", (int)r, (long long)rows,
-                  (long long)Kp);
+        set_error("fc_prefill: cuTensorMapEncodeTiled failed with %d (%lld rows of %lld bytes)", (int)r, (long long)rows,
+                  (long long)row_bytes);
         return Q4FC_ECUDA;
     }
     return Q4FC_OK;
@@ -862,8 +736,7 @@ int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, dim3 
 
 template <int FMT, int G>
 int launch_prefill_tile(int tile, const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
-    return tile == 128 ? launch_prefill_variant<FMT, G, 128>(p, map, grid, s)
-                       : launch_prefill_variant<FMT, G, 64>(p, map, grid, s);
+    return tile == 128 ? launch_prefill_wide(FMT, G, p, map, grid, s) : launch_prefill_variant<FMT, G, 64>(p, map, grid, s);
 }
 
 // tiles first .. end - 1, K divided by p.split
@@ -891,6 +764,65 @@ int launch_tiles(int fmt, int G, int tile, PrefillParams p, const CUtensorMap& m
 // scales and group sums of a format, padded to whole row tiles of either size
 size_t scale_bytes(int64_t rows, int64_t Kg, int sums) { return (size_t)((rows + 127) / 128 * 128) * Kg * sums * 4; }
 
+// How tiles of `tile` rows go over the SMs.
+struct TilePlan {
+    int tile = 0;
+    int64_t tiles = 0, split = 1;          // K divided over clusters of `split` CTAs ...
+    int64_t left = 0, left_split = 1;      // ... and of the last `left` tiles, in a launch of their own, over `left_split`
+    int64_t cost = 0;                      // rounds over the SMs in stages of 128 k, start-up and adding included
+    bool crowded = false;                  // two CTAs on an SM
+};
+// Clusters of 1 .. 8 CTAs that run at once on 148 SMs, one CTA on an SM (two: twice as many at least): by the number of
+// tiles left from which on the launch takes longer (rows x 4096, group 32: 33 tiles by four 100.5 us, 34 120.6; 22 by six 97.5,
+// 23 114.3; 42 by three 112, 44 129, of the wide kernel 44 148.8 and 48 173.8).
+int64_t clusters_at_once(int64_t c, bool wide, int64_t places) {
+    constexpr int kAtOnce[kMaxSplit] = {148, 74, 42, 33, 24, 22, 15, 15};
+    const int64_t n = (wide && c == 3 ? 44 : kAtOnce[c - 1]) * places / 148;
+    return n > 1 ? n : 1;
+}
+TilePlan plan_tiles(int tile, bool wide, int G, int64_t n_tiles, int64_t rows, int64_t nstage, int64_t sms) {
+    TilePlan t;
+    t.tile = tile, t.tiles = n_tiles * ((rows + tile - 1) / tile);
+    const int64_t places = (tile == 128 ? 1 : 2) * sms, most = nstage / 4 < 1 ? 1 : nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
+    const int64_t startup = G == 128 ? 8 : 4, start_few = wide ? startup + 2 : startup;
+    auto divided = [&](int64_t tiles, int64_t c, int64_t startup) {  // rounds x (stages of a CTA + start-up and adding)
+        const int64_t fit = clusters_at_once(c, wide, places);
+        return (tiles + fit - 1) / fit * ((nstage + c - 1) / c + startup);
+    };
+    if (t.tiles < places) {
+        // Few tiles: K is divided while a CTA keeps four stages.  64-row tiles: as often as fills the two places on every SM (37 rows x
+        // 11008: 78 us undivided, 62 by two, 41 by three, 55 by four, which needs a second wave).  The wide kernel: as the sum of
+        // rounds, stages and start-up says, with the clusters that run at once (192 x 1024 x 4096, 16 tiles, group 32: by eight 31.9 us,
+        // by six 21.4; 128 x 6000 x 3000, 47 tiles: by three 44.9, by two 31.4; 300 x 1500 x 4096, 36 tiles: by four 41.4, by
+        // three 31.4).
+        t.split = places / t.tiles < most ? places / t.tiles : most;
+        if (wide) {
+            t.split = 1;
+            for (int64_t c = 2; c <= most; c++)
+                if (divided(t.tiles, c, start_few) < divided(t.tiles, t.split, start_few)) t.split = c;
+        }
+        t.cost = wide ? divided(t.tiles, t.split, start_few) : (nstage + t.split - 1) / t.split + startup;
+        t.crowded = t.tiles * t.split > sms;
+        return t;
+    }
+    t.crowded = tile != 128;
+    t.cost = t.tiles / places * nstage + startup;
+    if (t.tiles % places != 0) {
+        // What is left after whole rounds over the places would take a round of its own, most places empty.  With K divided by c it
+        // takes 1/c of one, and some stages' time for start-up and the adding, where that many clusters run at once.  (11008
+        // columns, K = 4096: 512 rows, group 32, 48 of 344 tiles left, undivided 177 us, by two 156, by three, which takes two rounds,
+        // 174; 256 rows, Q8C, 24 of 172, 148 -> 100; 100 rows x 20000, group 32, 18 of 314, 174 -> 106.  Divided where
+        // this sum says no: 1024 x 4096 x 4096, 108 of 256 left, 125 -> 137.)
+        t.left = t.tiles % places;
+        int64_t best = nstage;  // undivided, in the launch of the others
+        for (int64_t c = 2; c <= most; c++)
+            if (divided(t.left, c, startup) < best) best = divided(t.left, c, startup), t.left_split = c;
+        if (t.left_split == 1) t.left = 0;
+        t.cost += best;
+    }
+    return t;
+}
+
 // Quantizer and GEMM; `codes` and `sc` are scratch for [rows][Kg * G] bytes and scale_bytes().
 int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t ldx, int8_t* codes, float* sc,
                 PrefillParams p, cudaStream_t s) {
@@ -904,48 +836,30 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     }
     const int64_t n_tiles = (p.N + kTileN - 1) / kTileN;
     const int64_t nstage = (Kp + kStageK - 1) / kStageK;
-    // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM: the large tile as soon as such tiles occupy
-    // every SM (512 rows x 4096 x 11008, group 32: 186 us, with 64 rows 209; 256 rows, Q8C: 102 and 108), the small one for less
-    // work (320 x 2048 x 2048, group 32: 27.8 us, with 128 rows 35.6).  Over 264 sizes (65 to 1024 rows, K x N from 1000 x 9000 to
-    // 11008 x 4096) that line costs 4.5 % against the better of the two, with group 128 9 %: from half the SMs on large tiles with K
-    // divided are ahead (group 128, 512 x 4096 x 4096: 44.2 us, with 128 rows 34.9; group 32, 512 x 11008 x 4096 225 and 201).  K is
-    // divided while that fills the two places on every SM and leaves a CTA four stages (37 rows x 11008: 78 us undivided, 62 by
-    // two, 41 by three, 55 by four, which needs a second wave).
-    const int tile = (rows > 64 && n_tiles * ((rows + 127) / 128) >= di->sm_count) ? 128 : 64;
-    const int64_t m_tiles = (rows + tile - 1) / tile;
-    const int64_t tiles = n_tiles * m_tiles, places = (tile == 128 ? 1 : 2) * (int64_t)di->sm_count;
-    const int64_t most = nstage / 4 < 1 ? 1 : nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
-    int64_t split = 1, left = 0, left_split = 1;  // of the tiles, the last `left` with K divided by `left_split`
-    if (tiles < places) {
-        split = places / tiles < most ? places / tiles : most;
-    } else if (tiles % places != 0) {
-        // What is left after whole rounds over the places would take a round of its own, most places empty.  With K divided by c it
-        // takes 1/c of one, and some stages' time for start-up and the adding, where that many clusters run at once.  (11008
-        // columns, K = 4096: 512 rows, group 32, 48 of 344 tiles left, 217 -> 186 us; 256 rows, Q8C, 24 of 172, 148 -> 100; 256 rows,
-        // group 128, 61 -> 47; 100 rows x 20000, group 32, 18 of 314, 174 -> 106.  Divided where this sum says no: 1000 rows, 96
-        // of 688, Q8C, 360 -> 394.)
-        left = tiles % places;
-        int64_t best = nstage;  // undivided, in the launch of the others
-        for (int64_t c = 2; c <= most; c++) {
-            // Clusters of 2 .. 8 CTAs that run at once on 148 SMs, one CTA on an SM (two: twice as many at least): by the number of
-            // tiles left from which on the launch takes longer (rows x 4096, group 32: 33 tiles by four 100.5 us, 34 120.6; 22 by
-            // six 97.5, 23 114.3; 42 by three 112, 44 129).
-            constexpr int kAtOnce[kMaxSplit - 1] = {74, 42, 33, 24, 22, 15, 15};
-            const int64_t fit = kAtOnce[c - 2] * places / 148;
-            const int64_t cost = (left + fit - 1) / fit * ((nstage + c - 1) / c + (G == 128 ? 8 : 4));
-            if (cost < best) best = cost, left_split = c;
-        }
-        if (left_split == 1) left = 0;
+    // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM.
+    TilePlan t = plan_tiles(64, false, G, n_tiles, rows, nstage, di->sm_count);
+    if (rows > 64 && fmt == kQ8C) {
+        // Q8C: the large tile as soon as such tiles occupy every SM (256 rows x 4096 x 11008: 102 us and 108).
+        if (n_tiles * ((rows + 127) / 128) >= di->sm_count) t = plan_tiles(128, false, G, n_tiles, rows, nstage, di->sm_count);
+    } else if (rows > 64) {
+        // A round of 64-row tiles, two on an SM, takes 1.5 times one of the wide kernel's tiles; alone on an SM as long as that.  Over 495
+        // calls (65 to 512 rows, K x N from 1000 x 1500 to 4096 x 11008) the choice costs 0.9 % against the better of the two, at most
+        // 16 % (192 x 700 x 11008: 38.9 and 33.6); always the wide kernel 3.2 %, from as many of its tiles on as SMs 11.6 %.
+        const TilePlan w = plan_tiles(128, true, G, n_tiles, rows, nstage, di->sm_count);
+        if (Kp <= 0x3fffffffLL && (w.tiles >= di->sm_count || 2 * w.cost <= (t.crowded ? 3 : 2) * t.cost)) t = w;
     }
+    const int tile = t.tile;
+    const int64_t m_tiles = (rows + tile - 1) / tile, tiles = t.tiles, split = t.split, left = t.left, left_split = t.left_split;
     if (n_tiles * split > 0x7fffffffLL || m_tiles > 65535 || tiles > 0x7fffffffLL / kMaxSplit) {
         set_error("fc_prefill: %lld x %lld tiles exceed the grid limit", (long long)n_tiles, (long long)m_tiles);
         return Q4FC_ELIMIT;
     }
     p.n_tiles = (int)n_tiles;
-    if (int rc = launch_quant_x_tile(x, rows, K, ldx, G, fmt == kQ4_1, tile, codes, sc, s)) return rc;
+    const bool f16 = G == 32 && fmt != kQ8C && tile == 128;  // operands of the wide kernel
+    if (int rc = launch_quant_x_tile(x, rows, K, ldx, G, fmt == kQ4_1, tile, f16, codes, sc, s)) return rc;
     CUtensorMap map = {};
     if (Kp > 0)  // (no K group: no stage reads the map)
-        if (int rc = make_codes_map(&map, codes, rows, Kp, tile)) return rc;
+        if (int rc = make_codes_map(&map, codes, rows, f16 ? 2 * Kp : Kp, tile)) return rc;
     p.split = (int)split, p.part = left == 0 ? kWhole : kFirst;
     if (int rc = launch_tiles(fmt, G, tile, p, map, 0, tiles - left, s)) return rc;
     if (left == 0) return Q4FC_OK;
@@ -954,7 +868,7 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
 }
 
 // workspace: [status 256][what the decode kernels keep between calls: decode_prequant_offset() bytes]
-//            [codes rows x Kp, 256-aligned][scales and group sums]
+//            [codes of all rows, 256-aligned][scales and group sums]
 // The quantized activations start where the decode path's own quantizer scratch starts: calls on one
 // workspace are ordered, so the two can share that space, and neither lands on the stream-K stripe
 // counters, which must stay zero between calls.
@@ -964,7 +878,8 @@ struct WsLayout {
 WsLayout ws_layout(int64_t rows, int64_t Kg, int G) {
     WsLayout l;
     l.codes = decode_prequant_offset();
-    l.sc = align_up(l.codes + (size_t)rows * Kg * G, 256);
+    // (group 32 beyond 64 rows, which is where 128-row tiles begin: fp16)
+    l.sc = align_up(l.codes + (size_t)rows * Kg * G * (G == 32 && rows > 64 ? 2 : 1), 256);
     l.total = align_up(l.sc + scale_bytes(rows, Kg, 2), 256);
     return l;
 }

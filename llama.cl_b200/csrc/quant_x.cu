@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_kernel(const float* __r
 // The prefill GEMM's quantizer: the codes and scales of quant_x_kernel, scales (and, `sums`, group sums, tree-ordered)
 // in the layout in which the GEMM's tiles of 2^log2tile rows read them: [row tile][Kg][scale | sum][row in tile].
 // The eight warps of a CTA take the same 128 k of eight neighbouring rows, whose scales share a 32-byte sector.
-template <int G>
+template <int G, bool F16>
 __global__ void __launch_bounds__(kQxWarps * 32) quant_x_tile_kernel(const float* __restrict__ x, int64_t rows, int64_t K,
                                                                      int64_t ldx, int64_t Kg, int vec_ok, int sums,
                                                                      int log2tile, int8_t* __restrict__ codes,
@@ -155,22 +155,32 @@ __global__ void __launch_bounds__(kQxWarps * 32) quant_x_tile_kernel(const float
     }
     const float d = div_const_rn(amax, 127.0f, 1.0f / 127.0f);
     const float id = inv_or_zero(d);
-    uint32_t packed = 0;
+    int q[4] = {};
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        int q = 0;
+    for (int j = 0; j < 4; j++)
         if (e0 + j < len) {
             const float t = __fmul_rn(v[j], id);
-            q = sat8(e0 + j < body ? __float2int_rn(t) : round_half_away(t));
+            q[j] = sat8(e0 + j < body ? __float2int_rn(t) : round_half_away(t));
         }
-        packed |= (uint32_t)(q & 0xFF) << (8 * j);
+    uint32_t w[2];  // F16: four codes, as two lanes hold eight k: the even one takes k = 0,2,4,6 (see launch_quant_x_tile)
+    if constexpr (F16) {
+        uint32_t h[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) h[j] = __half_as_ushort(__int2half_rn(q[j] * ((lane & 1) ? 16 : 256)));
+        const uint32_t even = h[0] | h[2] << 16, odd = h[1] | h[3] << 16;
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, (lane & 1) ? even : odd, 1);
+        w[0] = (lane & 1) ? other : even, w[1] = (lane & 1) ? odd : other;
     }
     if (exists) {
-        *reinterpret_cast<uint32_t*>(codes + row * (Kg * G) + k) = packed;
+        if constexpr (F16)
+            *reinterpret_cast<uint2*>(codes + (row * (Kg * G) + k) * 2) = make_uint2(w[0], w[1]);
+        else
+            *reinterpret_cast<uint32_t*>(codes + row * (Kg * G) + k) =
+                (q[0] & 0xFF) | (q[1] & 0xFF) << 8 | (q[2] & 0xFF) << 16 | (uint32_t)(q[3] & 0xFF) << 24;
         if (e0 == 0) {
             const int64_t tile = (int64_t)1 << log2tile, per = tile << sums;
             float* dst = sc + ((row >> log2tile) * Kg + kb) * per + (row & (tile - 1));
-            dst[0] = d;
+            dst[0] = F16 ? __fmul_rn(d, 64.0f) : d;
             if (sums) dst[tile] = sum;
         }
     }
@@ -413,8 +423,8 @@ int launch_quant_x_pre(const float* x, int rows, int64_t K, int64_t ldx, int G, 
     return Q4FC_OK;
 }
 
-int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, bool sums, int tile, int8_t* codes,
-                        float* sc, cudaStream_t s) {
+int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, int G, bool sums, int tile, bool f16,
+                        int8_t* codes, float* sc, cudaStream_t s) {
     const int64_t Kg = (K + G - 1) / G;
     if (rows == 0 || Kg == 0) return Q4FC_OK;
     const int64_t grid = (rows + kQxWarps - 1) / kQxWarps * ((Kg * G + 127) / 128);
@@ -424,7 +434,7 @@ int launch_quant_x_tile(const float* x, int64_t rows, int64_t K, int64_t ldx, in
     }
     const int vec_ok = (K % 4 == 0) && (ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const int l2 = tile == 128 ? 7 : 6;
-    auto* kernel = G == 32 ? quant_x_tile_kernel<32> : quant_x_tile_kernel<128>;
+    auto* kernel = G == 128 ? quant_x_tile_kernel<128, false> : f16 ? quant_x_tile_kernel<32, true> : quant_x_tile_kernel<32, false>;
     DependentLaunch l(dim3((unsigned)grid), kQxWarps * 32, s);
     Q4FC_CUDA_OK(cudaLaunchKernelEx(&l.cfg, kernel, x, rows, K, ldx, Kg, vec_ok, (int)sums, l2, codes, sc));
     return Q4FC_OK;

@@ -267,6 +267,34 @@ def test_many_rows_last_tiles_divided(pkg, oracle, fmt, rows, N, K):
     check_many_rows(pkg, oracle, fmt, rows, N, K, launches=3)  # the quantizer, whole rounds, the remainder
 
 
+@pytest.mark.parametrize("rows,N,K", [
+    # 148 column tiles and more: whole tiles, the last columns and K groups not full, fewer K stages than are unpacked ahead and
+    # more than the rings hold, rows that end in each of a warp's four chunks
+    (65, 18901, 33), (81, 18901, 96), (112, 18920, 224), (128, 18944, 1312), (129, 9473, 640), (185, 9473, 160),
+    (128, 1024, 4096), (192, 1000, 4096), (129, 4096, 2080), (300, 1500, 4096), (128, 6000, 3000),  # K divided by 8, 6, 2, 3, 2
+])
+@pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128"])
+def test_wide_tiles_against_64_row_tiles(pkg, fmt, rows, N, K):
+    """128-row tiles against calls of at most 64 rows, which go in 64-row tiles: the same codes and exact integers, products and
+    sums in another order (tolerance as in test_many_rows_on_tile_edges, row by row).  Among the rows the ends of the range."""
+    signed = isinstance(fmt, str)
+    qtype, G = (0, int(fmt[6:])) if signed else fmt
+    g = torch.Generator(device="cuda").manual_seed(rows + N + K)
+    wq = pkg.llmops.offline_FC_quant_Q4A(torch.randn(N, K, generator=g, device="cuda") * 0.02, qtype=f"q4_{qtype}", group_k=G)
+    x = torch.randn(1, rows, K, generator=g, device="cuda")
+    x[0, 3], x[0, 5:8] = 0, x[0, 5:8] * torch.tensor([[1e-30], [1e30], [1e-44]], device="cuda")
+    x[0, 9, 1], x[0, 10, 2], x[0, rows - 1, 0] = float("inf"), float("nan"), 1e6
+    got = pkg.llmops.fc_Q4A(x, wq, N, nibble_signed=signed)
+    want = torch.cat([pkg.llmops.fc_Q4A(part.contiguous(), wq, N, nibble_signed=signed) for part in x.split(60, dim=1)], dim=1)
+    again = pkg.llmops.fc_Q4A(x, wq, N, nibble_signed=signed)
+    assert torch.equal(got.view(torch.int32), again.view(torch.int32))  # fixed summation order
+    assert torch.equal(got.isfinite(), want.isfinite()) and torch.equal(got.isnan(), want.isnan())
+    got, want = got.nan_to_num(0, 0, 0), want.nan_to_num(0, 0, 0)
+    # (the row of subnormal values: its results are a few units of the smallest number)
+    assert ((got - want).abs() <= 2e-5 * want.abs().amax(-1, keepdim=True) + 1e-42).all()
+    pkg.llmops.check_device_status()
+
+
 def early_edges(graph):
     """Edges of a captured graph over which a kernel begins before the one in front of it has ended, and all of them."""
     cu, n = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t()
