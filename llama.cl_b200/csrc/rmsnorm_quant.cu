@@ -31,7 +31,7 @@
 namespace q4fc {
 namespace {
 
-constexpr int kRnThreads = 256;
+constexpr int kRnThreads = 1024;  // at most: a warp per 128 k where that is enough
 
 __device__ __forceinline__ int sat8(int v) { return min(127, max(-128, v)); }
 
@@ -52,15 +52,30 @@ __global__ void __launch_bounds__(kRnThreads) rmsnorm_quant_kernel(const float* 
     pdl_launch_dependents();
     pdl_wait_prior_grid();  // the activations may come from the kernel before
 
-    for (int64_t i = threadIdx.x * 4; i < K; i += kRnThreads * 4) {  // K % 8 == 0 (checked by the launcher)
-        float4 a = __ldcg(reinterpret_cast<const float4*>(src + i));
-        if (residual != nullptr) {
-            // the reference's iadd in front of the normalization (ops/op_misc.hpp:55-79): one IEEE add each
-            const float4 b = __ldcg(reinterpret_cast<const float4*>(residual + m * ldx + i));
-            a.x = __fadd_rn(a.x, b.x), a.y = __fadd_rn(a.y, b.y), a.z = __fadd_rn(a.z, b.z), a.w = __fadd_rn(a.w, b.w);
-            if (sum_out != nullptr) *reinterpret_cast<float4*>(sum_out + m * ldx + i) = a;
+    // the weights of this warp's first 128 k, asked for before anything else needs time
+    const int64_t k0 = warp * 128 + lane * 4;
+    const float4 w0 = k0 + 4 <= K ? ld_after_wait(reinterpret_cast<const float4*>(weight + k0)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int64_t step = blockDim.x * 4;
+    for (int64_t i0 = threadIdx.x * 4; i0 < K; i0 += 2 * step) {  // K % 8 == 0 (checked by the launcher)
+        float4 a[2], b[2];  // loads in front of the stores, which may be to the same row
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int64_t i = i0 + j * step;
+            if (i < K) a[j] = __ldcg(reinterpret_cast<const float4*>(src + i));
+            if (i < K && residual != nullptr) b[j] = __ldcg(reinterpret_cast<const float4*>(residual + m * ldx + i));
         }
-        *reinterpret_cast<float4*>(row + i) = a;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int64_t i = i0 + j * step;
+            if (i >= K) break;
+            if (residual != nullptr) {
+                // the reference's iadd in front of the normalization (ops/op_misc.hpp:55-79): one IEEE add each
+                a[j].x = __fadd_rn(a[j].x, b[j].x), a[j].y = __fadd_rn(a[j].y, b[j].y);
+                a[j].z = __fadd_rn(a[j].z, b[j].z), a[j].w = __fadd_rn(a[j].w, b[j].w);
+                if (sum_out != nullptr) *reinterpret_cast<float4*>(sum_out + m * ldx + i) = a[j];
+            }
+            *reinterpret_cast<float4*>(row + i) = a[j];
+        }
     }
     __syncthreads();
 
@@ -68,8 +83,27 @@ __global__ void __launch_bounds__(kRnThreads) rmsnorm_quant_kernel(const float* 
         float s = 0.0f;
         if (lane < 8) {
             // the reference's lane `lane` of its 8-wide running sum
-#pragma unroll 8
-            for (int64_t i = lane; i < K; i += 8) s = __fmaf_rn(row[i], row[i], s);
+            // (sixteen values on their way while the sixteen before are added: the chain waits for its additions alone)
+            const float* p = row + lane;
+            const int n = (int)(K / 8);
+            float cur[16] = {}, next[16];
+            int i = 0;
+            if (n >= 16) {
+#pragma unroll
+                for (int j = 0; j < 16; j++) cur[j] = p[8 * j];
+#pragma unroll 2
+                for (i = 16; i + 16 <= n; i += 16) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) next[j] = p[8 * (i + j)];
+#pragma unroll
+                    for (int j = 0; j < 16; j++) s = __fmaf_rn(cur[j], cur[j], s);
+#pragma unroll
+                    for (int j = 0; j < 16; j++) cur[j] = next[j];
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j++) s = __fmaf_rn(cur[j], cur[j], s);
+            }
+            for (; i < n; i++) s = __fmaf_rn(p[8 * i], p[8 * i], s);
         }
         // ((s4 + s0) + (s6 + s2)) + ((s5 + s1) + (s7 + s3))
         const float a = __fadd_rn(__shfl_sync(0xffffffffu, s, (lane & 3) + 4), __shfl_sync(0xffffffffu, s, lane & 3));
@@ -84,7 +118,7 @@ __global__ void __launch_bounds__(kRnThreads) rmsnorm_quant_kernel(const float* 
     const float r = row[K];
 
     const int64_t chunks = (Kg * G + 127) / 128;
-    for (int64_t c = warp; c < chunks; c += kRnThreads / 32) {
+    for (int64_t c = warp; c < chunks; c += blockDim.x / 32) {
         const int64_t k = c * 128 + lane * 4;
         const int64_t kb = c * GPC + lane / SEG;
         const bool exists = kb < Kg;
@@ -94,7 +128,7 @@ __global__ void __launch_bounds__(kRnThreads) rmsnorm_quant_kernel(const float* 
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         if (k + 4 <= K) {
             const float4 a = *reinterpret_cast<const float4*>(row + k);
-            const float4 w = __ldg(reinterpret_cast<const float4*>(weight + k));
+            const float4 w = c == warp ? w0 : __ldg(reinterpret_cast<const float4*>(weight + k));
             v[0] = __fmul_rn(__fmul_rn(a.x, r), w.x), v[1] = __fmul_rn(__fmul_rn(a.y, r), w.y);
             v[2] = __fmul_rn(__fmul_rn(a.z, r), w.z), v[3] = __fmul_rn(__fmul_rn(a.w, r), w.w);
             if (y != nullptr) *reinterpret_cast<float4*>(y + m * ldy + k) = make_float4(v[0], v[1], v[2], v[3]);
@@ -170,7 +204,8 @@ int launch_rmsnorm_quant(const float* x, const float* residual, float* sum_out, 
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)rows);
-    cfg.blockDim = dim3(kRnThreads);
+    const int64_t threads = (K + 127) / 128 * 32;
+    cfg.blockDim = dim3((unsigned)(threads < 128 ? 128 : threads < kRnThreads ? threads : kRnThreads));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
