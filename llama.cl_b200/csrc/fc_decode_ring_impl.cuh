@@ -801,15 +801,33 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
     // and store the codes into one another's shared memory, instead of each CTA repeating it.
     p.bq = 1;
     if (p.cs == 1 && !preq) {
-        int bq = kShare;
-        while (bq > 1 && nc < bq) bq /= 2;
-        if (bq > 1) {
+        // CTAs of a launch with `bq` sharers.  A CTA more than stripes does no harm, one less makes another take two (a row x 4096,
+        // Q4_1 group 32: 77 stripes on 76 CTAs 6.95 us, on 80 5.10; 110 7.01 and 5.20).  Clusters of four reach 132 of 148 SMs, of two
+        // all of them (140 stripes on 132 7.10, on 148 5.25; 290 stripes 9.6 and 9.0).
+        auto units_of = [&](int bq) {
             int l2 = 0;
             while ((1 << l2) < bq) l2++;
             const int cap = ring_max_clusters(v, dev, bq, l2, di);
-            if (cap < 0) return Q4FC_ECUDA;
-            int units = nc / bq * bq;
-            if (units > cap * bq) units = cap * bq;
+            if (cap < 0) return -1;
+            const int units = TP ? nc / bq * bq : (nc + bq - 1) / bq * bq;  // (the last of them may have no stripe)
+            return units < cap * bq ? units : cap * bq;
+        };
+        int bq = kShare;
+        while (bq > 1 && nc < bq) bq /= 2;
+        if (bq > 1) {
+            int units = units_of(bq);
+            if (units < 0) return Q4FC_ECUDA;
+            if (!TP && bq == 4) {
+                // Two sharers where the SMs that clusters of two reach besides save a round of stripes, and that is worth more than
+                // the quantizer's longer share (a stripe takes half a nanosecond per k, a pass of the 16 warps over 128 k of four rows
+                // each 0.4 us).
+                const int two = units_of(2);
+                if (two < 0) return Q4FC_ECUDA;
+                const int64_t K = p.in[0].K, chunks = (K + 127) / 128, sets = (rows_max + 3) / 4;
+                const int64_t saved = (ng_total + units - 1) / units - (ng_total + two - 1) / two;
+                const int64_t more = ((chunks + 2 * kRW - 1) / (2 * kRW) - (chunks + 4 * kRW - 1) / (4 * kRW)) * sets;
+                if (saved * K > more * 800 && saved > 0) bq = 2, units = two;
+            }
             p.bq = bq;
             nc = units;
         }

@@ -267,6 +267,18 @@ def test_many_rows_last_tiles_divided(pkg, oracle, fmt, rows, N, K):
     check_many_rows(pkg, oracle, fmt, rows, N, K, launches=3)  # the quantizer, whole rounds, the remainder
 
 
+@pytest.mark.parametrize("stripes", [75, 77, 131, 133, 148, 149, 266, 296, 297])
+@pytest.mark.parametrize("rows,K,qtype,G", [(1, 1000, 1, 32), (3, 2080, 0, 128), (1, 9000, 1, 128), (2, 4096, 0, 32)])
+def test_decode_ctas_that_share_the_quantizer(pkg, stripes, rows, K, qtype, G):
+    """Four or two CTAs to a share, CTAs without a stripe, one to three rounds of stripes: bit-equal to quantizing in front."""
+    g = torch.Generator(device="cuda").manual_seed(stripes + K)
+    N = stripes * 32 - 5
+    wq = pkg.llmops.offline_FC_quant_Q4A(torch.randn(N, K, generator=g, device="cuda") * 0.02, qtype=f"q4_{qtype}", group_k=G)
+    x = torch.randn(1, rows, K, generator=g, device="cuda")
+    want = pkg.llmops.fc_Q4A_q8(pkg.llmops.quantize_activations(x, G), wq, N)
+    assert torch.equal(pkg.llmops.fc_Q4A(x, wq, N, path="decode"), want)
+
+
 @pytest.mark.parametrize("rows,N,K", [
     # 148 column tiles and more: whole tiles, the last columns and K groups not full, fewer K stages than are unpacked ahead and
     # more than the rings hold, rows that end in each of a warp's four chunks
