@@ -13,9 +13,9 @@
 //     so that nothing converts them, with int8 integers (group 128's MMAs alone would take 512 cycles with fp16).
 //
 // Measured (whole calls, in the 64-row kernel's form before -> here):
-//   512 x 4096 x 11008, Q4_0 g32 186 -> 154 us (299 TOPS), Q4_1 g32 235 -> 197;  2048 rows, Q4_1 g128 296 -> 282 (655 TOPS)
-//   one round of 148 tiles, K = 4096 (the quantizer included): Q4_0 g32 76 -> 61 us, Q4_1 g32 96 -> 78, Q4_1 g128 33 -> 31
-// A K group of 32 takes 820 cycles (from K = 2048 to 8192), in which a scheduler issues 400 instructions.  What bounds it: the
+//   512 x 4096 x 11008, Q4_0 g32 186 -> 150 us (308 TOPS), Q4_1 g32 235 -> 197;  2048 rows, Q4_1 g128 296 -> 282 (655 TOPS)
+//   one round of 148 tiles, K = 4096 (the quantizer included): Q4_0 g32 76 -> 60 us, Q4_1 g32 96 -> 78, Q4_1 g128 33 -> 31
+// A K group of 32 takes 790 cycles (from K = 2048 to 8192), in which a scheduler issues 400 instructions.  What bounds it: the
 // latencies of two warps a scheduler that meet at the same buffers.  The FMA pipe has 330 cycles to do (a packed multiplication 2.4, a
 // packed fma with three register operands 2.8), broadcasting the scales takes shared memory 260, the MMAs 128; an epilogue
 // alone, without unpacking and with a constant for the column's scale, takes 435.  That total moves little with its parts
@@ -266,6 +266,9 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
         const uint32_t share = quarter * S::kRawStripe + half * (S::kF16 ? BS : 1024) + lane * 4;
         constexpr int kWords = S::kF16 ? 4 : 8, kOut = 16 / kWords;
         uint32_t words[kWords];
+        // behind the first or the second of the four chunks: 512 x 4096 x 11008, Q4_0 g32 154 and 150 us, Q4_1 g32 197 and 201; one round,
+        // Q4_1 g128, 732 and 749 ns a group
+        constexpr int kUnpackAt = G == 32 && FMT != kQ4_1 ? 1 : 0;
         auto load_words = [&](int slot) {
             const uint8_t* src = smem + S::kSlotOff + slot * S::kSlotBytes + share;
 #pragma unroll
@@ -354,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
                         if (more) tc_ld(at + (c + 1) * (2 * W), v[(c + 1) & 1]);
                         if (c == 0) ask();
                         if (some) scale(c);
-                        if (c == 0 && gi == 0) unpack(place_now);
+                        if (c == kUnpackAt && gi == 0) unpack(place_now);
                         if (more) tc_wait_ld(v[(c + 1) & 1]);
                     }
                     if (gi == 0) tc_wait_st();
