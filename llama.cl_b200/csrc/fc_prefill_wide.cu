@@ -13,7 +13,7 @@
 //     so that nothing converts them, with int8 integers (group 128's MMAs alone would take 512 cycles with fp16).
 //
 // Measured (whole calls, in the 64-row kernel's form before -> here):
-//   512 x 4096 x 11008, Q4_0 g32 186 -> 150 us (308 TOPS), Q4_1 g32 235 -> 197;  2048 rows, Q4_1 g128 296 -> 282 (655 TOPS)
+//   512 x 4096 x 11008, Q4_0 g32 186 -> 150 us (308 TOPS), Q4_1 g32 235 -> 197;  2048 rows, Q4_1 g128 296 -> 278 (664 TOPS)
 //   one round of 148 tiles, K = 4096 (the quantizer included): Q4_0 g32 76 -> 60 us, Q4_1 g32 96 -> 78, Q4_1 g128 33 -> 31
 // A K group of 32 takes 790 cycles (from K = 2048 to 8192), in which a scheduler issues 400 instructions.  What bounds it: the
 // latencies of two warps a scheduler that meet at the same buffers.  The FMA pipe has 330 cycles to do (a packed multiplication 2.4, a
@@ -167,8 +167,10 @@ __device__ __forceinline__ void accumulate(uint64_t (&acc)[W / 2], const uint32_
         const ulonglong2 x4 = *reinterpret_cast<const ulonglong2*>(xs + 4 * j);
         const uint64_t i01 = pack2(number(4 * j), number(4 * j + 1)), i23 = pack2(number(4 * j + 2), number(4 * j + 3));
         uint64_t &a = acc[2 * j], &b = acc[2 * j + 1];
-        a = ffma2(wd2, fmul2(x4.x, i01), a);
-        b = ffma2(wd2, fmul2(x4.y, i23), b);
+        // which factor comes first decides which operands stay at hand: a group of one round's tiles, Q4_1, 128 k 736 and 718 ns, 32 k
+        // 549 and 563
+        a = F16 ? ffma2(wd2, fmul2(x4.x, i01), a) : ffma2(x4.x, fmul2(wd2, i01), a);
+        b = F16 ? ffma2(wd2, fmul2(x4.y, i23), b) : ffma2(x4.y, fmul2(wd2, i23), b);
         if (FMT == kQ4_1) {
             const ulonglong2 g4 = *reinterpret_cast<const ulonglong2*>(xs + TM + 4 * j);
             a = ffma2(wm2, g4.x, a);
