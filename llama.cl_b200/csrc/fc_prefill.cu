@@ -772,15 +772,32 @@ struct TilePlan {
     int64_t cost = 0;                      // rounds over the SMs in stages of 128 k, start-up and adding included
     bool crowded = false;                  // two CTAs on an SM
 };
-// Clusters of 1 .. 8 CTAs that run at once on 148 SMs, one CTA on an SM (two: twice as many at least): by the number of
+// Clusters of 1 .. 8 CTAs that run at once on 148 SMs, one CTA on an SM: by the number of
 // tiles left from which on the launch takes longer (rows x 4096, group 32: 33 tiles by four 100.5 us, 34 120.6; 22 by six 97.5,
-// 23 114.3; 42 by three 112, 44 129, of the wide kernel 44 148.8 and 48 173.8).
+// 23 114.3; 42 by three 112, 44 129, of the wide kernel 44 148.8 and 48 173.8).  Two CTAs on an SM: twice as many at least.
 int64_t clusters_at_once(int64_t c, bool wide, int64_t places) {
     constexpr int kAtOnce[kMaxSplit] = {148, 74, 42, 33, 24, 22, 15, 15};
     const int64_t n = (wide && c == 3 ? 44 : kAtOnce[c - 1]) * places / 148;
     return n > 1 ? n : 1;
 }
-TilePlan plan_tiles(int tile, bool wide, int G, int64_t n_tiles, int64_t rows, int64_t nstage, int64_t sms) {
+// Over how many CTAs few 64-row tiles, one for each 128 columns, divide K: rounds x (stages of a CTA + start-up and adding), where a stage takes half as long
+// again, and the rest a fifth, once two CTAs share an SM.  By the times of 84 calls (12 to 64 rows, 8 to 141 tiles) divided by 1 to 8: 0.1 %
+// behind the best of them, at most 2 %; as often as fills two places on every SM 7 % and 50 % (64 x 5120 x 4096, 40 tiles, group
+// 128: by seven 22.4 us, by six 15.8; 64 x 4096 x 4096: by eight 14.9, by four 13.1; group 32, 47 tiles: by six 41.7, by five 29.8).
+// Clusters of two CTAs on an SM that were seen to run at once: kTwo.
+int64_t split_of_few(int64_t tiles, int64_t most, int G, bool q8c, int64_t nstage, int64_t sms) {
+    constexpr int kTwo[kMaxSplit] = {296, 148, 86, 66, 48, 44, 32, 32};
+    const int64_t startup = G == 128 ? 16 : 4;
+    int64_t best = 0, best_cost = 0;
+    for (int64_t c = 1; c <= most; c++) {
+        const int64_t fit = kTwo[c - 1] * sms / 148 > 1 ? kTwo[c - 1] * sms / 148 : 1, rounds = (tiles + fit - 1) / fit;
+        const bool shared = tiles > clusters_at_once(c, false, sms) + (q8c ? 1 : 0);  // (Q8C, 50 x 2048, 16 tiles: by eight 18.5, by six 19.2)
+        const int64_t cost = rounds * ((nstage + c - 1) / c * (shared ? 15 : 10) + startup * (shared ? 12 : 10));
+        if (best == 0 || cost <= best_cost) best = c, best_cost = cost;
+    }
+    return best;
+}
+TilePlan plan_tiles(int tile, bool wide, int G, bool q8c, int64_t n_tiles, int64_t rows, int64_t nstage, int64_t sms) {
     TilePlan t;
     t.tile = tile, t.tiles = n_tiles * ((rows + tile - 1) / tile);
     const int64_t places = (tile == 128 ? 1 : 2) * sms, most = nstage / 4 < 1 ? 1 : nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
@@ -790,14 +807,13 @@ TilePlan plan_tiles(int tile, bool wide, int G, int64_t n_tiles, int64_t rows, i
         return (tiles + fit - 1) / fit * ((nstage + c - 1) / c + startup);
     };
     if (t.tiles < places) {
-        // Few tiles: K is divided while a CTA keeps four stages.  64-row tiles: as often as fills the two places on every SM (37 rows x
-        // 11008: 78 us undivided, 62 by two, 41 by three, 55 by four, which needs a second wave).  The wide kernel: as the sum of
+        // Few tiles: K is divided while a CTA keeps four stages.  The wide kernel: as the sum of
         // rounds, stages and start-up says, with the clusters that run at once (192 x 1024 x 4096, 16 tiles, group 32: by eight 31.9 us,
         // by six 21.4; 128 x 6000 x 3000, 47 tiles: by three 44.9, by two 31.4; 300 x 1500 x 4096, 36 tiles: by four 41.4, by
-        // three 31.4).
-        t.split = places / t.tiles < most ? places / t.tiles : most;
+        // three 31.4).  More than one row of 64-row tiles: as often as fills the two places on every SM (the last row is seldom full, and its
+        // CTAs leave early: 150 x 3000 x 4096, 72 tiles: by four 40, by three, which that sum says, 52).
+        t.split = wide ? 1 : rows <= 64 ? split_of_few(t.tiles, most, G, q8c, nstage, sms) : places / t.tiles < most ? places / t.tiles : most;
         if (wide) {
-            t.split = 1;
             for (int64_t c = 2; c <= most; c++)
                 if (divided(t.tiles, c, start_few) < divided(t.tiles, t.split, start_few)) t.split = c;
         }
@@ -837,15 +853,15 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     const int64_t n_tiles = (p.N + kTileN - 1) / kTileN;
     const int64_t nstage = (Kp + kStageK - 1) / kStageK;
     // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM.
-    TilePlan t = plan_tiles(64, false, G, n_tiles, rows, nstage, di->sm_count);
+    TilePlan t = plan_tiles(64, false, G, fmt == kQ8C, n_tiles, rows, nstage, di->sm_count);
     if (rows > 64 && fmt == kQ8C) {
         // Q8C: the large tile as soon as such tiles occupy every SM (256 rows x 4096 x 11008: 102 us and 108).
-        if (n_tiles * ((rows + 127) / 128) >= di->sm_count) t = plan_tiles(128, false, G, n_tiles, rows, nstage, di->sm_count);
+        if (n_tiles * ((rows + 127) / 128) >= di->sm_count) t = plan_tiles(128, false, G, true, n_tiles, rows, nstage, di->sm_count);
     } else if (rows > 64) {
         // A round of 64-row tiles, two on an SM, takes 1.5 times one of the wide kernel's tiles; alone on an SM as long as that.  Over 495
         // calls (65 to 512 rows, K x N from 1000 x 1500 to 4096 x 11008) the choice costs 0.9 % against the better of the two, at most
         // 16 % (192 x 700 x 11008: 38.9 and 33.6); always the wide kernel 3.2 %, from as many of its tiles on as SMs 11.6 %.
-        const TilePlan w = plan_tiles(128, true, G, n_tiles, rows, nstage, di->sm_count);
+        const TilePlan w = plan_tiles(128, true, G, false, n_tiles, rows, nstage, di->sm_count);
         if (Kp <= 0x3fffffffLL && (w.tiles >= di->sm_count || 2 * w.cost <= (t.crowded ? 3 : 2) * t.cost)) t = w;
     }
     const int tile = t.tile;
