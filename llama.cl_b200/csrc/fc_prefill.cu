@@ -69,7 +69,10 @@ constexpr int kTmemBufs = 4;   // of a tile's columns each
 constexpr int kProdWarps = 4;  // one stripe of the tile each
 constexpr int kMaxSplit = 8;
 
-template <int FMT, int G, int TM>
+// FOLD: Q8C, the K groups of a running sum; Q4, whether the sums move after p.fold stages (see fold_of), kFewRows or kManyRows of a
+// 64-row tile in use
+enum { kFewRows = 1, kManyRows = 2 };
+template <int FMT, int G, int TM, int FOLD>
 struct PrefillShape {
     static constexpr int kBlock = FMT == kQ8C ? 1024 : block_bytes(FMT == kQ4_1, G);
     static constexpr int kGroups = kStageK / G;           // K groups per stage: 4 (group 32) or 1 (group 128)
@@ -82,8 +85,11 @@ struct PrefillShape {
     static constexpr int kB = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;    // stages of activation codes
     static constexpr int kRaw = FMT == kQ8C || (TM == 64 && G == 32) ? 3 : 4;  // stages of packed bytes
     static constexpr int kScs = 4;                        // stages of scales
-    // buffers of integers in the kTmemBufs x TM columns (Q8C in 64-row tiles keeps its sums in the last one's place)
-    static constexpr int kBufs = FMT == kQ8C && TM == 64 ? kTmemBufs - 1 : kTmemBufs;
+    // Buffers of integers in the kTmemBufs x TM columns.  Sums that move, of 64-row tiles, take the last one's place, or where at most
+    // 48 rows are in use the last quarters of the buffers, which no MMA then writes.
+    static constexpr int kBufs = TM == 64 && FOLD > (FMT == kQ8C ? 0 : kFewRows) ? kTmemBufs - 1 : kTmemBufs;
+    static constexpr int kSumCol = kBufs == kTmemBufs ? 48 : kBufs * TM;      // of the first 16 rows' sums
+    static constexpr int kSumStep = kBufs == kTmemBufs ? TM : 16;             // from 16 rows to the next 16
     static constexpr int kRawStripe = kGroups * kBlock;   // packed bytes of one stripe in a stage
     static constexpr int kABytes = kTileN * kStageK, kBBytes = TM * kStageK;
     static constexpr int kXscBytes = kGroups * kSums * TM * 4;                // [group][scale | sum][row] fp32
@@ -266,15 +272,47 @@ __device__ __forceinline__ void unfold(uint64_t (&run)[8], uint32_t at) {  // `r
     }
 }
 
+
+// Q4 where sums move: the running sums of a thread's rows (sixteen, or `two` times sixteen) and the sums behind `at` added, into there,
+// and the running sums start anew; the `last` time into the running sums.  One piece of code for both: a CTA runs it once or twice,
+// and what it takes is its instructions' way to the SM (0.3 us for both; in front of the groups' loop's own branches 1 us).
+__device__ __forceinline__ void merge_sums(uint64_t (&run)[2][8], uint32_t at, uint32_t step, bool two, bool last) {
+    tc_wait_st();
+    auto add = [&](uint64_t (&r)[8], uint32_t at) {
+        uint32_t v[16];
+        tc_ld(at, v);
+        tc_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 8; j++) r[j] = fadd2(pack2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), r[j]);
+    };
+    auto store = [&](uint64_t (&r)[8], uint32_t at) {
+        uint32_t v[16];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            float lo, hi;
+            unpack2(r[j], lo, hi);
+            v[2 * j] = __float_as_uint(lo), v[2 * j + 1] = __float_as_uint(hi);
+            r[j] = 0;
+        }
+        q4fc::tc_st(at, v);
+    };
+    add(run[0], at);
+    if (two) add(run[1], at + step);
+    if (last) return;
+    store(run[0], at);
+    if (two) store(run[1], at + step);
+}
+
 template <int FMT, int G, int TM, int FOLD>
-__global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 ? 1 : 2)
+__global__ void __launch_bounds__(PrefillShape<FMT, G, TM, FOLD>::kThreads, TM == 128 ? 1 : 2)
     fc_prefill_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap codes_map) {
-    using S = PrefillShape<FMT, G, TM>;
+    using S = PrefillShape<FMT, G, TM, FOLD>;
     constexpr int BS = S::kBlock;
     constexpr int GPS = S::kGroups;
     constexpr int MMAS = G / 32;  // K=32 instructions per group
     constexpr int CGN = S::kEpiWarps / 4;
     constexpr int kUnpackWarp = S::kEpiWarps, kMmaWarp = kUnpackWarp + kProdWarps;
+    constexpr bool kMoves = FMT != kQ8C && FOLD > 0;
 
     extern __shared__ uint8_t smem_raw[];
     // (the same offset in every CTA of a cluster: the dynamic shared memory starts at the same address)
@@ -290,6 +328,7 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
     const uint32_t bar_tfull = bar_sempty + 8 * S::kScs, bar_tempty = bar_tfull + 8 * kTmemBufs;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 496);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 500);
+    [[maybe_unused]] volatile int* noted = reinterpret_cast<volatile int*>(bars + 504);  // kMoves: the CTA's groups, and rows
     static_assert(8 * (4 * S::kRaw + 2 * S::kA + 2 * S::kB + 2 * S::kScs + 2 * kTmemBufs) <= 496, "barriers");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -322,6 +361,7 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
             mbar_init(bar_tempty + 8 * i, S::kEpiWarps);
         }
         *abort_flag = 0;
+        if (kMoves) noted[0] = min(p.Kg, it1 * GPS) - it0 * GPS, noted[1] = live;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
     }
@@ -352,61 +392,85 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM>::kThreads, TM == 128 
         const uint32_t sum0 = TM == 128 ? smem0 + S::kSumOff + threadIdx.x * 16 : taddr + S::kBufs * TM;
         const uint32_t sum1 = sum0 + (TM == 128 ? 4 * 16 * kEpi : CGN * 16);
         const int groups = min(p.Kg, it1 * GPS) - it0 * GPS;
+        // groups g .. end - 1 into the running sums; false when a wait ran out
+        auto add_groups = [&](int g, int end) {
 #pragma unroll 1
-        for (int g = 0; g < groups; g++) {
-            const int i = g / GPS, sl = i % S::kScs, gi = g % GPS, b = g % S::kBufs;
-            if (gi == 0 && !wait_or_abort(bar_sfull + 8 * sl, (i / S::kScs) & 1, abort_flag)) break;
-            const uint8_t* sc = smem + S::kScOff + sl * S::kScBytes;
-            const float* xs = reinterpret_cast<const float*>(sc) + gi * (S::kSums * TM) + cgrp * 16;
-            uint64_t wd2 = 0, wm2 = 0;
-            if constexpr (FMT != kQ8C) {
-                const uint32_t w = reinterpret_cast<const uint32_t*>(sc + S::kXscBytes)[gi * kTileN + nrow];
-                const float wd = h2f((uint16_t)w), wm = h2f((uint16_t)(w >> 16));
-                wd2 = pack2(wd, wd), wm2 = pack2(wm, wm);
-            }
-            if (!wait_or_abort(bar_tfull + 8 * b, (g / S::kBufs) & 1, abort_flag)) break;
-            tc_fence_after();
-            // W integers at a time: what the two chunks would take together is what the register file has left, and the
-            // compiler then serialises the arithmetic (37 rows, one CTA an SM: 84 us with W = 16 in 72 registers, 78 with 8)
-            auto release = [&] {  // the buffer can be overwritten
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_tempty + 8 * b);
-            };
-            constexpr int W = S::kLoadWidth;
-            uint32_t v[W];
-            if (live0) {
-                tc_ld(taddr + b * TM, v);
-                tc_wait_ld();
-                accumulate<FMT, TM, 0, W>(acc[0], v, xs, wd2, wm2);
-                if constexpr (W == 8) {
-                    tc_ld(taddr + b * TM + 8, v);
+            for (; g < end; g++) {
+                const int i = g / GPS, sl = i % S::kScs, gi = g % GPS, b = g % S::kBufs;
+                if (gi == 0 && !wait_or_abort(bar_sfull + 8 * sl, (i / S::kScs) & 1, abort_flag)) return false;
+                const uint8_t* sc = smem + S::kScOff + sl * S::kScBytes;
+                const float* xs = reinterpret_cast<const float*>(sc) + gi * (S::kSums * TM) + cgrp * 16;
+                uint64_t wd2 = 0, wm2 = 0;
+                if constexpr (FMT != kQ8C) {
+                    const uint32_t w = reinterpret_cast<const uint32_t*>(sc + S::kXscBytes)[gi * kTileN + nrow];
+                    const float wd = h2f((uint16_t)w), wm = h2f((uint16_t)(w >> 16));
+                    wd2 = pack2(wd, wd), wm2 = pack2(wm, wm);
+                }
+                if (!wait_or_abort(bar_tfull + 8 * b, (g / S::kBufs) & 1, abort_flag)) return false;
+                tc_fence_after();
+                // W integers at a time: what the two chunks would take together is what the register file has left, and the
+                // compiler then serialises the arithmetic (37 rows, one CTA an SM: 84 us with W = 16 in 72 registers, 78 with 8)
+                auto release = [&] {  // the buffer can be overwritten
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_tempty + 8 * b);
+                };
+                constexpr int W = S::kLoadWidth;
+                uint32_t v[W];
+                if (live0) {
+                    tc_ld(taddr + b * TM, v);
                     tc_wait_ld();
-                    accumulate<FMT, TM, 4, W>(acc[0], v, xs + 8, wd2, wm2);
+                    accumulate<FMT, TM, 0, W>(acc[0], v, xs, wd2, wm2);
+                    if constexpr (W == 8) {
+                        tc_ld(taddr + b * TM + 8, v);
+                        tc_wait_ld();
+                        accumulate<FMT, TM, 4, W>(acc[0], v, xs + 8, wd2, wm2);
+                    }
                 }
-            }
-            if (live1) {
-                tc_ld(taddr + b * TM + CGN * 16, v);
-                tc_wait_ld();
-                if constexpr (W == 8) {
-                    accumulate<FMT, TM, 0, W>(acc[1], v, xs + CGN * 16, wd2, wm2);
-                    tc_ld(taddr + b * TM + CGN * 16 + 8, v);
+                if (live1) {
+                    tc_ld(taddr + b * TM + CGN * 16, v);
                     tc_wait_ld();
+                    if constexpr (W == 8) {
+                        accumulate<FMT, TM, 0, W>(acc[1], v, xs + CGN * 16, wd2, wm2);
+                        tc_ld(taddr + b * TM + CGN * 16 + 8, v);
+                        tc_wait_ld();
+                    }
                 }
-            }
-            release();
-            if (live1) accumulate<FMT, TM, W == 8 ? 4 : 0, W>(acc[1], v, xs + CGN * 16 + 16 - W, wd2, wm2);
-            if (gi == GPS - 1) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_sempty + 8 * sl);  // done with the stage's scales
-            }
-            if constexpr (FOLD > 0)
-                if (g % FOLD == FOLD - 1) {
-                    if (live0) fold<TM, kEpi>(acc[0], sum0, g == FOLD - 1);
-                    if (live1) fold<TM, kEpi>(acc[1], sum1, g == FOLD - 1);
+                release();
+                if (live1) accumulate<FMT, TM, W == 8 ? 4 : 0, W>(acc[1], v, xs + CGN * 16 + 16 - W, wd2, wm2);
+                if (gi == GPS - 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_sempty + 8 * sl);  // done with the stage's scales
                 }
+                if constexpr (FMT == kQ8C && FOLD > 0)
+                    if (g % FOLD == FOLD - 1) {
+                        if (live0) fold<TM, kEpi>(acc[0], sum0, g == FOLD - 1);
+                        if (live1) fold<TM, kEpi>(acc[1], sum1, g == FOLD - 1);
+                    }
+            }
+            return true;
+        };
+        if constexpr (!kMoves) {
+            add_groups(0, groups);
+        } else {
+            const uint32_t kZero[16] = {};
+            const uint32_t first = taddr + S::kSumCol + cgrp * (S::kSumStep - 16);
+            q4fc::tc_st(first, kZero);
+            if (live1) q4fc::tc_st(first + CGN * S::kSumStep, kZero);
+            // A loop around the groups' loop, which finds anew what it needs, so that the groups' loop keeps its registers (3584 columns, 16
+            // rows, K = 2816, group 32: moving nothing 12.8 us, so 13.5, as a branch in the groups' loop 14.8).
+            int end = 0;
+#pragma unroll 1
+            do {
+                const int g = end;
+                end = min(g + p.fold * GPS, noted[0]);
+                if (!add_groups(g, end)) break;
+                const uint32_t at = *reinterpret_cast<volatile uint32_t*>(tmem_slot) + ((threadIdx.x & 96u) << 16) + S::kSumCol;
+                const uint32_t w = threadIdx.x >> 7;
+                merge_sums(acc, at + w * S::kSumStep, CGN * S::kSumStep, (int)(w + CGN) * 16 < noted[1], end >= noted[0]);
+            } while (end < noted[0]);
         }
-        if (FOLD > 0 && groups >= FOLD) {
+        if (FMT == kQ8C && groups >= FOLD) {
             if (live0) unfold<TM, kEpi>(acc[0], sum0);
             if (live1) unfold<TM, kEpi>(acc[1], sum1);
         }
@@ -705,7 +769,7 @@ int make_codes_map(CUtensorMap* map, const int8_t* codes, int64_t rows, int64_t 
 
 template <int FMT, int G, int TM, int FOLD = 0>
 int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
-    using S = PrefillShape<FMT, G, TM>;
+    using S = PrefillShape<FMT, G, TM, FOLD>;
     static std::atomic<bool> attr_done[64] = {};  // set once per device; a second setter repeats the same call
     int dev = 0;
     Q4FC_CUDA_OK(cudaGetDevice(&dev));
@@ -736,7 +800,10 @@ int launch_prefill_variant(const PrefillParams& p, const CUtensorMap& map, dim3 
 
 template <int FMT, int G>
 int launch_prefill_tile(int tile, const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
-    return tile == 128 ? launch_prefill_wide(FMT, G, p, map, grid, s) : launch_prefill_variant<FMT, G, 64>(p, map, grid, s);
+    if (tile == 128) return launch_prefill_wide(FMT, G, p, map, grid, s);
+    if (p.fold == 0) return launch_prefill_variant<FMT, G, 64>(p, map, grid, s);
+    return p.rows <= 48 ? launch_prefill_variant<FMT, G, 64, kFewRows>(p, map, grid, s)
+                        : launch_prefill_variant<FMT, G, 64, kManyRows>(p, map, grid, s);
 }
 
 // tiles first .. end - 1, K divided by p.split
@@ -839,6 +906,18 @@ TilePlan plan_tiles(int tile, bool wide, int G, bool q8c, int64_t n_tiles, int64
     return t;
 }
 
+// Stages of a running sum (Q4), 0: all of a CTA's.  The rounding error of a sum grows with the root of its terms, so that a division of
+// K into few parts, where it is the fastest, would be less exact than one into many (49 x 10740 x 9384, group 32: by two 2.38e-7 of
+// the result in the 2-norm, by four 1.80e-7).  So no running sum is longer than if K were divided as often as fills two places on every
+// SM, and the parts of a CTA are added as those of several would be.
+int64_t fold_of(int64_t split, int64_t n_tiles, int64_t rows, int64_t nstage, int64_t sms) {
+    const int64_t tiles = n_tiles * ((rows + 63) / 64), most = nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
+    const int64_t parts = 2 * sms / tiles < most ? 2 * sms / tiles : most;
+    if (parts <= split) return 0;
+    const int64_t fold = (nstage + parts - 1) / parts;
+    return fold < (nstage + split - 1) / split ? fold : 0;
+}
+
 // Quantizer and GEMM; `codes` and `sc` are scratch for [rows][Kg * G] bytes and scale_bytes().
 int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t ldx, int8_t* codes, float* sc,
                 PrefillParams p, cudaStream_t s) {
@@ -877,6 +956,7 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     if (Kp > 0)  // (no K group: no stage reads the map)
         if (int rc = make_codes_map(&map, codes, rows, f16 ? 2 * Kp : Kp, tile)) return rc;
     p.split = (int)split, p.part = left == 0 ? kWhole : kFirst;
+    p.fold = fmt == kQ8C || left > 0 ? 0 : (int)fold_of(split, n_tiles, rows, nstage, di->sm_count);
     if (int rc = launch_tiles(fmt, G, tile, p, map, 0, tiles - left, s)) return rc;
     if (left == 0) return Q4FC_OK;
     p.split = (int)left_split, p.part = kRemainder;

@@ -62,8 +62,11 @@ struct WideShape {
     static constexpr int kSlotBytes = kRawBytes + kXscBytes;
     static constexpr int kSlotOff = kB * kBBytes;
     static constexpr int kBarOff = kSlotOff + kSlots * kSlotBytes;
-    static constexpr int kSmem = kBarOff + 512 + 1024 /*alignment slack*/;
-    static_assert(kSmem <= 227 * 1024, "one CTA on an SM");
+    static constexpr int kSumOff = kBarOff + 512;
+    // where the sums move (FOLD), their second place is behind the barriers
+    template <bool FOLD>
+    static constexpr int kSmem = kSumOff + (FOLD ? TM * kTileN * 4 : 0) + 1024 /*alignment slack*/;
+    static_assert(kSmem<true> <= 227 * 1024, "one CTA on an SM");
     static_assert(TM * kTileN * 4 <= kSlotOff, "the partial tile of a K split takes the place of the codes");
 };
 
@@ -179,7 +182,8 @@ __device__ __forceinline__ void accumulate(uint64_t (&acc)[W / 2], const uint32_
     }
 }
 
-template <int FMT, int G>
+// FOLD: the running sums move to a second place, once, after p.fold stages of 128 k (0.9 us for that and adding them at the end)
+template <int FMT, int G, bool FOLD>
 __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap codes_map) {
     using S = WideShape<FMT, G>;
     constexpr int BS = S::kBlock;
@@ -259,12 +263,19 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
         uint32_t v[2][W];
         uint32_t xs = 0;  // the group's scales, as an offset: the compiler keeps to shared-memory loads
         uint64_t wd2 = 0, wm2 = 0;
+        // a thread's sums behind the barriers, in 16-byte places of its own: `then`(place, two pairs of rows) for each of them
+        [[maybe_unused]] auto sums = [&](auto then) {
+            ulonglong2* at = reinterpret_cast<ulonglong2*>(smem + S::kSumOff) + threadIdx.x;
+#pragma unroll
+            for (int j = 0; j < kChunks * W / 4; j++) then(at[j * kEpiWarps * 32], acc[j / (W / 4)][2 * j % (W / 2)], acc[j / (W / 4)][2 * j % (W / 2) + 1]);
+        };
         auto scale = [&](int c) {
             accumulate<FMT, S::kF16>(acc[c], v[c & 1], reinterpret_cast<const float*>(smem + xs) + c * (2 * W), wd2, wm2);
         };
         // Weights: a warp unpacks half of its 32 columns' share of a stage, kA - 1 stages in front of the one it scales.  (The MMAs
         // that read that place before have ended: this warp has seen the sums of a later one.)
         constexpr int kLead = kA - 1;
+        constexpr int kPerFold = 128 / (GPS * G);  // stages of 128 k
         const uint32_t share = quarter * S::kRawStripe + half * (S::kF16 ? BS : 1024) + lane * 4;
         constexpr int kWords = S::kF16 ? 4 : 8, kOut = 16 / kWords;
         uint32_t words[kWords];
@@ -334,6 +345,8 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
                     const uint16_t wd16 = *reinterpret_cast<const uint16_t*>(tail);
                     const uint16_t wm16 = FMT == kQ4_1 ? *reinterpret_cast<const uint16_t*>(tail + 64) : 0;
                     if (ALL && later) scale(kChunks - 1);  // of the group before
+                    if constexpr (FOLD)
+                        if (gi == 0 && i == p.fold * kPerFold) sums([](ulonglong2& s, uint64_t& a, uint64_t& b) { s.x = a, s.y = b, a = b = 0; });
                     xs = sc + S::kRawBytes + (gi * (S::kSums * TM) + half * W) * 4;
                     const float wd = h2f(wd16) * (S::kF16 ? kWdScale : 1.0f), wm = h2f(wm16);
                     wd2 = pack2(wd, wd), wm2 = pack2(wm, wm);
@@ -383,6 +396,8 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
             run(std::true_type{});
         else
             run(std::false_type{});
+        if constexpr (FOLD)
+            if (iters > p.fold * kPerFold) sums([](ulonglong2& s, uint64_t& a, uint64_t& b) { a = fadd2(s.x, a), b = fadd2(s.y, b); });
         if (cs > 1) asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");  // (the partial tile takes the place of what they read)
         if (cs == 1) {
             const int64_t n = n0 + nrow;
@@ -579,22 +594,22 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
     }
 }
 
-template <int FMT, int G>
+template <int FMT, int G, bool FOLD>
 int launch_variant(const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
     using S = WideShape<FMT, G>;
     static std::atomic<bool> attr_done[64] = {};  // set once per device; a second setter repeats the same call
     int dev = 0;
     Q4FC_CUDA_OK(cudaGetDevice(&dev));
-    auto* fn = fc_prefill_wide_kernel<FMT, G>;
+    auto* fn = fc_prefill_wide_kernel<FMT, G, FOLD>;
     if (dev >= 64 || !attr_done[dev]) {
-        Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSmem));
+        Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::template kSmem<FOLD>));
         Q4FC_CUDA_OK(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         if (dev < 64) attr_done[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = S::kSmem;
+    cfg.dynamicSmemBytes = S::template kSmem<FOLD>;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     // starts beside the quantizer in front of it and waits for that one's results where it needs them
@@ -610,12 +625,17 @@ int launch_variant(const PrefillParams& p, const CUtensorMap& map, dim3 grid, cu
     return Q4FC_OK;
 }
 
+template <int FMT, int G>
+int launch_fold(const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
+    return p.fold > 0 ? launch_variant<FMT, G, true>(p, map, grid, s) : launch_variant<FMT, G, false>(p, map, grid, s);
+}
+
 }  // namespace
 
 int launch_prefill_wide(int fmt, int G, const PrefillParams& p, const CUtensorMap& map, dim3 grid, cudaStream_t s) {
-    if (fmt == kQ4_1) return G == 32 ? launch_variant<kQ4_1, 32>(p, map, grid, s) : launch_variant<kQ4_1, 128>(p, map, grid, s);
-    if (fmt == kQ4_0) return G == 32 ? launch_variant<kQ4_0, 32>(p, map, grid, s) : launch_variant<kQ4_0, 128>(p, map, grid, s);
-    return G == 32 ? launch_variant<kQ4_0Signed, 32>(p, map, grid, s) : launch_variant<kQ4_0Signed, 128>(p, map, grid, s);
+    if (fmt == kQ4_1) return G == 32 ? launch_fold<kQ4_1, 32>(p, map, grid, s) : launch_fold<kQ4_1, 128>(p, map, grid, s);
+    if (fmt == kQ4_0) return G == 32 ? launch_fold<kQ4_0, 32>(p, map, grid, s) : launch_fold<kQ4_0, 128>(p, map, grid, s);
+    return G == 32 ? launch_fold<kQ4_0Signed, 32>(p, map, grid, s) : launch_fold<kQ4_0Signed, 128>(p, map, grid, s);
 }
 
 }  // namespace q4fc

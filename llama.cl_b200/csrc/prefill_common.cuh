@@ -23,6 +23,7 @@ struct PrefillParams {
     int n_tiles;         // column tiles; tiles are counted along them
     int n_off, m_off;    // this launch's first tile
     int n_end, m_end;    // and the one behind its last
+    int fold;            // Q4: stages of 128 k of a running sum, 0: one sum over all of a CTA's stages
     int part;            // kWhole, or of two launches kFirst (whole rounds) and kRemainder (the tiles that are left)
 };
 
