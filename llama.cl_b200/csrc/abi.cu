@@ -46,6 +46,7 @@ const DeviceInfo* device_info() {
             set_error("cannot query device %d", dev);
             return nullptr;
         }
+        info[dev].index = dev;
         info[dev].sm_count = sms;
         info[dev].max_smem_optin = smem;
         ready[dev] = true;

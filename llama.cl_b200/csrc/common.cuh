@@ -34,6 +34,7 @@ int cuda_fail(cudaError_t e, const char* what);
     } while (0)
 
 struct DeviceInfo {
+    int index;
     int sm_count;
     int max_smem_optin;
 };

@@ -56,6 +56,7 @@
 
 #include <atomic>
 #include <cfloat>
+#include <mutex>
 
 #include "prefill_common.cuh"
 
@@ -68,6 +69,7 @@ constexpr int kStageK = 128;   // k per shared-memory stage (one 128-byte swizzl
 constexpr int kTmemBufs = 4;   // of a tile's columns each
 constexpr int kProdWarps = 4;  // one stripe of the tile each
 constexpr int kMaxSplit = 8;
+constexpr int64_t kMaxTileRows = 65535;  // rows of tiles, a grid's y
 
 // FOLD: Q8C, the K groups of a running sum; Q4, whether the sums move after p.fold stages (see fold_of), kFewRows or kManyRows of a
 // 64-row tile in use
@@ -831,78 +833,132 @@ int launch_tiles(int fmt, int G, int tile, PrefillParams p, const CUtensorMap& m
 // scales and group sums of a format, padded to whole row tiles of either size
 size_t scale_bytes(int64_t rows, int64_t Kg, int sums) { return (size_t)((rows + 127) / 128 * 128) * Kg * sums * 4; }
 
+// Clusters of 1 .. kMaxSplit CTAs that run at once, one CTA on an SM and two.  Cards differ in where their SMs lie (clusters of three and
+// five CTAs: 42 and 24 on one B200, 45 and 26 on another), so the runtime is asked; for an empty kernel, since of a
+// 64-row tile's own kernel it counts one CTA on an SM where two run.
+__global__ void cluster_room_kernel() {}
+struct ClusterRoom {
+    int one[kMaxSplit], two[kMaxSplit];
+};
+const ClusterRoom& cluster_room(const DeviceInfo* di) {
+    static std::atomic<bool> known[64] = {};
+    static ClusterRoom rooms[64];
+    static std::mutex mutex;
+    ClusterRoom& room = rooms[di->index];
+    if (known[di->index].load(std::memory_order_acquire)) return room;
+    std::lock_guard<std::mutex> lock(mutex);
+    for (int places = 1; places <= 2; places++)
+        for (int c = 1; c <= kMaxSplit; c++) {
+            const int smem = places == 1 ? di->max_smem_optin : 113 * 1024;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(c * di->sm_count)), cfg.blockDim = dim3(64), cfg.dynamicSmemBytes = (size_t)smem;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned)c, attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr, cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaFuncSetAttribute(cluster_room_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+                cudaFuncSetAttribute(cluster_room_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&n, cluster_room_kernel, &cfg) != cudaSuccess || n <= 0) {
+                cudaGetLastError();
+                n = places * di->sm_count / c * 7 / 8;  // a stand-in
+                if (n < 1) n = 1;
+            }
+            (places == 1 ? room.one : room.two)[c - 1] = n;
+        }
+    known[di->index].store(true, std::memory_order_release);
+    return room;
+}
+// Clusters of an odd number of CTAs find the last of their places late: by how much more the n-th takes (K = 4096, group 32, 64 rows, two
+// places on an SM: by three up to 87 tiles 35 us, 90 41, 93 54; 128 rows, one place, up to 43 tiles 30 us, 44 33, 45 38).
+float late(int n, int room, int c, float most) {
+    const int last = room / 14 > 0 ? room / 14 : 1;
+    return c > 1 && c % 2 == 1 && n > room - last ? 1.0f + most * (float)(n - (room - last)) / (float)last : 1.0f;
+}
+
 // How tiles of `tile` rows go over the SMs.
 struct TilePlan {
     int tile = 0;
-    int64_t tiles = 0, split = 1;          // K divided over clusters of `split` CTAs ...
-    int64_t left = 0, left_split = 1;      // ... and of the last `left` tiles, in a launch of their own, over `left_split`
-    int64_t cost = 0;                      // rounds over the SMs in stages of 128 k, start-up and adding included
-    bool crowded = false;                  // two CTAs on an SM
+    int tiles = 0, split = 1;          // K divided over clusters of `split` CTAs ...
+    int left = 0, left_split = 1;      // ... and of the last `left` tiles, in a launch of their own, over `left_split`
+    float cost = 0;                    // us
 };
-// Clusters of 1 .. 8 CTAs that run at once on 148 SMs, one CTA on an SM: by the number of
-// tiles left from which on the launch takes longer (rows x 4096, group 32: 33 tiles by four 100.5 us, 34 120.6; 22 by six 97.5,
-// 23 114.3; 42 by three 112, 44 129, of the wide kernel 44 148.8 and 48 173.8).  Two CTAs on an SM: twice as many at least.
-int64_t clusters_at_once(int64_t c, bool wide, int64_t places) {
-    constexpr int kAtOnce[kMaxSplit] = {148, 74, 42, 33, 24, 22, 15, 15};
-    const int64_t n = (wide && c == 3 ? 44 : kAtOnce[c - 1]) * places / 148;
-    return n > 1 ? n : 1;
-}
-// Over how many CTAs few 64-row tiles, one for each 128 columns, divide K: rounds x (stages of a CTA + start-up and adding), where a stage takes half as long
-// again, and the rest a fifth, once two CTAs share an SM.  By the times of 84 calls (12 to 64 rows, 8 to 141 tiles) divided by 1 to 8: 0.1 %
-// behind the best of them, at most 2 %; as often as fills two places on every SM 7 % and 50 % (64 x 5120 x 4096, 40 tiles, group
-// 128: by seven 22.4 us, by six 15.8; 64 x 4096 x 4096: by eight 14.9, by four 13.1; group 32, 47 tiles: by six 41.7, by five 29.8).
-// Clusters of two CTAs on an SM that were seen to run at once: kTwo.
-int64_t split_of_few(int64_t tiles, int64_t most, int G, bool q8c, int64_t nstage, int64_t sms) {
-    constexpr int kTwo[kMaxSplit] = {296, 148, 86, 66, 48, 44, 32, 32};
-    const int64_t startup = G == 128 ? 16 : 4;
-    int64_t best = 0, best_cost = 0;
-    for (int64_t c = 1; c <= most; c++) {
-        const int64_t fit = kTwo[c - 1] * sms / 148 > 1 ? kTwo[c - 1] * sms / 148 : 1, rounds = (tiles + fit - 1) / fit;
-        const bool shared = tiles > clusters_at_once(c, false, sms) + (q8c ? 1 : 0);  // (Q8C, 50 x 2048, 16 tiles: by eight 18.5, by six 19.2)
-        const int64_t cost = rounds * ((nstage + c - 1) / c * (shared ? 15 : 10) + startup * (shared ? 12 : 10));
-        if (best == 0 || cost <= best_cost) best = c, best_cost = cost;
+// What a stage of 128 k takes, us: a 64-row tile's alone on an SM, and for each 16 rows in use; with a second CTA on the SM; a
+// tile's of the wide kernel.  These and the constants in plan_tiles are fitted to the times of 844 calls of 9 to 2048 rows, each in both
+// tiles and with every division of K.  What they choose took 0.3 % longer than the best of these in the mean, at most 12 % (rules of their own
+// for at most 64 rows, for more and between the tiles, by the clusters that one card holds at once: 2 %, of Q8C 4 %, at most 53 %).
+struct StageCost {
+    float alone, alone_rows, shared, shared_rows, wide;
+};
+constexpr StageCost kStageQ4[2][2] = {{{0.51f, 0.04f, 0.62f, 0.07f, 0.57f}, {0.44f, 0.06f, 0.59f, 0.11f, 0.64f}},    // group 128: Q4_0, Q4_1
+                                      {{0.97f, 0.20f, 1.16f, 0.29f, 1.65f}, {1.11f, 0.24f, 1.29f, 0.38f, 2.20f}}};   // group 32
+constexpr StageCost kStageQ8C = {0.95f, 0.20f, 1.06f, 0.29f, 0};
+
+// The last tiles of many: K divided over clusters where that takes less than a round more.  In stages: rounds x (stages of a CTA +
+// start-up and adding).  (11008 columns, K = 4096: 512 rows, group 32, 48 of 344 tiles left, undivided 177 us, by two 156, by three,
+// which takes two rounds, 174; 256 rows, Q8C, 24 of 172, 148 -> 100; 100 rows x 20000, group 32, 18 of 314, 174 -> 106.  Divided where
+// this sum says no: 1024 x 4096 x 4096, 108 of 256 left, 125 -> 137.)
+int split_of_left(int left, const int* room, int most, int nstage, int startup) {
+    float best = (float)nstage;  // undivided, in the launch of the others
+    int split = 1;
+    for (int c = 2; c <= most; c++) {
+        const int full = (left - 1) / room[c - 1], rest = left - full * room[c - 1];
+        const float cost = ((float)full + late(rest, room[c - 1], c, 0.25f)) * (float)((nstage + c - 1) / c + startup);
+        if (cost < best) best = cost, split = c;
     }
-    return best;
+    return split;
 }
-TilePlan plan_tiles(int tile, bool wide, int G, bool q8c, int64_t n_tiles, int64_t rows, int64_t nstage, int64_t sms) {
+// Into how many running sums the K of a tile is divided at least (see fold_of).
+int least_parts(int n_tiles, int64_t rows, int nstage, int sms) {
+    const int64_t tiles = n_tiles * ((rows + 63) / 64);
+    const int most = nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
+    return 2 * sms / tiles < most ? (int)(2 * sms / tiles) : most;
+}
+TilePlan plan_tiles(int tile, int fmt, int G, int n_tiles, int64_t rows, int nstage, const ClusterRoom& at_once, int sms) {
+    const bool q8c = fmt == kQ8C, wide = tile == 128 && !q8c;
+    const StageCost& stage = q8c ? kStageQ8C : kStageQ4[G == 32][fmt == kQ4_1];
+    const int m_tiles = (int)((rows + tile - 1) / tile);
     TilePlan t;
-    t.tile = tile, t.tiles = n_tiles * ((rows + tile - 1) / tile);
-    const int64_t places = (tile == 128 ? 1 : 2) * sms, most = nstage / 4 < 1 ? 1 : nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
-    const int64_t startup = G == 128 ? 8 : 4, start_few = wide ? startup + 2 : startup;
-    auto divided = [&](int64_t tiles, int64_t c, int64_t startup) {  // rounds x (stages of a CTA + start-up and adding)
-        const int64_t fit = clusters_at_once(c, wide, places);
-        return (tiles + fit - 1) / fit * ((nstage + c - 1) / c + startup);
-    };
-    if (t.tiles < places) {
-        // Few tiles: K is divided while a CTA keeps four stages.  The wide kernel: as the sum of
-        // rounds, stages and start-up says, with the clusters that run at once (192 x 1024 x 4096, 16 tiles, group 32: by eight 31.9 us,
-        // by six 21.4; 128 x 6000 x 3000, 47 tiles: by three 44.9, by two 31.4; 300 x 1500 x 4096, 36 tiles: by four 41.4, by
-        // three 31.4).  More than one row of 64-row tiles: as often as fills the two places on every SM (the last row is seldom full, and its
-        // CTAs leave early: 150 x 3000 x 4096, 72 tiles: by four 40, by three, which that sum says, 52).
-        t.split = wide ? 1 : rows <= 64 ? split_of_few(t.tiles, most, G, q8c, nstage, sms) : places / t.tiles < most ? places / t.tiles : most;
+    t.tile = tile, t.tiles = n_tiles * m_tiles;
+    const int places = (tile == 128 ? 1 : 2) * sms, most = nstage / 4 < 1 ? 1 : nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
+    const bool few = t.tiles < places;
+    const int* room = tile == 128 ? at_once.one : at_once.two;
+    // 64-row tiles: 16-row pieces in use, of the fullest tile and in the mean
+    const float fullest = rows < 64 ? (float)((rows + 15) / 16) : 4.0f, mean = (float)((rows + 15) / 16) / (float)m_tiles;
+    const float alone = stage.alone + stage.alone_rows * fullest;
+    const float shared = stage.shared + stage.shared_rows * (few && m_tiles > 1 ? 0.5f * (mean + fullest) : mean);
+    // the wide kernel: a tile with fewer rows takes other loads, and by what it lets stand hardly less (129 to 256 rows x 6144 x 18944, two rounds,
+    // the second of tiles with 1, 33, 65, 97 and 128 rows: Q4_0 group 32 68, 78, 90, 95 and 83 us, Q4_1 group 128 29, 30, 33, 37 and 39)
+    const int last = (int)((rows - (int64_t)(m_tiles - 1) * tile + 15) / 16);
+    const float partial = last == 8 ? 1.0f : 0.75f + 0.05f * (float)last;
+    // n tiles, K divided by c: rounds x (start + stages)
+    auto launch = [&](int n, int c) {
+        const float stages = (float)((nstage + c - 1) / c);
+        const int full = (n - 1) / room[c - 1], rest = n - full * room[c - 1];
         if (wide) {
-            for (int64_t c = 2; c <= most; c++)
-                if (divided(t.tiles, c, start_few) < divided(t.tiles, t.split, start_few)) t.split = c;
+            const float used = full > 0 ? ((float)(m_tiles - 1) + partial) / (float)m_tiles : m_tiles > 1 && partial < 1 ? 1.0f : partial;
+            return (6.4f + stages * stage.wide * used) * ((float)full + late(rest, room[c - 1], c, 0.4f));
         }
-        t.cost = wide ? divided(t.tiles, t.split, start_few) : (nstage + t.split - 1) / t.split + startup;
-        t.crowded = t.tiles * t.split > sms;
-        return t;
+        const float pair = 4.6f + stages * shared, one = 3.3f + stages * alone;
+        if (rest > at_once.one[c - 1]) return pair * ((float)full + late(rest, room[c - 1], c, 0.5f));
+        return pair * (float)full + one * (full == 0 ? late(rest, at_once.one[c - 1], c, 0.05f) : 1.0f);
+    };
+    const float clusters = wide ? 1.9f : 2.3f;  // their start, and adding their parts
+    if (few) {
+        // K is divided while a CTA keeps four stages
+        const int parts = q8c ? 0 : least_parts(n_tiles, rows, nstage, sms);
+        for (int c = 1; c <= most; c++) {
+            if (wide && parts > 2 * c) continue;  // (whose sums move once)
+            const float cost = launch(t.tiles, c) + (c > 1 ? clusters : 0.0f) + (parts > c ? 0.8f : 0.0f);
+            if (t.cost == 0 || cost <= t.cost) t.split = c, t.cost = cost;
+        }
+    } else {
+        if (t.tiles % places != 0) t.left_split = split_of_left(t.tiles % places, room, most, nstage, G == 128 ? 8 : 4);
+        if (t.left_split > 1) t.left = t.tiles % places;
+        t.cost = launch(t.tiles - t.left, 1) + (t.left > 0 ? launch(t.left, t.left_split) + clusters : 0.0f);
     }
-    t.crowded = tile != 128;
-    t.cost = t.tiles / places * nstage + startup;
-    if (t.tiles % places != 0) {
-        // What is left after whole rounds over the places would take a round of its own, most places empty.  With K divided by c it
-        // takes 1/c of one, and some stages' time for start-up and the adding, where that many clusters run at once.  (11008
-        // columns, K = 4096: 512 rows, group 32, 48 of 344 tiles left, undivided 177 us, by two 156, by three, which takes two rounds,
-        // 174; 256 rows, Q8C, 24 of 172, 148 -> 100; 100 rows x 20000, group 32, 18 of 314, 174 -> 106.  Divided where
-        // this sum says no: 1024 x 4096 x 4096, 108 of 256 left, 125 -> 137.)
-        t.left = t.tiles % places;
-        int64_t best = nstage;  // undivided, in the launch of the others
-        for (int64_t c = 2; c <= most; c++)
-            if (divided(t.left, c, startup) < best) best = divided(t.left, c, startup), t.left_split = c;
-        if (t.left_split == 1) t.left = 0;
-        t.cost += best;
-    }
+    if (wide) t.cost -= 0.6f;
     return t;
 }
 
@@ -910,11 +966,9 @@ TilePlan plan_tiles(int tile, bool wide, int G, bool q8c, int64_t n_tiles, int64
 // K into few parts, where it is the fastest, would be less exact than one into many (49 x 10740 x 9384, group 32: by two 2.38e-7 of
 // the result in the 2-norm, by four 1.80e-7).  So no running sum is longer than if K were divided as often as fills two places on every
 // SM, and the parts of a CTA are added as those of several would be.
-int64_t fold_of(int64_t split, int64_t n_tiles, int64_t rows, int64_t nstage, int64_t sms) {
-    const int64_t tiles = n_tiles * ((rows + 63) / 64), most = nstage / 4 < kMaxSplit ? nstage / 4 : kMaxSplit;
-    const int64_t parts = 2 * sms / tiles < most ? 2 * sms / tiles : most;
+int fold_of(int split, int parts, int nstage) {
     if (parts <= split) return 0;
-    const int64_t fold = (nstage + parts - 1) / parts;
+    const int fold = (nstage + parts - 1) / parts;
     return fold < (nstage + split - 1) / split ? fold : 0;
 }
 
@@ -929,37 +983,44 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
         set_error("fc_prefill: rows=%lld or K=%lld beyond the 2^31 coordinate range", (long long)rows, (long long)K);
         return Q4FC_ELIMIT;
     }
-    const int64_t n_tiles = (p.N + kTileN - 1) / kTileN;
-    const int64_t nstage = (Kp + kStageK - 1) / kStageK;
-    // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM.
-    TilePlan t = plan_tiles(64, false, G, fmt == kQ8C, n_tiles, rows, nstage, di->sm_count);
-    if (rows > 64 && fmt == kQ8C) {
-        // Q8C: the large tile as soon as such tiles occupy every SM (256 rows x 4096 x 11008: 102 us and 108).
-        if (n_tiles * ((rows + 127) / 128) >= di->sm_count) t = plan_tiles(128, false, G, true, n_tiles, rows, nstage, di->sm_count);
-    } else if (rows > 64) {
-        // A round of 64-row tiles, two on an SM, takes 1.5 times one of the wide kernel's tiles; alone on an SM as long as that.  Over 495
-        // calls (65 to 512 rows, K x N from 1000 x 1500 to 4096 x 11008) the choice costs 0.9 % against the better of the two, at most
-        // 16 % (192 x 700 x 11008: 38.9 and 33.6); always the wide kernel 3.2 %, from as many of its tiles on as SMs 11.6 %.
-        const TilePlan w = plan_tiles(128, true, G, false, n_tiles, rows, nstage, di->sm_count);
-        if (Kp <= 0x3fffffffLL && (w.tiles >= di->sm_count || 2 * w.cost <= (t.crowded ? 3 : 2) * t.cost)) t = w;
-    }
-    const int tile = t.tile;
-    const int64_t m_tiles = (rows + tile - 1) / tile, tiles = t.tiles, split = t.split, left = t.left, left_split = t.left_split;
-    if (n_tiles * split > 0x7fffffffLL || m_tiles > 65535 || tiles > 0x7fffffffLL / kMaxSplit) {
-        set_error("fc_prefill: %lld x %lld tiles exceed the grid limit", (long long)n_tiles, (long long)m_tiles);
+    const int64_t all_columns = (p.N + kTileN - 1) / kTileN;
+    if (all_columns > 0x7fffffffLL / kMaxSplit || (rows + 63) / 64 > 0x7fffffffLL / kMaxSplit / all_columns) {
+        set_error("fc_prefill: %lld rows x %lld columns exceed the grid limit", (long long)rows, (long long)p.N);
         return Q4FC_ELIMIT;
     }
-    p.n_tiles = (int)n_tiles;
+    const int n_tiles = (int)all_columns, nstage = (int)((Kp + kStageK - 1) / kStageK), sms = di->sm_count;
+    const ClusterRoom& room = cluster_room(di);
+    // 128-row tiles unpack the weights half as often, 64-row tiles run two to an SM.
+    TilePlan t;
+    if (fmt == kQ8C) {
+        // Q8C: the large tile as soon as such tiles occupy every SM (256 rows x 4096 x 11008: 102 us and 108).
+        const int tile = rows > 64 && n_tiles * ((rows + 127) / 128) >= sms ? 128 : 64;
+        t = plan_tiles(tile, fmt, G, n_tiles, rows, nstage, room, sms);
+    } else {
+        t = plan_tiles(64, fmt, G, n_tiles, rows, nstage, room, sms);
+        if (rows > 64 && Kp <= 0x3fffffffLL) {
+            // The large tile too where its last tiles are divided, which takes less than the sum (they start beside the others' ends: 129 rows
+            // x 2080 x 9500, Q4_0 group 32, 38 us, sum 50, and 45 in 64-row tiles; over 180 calls of many tiles 0.04 % are lost).
+            const TilePlan w = plan_tiles(128, fmt, G, n_tiles, rows, nstage, room, sms);
+            if (w.cost < t.cost || w.left > 0 || rows > kMaxTileRows * 64) t = w;
+        }
+    }
+    const int tile = t.tile, tiles = t.tiles, split = t.split, left = t.left;
+    if (rows > kMaxTileRows * tile) {
+        set_error("fc_prefill: %lld rows exceed the grid limit", (long long)rows);
+        return Q4FC_ELIMIT;
+    }
+    p.n_tiles = n_tiles;
     const bool f16 = G == 32 && fmt != kQ8C && tile == 128;  // operands of the wide kernel
     if (int rc = launch_quant_x_tile(x, rows, K, ldx, G, fmt == kQ4_1, tile, f16, codes, sc, s)) return rc;
     CUtensorMap map = {};
     if (Kp > 0)  // (no K group: no stage reads the map)
         if (int rc = make_codes_map(&map, codes, rows, f16 ? 2 * Kp : Kp, tile)) return rc;
-    p.split = (int)split, p.part = left == 0 ? kWhole : kFirst;
-    p.fold = fmt == kQ8C || left > 0 ? 0 : (int)fold_of(split, n_tiles, rows, nstage, di->sm_count);
+    p.split = split, p.part = left == 0 ? kWhole : kFirst;
+    p.fold = fmt == kQ8C || left > 0 ? 0 : fold_of(split, least_parts(n_tiles, rows, nstage, sms), nstage);
     if (int rc = launch_tiles(fmt, G, tile, p, map, 0, tiles - left, s)) return rc;
     if (left == 0) return Q4FC_OK;
-    p.split = (int)left_split, p.part = kRemainder;
+    p.split = t.left_split, p.part = kRemainder;
     return launch_tiles(fmt, G, tile, p, map, tiles - left, tiles, s);
 }
 

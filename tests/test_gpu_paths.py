@@ -267,6 +267,79 @@ def test_many_rows_last_tiles_divided(pkg, oracle, fmt, rows, N, K):
     check_many_rows(pkg, oracle, fmt, rows, N, K, launches=3)  # the quantizer, whole rounds, the remainder
 
 
+class _KernelNode(ctypes.Structure):
+    _fields_ = [("func", ctypes.c_void_p), ("grid", ctypes.c_uint * 3), ("block", ctypes.c_uint * 3), ("shared", ctypes.c_uint),
+                ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p), ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
+
+
+def gemm_launches(run):
+    """What a call of the many-row FC launches behind the quantizer: for each kernel its blocks' threads and its clusters' blocks."""
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        run()  # the stream's workspace
+        stream.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            run()
+    cu, n = ctypes.CDLL("libcuda.so.1"), ctypes.c_size_t()
+    g = ctypes.c_void_p(graph.raw_cuda_graph())
+    assert cu.cuGraphGetNodes(g, None, ctypes.byref(n)) == 0
+    nodes, seen = (ctypes.c_void_p * n.value)(), []
+    assert cu.cuGraphGetNodes(g, nodes, ctypes.byref(n)) == 0
+    for node in map(ctypes.c_void_p, nodes):
+        kernel, value = _KernelNode(), (ctypes.c_uint * 16)()
+        assert cu.cuGraphKernelNodeGetParams_v2(node, ctypes.byref(kernel)) == 0
+        assert cu.cuGraphKernelNodeGetAttribute(node, 4, value) == 0  # the cluster's dimension
+        if kernel.block[0] != 256:  # (the quantizer)
+            seen.append((kernel.block[0], value[0]))
+    return sorted(seen, key=lambda launch: launch[1])
+
+
+ROWS64, ROWS128 = 448, 320  # threads of a block: of 64-row tiles, and of 128-row tiles of Q4 weights
+
+
+@pytest.mark.parametrize("rows,N,K,launches", [
+    # few tiles: K by one to eight, the last stage not full; 69 tiles, which run at once by four on every card
+    *[(20 if c % 2 else 50, 300, 512 * c + 300, [(ROWS64, c)]) for c in range(1, 9)], (31, 8707, 6030, [(ROWS64, 4)]),
+    # a few more than two on each of 148 SMs
+    *[(40, (296 + left) * 128 - 59, K, [(ROWS64, 1), (ROWS64, c)])
+      for left, K, c in [(100, 4096, 2), (80, 4096, 3), (65, 4096, 4), (47, 4096, 5), (44, 4096, 6), (30, 3564, 7), (30, 4076, 8)]],
+    # 128-row tiles, whole calls (the second, fourth, sixth and eighth: rows that are not there, more of them columns)
+    *[(rows, tiles * 128 - 20, K, [(ROWS128, c)]) for c, (rows, tiles, K) in enumerate([
+        (256, 74, 2000), (200, 35, 3000), (128, 38, 6500), (113, 31, 4000), (128, 23, 8000), (113, 22, 6500), (128, 14, 3900),
+        (113, 15, 8000)], 1)],
+    # and a few more than one on each SM
+    *[(65, (148 + left) * 128 - 59, K, [(ROWS128, 1), (ROWS128, c)])
+      for left, K, c in [(50, 4096, 2), (40, 4096, 3), (30, 4096, 4), (23, 4096, 5), (20, 4096, 6), (10, 3564, 7), (10, 4076, 8)]],
+])
+@pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128", "q8c"])
+def test_every_division_of_k(pkg, fmt, rows, N, K, launches):
+    """Every way to divide K, in either tile and for the last of many tiles, and that it is the one a call takes; against calls of
+    at most eight rows, which other kernels serve: the same exact integers, other products and sums (tolerance as above)."""
+    ops = pkg.llmops
+    g = torch.Generator(device="cuda").manual_seed(rows + N + K)
+    W, x = torch.randn(N, K, generator=g, device="cuda") * 0.02, torch.randn(1, rows, K, generator=g, device="cuda")
+    if fmt == "q8c":
+        if launches[0][0] == ROWS128:
+            pytest.skip("Q8C has 128-row tiles of its own")
+        w8, s8 = pkg.c_ext.FC_quant_Q8C(W)
+        run, few = (lambda x: pkg.c_ext.FC_evaluate_Q8C(x, w8, s8, N),) * 2
+    else:
+        signed = isinstance(fmt, str)
+        qtype, G = (0, int(fmt[6:])) if signed else fmt
+        wq = ops.offline_FC_quant_Q4A(W, qtype=f"q4_{qtype}", group_k=G)
+        run = lambda x: ops.fc_Q4A(x, wq, N, nibble_signed=signed)
+        few = lambda x: ops.fc_Q4A(x, wq, N, nibble_signed=signed, path="decode")
+    del W
+    got = run(x)
+    assert torch.equal(got, run(x))  # fixed summation order
+    want = torch.cat([few(part.contiguous()) for part in x.split(8, dim=1)], dim=1)
+    assert (got - want).abs().max() <= 2e-5 * want.abs().max()
+    if fmt != "q8c" or N > 1000:  # (which leaves small problems to its own kernel)
+        assert gemm_launches(lambda: run(x)) == launches
+    ops.check_device_status()
+
+
 def fc_in_64_bits(oracle, wq, x, N, G):
     """Q4_0, signed nibbles, on the oracle's activation codes and scales, summed in 64 bits."""
     Ng, Kg, rows = wq.shape[0], wq.shape[1], x.shape[1]
