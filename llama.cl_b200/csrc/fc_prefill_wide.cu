@@ -218,7 +218,6 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < S::kSlots; i++) {
-            mbar_init(bar_raw + 8 * i, 1);
             mbar_init(bar_scales + 8 * i, 1);
             mbar_init(bar_free + 8 * i, kEpiWarps);
         }
@@ -234,6 +233,21 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
         *aborted = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
+    }
+    if (warp == kMmaWarp + 1) {
+        if (lane < S::kSlots) mbar_init(bar_raw + 8 * lane, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_proxy_async();
+        __syncwarp();
+        // The first stages' packed bytes, a lane per stage and stripe, while tensor memory is allocated and the warps meet.  (One thread,
+        // behind that: 1398 rows x 694 x 25344, Q4_1 group 128, 135.2 us, so 130.7; 2048 x 4096 x 11008 279.0 and 277.1.)
+        const int i = lane >> 2, j = lane & 3, stripes = min(4, p.Ng - n_tile * 4);
+        if (i < min(S::kSlots / 2, iters) && j < stripes) {
+            const uint32_t bytes = (uint32_t)(min(GPS, p.Kg - (it0 + i) * GPS) * BS), bar = bar_raw + 8 * i;
+            if (j == 0) mbar_expect_tx(bar, bytes * stripes);
+            bulk_g2s(smem0 + S::kSlotOff + i * S::kSlotBytes + j * S::kRawStripe,
+                     p.wq + ((int64_t)(n_tile * 4 + j) * p.Kg + (int64_t)(it0 + i) * GPS) * BS, bytes, bar);
+        }
     }
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -495,8 +509,6 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
                          p.sc + ((int64_t)m_tile * p.Kg + (int64_t)it * GPS) * (S::kSums * TM), bytes, bar);
             };
             const int first = min(S::kSlots / 2, iters);
-#pragma unroll 1
-            for (int i = 0; i < first; i++) load_raw(i);
             // The quantizer's results are complete.  (It has let this launch, or the one whose remainder this one does, begin only
             // when everything in front of it was complete.)  A remainder has the quantizer two launches in front of it and does not
             // wait yet for the one between, of whose tiles it reads and writes none.  Why it sees codes and scales all the same:
