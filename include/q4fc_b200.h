@@ -116,7 +116,7 @@ int q4fc_quant_x(const float* x, int64_t rows, int64_t K, int64_t ldx, int group
  * ldy).  rows is the reference's B*M.  The activation quantization happens
  * inside, as in the reference.
  *   q4fc_fc_decode  rows <= 8: weight-streaming GEMV, HBM-bound.
- *   q4fc_fc_prefill any rows:  int8 tensor-core GEMM.
+ *   q4fc_fc_prefill any rows:  tensor-core GEMM, integer products and group sums exact.
  *   q4fc_fc         picks one of the two.
  * The sums over K groups have a fixed order, the same from run to run.  It
  * depends on the sizes and, in the GEMM (q4fc_q8c_fc's too), on where in y an

@@ -972,8 +972,11 @@ int fold_of(int split, int parts, int nstage) {
     return fold < (nstage + split - 1) / split ? fold : 0;
 }
 
-// Quantizer and GEMM; `codes` and `sc` are scratch for [rows][Kg * G] bytes and scale_bytes().
-int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t ldx, int8_t* codes, float* sc,
+// The wide kernel's codes are fp16 (group 32), twice the bytes.
+bool wide_codes_f16(int G) { return G == 32; }
+// Quantizer and GEMM; `codes` and `sc` are scratch for [rows][Kg * G] codes of a byte, or two bytes where `wide` allows the wide kernel
+// and wide_codes_f16() says so, and for scale_bytes().
+int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t ldx, int8_t* codes, float* sc, bool wide,
                 PrefillParams p, cudaStream_t s) {
     const DeviceInfo* di = device_info();
     if (!di) return Q4FC_ECUDA;
@@ -998,7 +1001,7 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
         t = plan_tiles(tile, fmt, G, n_tiles, rows, nstage, room, sms);
     } else {
         t = plan_tiles(64, fmt, G, n_tiles, rows, nstage, room, sms);
-        if (rows > 64 && Kp <= 0x3fffffffLL) {
+        if (wide && Kp <= 0x3fffffffLL) {
             // The large tile too where its last tiles are divided, which takes less than the sum (they start beside the others' ends: 129 rows
             // x 2080 x 9500, Q4_0 group 32, 38 us, sum 50, and 45 in 64-row tiles; over 180 calls of many tiles 0.04 % are lost).
             const TilePlan w = plan_tiles(128, fmt, G, n_tiles, rows, nstage, room, sms);
@@ -1011,7 +1014,7 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
         return Q4FC_ELIMIT;
     }
     p.n_tiles = n_tiles;
-    const bool f16 = G == 32 && fmt != kQ8C && tile == 128;  // operands of the wide kernel
+    const bool f16 = fmt != kQ8C && tile == 128 && wide_codes_f16(G);
     if (int rc = launch_quant_x_tile(x, rows, K, ldx, G, fmt == kQ4_1, tile, f16, codes, sc, s)) return rc;
     CUtensorMap map = {};
     if (Kp > 0)  // (no K group: no stage reads the map)
@@ -1032,27 +1035,30 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
 struct WsLayout {
     size_t codes, sc, total;
 };
-WsLayout ws_layout(int64_t rows, int64_t Kg, int G) {
+WsLayout ws_layout(int64_t rows, int64_t Kg, int G, bool wide) {
     WsLayout l;
     l.codes = decode_prequant_offset();
-    // (group 32 beyond 64 rows, which is where 128-row tiles begin: fp16)
-    l.sc = align_up(l.codes + (size_t)rows * Kg * G * (G == 32 && rows > 64 ? 2 : 1), 256);
+    l.sc = align_up(l.codes + (size_t)rows * Kg * G * (wide && wide_codes_f16(G) ? 2 : 1), 256);
     l.total = align_up(l.sc + scale_bytes(rows, Kg, 2), 256);
     return l;
 }
+bool may_be_wide(int64_t rows) { return rows > 64; }
 
 }  // namespace
 
 size_t prefill_workspace_bytes(int64_t rows, int64_t K, int64_t N, int qtype, int G) {
     (void)N, (void)qtype;
-    return ws_layout(rows, (K + G - 1) / G, G).total;
+    return ws_layout(rows, (K + G - 1) / G, G, may_be_wide(rows)).total;
 }
 
 int launch_fc_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, const uint8_t* wq, int64_t Ng,
                       int64_t Kg, int qtype, int G, int64_t N, float* y, int64_t ldy, void* ws, size_t ws_bytes,
                       unsigned flags, cudaStream_t s) {
     if (rows == 0 || N == 0) return Q4FC_OK;
-    const WsLayout l = ws_layout(rows, Kg, G);
+    // A workspace without room for fp16 codes (of a size from when there were none, say) does for 64-row tiles.
+    bool wide = may_be_wide(rows);
+    if (wide && ws_bytes < ws_layout(rows, Kg, G, true).total && rows <= kMaxTileRows * 64) wide = false;
+    const WsLayout l = ws_layout(rows, Kg, G, wide);
     if (ws == nullptr || ws_bytes < l.total) {
         set_error("fc_prefill: workspace of %zu bytes given, %zu needed", ws_bytes, l.total);
         return Q4FC_EWORKSPACE;
@@ -1064,7 +1070,7 @@ int launch_fc_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, cons
     const bool sgn = (flags & Q4FC_FLAG_NIBBLE_SIGNED) && qtype == 0;
     // the reference's 1/16 activation scale of Q4_0 pairs with its x16 nibble shift; neither is materialised
     return launch_gemm(qtype == 1 ? kQ4_1 : sgn ? kQ4_0Signed : kQ4_0, G, x, rows, K, ldx,
-                       reinterpret_cast<int8_t*>(base + l.codes), reinterpret_cast<float*>(base + l.sc), p, s);
+                       reinterpret_cast<int8_t*>(base + l.codes), reinterpret_cast<float*>(base + l.sc), wide, p, s);
 }
 
 size_t q8c_prefill_scale_bytes(int64_t rows, int64_t Kg) { return scale_bytes(rows, Kg, 1); }
@@ -1076,7 +1082,7 @@ int launch_q8c_prefill(const float* x, int64_t rows, int64_t K, int64_t ldx, con
     if (!p.status) return Q4FC_ECUDA;
     p.wq = reinterpret_cast<const uint8_t*>(wq), p.wscales = wscales, p.y = y;
     p.N = N, p.ldy = ldy, p.Ng = (int)Ng, p.Kg = (int)Kg;
-    return launch_gemm(kQ8C, 32, x, rows, K, ldx, codes, sc, p, s);
+    return launch_gemm(kQ8C, 32, x, rows, K, ldx, codes, sc, false, p, s);
 }
 
 }  // namespace q4fc

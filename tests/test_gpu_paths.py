@@ -228,6 +228,31 @@ def test_few_rows_on_the_prefill_path(pkg, rows, qtype, G):
     assert torch.equal(pkg.host.HostFC(wq, N, max_rows=rows, path="prefill")(x), got)
 
 
+@pytest.mark.parametrize("rows,N,K", [(65, 96, 4100), (128, 4096, 2080), (300, 12800, 1000)])
+@pytest.mark.parametrize("qtype,G", [(0, 32), (1, 32), (1, 128)])
+def test_many_rows_with_a_workspace_for_byte_codes(pkg, rows, N, K, qtype, G):
+    """Room for a byte per activation code is enough: with group 32 for 64-row tiles, else for what a full workspace gives.  Less
+    is refused."""
+    ops = pkg.llmops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    wq = ops.offline_FC_quant_Q4A(torch.randn(N, K, generator=g, device="cuda") * 0.02, qtype=qtype, group_k=G)
+    x = torch.randn(1, rows, K, generator=g, device="cuda")
+    codes = rows * -(-K // G) * G
+    size = pkg._cabi.lib().q4fc_fc_workspace_bytes(rows, K, N, qtype, G)
+    whole = lambda nbytes: -(-nbytes // 256) * 256
+    small = size - whole(2 * codes) + whole(codes) if G == 32 else size
+    want = ops.fc_Q4A(x, wq, N)
+    ws = ops.Workspace(small, torch.device("cuda"))
+    got = ops.fc_Q4A(x, wq, N, workspace=ws)
+    ws.check()
+    # 2 x 129 roundings of 2^-24 at most on either side, as a random walk: 1.4e-6 of the largest sum; a factor of ten on top
+    assert (got - want).abs().max() <= 2e-5 * want.abs().max()
+    if G == 32:
+        assert gemm_launches(lambda: ops.fc_Q4A(x, wq, N, workspace=ws))[0][0] == ROWS64
+    with pytest.raises(RuntimeError, match="workspace"):
+        ops.fc_Q4A(x, wq, N, workspace=ops.Workspace(small - 256, torch.device("cuda")))
+
+
 @pytest.mark.parametrize("rows,N,K", [
     (9, 4096, 512),     # one 16-row chunk
     (16, 130, 4128),    # a last stage with one K group; K divided unevenly; stripes that fill no tile of four
