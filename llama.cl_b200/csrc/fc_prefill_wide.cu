@@ -412,7 +412,6 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
             run(std::false_type{});
         if constexpr (FOLD)
             if (iters > p.fold * kPerFold) sums([](ulonglong2& s, uint64_t& a, uint64_t& b) { a = fadd2(s.x, a), b = fadd2(s.y, b); });
-        if (cs > 1) asm volatile("bar.sync 1, %0;" ::"n"(kEpiWarps * 32) : "memory");  // (the partial tile takes the place of what they read)
         if (cs == 1) {
             const int64_t n = n0 + nrow;
             if (n < p.N && !*aborted) {
@@ -432,7 +431,8 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
                 }
             }
         } else if (!*aborted) {
-            // this CTA's partial tile; every operand of this CTA has been consumed (all groups' sums were seen)
+            // This CTA's partial tile, in the place of the codes.  Only MMAs read those, and a warp that has seen the last sums knows them all
+            // to have ended.
             float* red = reinterpret_cast<float*>(smem);
 #pragma unroll
             for (int h = 0; h < kChunks; h++)
