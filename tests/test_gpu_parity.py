@@ -586,6 +586,34 @@ def test_rmsnorm_quantize_matches_the_reference_rows(lib_built):
         pkg.llmops.rmsnorm_quantize(torch.zeros(1, 1, 12, device="cuda"), torch.ones(12, device="cuda"), 1e-5, 32)
 
 
+@pytest.mark.parametrize("K", [8, 120, 200, 1048, 4096, 4104, 4128, 5120, 8192, 8200, 11008])
+@pytest.mark.parametrize("rows", [1, 3, 8])
+@pytest.mark.parametrize("G", [32, 128])
+def test_rmsnorm_quantize_row_lengths(lib_built, oracle, K, rows, G):
+    """Rows shorter and longer than what a block's threads load at once and its warps quantize at once, sums whose pipelined part
+    leaves a remainder, K that is no whole number of groups; with the sum written elsewhere, onto the input, or onto the residual."""
+    import llama_cl_b200 as pkg
+
+    g = torch.Generator().manual_seed(K + rows)
+    x, res = torch.randn(1, rows, K, generator=g), torch.randn(1, rows, K, generator=g)
+    w, eps = torch.randn(K, generator=g) * 0.1 + 1, 1e-5
+    for residual in (False, True):
+        row = (x + res if residual else x).numpy()
+        want = oracle.restated.rmsnorm(row, w.numpy(), eps)
+        codes, scales, _ = oracle.restated.quant_x(want, G, 1.0)
+        for where in ("elsewhere", "input", "residual") if residual else (None,):
+            xd, rd = x.cuda(), res.cuda()
+            normalized = torch.empty_like(xd)
+            total = {"elsewhere": torch.empty_like(xd), "input": xd, "residual": rd, None: None}[where]
+            xq = pkg.llmops.rmsnorm_quantize(xd, w.cuda(), eps, G, residual=rd if residual else None, sum_out=total,
+                                             normalized=normalized)
+            assert np.array_equal(normalized.cpu().numpy(), want), where
+            assert np.array_equal(xq.codes().cpu().numpy(), codes.reshape(rows, -1)), where
+            assert np.array_equal(xq.scales_and_sums()[0].cpu().numpy(), scales.reshape(rows, -1)), where
+            if residual:
+                assert np.array_equal(total.cpu().numpy(), row), where
+
+
 @pytest.mark.parametrize("qname,G", [("q4_1", 128), ("q4_0", 32)])
 def test_fc_decode_with_addend(lib_built, qname, G):
     """Bias or residual folded into the decode kernel: the same bytes as the FC followed by one fp32 add
