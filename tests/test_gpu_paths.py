@@ -1,6 +1,7 @@
 """Branches of the host and kernel dispatch, each at the sizes where it can go wrong, against the other entry points or
 the oracle."""
 import ctypes
+import re
 import weakref
 
 import numpy as np
@@ -270,13 +271,13 @@ def test_many_rows_on_tile_edges(pkg, oracle, fmt, rows, N, K):
 
 
 @pytest.mark.parametrize("rows,N,K", [
-    # 64-row tiles, 148 SMs: 296 places over the column tiles divide K by 3, 5, 6 and 7; 29 stages, the last one group
+    # 64-row tiles; 29 stages, the last one group (which divisions there are, and that calls take them: test_every_division_of_k)
     (20, 11000, 3600), (17, 7550, 3600), (17, 6270, 3600), (17, 5370, 3600),
     (129, 10000, 1184),  # 128-row tiles on every SM: ten stages go around every ring, the last one group
 ])
 @pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128", "q8c"])
 def test_many_rows_divisions_and_long_k(pkg, oracle, fmt, rows, N, K):
-    """Clusters that are no power of two, and tiles whose shared-memory rings wrap, in every format."""
+    """Divided K, and tiles whose shared-memory rings wrap, in every format, against the oracle."""
     check_many_rows(pkg, oracle, fmt, rows, N, K)
 
 
@@ -297,8 +298,12 @@ class _KernelNode(ctypes.Structure):
                 ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p), ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
 
 
-def gemm_launches(run):
-    """What a call of the many-row FC launches behind the quantizer: for each kernel its blocks' threads and its clusters' blocks."""
+ROWS64, ROWS128 = 64, 128  # rows of a tile: fc_prefill_kernel's (of Q8C also 128), and fc_prefill_wide_kernel's
+
+
+def gemm_launches(run, moves=False):
+    """What a call of the many-row FC launches behind the quantizer: for each kernel the rows of a tile and the blocks of a cluster;
+    `moves`: also whether running sums move (of 64-row tiles 1 with at most 48 rows, else 2)."""
     stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
     stream.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
@@ -315,12 +320,13 @@ def gemm_launches(run):
         kernel, value = _KernelNode(), (ctypes.c_uint * 16)()
         assert cu.cuGraphKernelNodeGetParams_v2(node, ctypes.byref(kernel)) == 0
         assert cu.cuGraphKernelNodeGetAttribute(node, 4, value) == 0  # the cluster's dimension
-        if kernel.block[0] != 256:  # (the quantizer)
-            seen.append((kernel.block[0], value[0]))
-    return sorted(seen, key=lambda launch: launch[1])
-
-
-ROWS64, ROWS128 = 448, 320  # threads of a block: of 64-row tiles, and of 128-row tiles of Q4 weights
+        name = ctypes.c_char_p()
+        assert cu.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(kernel.func)) == 0
+        if tile := re.search(rb"fc_prefill_kernelILi\dELi\d+ELi(\d+)ELi(\d+)E", name.value):
+            seen.append((int(tile[1]), value[0], int(tile[2])))
+        elif tile := re.search(rb"fc_prefill_wide_kernelILi\dELi\d+ELb([01])E", name.value):
+            seen.append((ROWS128, value[0], int(tile[1])))
+    return [launch if moves else launch[:2] for launch in sorted(seen, key=lambda launch: launch[1])]
 
 
 @pytest.mark.parametrize("rows,N,K,launches", [
@@ -365,6 +371,52 @@ def test_every_division_of_k(pkg, fmt, rows, N, K, launches):
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("rows,N,K,launch", [
+    (20, 40 * 128 - 20, 7600, (ROWS64, 6, 1)), (48, 40 * 128 - 20, 7600, (ROWS64, 6, 1)),  # 40 tiles by six instead of by seven
+    (49, 40 * 128 - 20, 7600, (ROWS64, 6, 2)), (64, 40 * 128 - 20, 7600, (ROWS64, 6, 2)),
+    (128, 36 * 128 - 20, 6500, (ROWS128, 3, 1)), (100, 36 * 128 - 20, 6500, (ROWS128, 3, 1)),  # 72 of 64 rows by four
+    (20, 97 * 128, 1500, None),  # group 128: undivided instead of by three, two moves
+])
+@pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128"])
+def test_running_sums_that_move(pkg, fmt, rows, N, K, launch):
+    """Where K is divided by less than fills the GPU, the running sums move in between: each place they move to (tolerance as
+    above)."""
+    ops, signed = pkg.llmops, isinstance(fmt, str)
+    qtype, G = (0, int(fmt[6:])) if signed else fmt
+    g = torch.Generator(device="cuda").manual_seed(rows + N + K)
+    wq = ops.offline_FC_quant_Q4A(torch.randn(N, K, generator=g, device="cuda") * 0.02, qtype=f"q4_{qtype}", group_k=G)
+    x = torch.randn(1, rows, K, generator=g, device="cuda")
+    x[0, 3], x[0, 5, 7], x[0, 9, 1], x[0, 10, 2] = 0, 1e6, float("inf"), float("nan")
+    run = lambda x, path=None: ops.fc_Q4A(x, wq, N, nibble_signed=signed, **({"path": path} if path else {}))
+    got, want = run(x), torch.cat([run(part.contiguous(), "decode") for part in x.split(8, dim=1)], dim=1)
+    assert torch.equal(got.view(torch.int32), run(x).view(torch.int32))
+    assert torch.equal(got.isfinite(), want.isfinite()) and torch.equal(got.isnan(), want.isnan())
+    got, want = got.nan_to_num(0, 0, 0), want.nan_to_num(0, 0, 0)
+    assert ((got - want).abs() <= 2e-5 * want.abs().amax(-1, keepdim=True)).all()
+    seen = gemm_launches(lambda: run(x), moves=True)
+    assert seen == [launch or ((ROWS64, 1, 1) if G == 128 else (ROWS64, 2, 1))]
+    ops.check_device_status()
+
+
+@pytest.mark.parametrize("rows,N,K", [(113, 18944, 640), (128, 18924, 640), (97, 18944, 3000), (65535 * 64 + 1, 20, 33)])
+@pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128)])
+def test_wide_tiles_with_few_stages(pkg, fmt, rows, N, K):
+    """128-row tiles with the fewest K stages that go in them, and beyond the rows that a grid of 64-row tiles has, where even
+    less than one stage does; against calls that go in 64-row tiles (tolerance as above)."""
+    ops, (qtype, G) = pkg.llmops, fmt
+    g = torch.Generator(device="cuda").manual_seed(K)
+    wq = ops.offline_FC_quant_Q4A(torch.randn(N, K, generator=g, device="cuda") * 0.02, qtype=f"q4_{qtype}", group_k=G)
+    x = torch.randn(1, rows, K, generator=g, device="cuda")
+    run = lambda x: ops.fc_Q4A(x, wq, N)
+    got = run(x)
+    few = 60 if rows < 1000 else 1 << 21
+    want = torch.cat([run(part.contiguous()) for part in x.split(few, dim=1)], dim=1)
+    assert (got - want).abs().max() <= 2e-5 * want.abs().max()
+    assert gemm_launches(lambda: run(x)) == [(ROWS128, 1)]
+    assert gemm_launches(lambda: run(x[:, :few].contiguous()))[0][0] == ROWS64
+    ops.check_device_status()
+
+
 def fc_in_64_bits(oracle, wq, x, N, G):
     """Q4_0, signed nibbles, on the oracle's activation codes and scales, summed in 64 bits."""
     Ng, Kg, rows = wq.shape[0], wq.shape[1], x.shape[1]
@@ -406,15 +458,15 @@ def test_decode_ctas_that_share_the_quantizer(pkg, stripes, rows, K, qtype, G):
 
 
 @pytest.mark.parametrize("rows,N,K", [
-    # 148 column tiles and more: whole tiles, the last columns and K groups not full, fewer K stages than are unpacked ahead and
-    # more than the rings hold, rows that end in each of a warp's four chunks
+    # 148 column tiles and more: whole tiles, the last columns and K groups not full, few K stages and more than the rings hold, rows
+    # that end in each of a warp's four chunks (which calls go in 128-row tiles: test_every_division_of_k and the one behind it)
     (65, 18901, 33), (81, 18901, 96), (112, 18920, 224), (128, 18944, 1312), (129, 9473, 640), (185, 9473, 160),
-    (128, 1024, 4096), (192, 1000, 4096), (129, 4096, 2080), (300, 1500, 4096), (128, 6000, 3000),  # K divided by 8, 6, 2, 3, 2
+    (128, 1024, 4096), (192, 1000, 4096), (129, 4096, 2080), (300, 1500, 4096), (128, 6000, 3000),  # K divided
 ])
 @pytest.mark.parametrize("fmt", [(0, 32), (0, 128), (1, 32), (1, 128), "signed32", "signed128"])
 def test_wide_tiles_against_64_row_tiles(pkg, fmt, rows, N, K):
-    """128-row tiles against calls of at most 64 rows, which go in 64-row tiles: the same codes and exact integers, products and
-    sums in another order (tolerance as in test_many_rows_on_tile_edges, row by row).  Among the rows the ends of the range."""
+    """More than 64 rows, in either tile, against calls of at most 64 rows, which go in 64-row tiles: the same codes and exact
+    integers, products and sums in another order (tolerance as in test_many_rows_on_tile_edges, row by row).  Among the rows the ends of the range."""
     signed = isinstance(fmt, str)
     qtype, G = (0, int(fmt[6:])) if signed else fmt
     g = torch.Generator(device="cuda").manual_seed(rows + N + K)
