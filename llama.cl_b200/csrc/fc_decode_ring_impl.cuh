@@ -797,6 +797,7 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
         }
     }
     p.ring_off = (int)fixed;
+    p.x_vec_ok = any_fp32 && (p.in[0].K % 4 == 0) && (p.ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.x) & 15) == 0);
     // Without a K split every CTA needs all of the quantized activations: clusters of kShare CTAs split that work
     // and store the codes into one another's shared memory, instead of each CTA repeating it.
     p.bq = 1;
@@ -809,7 +810,7 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
             while ((1 << l2) < bq) l2++;
             const int cap = ring_max_clusters(v, dev, bq, l2, di);
             if (cap < 0) return -1;
-            const int units = TP ? nc / bq * bq : (nc + bq - 1) / bq * bq;  // (the last of them may have no stripe)
+            const int units = TP ? nc / bq * bq : (nc + bq - 1) / bq * bq;  // (some of them, of any rank in a cluster, may have no stripe)
             return units < cap * bq ? units : cap * bq;
         };
         int bq = kShare;
@@ -819,14 +820,20 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
             if (units < 0) return Q4FC_ECUDA;
             if (!TP && bq == 4) {
                 // Two sharers where the SMs that clusters of two reach besides save a round of stripes, and that is worth more than
-                // the quantizer's longer share (a stripe takes half a nanosecond per k, a pass of the 16 warps over 128 k of four rows
-                // each 0.4 us).
+                // the quantizer's longer share.  A round of stripes takes 0.45 ns per k (group 128: 0.25) and 0.6 us, with more than
+                // four rows 0.36 (0.18) and 1.05; a pass of the 16 warps over 128 k of up to four rows each 0.6 us, 1.2 with two rows,
+                // 1.8 with more, and a third more where rows are read value by value.  Fitted to 700 calls measured with two and with
+                // four: 0.7 % behind the better (always four 10 %, always two 2.6 %).  5 rows x 2560, 288 stripes, Q4_1 group 128:
+                // by four 9.6 us, by two 10.0; 6 x 2730, 271 stripes, 10.8 and 12.4; 1 x 4096, 140 stripes, group 32, 7.1 and 5.3.
                 const int two = units_of(2);
                 if (two < 0) return Q4FC_ECUDA;
-                const int64_t K = p.in[0].K, chunks = (K + 127) / 128, sets = (rows_max + 3) / 4;
+                const int64_t K = p.in[0].K, items = (K + 127) / 128 * ((rows_max + 3) / 4);
                 const int64_t saved = (ng_total + units - 1) / units - (ng_total + two - 1) / two;
-                const int64_t more = ((chunks + 2 * kRW - 1) / (2 * kRW) - (chunks + 4 * kRW - 1) / (4 * kRW)) * sets;
-                if (saved * K > more * 800 && saved > 0) bq = 2, units = two;
+                const int64_t passes = (items + 2 * kRW - 1) / (2 * kRW) - (items + 4 * kRW - 1) / (4 * kRW);
+                const int64_t gain =
+                    saved * (rows_max > 4 ? K * (G == 32 ? 36 : 18) / 100 + 1050 : K * (G == 32 ? 45 : 25) / 100 + 600);
+                const int64_t loss = passes * (p.x_vec_ok ? 600 : 800) * (rows_max < 3 ? rows_max : 3);
+                if (saved > 0 && gain > loss) bq = 2, units = two;
             }
             p.bq = bq;
             nc = units;
@@ -873,7 +880,6 @@ int launch_ring_impl(const RingCall* calls, int ncalls, int qtype, int G, unsign
         p.depth = (int)depth;
     }
     const size_t smem = fixed + (size_t)p.depth * p.slot_bytes;
-    p.x_vec_ok = any_fp32 && (p.in[0].K % 4 == 0) && (p.ldx % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.x) & 15) == 0);
     {
         std::lock_guard<std::mutex> lk(g_setup_mutex);
         if (!v->attr_done[dev]) {

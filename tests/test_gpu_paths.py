@@ -298,12 +298,8 @@ class _KernelNode(ctypes.Structure):
                 ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p), ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
 
 
-ROWS64, ROWS128 = 64, 128  # rows of a tile: fc_prefill_kernel's (of Q8C also 128), and fc_prefill_wide_kernel's
-
-
-def gemm_launches(run, moves=False):
-    """What a call of the many-row FC launches behind the quantizer: for each kernel the rows of a tile and the blocks of a cluster;
-    `moves`: also whether running sums move (of 64-row tiles 1 with at most 48 rows, else 2)."""
+def kernels_of(run):
+    """The kernels of a captured call: name, and blocks of a cluster."""
     stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
     stream.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
@@ -317,15 +313,26 @@ def gemm_launches(run, moves=False):
     nodes, seen = (ctypes.c_void_p * n.value)(), []
     assert cu.cuGraphGetNodes(g, nodes, ctypes.byref(n)) == 0
     for node in map(ctypes.c_void_p, nodes):
-        kernel, value = _KernelNode(), (ctypes.c_uint * 16)()
+        kernel, value, name = _KernelNode(), (ctypes.c_uint * 16)(), ctypes.c_char_p()
         assert cu.cuGraphKernelNodeGetParams_v2(node, ctypes.byref(kernel)) == 0
         assert cu.cuGraphKernelNodeGetAttribute(node, 4, value) == 0  # the cluster's dimension
-        name = ctypes.c_char_p()
         assert cu.cuFuncGetName(ctypes.byref(name), ctypes.c_void_p(kernel.func)) == 0
-        if tile := re.search(rb"fc_prefill_kernelILi\dELi\d+ELi(\d+)ELi(\d+)E", name.value):
-            seen.append((int(tile[1]), value[0], int(tile[2])))
-        elif tile := re.search(rb"fc_prefill_wide_kernelILi\dELi\d+ELb([01])E", name.value):
-            seen.append((ROWS128, value[0], int(tile[1])))
+        seen.append((name.value, value[0]))
+    return seen
+
+
+ROWS64, ROWS128 = 64, 128  # rows of a tile: fc_prefill_kernel's (of Q8C also 128), and fc_prefill_wide_kernel's
+
+
+def gemm_launches(run, moves=False):
+    """What a call of the many-row FC launches behind the quantizer: for each kernel the rows of a tile and the blocks of a cluster;
+    `moves`: also whether running sums move (of 64-row tiles 1 with at most 48 rows, else 2)."""
+    seen = []
+    for name, cluster in kernels_of(run):
+        if tile := re.search(rb"fc_prefill_kernelILi\dELi\d+ELi(\d+)ELi(\d+)E", name):
+            seen.append((int(tile[1]), cluster, int(tile[2])))
+        elif tile := re.search(rb"fc_prefill_wide_kernelILi\dELi\d+ELb([01])E", name):
+            seen.append((ROWS128, cluster, int(tile[1])))
     return [launch if moves else launch[:2] for launch in sorted(seen, key=lambda launch: launch[1])]
 
 
@@ -415,6 +422,18 @@ def test_wide_tiles_with_few_stages(pkg, fmt, rows, N, K):
     assert gemm_launches(lambda: run(x)) == [(ROWS128, 1)]
     assert gemm_launches(lambda: run(x[:, :few].contiguous()))[0][0] == ROWS64
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("rows,K,stripes,qtype,G,sharers", [
+    (1, 4096, 140, 1, 32, 2), (1, 4096, 131, 1, 32, 4), (4, 4000, 290, 0, 32, 2),  # a round saved, none, a round
+    (5, 2560, 288, 1, 128, 4), (6, 2730, 271, 1, 128, 4), (7, 2340, 138, 0, 128, 4),  # a round, but a second pass of the quantizer
+])
+def test_sharers_of_the_quantizer(pkg, rows, K, stripes, qtype, G, sharers):
+    """Two CTAs share the quantizer instead of four only where the SMs so reached are worth its longer share."""
+    g = torch.Generator(device="cuda").manual_seed(stripes)
+    wq = pkg.llmops.offline_FC_quant_Q4A(torch.randn(stripes * 32, K, generator=g, device="cuda") * 0.02, qtype=qtype, group_k=G)
+    x = torch.randn(1, rows, K, generator=g, device="cuda")
+    assert kernels_of(lambda: pkg.llmops.fc_Q4A(x, wq, stripes * 32))[0][1] == sharers
 
 
 def fc_in_64_bits(oracle, wq, x, N, G):
