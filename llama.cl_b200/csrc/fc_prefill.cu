@@ -16,7 +16,7 @@
 //   * operand B = activation codes (int8), same layout, straight from the code matrix by TMA;
 //   * D = int32 accumulators in tensor memory, lane = weight column, column = activation row.
 // Every K group has its own pair of scales, so a group's MMA(s) (one K=32 instruction for group 32, four for group
-// 128) write a fresh TMEM buffer (four of TM columns, three where the fourth's place holds Q8C's sums), and the
+// 128) write a fresh TMEM buffer (four of TM columns, three where the fourth's place holds sums), and the
 // epilogue warps read the buffer back with
 // tcgen05.ld, turn the exact integers into fp32, scale them and accumulate the tile in registers.
 //
@@ -27,10 +27,12 @@
 // reads four rows per load, and weights, codes and scales have rings of their own, so that operands are released by the
 // MMA and not by the epilogue.
 //
+// Sizes here and below are rows x K x N.
+//
 // Measured (whole call, quantizer included; unpacking straight from global memory without prefetch, one 128 x 128 tile per CTA
 // whatever the row count, epilogue of 5 operations per integer -> this form -> with the last tiles divided, below, and scales read by
 // shared-memory loads):
-//   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 -> 36.3 us   Q8C, 256 rows 296 -> 151 -> 99 us (233 TOPS)
+//   4096 -> 11008   Q4_1 g32, 37 rows 123.7 -> 41.0 -> 36.0 us   Q8C, 256 rows 296 -> 151 -> 99 us (233 TOPS)
 // With 128-row tiles of Q4 weights, before they had a kernel of their own: Q4_0 g32, 512 rows 186 us; Q4_1 g128, 2048 rows 296.
 // A group of 32 k takes about 1000 cycles for 128 x 128 integers, of which the MMA needs 64: the epilogue's chain of load,
 // convert, scale is latency-bound with the 16 warps that the registers allow.  Tried and dropped: handing registers
@@ -46,8 +48,11 @@
 // less exact than that (K = 4096: 2.0e-7 of the result in the 2-norm, with 8 warps' chains 9.6e-8; K = 11008: 3.3e-7 and
 // 1.3e-7).  After 8 groups, or 12 where a CTA has more than 64, a thread moves its running sums to a second place and keeps
 // what that addition rounds off: 6.5e-8 to 7.5e-8 for K from 512 to 11008, below the 8-warp sums at every size tried.  It
-// cost 131 -> 151 us at 256 rows x 4096 x 11008 (before the last tiles were divided) and 33 -> 35 at 37 rows; every 16 groups 146 us and 8.3e-8, at K = 3001 not
-// below the 8-warp sums.  (Staggering the moves over the warps: 156; as an outer loop around the groups' loop: 157.)
+// cost 131 -> 151 us at 256 rows x 4096 x 11008 (before the last tiles were divided) and 33 -> 35 at 37 rows; every 16 groups 146
+// us and 8.3e-8, at K = 3001 not below the 8-warp sums.  (Staggering the moves over the warps: 156; as an outer loop around the groups' loop: 157.)
+//
+// Q4 sums K in one chain for each CTA; where few CTAs share it the sums move to a second place in between, so that no chain is longer
+// than with many (see fold_of).
 //
 // Few tiles, or the last of many: a cluster of `split` CTAs shares a tile and divides its K stages; the partial tiles meet in shared memory
 // and are added in rank order (fixed order, no atomics).  So the outputs of one call can be sums in two orders: equal rows of x, or
@@ -177,7 +182,7 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, ui
 
 // acc[P .. P + W/2) += scaled integers of W rows (+ wm * their group sums); `xs`: the rows' scales, the group sums
 // follow at xs + TM
-template <int FMT, int TM, int P, int W>
+template <int FMT, int G, int TM, int P, int W>
 __device__ __forceinline__ void accumulate(uint64_t (&acc)[8], const uint32_t (&v)[W], const float* xs, uint64_t wd2,
                                            uint64_t wm2) {
 #pragma unroll
@@ -186,8 +191,11 @@ __device__ __forceinline__ void accumulate(uint64_t (&acc)[8], const uint32_t (&
         const uint64_t i01 = pack2(__int2float_rn((int)v[4 * j]), __int2float_rn((int)v[4 * j + 1]));
         const uint64_t i23 = pack2(__int2float_rn((int)v[4 * j + 2]), __int2float_rn((int)v[4 * j + 3]));
         uint64_t &a = acc[P + 2 * j], &b = acc[P + 2 * j + 1];
-        a = ffma2(FMT == kQ8C ? x4.x : fmul2(wd2, x4.x), i01, a);
-        b = ffma2(FMT == kQ8C ? x4.y : fmul2(wd2, x4.y), i23, b);
+        // The column's scale, fp16, and the integer first, whose product rounds off less than that of the scales: 3 to 4 % less error
+        // against 64 bits, and 0.5 % less time.  (Not for Q4_0 with group 32, where up to 32 rows then take 0.8 % longer.)
+        constexpr bool kIntegerFirst = FMT == kQ4_1 || G == 128;
+        a = FMT == kQ8C ? ffma2(x4.x, i01, a) : kIntegerFirst ? ffma2(x4.x, fmul2(wd2, i01), a) : ffma2(fmul2(wd2, x4.x), i01, a);
+        b = FMT == kQ8C ? ffma2(x4.y, i23, b) : kIntegerFirst ? ffma2(x4.y, fmul2(wd2, i23), b) : ffma2(fmul2(wd2, x4.y), i23, b);
         if (FMT == kQ4_1) {
             const ulonglong2 g4 = *reinterpret_cast<const ulonglong2*>(xs + TM + 4 * j);
             a = ffma2(wm2, g4.x, a);
@@ -422,24 +430,24 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM, FOLD>::kThreads, TM =
                 if (live0) {
                     tc_ld(taddr + b * TM, v);
                     tc_wait_ld();
-                    accumulate<FMT, TM, 0, W>(acc[0], v, xs, wd2, wm2);
+                    accumulate<FMT, G, TM, 0, W>(acc[0], v, xs, wd2, wm2);
                     if constexpr (W == 8) {
                         tc_ld(taddr + b * TM + 8, v);
                         tc_wait_ld();
-                        accumulate<FMT, TM, 4, W>(acc[0], v, xs + 8, wd2, wm2);
+                        accumulate<FMT, G, TM, 4, W>(acc[0], v, xs + 8, wd2, wm2);
                     }
                 }
                 if (live1) {
                     tc_ld(taddr + b * TM + CGN * 16, v);
                     tc_wait_ld();
                     if constexpr (W == 8) {
-                        accumulate<FMT, TM, 0, W>(acc[1], v, xs + CGN * 16, wd2, wm2);
+                        accumulate<FMT, G, TM, 0, W>(acc[1], v, xs + CGN * 16, wd2, wm2);
                         tc_ld(taddr + b * TM + CGN * 16 + 8, v);
                         tc_wait_ld();
                     }
                 }
                 release();
-                if (live1) accumulate<FMT, TM, W == 8 ? 4 : 0, W>(acc[1], v, xs + CGN * 16 + 16 - W, wd2, wm2);
+                if (live1) accumulate<FMT, G, TM, W == 8 ? 4 : 0, W>(acc[1], v, xs + CGN * 16 + 16 - W, wd2, wm2);
                 if (gi == GPS - 1) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar_sempty + 8 * sl);  // done with the stage's scales
@@ -459,8 +467,8 @@ __global__ void __launch_bounds__(PrefillShape<FMT, G, TM, FOLD>::kThreads, TM =
             const uint32_t first = taddr + S::kSumCol + cgrp * (S::kSumStep - 16);
             q4fc::tc_st(first, kZero);
             if (live1) q4fc::tc_st(first + CGN * S::kSumStep, kZero);
-            // A loop around the groups' loop, which finds anew what it needs, so that the groups' loop keeps its registers (3584 columns, 16
-            // rows, K = 2816, group 32: moving nothing 12.8 us, so 13.5, as a branch in the groups' loop 14.8).
+            // A loop around the groups' loop, which finds anew what it needs, so that the groups' loop keeps its registers
+            // (16 x 2816 x 3584, group 32: moving nothing 12.8 us, so 13.5, as a branch in the groups' loop 14.8).
             int end = 0;
 #pragma unroll 1
             do {
@@ -891,8 +899,9 @@ struct TilePlan {
 struct StageCost {
     float alone, alone_rows, shared, shared_rows, wide;
 };
-constexpr StageCost kStageQ4[2][2] = {{{0.51f, 0.04f, 0.62f, 0.07f, 0.57f}, {0.44f, 0.06f, 0.59f, 0.11f, 0.64f}},    // group 128: Q4_0, Q4_1
-                                      {{0.97f, 0.20f, 1.16f, 0.29f, 1.65f}, {1.11f, 0.24f, 1.29f, 0.38f, 2.20f}}};   // group 32
+constexpr StageCost kStageQ4[2][2] = {  // group 128 and 32, each Q4_0 and Q4_1
+    {{0.51f, 0.04f, 0.62f, 0.07f, 0.57f}, {0.44f, 0.06f, 0.59f, 0.11f, 0.64f}},
+    {{0.97f, 0.20f, 1.16f, 0.29f, 1.65f}, {1.11f, 0.24f, 1.29f, 0.38f, 2.20f}}};
 constexpr StageCost kStageQ8C = {0.95f, 0.20f, 1.06f, 0.29f, 0};
 
 // The last tiles of many: K divided over clusters where that takes less than a round more.  In stages: rounds x (stages of a CTA +
@@ -928,8 +937,9 @@ TilePlan plan_tiles(int tile, int fmt, int G, int n_tiles, int64_t rows, int nst
     const float fullest = rows < 64 ? (float)((rows + 15) / 16) : 4.0f, mean = (float)((rows + 15) / 16) / (float)m_tiles;
     const float alone = stage.alone + stage.alone_rows * fullest;
     const float shared = stage.shared + stage.shared_rows * (few && m_tiles > 1 ? 0.5f * (mean + fullest) : mean);
-    // the wide kernel: a tile with fewer rows takes other loads, and by what it lets stand hardly less (129 to 256 rows x 6144 x 18944, two rounds,
-    // the second of tiles with 1, 33, 65, 97 and 128 rows: Q4_0 group 32 68, 78, 90, 95 and 83 us, Q4_1 group 128 29, 30, 33, 37 and 39)
+    // the wide kernel: a tile with fewer rows takes other code, and what it lets stand saves it little (129 to 256 rows x 6144 x
+    // 18944, two rounds, the second of tiles with 1, 33, 65, 97 and 128 rows: Q4_0 group 32 68, 78, 90, 95 and 83 us, Q4_1 group
+    // 128 29, 30, 33, 37 and 39)
     const int last = (int)((rows - (int64_t)(m_tiles - 1) * tile + 15) / 16);
     const float partial = last == 8 ? 1.0f : 0.75f + 0.05f * (float)last;
     // n tiles, K divided by c: rounds x (start + stages)
@@ -1002,8 +1012,9 @@ int launch_gemm(int fmt, int G, const float* x, int64_t rows, int64_t K, int64_t
     } else {
         t = plan_tiles(64, fmt, G, n_tiles, rows, nstage, room, sms);
         if (wide && Kp <= 0x3fffffffLL) {
-            // The large tile too where its last tiles are divided, which takes less than the sum (they start beside the others' ends: 129 rows
-            // x 2080 x 9500, Q4_0 group 32, 38 us, sum 50, and 45 in 64-row tiles; over 180 calls of many tiles 0.04 % are lost).
+            // The large tile too where its last tiles are divided, which takes less than the sum (they start beside the others'
+            // ends: 129 rows x 2080 x 9500, Q4_0 group 32, 38 us, sum 50, and 45 in 64-row tiles; over 180 calls of many tiles
+            // 0.04 % are lost).
             const TilePlan w = plan_tiles(128, fmt, G, n_tiles, rows, nstage, room, sms);
             if (w.cost < t.cost || w.left > 0 || rows > kMaxTileRows * 64) t = w;
         }

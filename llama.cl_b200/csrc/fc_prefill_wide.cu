@@ -12,8 +12,8 @@
 //   * D = three buffers of 128 columns: with fp16 operands fp32 numbers n x code x 2^-16 summed without rounding (below 2^24 units),
 //     so that nothing converts them, with int8 integers (group 128's MMAs alone would take 512 cycles with fp16).
 //
-// Measured (whole calls, in the 64-row kernel's form before -> here):
-//   512 x 4096 x 11008, Q4_0 g32 186 -> 150 us (308 TOPS), Q4_1 g32 235 -> 197;  2048 rows, Q4_1 g128 296 -> 278 (664 TOPS)
+// Measured (whole calls, rows x K x N, in the 64-row kernel's form before -> here):
+//   512 x 4096 x 11008, Q4_0 g32 186 -> 148 us (312 TOPS), Q4_1 g32 235 -> 196;  2048 rows, Q4_1 g128 296 -> 274 (674 TOPS)
 //   one round of 148 tiles, K = 4096 (the quantizer included): Q4_0 g32 76 -> 60 us, Q4_1 g32 96 -> 78, Q4_1 g128 33 -> 31
 // A K group of 32 takes 790 cycles (from K = 2048 to 8192), in which a scheduler issues 400 instructions.  What bounds it: the
 // latencies of two warps a scheduler that meet at the same buffers.  The FMA pipe has 330 cycles to do (a packed multiplication 2.4, a
@@ -182,7 +182,8 @@ __device__ __forceinline__ void accumulate(uint64_t (&acc)[W / 2], const uint32_
     }
 }
 
-// FOLD: the running sums move to a second place, once, after p.fold stages of 128 k (0.9 us for that and adding them at the end)
+// FOLD: the running sums move to a second place, once, after p.fold stages of 128 k (0.9 us with adding them at the end; see fold_of in
+// fc_prefill.cu)
 template <int FMT, int G, bool FOLD>
 __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap codes_map) {
     using S = WideShape<FMT, G>;
@@ -281,7 +282,10 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
         [[maybe_unused]] auto sums = [&](auto then) {
             ulonglong2* at = reinterpret_cast<ulonglong2*>(smem + S::kSumOff) + threadIdx.x;
 #pragma unroll
-            for (int j = 0; j < kChunks * W / 4; j++) then(at[j * kEpiWarps * 32], acc[j / (W / 4)][2 * j % (W / 2)], acc[j / (W / 4)][2 * j % (W / 2) + 1]);
+            for (int j = 0; j < kChunks * W / 4; j++) {
+                uint64_t(&a)[W / 2] = acc[j / (W / 4)];
+                then(at[j * kEpiWarps * 32], a[2 * j % (W / 2)], a[2 * j % (W / 2) + 1]);
+            }
         };
         auto scale = [&](int c) {
             accumulate<FMT, S::kF16>(acc[c], v[c & 1], reinterpret_cast<const float*>(smem + xs) + c * (2 * W), wd2, wm2);
@@ -360,7 +364,8 @@ __global__ void __launch_bounds__(kThreads, 1) fc_prefill_wide_kernel(const Pref
                     const uint16_t wm16 = FMT == kQ4_1 ? *reinterpret_cast<const uint16_t*>(tail + 64) : 0;
                     if (ALL && later) scale(kChunks - 1);  // of the group before
                     if constexpr (FOLD)
-                        if (gi == 0 && i == p.fold * kPerFold) sums([](ulonglong2& s, uint64_t& a, uint64_t& b) { s.x = a, s.y = b, a = b = 0; });
+                        if (gi == 0 && i == p.fold * kPerFold)
+                            sums([](ulonglong2& s, uint64_t& a, uint64_t& b) { s.x = a, s.y = b, a = b = 0; });
                     xs = sc + S::kRawBytes + (gi * (S::kSums * TM) + half * W) * 4;
                     const float wd = h2f(wd16) * (S::kF16 ? kWdScale : 1.0f), wm = h2f(wm16);
                     wd2 = pack2(wd, wd), wm2 = pack2(wm, wm);
