@@ -855,6 +855,7 @@ const ClusterRoom& cluster_room(const DeviceInfo* di) {
     ClusterRoom& room = rooms[di->index];
     if (known[di->index].load(std::memory_order_acquire)) return room;
     std::lock_guard<std::mutex> lock(mutex);
+    if (known[di->index].load(std::memory_order_relaxed)) return room;
     for (int places = 1; places <= 2; places++)
         for (int c = 1; c <= kMaxSplit; c++) {
             const int smem = places == 1 ? di->max_smem_optin : 113 * 1024;
