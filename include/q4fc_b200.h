@@ -119,8 +119,10 @@ int q4fc_quant_x(const float* x, int64_t rows, int64_t K, int64_t ldx, int group
  *   q4fc_fc_prefill any rows:  tensor-core GEMM, integer products and group sums exact.
  *   q4fc_fc         picks one of the two.
  * The sums over K groups have a fixed order, the same from run to run.  It
- * depends on the sizes and, in the GEMM (q4fc_q8c_fc's too), on where in y an
- * output lies: equal rows of x in one call may differ in the last place.
+ * depends on the sizes, on how many clusters of thread blocks the card holds
+ * at once (cards of one model differ in that) and, in the GEMM (q4fc_q8c_fc's
+ * too), on where in y an output lies: equal rows of x in one call, and equal
+ * calls on two cards, may differ in the last place.
  * ws: workspace of at least q4fc_fc_workspace_bytes() bytes, 256-byte
  * aligned, zeroed once with q4fc_fc_workspace_init() before its first use;
  * the kernels leave it ready for the next call.  Calls that may overlap on
